@@ -51,9 +51,10 @@ def listed():
         # the large single scene: ten parts, 30% clutter, finer sampling
         dict(MATCH, name="match_large", points=918402, instances=10, noise=0.3, clutter=0.30,
              train_sd=0.03, sd=0.03),
-        # the largest scene, from page-locked host memory as a camera driver fills it
+        # the largest scene, from page-locked host memory as a camera driver fills it; so dense a
+        # cloud takes more neighbours per normal
         dict(MATCH, name="match_xl_pinned", model="bracket", model_points=30011, points=2600007,
-             instances=12, noise=0.35, clutter=0.25, source="pinned"),
+             instances=12, noise=0.2, clutter=0.25, source="pinned", knn=24),
         # the reference's example call: a finer model, many matches, a long refinement with a
         # wide search radius
         dict(MATCH, name="match_long_refine", points=350001, instances=6, clutter=0.2,
@@ -97,7 +98,7 @@ def draw(rng):
             source=rng.choice(["device", "device", "host", "pinned"]),
             normals=rng.random() < 0.25, viewpoint=rng.random() < 0.8, train_sd=sd, sd=sd,
             kp=rng.choice([0.1, 0.1, 0.2] if haze else [0.1, 0.2, 0.2, 0.3]), min_score=rng.choice([0.2, 0.25, 0.3]),
-            matches=rng.choice([1, 4, 16, 16]), knn=rng.choice([8, 10, 10, 16]),
+            matches=rng.choice([1, 4, 16, 16]), knn=rng.choice([8, 10, 10, 16, 24]),
             smooth=rng.random() < 0.8, dense=rng.random() < 0.8, steps=rng.choice([5, 5, 9, 15]),
             reject=rng.choice([0.1, 0.1, 0.2, 0.3] if kind == "match" else [0.1, 0.1, 0.2]))
     if kind == "train":

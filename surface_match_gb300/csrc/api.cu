@@ -583,9 +583,11 @@ void match(Ctx &c, const Model &m, const float *xyzIn, const float *nrmIn, int64
             float4 *tpR = d.arena.get<float4>("m.tpR", std::max(T.m, 1));
             float4 *tpF = d.arena.get<float4>("m.tpF", std::max(T.m, 1));
             kd_mark_nonempty(d, T, ioi, neS);
-            kd_mark_nonempty(d, T, ioi2, neR);
             kd_tree_positions(d, T, ioi, P, tpS);
-            kd_tree_positions(d, T, ioi2, P, tpR);
+            if (mp.densePoseRefinement) { // (ioi2 is written by the resampling only)
+                kd_mark_nonempty(d, T, ioi2, neR);
+                kd_tree_positions(d, T, ioi2, P, tpR);
+            }
             kd_tree_positions(d, T, nullptr, P, tpF);
             s.neS         = neS;
             s.neR         = neR;

@@ -582,13 +582,15 @@ void match(Ctx &c, const Model &m, const float *xyzIn, const float *nrmIn, int64
             float4 *tpS = d.arena.get<float4>("m.tpS", std::max(T.m, 1));
             float4 *tpR = d.arena.get<float4>("m.tpR", std::max(T.m, 1));
             float4 *tpF = d.arena.get<float4>("m.tpF", std::max(T.m, 1));
+            float  *exc = d.arena.get<float>("m.exc", 3);
             kd_mark_nonempty(d, T, ioi, neS);
-            kd_tree_positions(d, T, ioi, P, tpS);
+            kd_tree_positions(d, T, ioi, P, tpS, exc);
             if (mp.densePoseRefinement) { // (ioi2 is written by the resampling only)
                 kd_mark_nonempty(d, T, ioi2, neR);
-                kd_tree_positions(d, T, ioi2, P, tpR);
+                kd_tree_positions(d, T, ioi2, P, tpR, exc + 1);
             }
-            kd_tree_positions(d, T, nullptr, P, tpF);
+            kd_tree_positions(d, T, nullptr, P, tpF, exc + 2);
+            s.exc         = exc;
             s.neS         = neS;
             s.neR         = neR;
             s.tpS         = tpS;

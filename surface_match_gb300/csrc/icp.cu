@@ -58,6 +58,7 @@ struct Stage {
     // subset (rankOf maps a point id to its subset rank); tree.nd == nullptr: the grid G
     smk::KdView   tree;
     const int    *rankOf;
+    const float  *exc; // largest excursion of the subset's points from their leaves' boxes
 };
 
 struct Work {
@@ -135,7 +136,10 @@ __global__ void __launch_bounds__(kT, 4) k_corr(Work w, Stage s, int usePrev) {
 
 // K1 with the reference's search: one thread per source point, the nearest point of the
 // reduced k-d tree (findClosestPoint, util.cpp:603-626: a 1-nearest search from the root,
-// with the tree's pruning) - the same pair rules as k_corr.
+// with the tree's pruning) - the same pair rules as k_corr. A pair farther than the rejection
+// distance is dropped, so the search starts from that distance's bound (smk::nn_bound): a
+// model point without a scene point near it (a hidden side) then prunes at the root instead of
+// walking thousands of leaves for a far point nobody uses.
 __global__ void __launch_bounds__(kT) k_corr_tree(Work w, Stage s) {
     chain_enter(); // launched chained
     const int   ci = blockIdx.y;
@@ -144,6 +148,7 @@ __global__ void __launch_bounds__(kT) k_corr_tree(Work w, Stage s) {
         return;
     if (w.live && blockIdx.x == 0 && threadIdx.x == 0)
         atomicAdd(w.live, (unsigned long long)s.n);
+    const float start = smk::nn_bound(s.rej2, *s.exc);
     for (int i = blockIdx.x * kT + threadIdx.x; i < s.n; i += gridDim.x * kT) {
         const size_t o  = (size_t)ci * w.maxSrc + i;
         const float4 sp = s.src[i], sn = s.srcN[i];
@@ -152,7 +157,7 @@ __global__ void __launch_bounds__(kT) k_corr_tree(Work w, Stage s) {
         smi::pose_rotate(C.M, sn.x, sn.y, sn.z, y.x, y.y, y.z);
         const float q[3] = {x.x, x.y, x.z};
         smk::NnSet  rs;
-        rs.init();
+        rs.init(start);
         smk::kd_search(s.tree, q, rs);
         const int   j  = rs.count ? s.rankOf[rs.idx] : -1;
         const float d  = rs.dist;
@@ -169,13 +174,17 @@ __global__ void __launch_bounds__(kT) k_corr_tree(Work w, Stage s) {
     }
 }
 
-// K4 with the reference's search: residual of each pair, one thread per pair.
+// K4 with the reference's search: residual of each pair, one thread per pair. The pair's scene
+// point, at squared distance u, is in the tree: the reference's result lies within
+// (sqrt(u) + exc)^2 (its search either meets that point or prunes it against a nearer one),
+// so the search starts from the bound of that distance.
 __global__ void __launch_bounds__(kT) k_resid_tree(Work w, Stage s) {
     chain_enter(); // launched chained
     const int   ci = blockIdx.y;
     const Cand &C  = w.cand[ci];
     if (!cand_live(C, s) || C.cnt < 6)
         return;
+    const float exc = *s.exc;
     for (int i = blockIdx.x * kT + threadIdx.x; i < s.n; i += gridDim.x * kT) {
         const size_t o = (size_t)ci * w.maxSrc + i;
         if (w.nnId[o] < 0)
@@ -184,7 +193,7 @@ __global__ void __launch_bounds__(kT) k_resid_tree(Work w, Stage s) {
         float        y[3];
         smi::pose_apply(C.step, x.x, x.y, x.z, y[0], y[1], y[2]);
         smk::NnSet rs;
-        rs.init();
+        rs.init(smk::nn_bound(smk::nn_bound(smk::eval_metric(y, s.dPos[w.nnId[o]]), exc), exc));
         smk::kd_search(s.tree, y, rs);
         w.resid[o] = smm::fsqrt(rs.dist);
     }
@@ -603,21 +612,24 @@ __global__ void __launch_bounds__(kT, 6) k_inliers(Work w, const float4 *__restr
 }
 
 // Inliers with the reference's search: the nearest point of the full tree closer than the
-// scoring distance (inliner, util.cpp:628-641), one thread per source point.
+// scoring distance (inliner, util.cpp:628-641), one thread per source point; only that
+// distance matters, so the search starts from its bound.
 __global__ void __launch_bounds__(kT) k_inliers_tree(Work w, const float4 *__restrict__ src, int n,
-                                                     smk::KdView F, float r2) {
+                                                     smk::KdView F, float r2,
+                                                     const float *__restrict__ exc) {
     chain_enter(); // launched chained
     __shared__ int sc[kW];
     const int      ci = blockIdx.y;
     const Cand    &C  = w.cand[ci];
     if (!C.active)
         return;
-    int c = 0;
+    const float start = smk::nn_bound(r2, *exc);
+    int         c     = 0;
     for (int i = blockIdx.x * kT + threadIdx.x; i < n; i += gridDim.x * kT) {
         float q[3];
         smi::pose_apply(C.M, src[i].x, src[i].y, src[i].z, q[0], q[1], q[2]);
         smk::NnSet rs;
-        rs.init();
+        rs.init(start);
         smk::kd_search(F, q, rs);
         c += (rs.count && rs.dist < r2) ? 1 : 0;
     }
@@ -729,7 +741,8 @@ void icp_all(Ctx &c, const Model &m, const IcpScene &sc, const IcpParams &p, con
     auto inliers = [&](const float4 *src, int n) {
         if (tree)
             launch_chained(c, k_inliers_tree, dim3(std::max(1, nblocks(n, kT)), ncand), kT, 0,
-                           w, src, n, sc.tree->view(nullptr, sc.pos, nullptr, sc.tpF), sc2);
+                           w, src, n, sc.tree->view(nullptr, sc.pos, nullptr, sc.tpF), sc2,
+                           sc.exc + 2);
         else
             launch_chained(c, k_inliers, dim3(std::max(1, nblocks(n, kW)), ncand), kT, 0, w,
                            src, n, sc.full.view(), sc2);
@@ -740,6 +753,7 @@ void icp_all(Ctx &c, const Model &m, const IcpScene &sc, const IcpParams &p, con
         if (tree) {
             s.tree   = sc.tree->view(sc.ioiS, sc.pos, sc.neS, sc.tpS);
             s.rankOf = sc.rankS;
+            s.exc    = sc.exc;
         }
         run_stage(c, w, s, ncand);
         launch_chained(c, k_stage_end, nblocks(ncand, 128), 128, 0, w, ncand, 2);
@@ -752,6 +766,7 @@ void icp_all(Ctx &c, const Model &m, const IcpScene &sc, const IcpParams &p, con
             if (tree) {
                 d.tree   = sc.tree->view(sc.ioiR, sc.pos, sc.neR, sc.tpR);
                 d.rankOf = sc.rankR;
+                d.exc    = sc.exc + 1;
             }
             run_stage(c, w, d, ncand);
             launch_chained(c, k_stage_end, nblocks(ncand, 128), 128, 0, w, ncand, 4);

@@ -1045,18 +1045,27 @@ __global__ void k_kd_nonempty(const int4 *__restrict__ nd, const int *__restrict
             break;
 }
 
+// Leaf records, and with excMax (zeroed) the largest distance of a listed point from its
+// leaf's build-time box, rounded up (as float bits: they order like the floats).
 __global__ void k_kd_tpos(const int *__restrict__ vacc, int m, const float4 *__restrict__ pos,
-                          float4 *__restrict__ tpos) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m)
-        return;
-    const int id = vacc[i];
-    if (id < 0) {
+                          const float *__restrict__ nodeBox, const int *__restrict__ leafOf,
+                          float4 *__restrict__ tpos, float *__restrict__ excMax) {
+    const int i  = blockIdx.x * blockDim.x + threadIdx.x;
+    const int id = i < m ? vacc[i] : -1;
+    float     e  = 0.0f;
+    if (id >= 0) {
+        const float4 p = pos[id];
+        tpos[i]        = make_float4(p.x, p.y, p.z, __int_as_float(id));
+        if (excMax)
+            e = (float)(excursion(nodeBox + 6 * (size_t)leafOf[i], p) * (1.0 + 1e-6));
+    } else if (i < m) {
         tpos[i] = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
-        return;
     }
-    const float4 p = pos[id];
-    tpos[i]        = make_float4(p.x, p.y, p.z, __int_as_float(id));
+    if (excMax) {
+        const unsigned w = __reduce_max_sync(0xffffffffu, __float_as_uint(e));
+        if ((threadIdx.x & 31) == 0 && w)
+            atomicMax((unsigned *)excMax, w);
+    }
 }
 
 } // namespace
@@ -1297,11 +1306,13 @@ void kd_mark_nonempty(Ctx &c, const KdTree &T, const int *vaccActive, int *flags
 }
 
 void kd_tree_positions(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
-                       float4 *tpos) {
+                       float4 *tpos, float *excMax) {
+    if (excMax)
+        SM_CUDA(cudaMemsetAsync(excMax, 0, sizeof(float), c.stream));
     if (T.m <= 0)
         return;
     k_kd_tpos<<<nblocks(T.m, 256), 256, 0, c.stream>>>(vaccActive ? vaccActive : T.vacc, T.m, pos,
-                                                        tpos);
+                                                        T.box, T.leafOf, tpos, excMax);
     SM_LAUNCH_CHECK();
 }
 

@@ -114,14 +114,15 @@ template <int K> struct KnnSet {
     }
 };
 
-// The one-nearest result set (KNNResultSet with capacity 1).
+// The one-nearest result set (KNNResultSet with capacity 1). `bound` starts the worst
+// distance (the reference starts at the largest float; see nn_bound).
 struct NnSet {
     int   idx;
     float dist;
     int   count;
-    __device__ void init() {
+    __device__ void init(float bound = 3.402823466e38f) {
         idx   = -1;
-        dist  = 3.402823466e38f;
+        dist  = bound;
         count = 0;
     }
     __device__ __forceinline__ float worst() const { return dist; }
@@ -133,6 +134,23 @@ struct NnSet {
         count = 1;
     }
 };
+
+// Start bound of a one-nearest search whose result only matters up to squared distance d2,
+// on a tree whose points lie at most `exc` outside their leaves' build-time boxes. The search
+// from this bound ends with the same point as the reference's search from the largest float
+// whenever that point's squared distance is at most d2, and with a point farther than d2 (or
+// none) whenever the reference's is farther:
+// - every node on the way to a point at distance r has a lower bound of at most (r + exc)^2
+//   (the margin covers the float rounding of the running bound), so with the point's own
+//   bound start the search prunes nothing the reference's result lies in by the start bound;
+// - the points it meets are a subset of those the reference's search meets, in the same order,
+//   so its running worst is never smaller than the reference's except by the start bound.
+__device__ __forceinline__ float nn_bound(float d2, float exc) {
+    const float r = smm::fsqrt(d2) + exc;
+    // (a non-finite bound, from an unlimited d2, falls back to the reference's start; the
+    // addend keeps the bound above a result at distance zero)
+    return fminf(r * r * (1.0f + 1e-4f) + 1e-30f, 3.402823466e38f);
+}
 
 // findNeighbors + searchLevel (nanoflann.hpp:1846-1930) iteratively: a frame per pending
 // far child keeps the node's entry state, so the far child is entered exactly when and

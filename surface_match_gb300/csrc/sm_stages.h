@@ -321,9 +321,10 @@ void kd_knn(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
 void kd_mark_nonempty(Ctx &c, const KdTree &T, const int *vaccActive, int *flags);
 // tpos[i] = pos[id] with w = id bits for the tree positions i whose vaccActive entry id is
 // >= 0, else w = -1 bits: the leaf records of the searches (taken after the positions last
-// moved).
+// moved). excMax (nullable, device): the largest distance of those points from their leaves'
+// build-time boxes (smk::nn_bound).
 void kd_tree_positions(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
-                       float4 *tpos);
+                       float4 *tpos, float *excMax = nullptr);
 // The voting stage's radius searches (ppf.cpp:273-276) in the reduced tree: for each of the
 // K keypoints the candidates (cand[0..ncand), the sampled points) its search of radius^2 r2
 // returns, as CSR lists (*offOut: K + 1 offsets, *idsOut: ids) whose last (rows mod 8) rows
@@ -390,6 +391,7 @@ struct IcpScene {
     const int    *ioiS = nullptr, *ioiR = nullptr, *rankS = nullptr, *rankR = nullptr;
     const int    *neS = nullptr, *neR = nullptr;                  // non-empty node flags
     const float4 *tpS = nullptr, *tpR = nullptr, *tpF = nullptr; // leaf records
+    const float  *exc = nullptr; // largest excursion from the leaf boxes: S, R, all points
 };
 struct IcpParams {
     int   sparse, dense, denseSteps;

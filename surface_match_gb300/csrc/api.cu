@@ -116,17 +116,20 @@ __global__ void k_gather_poses(const float *__restrict__ poses, const int *__res
         out[(size_t)i * smi::kPoseFloats + e] = poses[(size_t)s * smi::kPoseFloats + e];
 }
 
-__global__ void k_rank_of(const int *__restrict__ ids, int m, int *__restrict__ rank) {
+__global__ void k_rank_of(const int *__restrict__ ids, int m, const int *__restrict__ treePos,
+                          int *__restrict__ rank, int *__restrict__ tpos) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < m)
-        rank[ids[r]] = r;
+    if (r >= m)
+        return;
+    rank[ids[r]] = r;
+    tpos[r]      = treePos[ids[r]];
 }
 
-// rank[ids[r]] = r for r < m
-void rank_of(Ctx &c, const int *ids, int m, int *rank) {
+// rank[ids[r]] = r and tpos[r] = treePos[ids[r]] for r < m
+void rank_of(Ctx &c, const int *ids, int m, const int *treePos, int *rank, int *tpos) {
     if (m <= 0)
         return;
-    k_rank_of<<<nblocks(m, 256), 256, 0, c.stream>>>(ids, m, rank);
+    k_rank_of<<<nblocks(m, 256), 256, 0, c.stream>>>(ids, m, treePos, rank, tpos);
     SM_LAUNCH_CHECK();
 }
 
@@ -319,33 +322,27 @@ void train(Ctx &c, Model &m, const float *xyzIn, const float *nrmIn, int64_t n64
     int        *idx1         = c.arena.get<int>("t.idx1", n);
     int        *idx2         = c.arena.get<int>("t.idx2", n);
     int         n1 = 0, n2 = 0;
+    KdTree      T;
     if (m.order == SM_ORDER_REFERENCE) {
         // the reference's tree over the model (ppf.cpp:77-83): both samplings in tree order
         // on the positions as given, then normals from the tree's k nearest
-        KdTree T;
         build_kdtree(c, pos, n, valid, nvalid, box, T, "t.tree");
         n1 = kd_sample(c, T, nullptr, pos, sampleStep, box, idx1, nullptr, "t.s1");
         n2 = kd_sample(c, T, nullptr, pos, reSampleStep, box, idx2, nullptr, "t.s2");
-        if (!nrmIn) {
-            HGrid none;
-            estimate_normals(c, pos, nrm, n, idx1, n1, none, tp.knnNormal, tp.smoothNormal != 0,
-                             false, nullptr, "t.n1", &T);
-            estimate_normals(c, pos, nrm, n, idx2, n2, none, tp.knnNormal, tp.smoothNormal != 0,
-                             false, nullptr, "t.n2", &T);
-        }
     } else {
         n1 = sample_points(c, pos, n, valid, nvalid, box, sampleStep, idx1, "t.s1");
         n2 = sample_points(c, pos, n, valid, nvalid, box, reSampleStep, idx2, "t.s2");
-        if (!nrmIn) {
-            HGrid q;
-            const float gq = knn_cell(nvalid, n1, sampleStep, tp.knnNormal);
-            build_hgrid(c, pos, valid, nvalid, box, gq, q, "t.q");
-            estimate_normals(c, pos, nrm, n, idx1, n1, q, tp.knnNormal, tp.smoothNormal != 0, false,
-                             nullptr, "t.n1");
-            build_hgrid(c, pos, valid, nvalid, box, gq, q, "t.q");
-            estimate_normals(c, pos, nrm, n, idx2, n2, q, tp.knnNormal, tp.smoothNormal != 0, false,
-                             nullptr, "t.n2");
-        }
+    }
+    if (!nrmIn) {
+        const KdTree *tree = m.order == SM_ORDER_REFERENCE ? &T : nullptr;
+        HGrid         q;
+        const float   gq = knn_cell(nvalid, n1, sampleStep, tp.knnNormal);
+        build_hgrid(c, pos, valid, nvalid, box, gq, q, "t.q");
+        estimate_normals(c, pos, nrm, n, idx1, n1, q, tp.knnNormal, tp.smoothNormal != 0, false,
+                         nullptr, "t.n1", tree);
+        build_hgrid(c, pos, valid, nvalid, box, gq, q, "t.q");
+        estimate_normals(c, pos, nrm, n, idx2, n2, q, tp.knnNormal, tp.smoothNormal != 0, false,
+                         nullptr, "t.n2", tree);
     }
     float4 *sp = c.arena.get<float4>("t.sp", std::max(n1, 1));
     float4 *sn = c.arena.get<float4>("t.sn", std::max(n1, 1));
@@ -510,17 +507,14 @@ void match(Ctx &c, const Model &m, const float *xyzIn, const float *nrmIn, int64
         build_kdtree(c, pos, n, valid, nvalid, box, T, "m.tree");
         ioi = c.arena.get<int>("m.ioi", std::max(nvalid, 1));
         ns  = kd_sample(c, T, nullptr, pos, sampleStep, box, sampled, ioi, "m.s1");
-        if (!hasN)
-            estimate_normals(c, pos, nrm, n, sampled, ns, q, mp.knnNormal, mp.smoothNormal != 0,
-                             mp.invertNormal != 0, vp, "m.n1", &T);
     } else {
         ns = sample_points(c, pos, n, valid, nvalid, box, sampleStep, sampled, "m.s1");
-        gq = knn_cell(nvalid, ns, sampleStep, mp.knnNormal);
-        if (!hasN) {
-            build_hgrid(c, pos, valid, nvalid, box, gq, q, "m.q");
-            estimate_normals(c, pos, nrm, n, sampled, ns, q, mp.knnNormal, mp.smoothNormal != 0,
-                             mp.invertNormal != 0, vp, "m.n1");
-        }
+    }
+    gq = knn_cell(nvalid, ns, sampleStep, mp.knnNormal);
+    if (!hasN) {
+        build_hgrid(c, pos, valid, nvalid, box, gq, q, "m.q");
+        estimate_normals(c, pos, nrm, n, sampled, ns, q, mp.knnNormal, mp.smoothNormal != 0,
+                         mp.invertNormal != 0, vp, "m.n1", ref ? &T : nullptr);
     }
     record(c, 2);
     float maxOverlap = 0;
@@ -558,25 +552,28 @@ void match(Ctx &c, const Model &m, const float *xyzIn, const float *nrmIn, int64
         int *resampled = d.arena.get<int>("m.resampled", std::max(n, 1));
         s.pos = P;
         s.nrm = N;
-        if (ref) {
-            // restore() and resample the whole tree, normals without smoothing (ppf.cpp:428-
-            // 434); the refinement searches the tree reduced to each subset, and scores on
-            // the whole tree
-            int *ioi2 = d.arena.get<int>("m.ioi2", std::max(nvalid, 1));
-            if (mp.densePoseRefinement) {
-                nres = kd_sample(d, T, nullptr, P, reSampleStep, box, resampled, ioi2, "m.s3");
-                if (!hasN) {
-                    HGrid none;
-                    estimate_normals(d, P, N, n, resampled, nres, none, mp.knnNormal, false,
-                                     mp.invertNormal != 0, vp, "m.n2", &T);
-                }
+        // restore() and resample the whole scene, normals without smoothing (ppf.cpp:428-434)
+        int *ioi2 = ref ? d.arena.get<int>("m.ioi2", std::max(nvalid, 1)) : nullptr;
+        if (mp.densePoseRefinement) {
+            nres = ref ? kd_sample(d, T, nullptr, P, reSampleStep, box, resampled, ioi2, "m.s3")
+                       : sample_points(d, P, n, valid, nvalid, box, reSampleStep, resampled, "m.s3");
+            if (!hasN) {
+                HGrid q2;
+                build_hgrid(d, P, valid, nvalid, box, gq, q2, "m.q");
+                estimate_normals(d, P, N, n, resampled, nres, q2, mp.knnNormal, false,
+                                 mp.invertNormal != 0, vp, "m.n2", ref ? &T : nullptr);
             }
-            int *rankS = d.arena.get<int>("m.rankS", std::max(n, 1));
-            int *rankR = d.arena.get<int>("m.rankR", std::max(n, 1));
-            rank_of(d, sampled, ns, rankS);
-            rank_of(d, resampled, nres, rankR);
-            // the refinement's searches: empty subtrees of the reduced trees are skipped,
-            // leaves read tree-ordered records of the positions as they are now
+        }
+        if (ref) {
+            // the refinement searches the tree reduced to each subset, and scores on the
+            // whole tree; empty subtrees of the reduced trees are skipped, leaves read
+            // tree-ordered records of the positions as they are now
+            int    *rankS = d.arena.get<int>("m.rankS", std::max(n, 1));
+            int    *rankR = d.arena.get<int>("m.rankR", std::max(n, 1));
+            int    *tposS = d.arena.get<int>("m.tposS", std::max(ns, 1));
+            int    *tposR = d.arena.get<int>("m.tposR", std::max(nres, 1));
+            rank_of(d, sampled, ns, T.treePos, rankS, tposS);
+            rank_of(d, resampled, nres, T.treePos, rankR, tposR);
             int    *neS = d.arena.get<int>("m.neS", std::max(T.nnodes, 1));
             int    *neR = d.arena.get<int>("m.neR", std::max(T.nnodes, 1));
             float4 *tpS = d.arena.get<float4>("m.tpS", std::max(T.m, 1));
@@ -590,41 +587,31 @@ void match(Ctx &c, const Model &m, const float *xyzIn, const float *nrmIn, int64
                 kd_tree_positions(d, T, ioi2, P, tpR, exc + 1);
             }
             kd_tree_positions(d, T, nullptr, P, tpF, exc + 2);
-            s.exc         = exc;
-            s.neS         = neS;
-            s.neR         = neR;
-            s.tpS         = tpS;
-            s.tpR         = tpR;
-            s.tpF         = tpF;
-            s.tree        = &T;
-            s.ioiS        = ioi;
-            s.ioiR        = ioi2;
-            s.rankS       = rankS;
-            s.rankR       = rankR;
-            s.sampled.m   = ns;
-            s.resampled.m = nres;
-        } else {
-            if (mp.densePoseRefinement) {
-                nres = sample_points(d, P, n, valid, nvalid, box, reSampleStep, resampled, "m.s3");
-                if (!hasN) {
-                    HGrid q2;
-                    build_hgrid(d, P, valid, nvalid, box, gq, q2, "m.q");
-                    estimate_normals(d, P, N, n, resampled, nres, q2, mp.knnNormal, false,
-                                     mp.invertNormal != 0, vp, "m.n2");
-                }
-            }
-            // Nearest-neighbour grids of the refinement: cells of about a third of the
-            // rejection distance (never finer than the subset's spacing), so three cell
-            // shells always cover it. The inlier grid's cell just exceeds the scoring
-            // distance, so two shells decide. The subset grids name points by subset rank
-            // (the subsets are ascending, so rank order is index order), and the refinement
-            // reads rank-ordered copies of the subsets.
-            build_hgrid(d, P, sampled, ns, box, std::max(sampleStep, refDist / 2.98f), s.sampled,
-                        "m.gS", true);
-            build_hgrid(d, P, resampled, nres, box, std::max(2.0f * reSampleStep, refDist / 2.98f),
-                        s.resampled, "m.gR", true);
-            build_hgrid(d, P, valid, nvalid, box, std::max(scoreDist * 1.02f, gq), s.full, "m.gF");
+            s.exc   = exc;
+            s.neS   = neS;
+            s.neR   = neR;
+            s.tpS   = tpS;
+            s.tpR   = tpR;
+            s.tpF   = tpF;
+            s.tree  = &T;
+            s.ioiS  = ioi;
+            s.ioiR  = ioi2;
+            s.rankS = rankS;
+            s.rankR = rankR;
+            s.tposS = tposS;
+            s.tposR = tposR;
         }
+        // Nearest-neighbour grids of the refinement: cells of about a third of the
+        // rejection distance (never finer than the subset's spacing), so three cell
+        // shells always cover it. The inlier grid's cell just exceeds the scoring
+        // distance, so two shells decide. The subset grids name points by subset rank
+        // (in grid order the subsets are ascending, so rank order is index order), and the
+        // refinement reads rank-ordered copies of the subsets.
+        build_hgrid(d, P, sampled, ns, box, std::max(sampleStep, refDist / 2.98f), s.sampled,
+                    "m.gS", true);
+        build_hgrid(d, P, resampled, nres, box, std::max(2.0f * reSampleStep, refDist / 2.98f),
+                    s.resampled, "m.gR", true);
+        build_hgrid(d, P, valid, nvalid, box, std::max(scoreDist * 1.02f, gq), s.full, "m.gF");
         float4 *posS = d.arena.get<float4>("m.posS", std::max(ns, 1));
         float4 *nrmS = d.arena.get<float4>("m.nrmS", std::max(ns, 1));
         float4 *posR = d.arena.get<float4>("m.posR", std::max(nres, 1));
@@ -1153,7 +1140,7 @@ SM_API int sm_kdtree_probe(sm_context ctx, const float *xyzIn, int64_t n64, floa
             int   *nb  = c.arena.get<int>("kp.nb", (size_t)nq * k);
             float *nd  = c.arena.get<float>("kp.nd", (size_t)nq * k);
             SM_CUDA(cudaMemcpyAsync(cnt, &nq, sizeof(int), cudaMemcpyHostToDevice, c.stream));
-            kd_knn(c, T, nullptr, pos, q4, nullptr, cnt, nq, k, nb, nd, nullptr);
+            kd_knn(c, T, nullptr, pos, q4, cnt, nq, k, nb, nd);
             c.sync_checked();
             SM_CUDA(cudaMemcpy(outKnn, nb, (size_t)nq * k * 4, cudaMemcpyDeviceToHost));
             if (outKnnDist)

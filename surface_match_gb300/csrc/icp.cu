@@ -20,6 +20,7 @@
 #include <cooperative_groups.h>
 
 #include "sm_icp.h"
+#include "sm_kdgrid.cuh"
 #include "sm_stages.h"
 
 namespace sm {
@@ -54,10 +55,12 @@ struct Stage {
     int           iters;
     float         mseMin, mseMax, rej2;
     int           traceOff; // 0 sparse, 1 dense
-    // reference search order: nearest points from the k-d tree reduced to the stage's
-    // subset (rankOf maps a point id to its subset rank); tree.nd == nullptr: the grid G
+    // reference search order: nearest points as the k-d tree reduced to the stage's subset
+    // finds them (rankOf maps a point id to its subset rank, tposOf a rank to its tree
+    // position); tree.nd == nullptr: the nearest points of the grid G
     smk::KdView   tree;
-    const int    *rankOf;
+    int           treeM; // tree positions
+    const int    *rankOf, *tposOf;
     const float  *exc; // largest excursion of the subset's points from their leaves' boxes
 };
 
@@ -84,8 +87,24 @@ __device__ __forceinline__ bool cand_live(const Cand &c, const Stage &s) {
     return c.active && !c.stop && c.iterations < s.iters;
 }
 
-// K1: correspondences, one warp per source point (warp-cooperative grid search)
-__global__ void __launch_bounds__(kT, 4) k_corr(Work w, Stage s, int usePrev) {
+// The nearest point of the stage's subset to (x, y, z) by a warp, exact where its squared
+// distance is at most lim: subset rank (-1: none found) and squared distance d. With TREE the
+// point that the reference's search finds (sm_kdgrid.cuh).
+template <bool TREE>
+__device__ __forceinline__ int stage_nearest(const Stage &s, float x, float y, float z, float lim,
+                                             float &d) {
+    if (TREE)
+        return smk::warp_kd_nearest(s.tree, s.treeM, s.G, s.tposOf, s.rankOf, *s.exc, x, y, z, lim,
+                                    &d);
+    return warp_nn_walk(s.G, x, y, z, lim, d);
+}
+
+// K1: correspondences, one warp per source point (warp-cooperative grid search). In reference
+// order (TREE) a pair is what findClosestPoint (util.cpp:603-626) returns: a one-nearest search
+// of the reduced k-d tree with the tree's pruning; one beyond the rejection distance is
+// dropped, so the search is needed up to that distance only.
+template <bool TREE>
+__global__ void __launch_bounds__(kT, TREE ? 3 : 4) k_corr(Work w, Stage s, int usePrev) {
     chain_enter(); // launched chained
     const int ci   = blockIdx.y;
     const int lane = threadIdx.x & 31;
@@ -118,7 +137,7 @@ __global__ void __launch_bounds__(kT, 4) k_corr(Work w, Stage s, int usePrev) {
         if (jp >= 0 && jp < s.nDst)
             lim = fminf(lim, smm::dist2(x.x, x.y, x.z, qp.x, qp.y, qp.z));
         float      d;
-        const int  j  = warp_nn_walk(s.G, x.x, x.y, x.z, lim, d); // subset rank
+        const int  j  = stage_nearest<TREE>(s, x.x, x.y, x.z, lim, d); // subset rank
         const bool ok = j >= 0 && d <= s.rej2;
         if (lane == 0) {
             w.nnPrev[o] = j;
@@ -131,71 +150,6 @@ __global__ void __launch_bounds__(kT, 4) k_corr(Work w, Stage s, int usePrev) {
             if (ok)
                 atomicMin(&w.win[(size_t)ci * w.maxDst + j], win_key(d, i));
         }
-    }
-}
-
-// K1 with the reference's search: one thread per source point, the nearest point of the
-// reduced k-d tree (findClosestPoint, util.cpp:603-626: a 1-nearest search from the root,
-// with the tree's pruning) - the same pair rules as k_corr. A pair farther than the rejection
-// distance is dropped, so the search starts from that distance's bound (smk::nn_bound): a
-// model point without a scene point near it (a hidden side) then prunes at the root instead of
-// walking thousands of leaves for a far point nobody uses.
-__global__ void __launch_bounds__(kT) k_corr_tree(Work w, Stage s) {
-    chain_enter(); // launched chained
-    const int   ci = blockIdx.y;
-    const Cand &C  = w.cand[ci];
-    if (!cand_live(C, s))
-        return;
-    if (w.live && blockIdx.x == 0 && threadIdx.x == 0)
-        atomicAdd(w.live, (unsigned long long)s.n);
-    const float start = smk::nn_bound(s.rej2, *s.exc);
-    for (int i = blockIdx.x * kT + threadIdx.x; i < s.n; i += gridDim.x * kT) {
-        const size_t o  = (size_t)ci * w.maxSrc + i;
-        const float4 sp = s.src[i], sn = s.srcN[i];
-        float4       x, y;
-        smi::pose_apply(C.M, sp.x, sp.y, sp.z, x.x, x.y, x.z);
-        smi::pose_rotate(C.M, sn.x, sn.y, sn.z, y.x, y.y, y.z);
-        const float q[3] = {x.x, x.y, x.z};
-        smk::NnSet  rs;
-        rs.init(start);
-        smk::kd_search(s.tree, q, rs);
-        const int   j  = rs.count ? s.rankOf[rs.idx] : -1;
-        const float d  = rs.dist;
-        const bool  ok = j >= 0 && d <= s.rej2;
-        w.nnPrev[o] = j;
-        x.w         = d;
-        y.w         = 0.0f;
-        w.x4[o]     = x;
-        w.n4[o]     = y;
-        w.nnId[o]   = ok ? j : -1;
-        w.nnR[o]    = ok ? j : -1;
-        if (ok)
-            atomicMin(&w.win[(size_t)ci * w.maxDst + j], win_key(d, i));
-    }
-}
-
-// K4 with the reference's search: residual of each pair, one thread per pair. The pair's scene
-// point, at squared distance u, is in the tree: the reference's result lies within
-// (sqrt(u) + exc)^2 (its search either meets that point or prunes it against a nearer one),
-// so the search starts from the bound of that distance.
-__global__ void __launch_bounds__(kT) k_resid_tree(Work w, Stage s) {
-    chain_enter(); // launched chained
-    const int   ci = blockIdx.y;
-    const Cand &C  = w.cand[ci];
-    if (!cand_live(C, s) || C.cnt < 6)
-        return;
-    const float exc = *s.exc;
-    for (int i = blockIdx.x * kT + threadIdx.x; i < s.n; i += gridDim.x * kT) {
-        const size_t o = (size_t)ci * w.maxSrc + i;
-        if (w.nnId[o] < 0)
-            continue;
-        const float4 x = w.x4[o];
-        float        y[3];
-        smi::pose_apply(C.step, x.x, x.y, x.z, y[0], y[1], y[2]);
-        smk::NnSet rs;
-        rs.init(smk::nn_bound(smk::nn_bound(smk::eval_metric(y, s.dPos[w.nnId[o]]), exc), exc));
-        smk::kd_search(s.tree, y, rs);
-        w.resid[o] = smm::fsqrt(rs.dist);
     }
 }
 
@@ -432,7 +386,8 @@ __global__ void __cluster_dims__(kRC, 1, 1) __launch_bounds__(kR) k_fit(Work w, 
 }
 
 // K4: residual distance of each pair after the step, one warp per pair
-__global__ void __launch_bounds__(kT, 5) k_resid(Work w, Stage s) {
+template <bool TREE>
+__global__ void __launch_bounds__(kT, TREE ? 3 : 5) k_resid(Work w, Stage s) {
     chain_enter(); // launched chained
     const int   ci = blockIdx.y;
     const Cand &C  = w.cand[ci];
@@ -447,7 +402,7 @@ __global__ void __launch_bounds__(kT, 5) k_resid(Work w, Stage s) {
         float        y0, y1, y2, d;
         smi::pose_apply(C.step, x.x, x.y, x.z, y0, y1, y2);
         // the pair's scene point bounds the search exactly
-        warp_nn_walk(s.G, y0, y1, y2, smm::dist2(y0, y1, y2, q.x, q.y, q.z), d);
+        stage_nearest<TREE>(s, y0, y1, y2, smm::dist2(y0, y1, y2, q.x, q.y, q.z), d);
         if ((threadIdx.x & 31) == 0)
             w.resid[(size_t)ci * w.maxSrc + i] = smm::fsqrt(d);
     }
@@ -583,9 +538,12 @@ __global__ void k_stage_end(Work w, int ncand, int failStatus) {
 }
 
 // Inliers of each candidate: source points with a scene point closer than the scoring
-// distance, one warp per point (warp_any_within).
-__global__ void __launch_bounds__(kT, 6) k_inliers(Work w, const float4 *__restrict__ src, int n,
-                                                HGridView F, float r2) {
+// distance, one warp per point (warp_any_within); with TREE the scene point that the
+// reference's search of the whole tree returns (inliner, util.cpp:628-641).
+template <bool TREE>
+__global__ void __launch_bounds__(kT, TREE ? 3 : 6)
+    k_inliers(Work w, const float4 *__restrict__ src, int n, HGridView F, float r2, smk::KdView t,
+              int treeM, const int *__restrict__ treePos, const float *__restrict__ exc) {
     chain_enter(); // launched chained
     __shared__ int sc[kW];
     const int      ci = blockIdx.y;
@@ -597,52 +555,24 @@ __global__ void __launch_bounds__(kT, 6) k_inliers(Work w, const float4 *__restr
     for (int i = blockIdx.x * kW + (threadIdx.x >> 5); i < n; i += gridDim.x * kW) {
         float x, y, z;
         smi::pose_apply(C.M, src[i].x, src[i].y, src[i].z, x, y, z);
-        c += warp_any_within(F, x, y, z, r2) ? 1 : 0;
+        if (TREE) {
+            float     d;
+            const int j =
+                smk::warp_kd_nearest(t, treeM, F, treePos, nullptr, *exc, x, y, z, r2, &d);
+            c += (j >= 0 && d < r2) ? 1 : 0;
+        } else {
+            c += warp_any_within(F, x, y, z, r2) ? 1 : 0;
+        }
     }
     if (lane == 0)
         sc[threadIdx.x >> 5] = c;
     __syncthreads();
     if (threadIdx.x == 0) {
-        int t = 0;
+        int t2 = 0;
         for (int k = 0; k < kW; k++)
-            t += sc[k];
-        if (t)
-            atomicAdd(&w.cand[ci].inl, t);
-    }
-}
-
-// Inliers with the reference's search: the nearest point of the full tree closer than the
-// scoring distance (inliner, util.cpp:628-641), one thread per source point; only that
-// distance matters, so the search starts from its bound.
-__global__ void __launch_bounds__(kT) k_inliers_tree(Work w, const float4 *__restrict__ src, int n,
-                                                     smk::KdView F, float r2,
-                                                     const float *__restrict__ exc) {
-    chain_enter(); // launched chained
-    __shared__ int sc[kW];
-    const int      ci = blockIdx.y;
-    const Cand    &C  = w.cand[ci];
-    if (!C.active)
-        return;
-    const float start = smk::nn_bound(r2, *exc);
-    int         c     = 0;
-    for (int i = blockIdx.x * kT + threadIdx.x; i < n; i += gridDim.x * kT) {
-        float q[3];
-        smi::pose_apply(C.M, src[i].x, src[i].y, src[i].z, q[0], q[1], q[2]);
-        smk::NnSet rs;
-        rs.init(start);
-        smk::kd_search(F, q, rs);
-        c += (rs.count && rs.dist < r2) ? 1 : 0;
-    }
-    c = __reduce_add_sync(0xffffffffu, c);
-    if ((threadIdx.x & 31) == 0)
-        sc[threadIdx.x >> 5] = c;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int t = 0;
-        for (int k = 0; k < kW; k++)
-            t += sc[k];
-        if (t)
-            atomicAdd(&w.cand[ci].inl, t);
+            t2 += sc[k];
+        if (t2)
+            atomicAdd(&w.cand[ci].inl, t2);
     }
 }
 
@@ -681,25 +611,24 @@ __global__ void k_finish(Work w, int ncand, int refine, float minScore, int *sta
 
 void run_stage(Ctx &c, Work &w, const Stage &s, int ncand) {
     const dim3 gc(ncand * kRC);                               // reductions: a cluster per candidate
-    const dim3 gw(std::max(1, nblocks(s.n, kW)), ncand); // warp kernels: a warp per point
-    const dim3 gt(std::max(1, nblocks(s.n, kT)), ncand); // tree searches: a thread per point
+    const dim3 gw(std::max(1, nblocks(s.n, kW)), ncand); // searches: a warp per point
     const bool tree = s.tree.nd != nullptr;
     launch_chained(c, k_stage_begin, nblocks(ncand, 128), 128, 0, w, ncand);
     for (int it = 0; it < s.iters; it++) {
         cudaEvent_t t0 = c.clock.begin(c.stream);
         if (tree)
-            launch_chained(c, k_corr_tree, gt, kT, 0, w, s);
+            launch_chained(c, k_corr<true>, gw, kT, 0, w, s, it > 0 ? 1 : 0);
         else
-            launch_chained(c, k_corr, gw, kT, 0, w, s, it > 0 ? 1 : 0);
+            launch_chained(c, k_corr<false>, gw, kT, 0, w, s, it > 0 ? 1 : 0);
         c.clock.end(c.stream, t0, KernelClock::kCorr, 0.0); // bytes from the live count
         t0 = c.clock.begin(c.stream);
         launch_chained(c, k_fit, gc, kR, 0, w, s);
         c.clock.end(c.stream, t0, KernelClock::kFit, 0.0);
         t0 = c.clock.begin(c.stream);
         if (tree)
-            launch_chained(c, k_resid_tree, gt, kT, 0, w, s);
+            launch_chained(c, k_resid<true>, gw, kT, 0, w, s);
         else
-            launch_chained(c, k_resid, gw, kT, 0, w, s);
+            launch_chained(c, k_resid<false>, gw, kT, 0, w, s);
         c.clock.end(c.stream, t0, KernelClock::kResid, 0.0);
         t0 = c.clock.begin(c.stream);
         launch_chained(c, k_update, gc, kR, 0, w, s);
@@ -739,20 +668,23 @@ void icp_all(Ctx &c, const Model &m, const IcpScene &sc, const IcpParams &p, con
     const float sc2  = p.scoreDist * p.scoreDist;
     const bool tree = sc.tree != nullptr;
     auto inliers = [&](const float4 *src, int n) {
+        const dim3 g(std::max(1, nblocks(n, kW)), ncand);
         if (tree)
-            launch_chained(c, k_inliers_tree, dim3(std::max(1, nblocks(n, kT)), ncand), kT, 0,
-                           w, src, n, sc.tree->view(nullptr, sc.pos, nullptr, sc.tpF), sc2,
-                           sc.exc + 2);
+            launch_chained(c, k_inliers<true>, g, kT, 0, w, src, n, sc.full.view(), sc2,
+                           sc.tree->view(nullptr, sc.pos, nullptr, sc.tpF), sc.tree->m,
+                           (const int *)sc.tree->treePos, sc.exc + 2);
         else
-            launch_chained(c, k_inliers, dim3(std::max(1, nblocks(n, kW)), ncand), kT, 0, w,
-                           src, n, sc.full.view(), sc2);
+            launch_chained(c, k_inliers<false>, g, kT, 0, w, src, n, sc.full.view(), sc2,
+                           smk::KdView{}, 0, (const int *)nullptr, (const float *)nullptr);
     };
     if (p.sparse) {
         Stage s{m.sp, m.sn, m.ns, nblocks(m.ns, kT), sc.sampled.view(), sc.posS, sc.nrmS, sc.sampled.m, 5,
                 p.sampleStep * 0.5f, p.sampleStep, rej2, 0};
         if (tree) {
             s.tree   = sc.tree->view(sc.ioiS, sc.pos, sc.neS, sc.tpS);
+            s.treeM  = sc.tree->m;
             s.rankOf = sc.rankS;
+            s.tposOf = sc.tposS;
             s.exc    = sc.exc;
         }
         run_stage(c, w, s, ncand);
@@ -765,7 +697,9 @@ void icp_all(Ctx &c, const Model &m, const IcpScene &sc, const IcpParams &p, con
                     sc.resampled.m, p.denseSteps, p.reSampleStep * 0.5f, p.sampleStep, rej2, 1};
             if (tree) {
                 d.tree   = sc.tree->view(sc.ioiR, sc.pos, sc.neR, sc.tpR);
+                d.treeM  = sc.tree->m;
                 d.rankOf = sc.rankR;
+                d.tposOf = sc.tposR;
                 d.exc    = sc.exc + 1;
             }
             run_stage(c, w, d, ncand);

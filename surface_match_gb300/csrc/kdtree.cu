@@ -34,6 +34,7 @@
 #include <climits>
 #include <cmath>
 
+#include "sm_kdgrid.cuh"
 #include "sm_kdtree.cuh"
 #include "sm_stages.h"
 
@@ -859,37 +860,72 @@ __global__ void k_sp_out(const int *__restrict__ flag, const int *__restrict__ p
         ioi[i] = kept ? vaccA[i] : -1;
 }
 
-// ---- k-nearest searches on the tree (one query per thread) -----------------------------
-// Query t: position qpos[t], or pos[list[t]] when qpos is null; t < *nq (device count).
-// Writes its k nearest ids in the reference's order (distance, then first found) and
-// their squared distances; cnt[t] = how many were found.
-__global__ void k_kd_knn(KdView t, const float4 *__restrict__ qpos, const int *__restrict__ list,
-                         const int *__restrict__ nq, int k, int *__restrict__ nbr,
-                         float *__restrict__ dist, int *__restrict__ cnt, int *__restrict__ err,
-                         const float4 *__restrict__ nrm, int *__restrict__ need) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= *nq)
-        return;
-    const float4 p    = qpos ? qpos[i] : t.pos[list[i]];
-    const float  q[3] = {p.x, p.y, p.z};
+// ---- k-nearest searches on the tree ------------------------------------------------------
+// The k nearest ids of query t < *nq (a device count) in the reference's order (distance, then
+// first found), and how many: by a thread over the tree.
+__device__ __forceinline__ void kd_knn_query(const KdView &t, const float q[3], int k,
+                                             int *__restrict__ nbr, float *__restrict__ dist,
+                                             int *__restrict__ cnt, int *__restrict__ err) {
     smk::KnnSet<kMaxKnn> rs;
     rs.init(k);
     if (!smk::kd_search(t, q, rs))
         atomicExch(err, 1);
     for (int j = 0; j < k; j++) {
-        const int id           = j < rs.count ? rs.idx[j] : -1;
-        nbr[(size_t)i * k + j] = id;
+        nbr[j] = j < rs.count ? rs.idx[j] : -1;
         if (dist)
-            dist[(size_t)i * k + j] = rs.dist[j];
-        // with smoothing, neighbours that still need a normal are marked for estimation
-        if (need && id >= 0 && need[id] == 0) {
-            const float4 n = nrm[id];
-            if (!(isfinite(n.x) && isfinite(n.y) && isfinite(n.z)))
-                need[id] = 1;
-        }
+            dist[j] = rs.dist[j];
     }
     if (cnt)
-        cnt[i] = rs.count;
+        *cnt = rs.count;
+}
+
+// One query per thread, at qpos[t].
+__global__ void k_kd_knn(KdView t, const float4 *__restrict__ qpos, const int *__restrict__ nq,
+                         int k, int *__restrict__ nbr, float *__restrict__ dist,
+                         int *__restrict__ err) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= *nq)
+        return;
+    const float4 p    = qpos[i];
+    const float  q[3] = {p.x, p.y, p.z};
+    kd_knn_query(t, q, k, nbr + (size_t)i * k, dist + (size_t)i * k, nullptr, err);
+}
+
+// One query per warp, the point list[t], answered on the grid of the tree's points
+// (sm_kdgrid.cuh). With smoothing, neighbours that still need a normal are marked.
+constexpr int kKnnBs = 256;
+__global__ void __launch_bounds__(kKnnBs)
+    k_kd_knn_grid(KdView t, int m, HGridView g, const int *__restrict__ treePos,
+                  const int *__restrict__ list, const int *__restrict__ nq, int k,
+                  int *__restrict__ nbr, int *__restrict__ cnt, int *__restrict__ err,
+                  const float4 *__restrict__ nrm, int *__restrict__ need) {
+    const int lane = threadIdx.x & 31;
+    const int i    = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (i >= *nq)
+        return;
+    const float4 p = t.pos[list[i]];
+    int          id;
+    int          n = smk::warp_kd_knearest(t, m, g, treePos, p.x, p.y, p.z, k, &id);
+    int         *L = nbr + (size_t)i * k;
+    if (n < 0) {
+        if (lane == 0) {
+            const float q[3] = {p.x, p.y, p.z};
+            kd_knn_query(t, q, k, L, nullptr, cnt + i, err);
+        }
+        __syncwarp();
+        n  = cnt[i];
+        id = lane < n ? L[lane] : -1;
+    } else {
+        if (lane < k)
+            L[lane] = lane < n ? id : -1;
+        if (lane == 0)
+            cnt[i] = n;
+    }
+    if (need && lane < n && need[id] == 0) {
+        const float4 v = nrm[id];
+        if (!(isfinite(v.x) && isfinite(v.y) && isfinite(v.z)))
+            need[id] = 1;
+    }
 }
 
 // ---- the voting stage's radius searches (ppf.cpp:273-276) -------------------------------
@@ -1254,8 +1290,7 @@ int kd_sample(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
 }
 
 void kd_knn(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
-            const float4 *qpos, const int *list, const int *nq, int nqMax, int k, int *nbr,
-            float *dist, int *cnt, const float4 *nrm, int *need) {
+            const float4 *qpos, const int *nq, int nqMax, int k, int *nbr, float *dist) {
     if (nqMax <= 0 || T.m <= 0)
         return;
     if (k < 1 || k > kMaxKnn)
@@ -1265,7 +1300,19 @@ void kd_knn(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
     SM_CUDA(cudaMemsetAsync(err, 0, sizeof(int), c.stream));
     kd_tree_positions(c, T, vaccActive, pos, tpos);
     k_kd_knn<<<nblocks(nqMax, 128), 128, 0, c.stream>>>(T.view(vaccActive, pos, nullptr, tpos), qpos,
-                                                        list, nq, k, nbr, dist, cnt, err, nrm, need);
+                                                        nq, k, nbr, dist, err);
+    SM_LAUNCH_CHECK();
+}
+
+void kd_knn_points(Ctx &c, const KdTree &T, const HGrid &g, const float4 *pos, const int *list,
+                   const int *nq, int nqMax, int k, int *nbr, int *cnt, const float4 *nrm,
+                   int *need) {
+    if (nqMax <= 0 || T.m <= 0)
+        return;
+    int *err = c.arena.get<int>("kd.knn.err", 1);
+    SM_CUDA(cudaMemsetAsync(err, 0, sizeof(int), c.stream));
+    k_kd_knn_grid<<<nblocks((long long)nqMax * 32, kKnnBs), kKnnBs, 0, c.stream>>>(
+        T.view(nullptr, pos), T.m, g.view(), T.treePos, list, nq, k, nbr, cnt, err, nrm, need);
     SM_LAUNCH_CHECK();
 }
 

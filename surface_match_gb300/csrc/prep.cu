@@ -1097,6 +1097,9 @@ static int *compact_grid_order(Ctx &c, const HGrid &H, const int *need, int eq, 
 
 void build_hgrid(Ctx &c, const float4 *pos, const int *ids, int m, const Box &box, float g,
                  HGrid &H, const std::string &tag, bool wIsRank) {
+    // (any cell side gives the same results: without a wanted one, some 1000 cells an axis)
+    if (!(g > 0.0f))
+        g = std::max(std::max(box.ext(0), box.ext(1)), std::max(box.ext(2), 1e-30f)) / 1024.0f;
     // cells per axis stay below 2^20 so that cell keys fit 60 bits (coarser cells if needed)
     while (smg::dim_of(box.ext(0), g) >= (1 << 20) || smg::dim_of(box.ext(1), g) >= (1 << 20) ||
            smg::dim_of(box.ext(2), g) >= (1 << 20))
@@ -1261,18 +1264,6 @@ int sample_points(Ctx &c, const float4 *pos, int npoints, const int *ids, int m,
     return c.hostCounts[0];
 }
 
-// The points p < n with need[p] == eq, ascending, into out; returns the device address of
-// their count (no host round trip).
-static int *compact_need(Ctx &c, const int *need, int n, int eq, int *out, const std::string &tag) {
-    int *total = c.arena.get<int>(tag + ".scantot", 1);
-    int *pre   = c.arena.get<int>(tag + ".pre", std::max(n, 1));
-    scan_into(c, need, pre, n, eq, total);
-    if (n > 0) {
-        launch_chained(c, k_scatter_flags, nblocks(n, 256), 256, 0, need, pre, n, eq, out);
-    }
-    return total;
-}
-
 void estimate_normals(Ctx &c, float4 *pos, float4 *nrm, int npoints, const int *ids, int m,
                       const HGrid &query, int k, bool smooth, bool invert, const float *vp,
                       const std::string &tag, const KdTree *tree) {
@@ -1288,29 +1279,25 @@ void estimate_normals(Ctx &c, float4 *pos, float4 *nrm, int npoints, const int *
     fill(c, clear);
     launch_chained(c, k_mark_todo, nblocks(m, 256), 256, 0, ids, m, nrm, need);
     // the query lists and their counts stay on the device; launches are sized by bounds
-    // with the reference's k-d tree the k nearest come from its depth-first search (ties:
-    // first found); the lists are then in index order (the results do not depend on it)
-    int       *todo   = c.arena.get<int>(tag + ".todo", std::max(tree ? npoints : m, 1));
-    const int *ntodo  = tree ? compact_need(c, need, npoints, 2, todo, tag + ".ct")
-                             : compact_grid_order(c, query, need, 2, todo, tag + ".ct");
+    int       *todo   = c.arena.get<int>(tag + ".todo", std::max(m, 1));
+    const int *ntodo  = compact_grid_order(c, query, need, 2, todo, tag + ".ct");
     int       *nbrT   = c.arena.get<int>(tag + ".nbrT", (size_t)m * k);
     int       *cntT   = c.arena.get<int>(tag + ".cntT", m);
     if (tree)
-        kd_knn(c, *tree, nullptr, pos, nullptr, todo, ntodo, m, k, nbrT, nullptr, cntT, nrm,
-               smooth ? need : nullptr);
+        kd_knn_points(c, *tree, query, pos, todo, ntodo, m, k, nbrT, cntT, nrm,
+                      smooth ? need : nullptr);
     else
         launch_knn(c, todo, ntodo, m, query.view(), pos, k, nbrT, cntT, smooth ? 1 : 0, nrm, need);
     const int  extraMax = smooth ? (int)std::min<long long>(npoints, (long long)m * k) : 0;
     int       *extra = nullptr, *nbrE = nullptr, *cntE = nullptr;
     const int *nextra = nullptr;
     if (extraMax > 0) {
-        extra  = c.arena.get<int>(tag + ".extra", std::max(tree ? npoints : extraMax, 1));
-        nextra = tree ? compact_need(c, need, npoints, 1, extra, tag + ".ce")
-                      : compact_grid_order(c, query, need, 1, extra, tag + ".ce");
+        extra  = c.arena.get<int>(tag + ".extra", std::max(extraMax, 1));
+        nextra = compact_grid_order(c, query, need, 1, extra, tag + ".ce");
         nbrE   = c.arena.get<int>(tag + ".nbrE", (size_t)extraMax * k);
         cntE   = c.arena.get<int>(tag + ".cntE", extraMax);
         if (tree)
-            kd_knn(c, *tree, nullptr, pos, nullptr, extra, nextra, extraMax, k, nbrE, nullptr, cntE);
+            kd_knn_points(c, *tree, query, pos, extra, nextra, extraMax, k, nbrE, cntE, nrm, nullptr);
         else
             launch_knn(c, extra, nextra, extraMax, query.view(), pos, k, nbrE, cntE, 0, nrm, need);
     }

@@ -355,6 +355,12 @@ __device__ __forceinline__ int band_end(int done, int ms, float b2, float g) {
     return hi;
 }
 
+// Whether a point's key may matter beside the current k-th: smaller, or (TIES) at its distance.
+template <bool TIES>
+__device__ __forceinline__ bool knn_enters(unsigned long long key, unsigned long long kth) {
+    return key < kth || (TIES && key != ~0ull && (unsigned)(key >> 32) == (unsigned)(kth >> 32));
+}
+
 // k nearest by a scan of every point of g, for a query whose shell walk gave up (a point
 // far from the others would walk shells up to the grid's extent). The scan starts over
 // (best and seen reset: each point is visited once, so the result is the same exact k
@@ -362,6 +368,7 @@ __device__ __forceinline__ int band_end(int done, int ms, float b2, float g) {
 // it saw k points, else the k-th of a strided sample of the points; a merge runs only for a
 // round with a point below the current k-th. It runs for few queries and is kept lean (two
 // loads in flight per lane) so that the walk's register count stays as it is.
+template <bool TIES>
 static __device__ __noinline__ void knn_scan_all(const HGridView &g, float qx, float qy, float qz, int k,
                                           unsigned long long &best, int &seen) {
     const int lane  = threadIdx.x & 31;
@@ -399,7 +406,7 @@ static __device__ __noinline__ void knn_scan_all(const HGridView &g, float qx, f
             if ((unsigned)(key >> 32) > bound)
                 key = ~0ull;
             seen += __popc(__ballot_sync(0xffffffffu, r < g.m));
-            if (__any_sync(0xffffffffu, key < __shfl_sync(0xffffffffu, best, k - 1)))
+            if (__any_sync(0xffffffffu, knn_enters<TIES>(key, __shfl_sync(0xffffffffu, best, k - 1))))
                 best = warp_merge_low(best, warp_bitonic_sort(key));
         }
     }
@@ -414,7 +421,9 @@ static __device__ __noinline__ void knn_scan_all(const HGridView &g, float qx, f
 // after shell s once k points were seen and the k-th distance is below the ring bound of s
 // (every unvisited point is farther); further shells are walked one by one. Returns the
 // number found (<= k); lane j < that count gets the j-th neighbour's index in *id and
-// squared distance in *d.
+// squared distance in *d. With TIES points at the k-th distance are never skipped: for k < 32
+// lane k holds one more of them (index >= 0, the same distance) if there is one.
+template <bool TIES = false>
 __device__ __forceinline__ int warp_knn_sorted(const HGridView &g, float qx, float qy, float qz,
                                                int k, int *id, float *d) {
     const int          lane = threadIdx.x & 31;
@@ -428,7 +437,7 @@ __device__ __forceinline__ int warp_knn_sorted(const HGridView &g, float qx, flo
             const float dd = smm::dist2(qx, qy, qz, p.x, p.y, p.z);
             key = ((unsigned long long)__float_as_uint(dd) << 32) | (unsigned)__float_as_int(p.w);
         }
-        if (__any_sync(0xffffffffu, key < kth()))
+        if (__any_sync(0xffffffffu, knn_enters<TIES>(key, kth())))
             best = warp_merge_low(best, warp_bitonic_sort(key));
     };
     int c[3];
@@ -482,7 +491,7 @@ __device__ __forceinline__ int warp_knn_sorted(const HGridView &g, float qx, flo
         return __uint_as_float((unsigned)(kth() >> 32)) < bnd * bnd;
     };
     if (!done(1) && ms >= 2 && !warp_walk(g, qx, qy, qz, visit, done, 2, kKnnMaxShell))
-        knn_scan_all(g, qx, qy, qz, k, best, seen);
+        knn_scan_all<TIES>(g, qx, qy, qz, k, best, seen);
     const int n = min(seen, k);
     *id         = (int)(unsigned)(best & 0xffffffffu);
     *d          = __uint_as_float((unsigned)(best >> 32));

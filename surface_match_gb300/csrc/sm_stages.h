@@ -260,8 +260,8 @@ int sample_points(Ctx &c, const float4 *pos, int npoints, const int *ids, int m,
 struct KdTree;
 // Two-phase normal estimation of ids[0..m) (estimateNormal, util.cpp:234-334; all
 // neighbourhoods from the positions at the start of the call, then smoothing). The k
-// nearest come from the grid `query`, or, when `tree` is given, from the reference's k-d
-// tree (over all points, searched on the live positions `pos`).
+// nearest come from the grid `query` of the searched points; when `tree` is given they are
+// those of the reference's k-d tree over these points, in its order.
 void estimate_normals(Ctx &c, float4 *pos, float4 *nrm, int npoints, const int *ids, int m,
                       const HGrid &query, int k, bool smooth, bool invert, const float *vp,
                       const std::string &tag, const KdTree *tree = nullptr);
@@ -309,13 +309,16 @@ void build_kdtree(Ctx &c, const float4 *pos, int npoints, const int *ids, int m,
 // are clamped into its border cells).
 int kd_sample(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos, float step,
               const Box &box, int *outIds, int *ioi, const std::string &tag);
-// KNNResultSet searches (nanoflann findNeighbors) on the tree, one per query: query t is at
-// qpos[t] (or pos[list[t]] when qpos is null) for t < *nq (a device count, nqMax bounds the
-// launch); nbr[t*k + j] / dist[t*k + j] (dist nullable) its j-th nearest, cnt[t] (nullable)
-// how many there are.
+// KNNResultSet searches (nanoflann findNeighbors) on the tree, one per query: query t at
+// qpos[t] for t < *nq (a device count, nqMax bounds the launch); nbr[t*k + j] / dist[t*k + j]
+// its j-th nearest.
 void kd_knn(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
-            const float4 *qpos, const int *list, const int *nq, int nqMax, int k, int *nbr,
-            float *dist, int *cnt, const float4 *nrm = nullptr, int *need = nullptr);
+            const float4 *qpos, const int *nq, int nqMax, int k, int *nbr, float *dist);
+// The same for the points list[t] of the whole tree, given a grid of its points at their live
+// positions `pos`; need (nullable): neighbours without a finite normal are marked 1 where 0.
+void kd_knn_points(Ctx &c, const KdTree &T, const HGrid &g, const float4 *pos, const int *list,
+                   const int *nq, int nqMax, int k, int *nbr, int *cnt, const float4 *nrm,
+                   int *need);
 // flags[v] = 1 when node v's subtree holds a position whose vaccActive entry is >= 0
 // (the searches of a reduce()d tree skip the others).
 void kd_mark_nonempty(Ctx &c, const KdTree &T, const int *vaccActive, int *flags);
@@ -384,11 +387,12 @@ struct IcpScene {
     const float4 *pos, *nrm;
     HGrid         sampled, resampled, full; // the subset grids carry subset ranks in pts.w
     const float4 *posS, *nrmS, *posR, *nrmR; // the sampled / resampled subsets, rank order
-    // reference search order (tree != nullptr): searches in the k-d tree, reduced to the
+    // reference search order (tree != nullptr): the searches of the k-d tree, reduced to the
     // sampled (ioiS) or resampled (ioiR) points, whose ids map to subset ranks by rankS /
-    // rankR; the grids are then unused (only their point counts m are read)
+    // rankR and whose ranks map to tree positions by tposS / tposR
     const KdTree *tree = nullptr;
     const int    *ioiS = nullptr, *ioiR = nullptr, *rankS = nullptr, *rankR = nullptr;
+    const int    *tposS = nullptr, *tposR = nullptr;
     const int    *neS = nullptr, *neR = nullptr;                  // non-empty node flags
     const float4 *tpS = nullptr, *tpR = nullptr, *tpF = nullptr; // leaf records
     const float  *exc = nullptr; // largest excursion from the leaf boxes: S, R, all points

@@ -541,29 +541,41 @@ __global__ void k_kd_finish(int4 *__restrict__ nd, const int *__restrict__ paren
 }
 
 // ---- greedy sampling in tree order ---------------------------------------------------
-constexpr uint32_t  kNoCell   = 1u << 23; // sort key of positions reduce() excluded
+// A point is kept once every earlier point (tree order) within the step is decided and none of
+// the kept ones dropped it; a kept point drops the later points its search reaches. So only
+// kept points search their neighbourhood, and what is left is the dependency chain. Points sit
+// in cells of about the step, in tree order within a cell; only a cell's first open point can
+// be the next decided. A cell is a work item: the warp that holds it looks for a blocker of
+// its first open point - an open earlier point within the step - and either files the cell
+// under the blocker (the blocker's decision queues it again) or keeps the point, drops what it
+// reaches, queues the cells filed under any of these, and goes on with the next point. A cell
+// is in one place at a time: queued, held, or filed. The earliest open point of all has no
+// blocker, so there is always a cell to go on with, and a warp waits for queue slots only.
+// (Handling every point through the queue, with a neighbourhood pass per point to count its
+// earlier neighbours and one when it was decided, took 7.8 + 7.3 ms for the large scene's
+// 0.92 M points at steps 4.3 and 1.4 mm, where 7,000 and 56,000 are kept.)
 constexpr int       kSpBs     = 256;
 constexpr long long kSpIdle   = 1ll << 22; // polls of an unwritten queue slot before giving up
 constexpr int       kSpUnroll = 4;         // neighbourhood entries in flight per lane
+constexpr int       kSpCtas   = 4;         // CTAs per SM: the warps that hold cells at once
+constexpr long long kSpCells  = 1ll << 25; // most cells of the dense table (128 MB)
 
 struct SampleArgs {
     KdView          t;
-    float           org[3], g;
     int             dim[3];
     const float4   *ent;      // cell runs: {x, y, z, tree position bits}, tree order in a run
     const float    *ex;       // the entries' excursions from their leaves' build-time boxes
-    const int      *cellOf;   // per entry: its cell's occupied rank (-1 past the active ones)
     const int      *cellRank; // dense cell -> occupied rank (-1: empty)
     const int      *cellList; // occupied rank -> dense cell
-    const int      *cellBeg;  // occupied rank -> its run [beg, end) of the entries
-    const int      *cellEnd;
-    int            *open;     // occupied rank -> its points not yet decided
-    int            *cnt;      // per entry: earlier points within the step not yet decided
+    const int      *cellEnd;  // occupied rank -> end of its run of the entries
+    int            *cur;      // occupied rank -> no entry of its run before this one is open
     int            *dec;      // per entry: 0 open, 1 kept, 2 dropped
-    int            *queue;    // entries in the order they were decided (-1: not written)
+    int            *filed;    // per entry: first cell filed under it (-1: none)
+    int            *nextCell; // per occupied rank: the next cell filed under the same entry
+    int            *ring;     // queue of cells (-1: slot not written)
+    unsigned        ringMask;
     int            *head, *tail;
-    const int      *nact;     // number of entries of active points (device)
-    int             m;
+    int            *open;     // cells with points not yet decided
     float           r2;
     double          safe2;
     int            *keptFlag; // per tree position
@@ -602,13 +614,15 @@ __device__ __forceinline__ bool reaches(const SampleArgs &a, const float4 &q, co
     return smk::kd_reaches(a.t, qq, ip, a.r2, &key);
 }
 
+// The cell of each tree position (noCell where reduce() excluded it).
 __global__ void k_sp_keys(const int *__restrict__ vaccA, const float4 *__restrict__ pos, int m,
-                          GridParamsK gp, uint32_t *__restrict__ key, uint32_t *__restrict__ val) {
+                          GridParamsK gp, uint32_t noCell, uint32_t *__restrict__ key,
+                          uint32_t *__restrict__ val) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m)
         return;
     const int id = vaccA[i];
-    uint32_t  k  = kNoCell;
+    uint32_t  k  = noCell;
     if (id >= 0) {
         const float4 p  = pos[id];
         const int    cx = smg::coord(p.x, gp.org[0], gp.g, gp.dim[0]);
@@ -620,63 +634,55 @@ __global__ void k_sp_keys(const int *__restrict__ vaccA, const float4 *__restric
     val[i] = (uint32_t)i;
 }
 
-__global__ void k_sp_heads(const uint32_t *__restrict__ key, int m, int *__restrict__ head) {
+__global__ void k_sp_heads(const uint32_t *__restrict__ key, int m, uint32_t noCell,
+                           int *__restrict__ head) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k > m)
         return;
-    head[k] = (k < m && key[k] != kNoCell && (k == 0 || key[k - 1] != key[k])) ? 1 : 0;
+    head[k] = (k < m && key[k] != noCell && (k == 0 || key[k - 1] != key[k])) ? 1 : 0;
 }
 
-__global__ void k_sp_cells(const uint32_t *__restrict__ key, int m, const int *__restrict__ head,
-                           const int *__restrict__ rank, int *__restrict__ cellRank,
-                           int *__restrict__ cellList, int *__restrict__ cellBeg,
-                           int *__restrict__ cellEnd, int *__restrict__ cellOf,
-                           int *__restrict__ open, int *__restrict__ nact) {
+// The cells' runs (every occupied cell queued, in run order), and the runs' points in run
+// order: {x, y, z, tree position bits}, with the point's excursion from its leaf's build-time
+// box.
+__global__ void k_sp_cells(const uint32_t *__restrict__ key, const uint32_t *__restrict__ sortPos,
+                           int m, uint32_t noCell, const int *__restrict__ head,
+                           const int *__restrict__ rank, const float *__restrict__ nodeBox,
+                           const int *__restrict__ leafOf, int *__restrict__ cellRank,
+                           int *__restrict__ cellList, int *__restrict__ cellEnd,
+                           float4 *__restrict__ ent, float *__restrict__ ex, SampleArgs a) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= m)
+    if (k >= m || key[k] == noCell)
         return;
-    if (key[k] == kNoCell) {
-        cellOf[k] = -1;
-        return;
-    }
     const int r = rank[k] + head[k] - 1; // the run's occupied rank
-    cellOf[k]   = r;
-    atomicAdd(&open[r], 1);
     if (head[k]) {
         cellRank[key[k]] = r;
         cellList[r]      = (int)key[k];
-        cellBeg[r]       = k;
+        a.cur[r]         = k;
+        a.ring[r]        = r;
     }
     if (k == m - 1 || key[k + 1] != key[k])
         cellEnd[r] = k + 1;
-    if (k == m - 1 || key[k + 1] == kNoCell)
-        *nact = k + 1; // the active entries sort first
+    if (k == m - 1 || key[k + 1] == noCell) { // (the active entries sort first)
+        *a.tail = r + 1;
+        *a.open = r + 1;
+    }
+    const int    ip = (int)sortPos[k];
+    const float4 p  = a.t.pos[a.t.vacc[ip]];
+    ent[k]          = make_float4(p.x, p.y, p.z, __int_as_float(ip));
+    ex[k]           = (float)excursion(nodeBox + 6 * (size_t)leafOf[ip], p);
+    a.dec[k]        = 0;
+    a.filed[k]      = -1;
 }
 
-// The cell runs' points in run order: {x, y, z, tree position bits} and the point's
-// excursion from its leaf's build-time box.
-__global__ void k_sp_entries(const uint32_t *__restrict__ sortPos, int m, KdView t,
-                             const float *__restrict__ nodeBox, const int *__restrict__ leafOf,
-                             float4 *__restrict__ ent, float *__restrict__ ex) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= m)
-        return;
-    const int ip = (int)sortPos[k];
-    const int id = t.vacc[ip];
-    if (id < 0)
-        return;
-    const float4 p = t.pos[id];
-    ent[k]         = make_float4(p.x, p.y, p.z, __int_as_float(ip));
-    ex[k]          = (float)excursion(nodeBox + 6 * (size_t)leafOf[ip], p);
-}
-
-// The 27 cells around a cell: lane l < 27 gets the first entry of neighbour l's run; returns
-// the lane's exclusive prefix of the runs' lengths and writes their total to tot.
-// With onlyOpen, cells whose points are all decided count as empty: a decided point needs
-// nothing from its neighbours any more.
-__device__ __forceinline__ int nb_runs(const SampleArgs &a, int cid, int &nb, int &tot,
-                                       bool onlyOpen) {
+// The 27 cells around cell r: lane l < 27 gets the first open entry (or one before it) of
+// neighbour l's run, own cell from entry `own`; returns the lane's exclusive prefix of the
+// runs' lengths and writes their total to tot. With before >= 0, runs whose first open
+// point's tree position is above it count as empty.
+__device__ __forceinline__ int nb_runs(const SampleArgs &a, int r, int own, int before, int &nb,
+                                       int &tot) {
     const int lane = threadIdx.x & 31;
+    const int cid  = a.cellList[r];
     const int cx = cid % a.dim[0], cy = (cid / a.dim[0]) % a.dim[1], cz = cid / (a.dim[0] * a.dim[1]);
     nb      = 0;
     int len = 0;
@@ -684,9 +690,11 @@ __device__ __forceinline__ int nb_runs(const SampleArgs &a, int cid, int &nb, in
         const int x = cx + lane % 3 - 1, y = cy + (lane / 3) % 3 - 1, z = cz + lane / 9 - 1;
         if (x >= 0 && y >= 0 && z >= 0 && x < a.dim[0] && y < a.dim[1] && z < a.dim[2]) {
             const int nr = a.cellRank[(z * a.dim[1] + y) * a.dim[0] + x];
-            if (nr >= 0 && !(onlyOpen && ld_vol(&a.open[nr]) == 0)) {
-                nb  = a.cellBeg[nr];
+            if (nr >= 0) {
+                nb  = nr == r ? own : ld_vol(&a.cur[nr]);
                 len = a.cellEnd[nr] - nb;
+                if (len > 0 && before >= 0 && __float_as_int(a.ent[nb].w) > before)
+                    len = 0;
             }
         }
     }
@@ -708,141 +716,188 @@ __device__ __forceinline__ int nb_entry(int t, int excl, int nb) {
     return __shfl_sync(0xffffffffu, nb, lo) + (t - __shfl_sync(0xffffffffu, excl, lo));
 }
 
-// Step 1, a warp per point p: the earlier points (lower tree position) within the step of
-// p - squared distance from that point to p below step^2, the first test of its radius
-// search. p's decision waits for theirs. Points without any are kept at once and queued.
-__global__ void __launch_bounds__(kSpBs) k_sp_count(SampleArgs a) {
-    const int lane = threadIdx.x & 31;
-    const int nw   = (int)(((long long)gridDim.x * blockDim.x) >> 5);
-    for (int k = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5); k < a.m; k += nw) {
-        if (a.cellOf[k] < 0)
-            break; // past the active entries
-        const float4 p  = a.ent[k];
-        const int    ip = __float_as_int(p.w);
-        int          nb, tot;
-        const int    excl = nb_runs(a, a.cellList[a.cellOf[k]], nb, tot, false);
-        int          cnt  = 0;
-        for (int base = 0; base < tot; base += 32 * kSpUnroll) {
-            int    kb[kSpUnroll];
-            float4 b[kSpUnroll];
-#pragma unroll
-            for (int u = 0; u < kSpUnroll; u++)
-                kb[u] = nb_entry(min(base + u * 32 + lane, tot - 1), excl, nb);
-#pragma unroll
-            for (int u = 0; u < kSpUnroll; u++)
-                b[u] = a.ent[max(kb[u], 0)];
-#pragma unroll
-            for (int u = 0; u < kSpUnroll; u++)
-                if (base + u * 32 + lane < tot && __float_as_int(b[u].w) < ip) {
-                    const float bq[3] = {b[u].x, b[u].y, b[u].z};
-                    cnt += smk::eval_metric(bq, p) < a.r2 ? 1 : 0;
-                }
+// (store; fence; load of the other's word) on both sides of a filing: whichever of the filing
+// warp and the deciding one comes second sees the other
+__device__ __forceinline__ void fence_sc() { asm volatile("fence.sc.gpu;" ::: "memory"); }
+
+// Queues the cells filed under entry j. A slot is written once its last reader has emptied it:
+// at most every cell is queued, and the ring holds twice as many.
+__device__ __forceinline__ void sp_wake(const SampleArgs &a, int j) {
+    int c = atomicExch(&a.filed[j], -1);
+    if (c < 0)
+        return;
+    __threadfence();
+    while (c >= 0) {
+        const int nx = ld_vol(&a.nextCell[c]); // (its holder may file it anew once it is queued)
+        int      *s  = &a.ring[(unsigned)atomicAdd(a.tail, 1) & a.ringMask];
+        for (long long it = 0; atomicCAS(s, -1, c) != -1; it++)
+            if (it > kSpIdle) {
+                atomicExch(a.err, 1);
+                return;
+            }
+        c = nx;
+    }
+}
+
+// The next queued cell, by lane 0: -1 when every point is decided (or a wait expired).
+__device__ __forceinline__ int sp_take(const SampleArgs &a) {
+    int *s = &a.ring[(unsigned)atomicAdd(a.head, 1) & a.ringMask];
+    for (long long it = 0;; it++) {
+        if (ld_vol(s) >= 0) {
+            const int c = atomicExch(s, -1);
+            if (c >= 0)
+                return c;
         }
-        cnt = __reduce_add_sync(0xffffffffu, cnt);
-        if (lane == 0) {
-            a.cnt[k] = cnt;
-            if (cnt == 0) {
-                a.dec[k]                      = 1;
-                a.queue[atomicAdd(a.tail, 1)] = k;
-                atomicSub(&a.open[a.cellOf[k]], 1);
+        if (ld_vol(a.open) <= 0 || ld_vol(a.err))
+            return -1;
+        if (it > kSpIdle) {
+            atomicExch(a.err, 1);
+            return -1;
+        }
+        __nanosleep(64);
+    }
+}
+
+// An open entry with tree position below ip within the step of p: -1 when there is none.
+__device__ __forceinline__ int sp_blocker(const SampleArgs &a, int r, int k, const float4 &p,
+                                          int ip) {
+    const int lane = threadIdx.x & 31;
+    int       nb, tot;
+    const int excl = nb_runs(a, r, k, ip - 1, nb, tot);
+    for (int base = 0; base < tot; base += 32 * kSpUnroll) {
+        int    kb[kSpUnroll], dec[kSpUnroll];
+        float4 b[kSpUnroll];
+#pragma unroll
+        for (int u = 0; u < kSpUnroll; u++)
+            kb[u] = nb_entry(min(base + u * 32 + lane, tot - 1), excl, nb);
+#pragma unroll
+        for (int u = 0; u < kSpUnroll; u++) {
+            b[u]   = a.ent[kb[u]];
+            dec[u] = ld_vol(&a.dec[kb[u]]);
+        }
+        int last = -1; // the lane's latest blocker: it waits longest, so it is the one to wait for
+        int at   = -1;
+#pragma unroll
+        for (int u = 0; u < kSpUnroll; u++) {
+            const int   ib    = __float_as_int(b[u].w);
+            const float bq[3] = {b[u].x, b[u].y, b[u].z};
+            if (base + u * 32 + lane < tot && dec[u] == 0 && ib < ip && ib > last &&
+                smk::eval_metric(bq, p) < a.r2) {
+                last = ib;
+                at   = kb[u];
             }
         }
+        const int w = __reduce_max_sync(0xffffffffu, last);
+        if (w >= 0)
+            return __shfl_sync(0xffffffffu, at, __ffs(__ballot_sync(0xffffffffu, last == w)) - 1);
+    }
+    return -1;
+}
+
+// Drops the open later points that the search of kept point q (entry k of cell r) reaches.
+__device__ __forceinline__ void sp_drop(const SampleArgs &a, int r, int k, const float4 &q, int iq) {
+    const int   lane  = threadIdx.x & 31;
+    const float qq[3] = {q.x, q.y, q.z};
+    int         nb, tot;
+    const int   excl = nb_runs(a, r, k + 1, -1, nb, tot);
+    for (int base = 0; base < tot; base += 32 * kSpUnroll) {
+        int    kp[kSpUnroll], dec[kSpUnroll];
+        float4 p[kSpUnroll];
+#pragma unroll
+        for (int u = 0; u < kSpUnroll; u++)
+            kp[u] = nb_entry(min(base + u * 32 + lane, tot - 1), excl, nb);
+#pragma unroll
+        for (int u = 0; u < kSpUnroll; u++) {
+            p[u]   = a.ent[kp[u]];
+            dec[u] = ld_vol(&a.dec[kp[u]]);
+        }
+        bool gone[kSpUnroll], any = false;
+#pragma unroll
+        for (int u = 0; u < kSpUnroll; u++) {
+            gone[u] = base + u * 32 + lane < tot && dec[u] == 0 && __float_as_int(p[u].w) > iq &&
+                      smk::eval_metric(qq, p[u]) < a.r2 &&
+                      reaches(a, q, p[u], __float_as_int(p[u].w), (double)a.ex[kp[u]]);
+            if (gone[u]) {
+                *(volatile int *)&a.dec[kp[u]] = 2;
+                any                            = true;
+            }
+        }
+        if (!any)
+            continue;
+        fence_sc();
+#pragma unroll
+        for (int u = 0; u < kSpUnroll; u++)
+            if (gone[u] && ld_vol(&a.filed[kp[u]]) >= 0)
+                sp_wake(a, kp[u]);
     }
 }
 
-// Decide entry p (open -> fate) and queue it, unless it is decided already.
-__device__ __forceinline__ void sp_push(const SampleArgs &a, int p, int fate) {
-    if (atomicCAS(&a.dec[p], 0, fate) == 0) {
-        atomicSub(&a.open[a.cellOf[p]], 1);
-        const int slot = atomicAdd(a.tail, 1);
-        __threadfence();
-        atomicExch(&a.queue[slot], p);
-    }
-}
-
-// Step 2, a warp per queued point b, in queue order (every active point is queued exactly
-// once). A kept b drops every later point its search reaches (and queues it); every other
-// later point within the step that is still open counts b as decided, and the last of its
-// earlier points to be decided queues it as kept. Dropping happens before counting, so a
-// point that a kept point reaches never runs out of count. Each queued point waits only on
-// points queued before it, so the warps that took the earliest slots always progress.
 __global__ void __launch_bounds__(kSpBs) k_sp_run(SampleArgs a) {
     const int lane = threadIdx.x & 31;
     for (;;) {
-        int slot = 0;
-        if (lane == 0)
-            slot = atomicAdd(a.head, 1);
-        slot = __shfl_sync(0xffffffffu, slot, 0);
-        if (slot >= *a.nact)
+        const int r = __shfl_sync(0xffffffffu, lane == 0 ? sp_take(a) : 0, 0);
+        if (r < 0)
             return;
-        int b = -1;
-        if (lane == 0) {
-            for (long long it = 0;; it++) {
-                b = ld_vol(&a.queue[slot]);
-                if (b >= 0)
+        __threadfence(); // the decisions before the cell was queued are visible
+        int       k = ld_vol(&a.cur[r]);
+        const int e = a.cellEnd[r];
+        for (;;) {
+            // the cell's first open entry
+            unsigned open = 0u;
+            for (; k < e; k += 32) {
+                open = __ballot_sync(0xffffffffu, k + lane < e && ld_vol(&a.dec[k + lane]) == 0);
+                if (open)
                     break;
-                if (ld_vol(a.err) || it > kSpIdle) {
-                    atomicExch(a.err, 1);
-                    break;
-                }
-                __nanosleep(32);
             }
-        }
-        b = __shfl_sync(0xffffffffu, b, 0);
-        if (b < 0)
-            return;
-        __threadfence();
-        const int    fate = ld_vol(&a.dec[b]);
-        const float4 q    = a.ent[b];
-        const int    iq   = __float_as_int(q.w);
-        if (fate == 1 && lane == 0)
-            a.keptFlag[iq] = 1;
-        int         nb, tot;
-        // only neighbour cells that still hold an undecided point: after a kept point's
-        // wave of drops most cells around a dropped point are settled
-        const int   excl  = nb_runs(a, a.cellList[a.cellOf[b]], nb, tot, true);
-        const float qq[3] = {q.x, q.y, q.z};
-        for (int base = 0; base < tot; base += 32 * kSpUnroll) {
-            int    kp[kSpUnroll];
-            float4 p[kSpUnroll];
-#pragma unroll
-            for (int u = 0; u < kSpUnroll; u++)
-                kp[u] = nb_entry(min(base + u * 32 + lane, tot - 1), excl, nb);
-#pragma unroll
-            for (int u = 0; u < kSpUnroll; u++)
-                p[u] = a.ent[max(kp[u], 0)];
-            // the later points within the step that are still open
-            bool live[kSpUnroll];
-#pragma unroll
-            for (int u = 0; u < kSpUnroll; u++)
-                live[u] = base + u * 32 + lane < tot && __float_as_int(p[u].w) > iq &&
-                          smk::eval_metric(qq, p[u]) < a.r2;
-#pragma unroll
-            for (int u = 0; u < kSpUnroll; u++)
-                live[u] = live[u] && ld_vol(&a.dec[kp[u]]) == 0;
-            bool count[kSpUnroll];
-#pragma unroll
-            for (int u = 0; u < kSpUnroll; u++) {
-                count[u] = false;
-                if (!live[u])
-                    continue;
-                if (fate == 1 && reaches(a, q, p[u], __float_as_int(p[u].w), (double)a.ex[kp[u]])) {
-                    sp_push(a, kp[u], 2);
-                    continue;
+            if (!open) {
+                if (lane == 0) {
+                    *(volatile int *)&a.cur[r] = e;
+                    atomicSub(a.open, 1);
                 }
-                count[u] = true;
+                break;
             }
+            k += __ffs(open) - 1;
+            if (lane == 0)
+                *(volatile int *)&a.cur[r] = k;
+            const float4 p  = a.ent[k];
+            const int    ip = __float_as_int(p.w);
+            const int    j  = sp_blocker(a, r, k, p, ip);
+            if (j >= 0) {
+                if (lane == 0) {
+                    // file the cell under j, unless j was decided meanwhile: then whoever takes
+                    // j's list (this warp or the one that decided j) queues it
+                    int old = ld_vol(&a.filed[j]);
+                    for (;;) {
+                        *(volatile int *)&a.nextCell[r] = old;
+                        __threadfence();
+                        const int seen = atomicCAS(&a.filed[j], old, r);
+                        if (seen == old)
+                            break;
+                        old = seen;
+                    }
+                    fence_sc();
+                    if (ld_vol(&a.dec[j]) != 0)
+                        sp_wake(a, j);
+                }
+                __syncwarp();
+                break;
+            }
+            // no open earlier point within the step. A kept point drops before it counts as
+            // decided, so p's own state is final now
             __threadfence();
-            int old[kSpUnroll];
-#pragma unroll
-            for (int u = 0; u < kSpUnroll; u++)
-                old[u] = count[u] ? atomicSub(&a.cnt[kp[u]], 1) : 0;
-#pragma unroll
-            for (int u = 0; u < kSpUnroll; u++)
-                if (old[u] == 1) {
-                    __threadfence();
-                    sp_push(a, kp[u], 1);
-                }
+            if (__shfl_sync(0xffffffffu, lane == 0 ? ld_vol(&a.dec[k]) : 0, 0) != 0)
+                continue; // dropped meanwhile: on to the cell's next open entry
+            sp_drop(a, r, k, p, ip);
+            __threadfence();
+            __syncwarp();
+            if (lane == 0) {
+                a.keptFlag[ip]               = 1;
+                *(volatile int *)&a.dec[k]   = 1;
+                fence_sc();
+                if (ld_vol(&a.filed[k]) >= 0)
+                    sp_wake(a, k);
+            }
+            __syncwarp();
         }
     }
 }
@@ -1200,83 +1255,70 @@ int kd_sample(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
     const int *vaccA = vaccActive ? vaccActive : T.vacc;
     float      ext[3] = {box.ext(0), box.ext(1), box.ext(2)};
     GridParamsK gp;
-    gp.g = smg::sample_cell(step, ext);
+    // cells just above the step, coarser where a dense table would not fit
+    gp.g = smg::sample_cell(step, ext, kSpCells);
     for (int a = 0; a < 3; a++) {
         gp.org[a] = box.mn[a];
         gp.dim[a] = smg::dim_of(ext[a], gp.g);
     }
-    const long long nc = (long long)gp.dim[0] * gp.dim[1] * gp.dim[2];
+    const long long nc     = (long long)gp.dim[0] * gp.dim[1] * gp.dim[2];
+    const uint32_t  noCell = (uint32_t)nc;
+    int             bits   = 1;
+    while ((nc >> bits) != 0)
+        bits++;
+    unsigned ring = 1024;
+    while (ring < 2u * (unsigned)m)
+        ring <<= 1;
     uint32_t *key   = c.arena.get<uint32_t>(tag + ".key", m);
     uint32_t *val   = c.arena.get<uint32_t>(tag + ".val", m);
     int      *head  = c.arena.get<int>(tag + ".head", (size_t)m + 1);
     int      *rank  = c.arena.get<int>(tag + ".rank", (size_t)m + 1);
     int      *cRank = c.arena.get<int>(tag + ".crank", nc);
-    k_sp_keys<<<nblocks(m, 256), 256, 0, c.stream>>>(vaccA, pos, m, gp, key, val);
-    SM_LAUNCH_CHECK();
-    radix_sort_pairs(c, key, val, m, 24, tag);
-    k_sp_heads<<<nblocks((long long)m + 1, 256), 256, 0, c.stream>>>(key, m, head);
-    SM_LAUNCH_CHECK();
-    const int ncells = scan_excl(c, head, rank, (long long)m + 1, tag + ".hs", true);
-    int    *cellList = c.arena.get<int>(tag + ".clist", std::max(ncells, 1));
-    int    *cellBeg  = c.arena.get<int>(tag + ".cbeg", std::max(ncells, 1));
-    int    *cellEnd  = c.arena.get<int>(tag + ".cend", std::max(ncells, 1));
-    int    *cellOf   = c.arena.get<int>(tag + ".cof", m);
-    float4 *ent      = c.arena.get<float4>(tag + ".ent", m);
-    float  *ex       = c.arena.get<float>(tag + ".ex", m);
-    int    *cnt      = c.arena.get<int>(tag + ".cnt", m);
-    int    *open     = c.arena.get<int>(tag + ".open", std::max(ncells, 1));
-    int    *dec      = c.arena.get<int>(tag + ".dec", m);
-    int    *queue    = c.arena.get<int>(tag + ".q", m);
-    int    *flag     = c.arena.get<int>(tag + ".flag", (size_t)m + 1);
-    int    *ctl      = c.arena.get<int>(tag + ".ctl", 4); // head, tail, active entries, error
-    SM_CUDA(cudaMemsetAsync(cRank, 0xff, (size_t)nc * 4, c.stream));
-    SM_CUDA(cudaMemsetAsync(flag, 0, ((size_t)m + 1) * 4, c.stream));
-    SM_CUDA(cudaMemsetAsync(ctl, 0, 4 * sizeof(int), c.stream));
-    SM_CUDA(cudaMemsetAsync(dec, 0, (size_t)m * 4, c.stream));
-    SM_CUDA(cudaMemsetAsync(open, 0, (size_t)std::max(ncells, 1) * 4, c.stream));
-    SM_CUDA(cudaMemsetAsync(queue, 0xff, (size_t)m * 4, c.stream));
-    k_sp_cells<<<nblocks(m, 256), 256, 0, c.stream>>>(key, m, head, rank, cRank, cellList, cellBeg,
-                                                     cellEnd, cellOf, open, ctl + 2);
-    SM_LAUNCH_CHECK();
-    k_sp_entries<<<nblocks(m, 256), 256, 0, c.stream>>>(val, m, T.view(vaccA, pos), T.box,
-                                                        T.leafOf, ent, ex);
-    SM_LAUNCH_CHECK();
+    int      *cList = c.arena.get<int>(tag + ".clist", m); // at most a cell per point
+    int      *cEnd  = c.arena.get<int>(tag + ".cend", m);
+    float4   *ent   = c.arena.get<float4>(tag + ".ent", m);
+    float    *ex    = c.arena.get<float>(tag + ".ex", m);
+    int      *flag  = c.arena.get<int>(tag + ".flag", (size_t)m + 1);
+    int      *ctl   = c.arena.get<int>(tag + ".ctl", 4); // head, tail, open cells, error
     SampleArgs a{};
     a.t = T.view(vaccA, pos);
-    for (int d = 0; d < 3; d++) {
-        a.org[d] = gp.org[d];
+    for (int d = 0; d < 3; d++)
         a.dim[d] = gp.dim[d];
-    }
-    a.g        = gp.g;
     a.ent      = ent;
     a.ex       = ex;
-    a.cellOf   = cellOf;
     a.cellRank = cRank;
-    a.cellList = cellList;
-    a.cellBeg  = cellBeg;
-    a.cellEnd  = cellEnd;
-    a.cnt      = cnt;
-    a.open     = open;
-    a.dec      = dec;
-    a.queue    = queue;
+    a.cellList = cList;
+    a.cellEnd  = cEnd;
+    a.cur      = c.arena.get<int>(tag + ".cur", m);
+    a.dec      = c.arena.get<int>(tag + ".dec", m);
+    a.filed    = c.arena.get<int>(tag + ".filed", m);
+    a.nextCell = c.arena.get<int>(tag + ".next", m);
+    a.ring     = c.arena.get<int>(tag + ".ring", ring);
+    a.ringMask = ring - 1;
     a.head     = ctl;
     a.tail     = ctl + 1;
-    a.nact     = ctl + 2;
-    a.m        = m;
+    a.open     = ctl + 2;
     a.r2       = step * step;
     a.safe2    = (double)a.r2 * (1.0 - 1e-4);
     a.keptFlag = flag;
     a.err      = ctl + 3;
-    if (ncells > 0) {
-        int nsm = 0;
-        SM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device));
-        const int wpb = kSpBs / 32;
-        k_sp_count<<<std::min(nblocks(m, wpb), nsm * 16), kSpBs, 0, c.stream>>>(a);
-        SM_LAUNCH_CHECK();
-        // the queue's consumers: each queued point is taken by one warp, in queue order
-        k_sp_run<<<std::min(nblocks(m, wpb), nsm * 4), kSpBs, 0, c.stream>>>(a);
-        SM_LAUNCH_CHECK();
-    }
+    k_sp_keys<<<nblocks(m, 256), 256, 0, c.stream>>>(vaccA, pos, m, gp, noCell, key, val);
+    SM_LAUNCH_CHECK();
+    radix_sort_pairs(c, key, val, m, bits, tag);
+    k_sp_heads<<<nblocks((long long)m + 1, 256), 256, 0, c.stream>>>(key, m, noCell, head);
+    SM_LAUNCH_CHECK();
+    scan_excl(c, head, rank, (long long)m + 1, tag + ".hs", false);
+    SM_CUDA(cudaMemsetAsync(cRank, 0xff, (size_t)nc * 4, c.stream));
+    SM_CUDA(cudaMemsetAsync(flag, 0, ((size_t)m + 1) * 4, c.stream));
+    SM_CUDA(cudaMemsetAsync(ctl, 0, 4 * sizeof(int), c.stream));
+    SM_CUDA(cudaMemsetAsync(a.ring, 0xff, (size_t)ring * 4, c.stream));
+    k_sp_cells<<<nblocks(m, 256), 256, 0, c.stream>>>(key, val, m, noCell, head, rank, T.box,
+                                                     T.leafOf, cRank, cList, cEnd, ent, ex, a);
+    SM_LAUNCH_CHECK();
+    int nsm = 0;
+    SM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device));
+    k_sp_run<<<std::min(nblocks(m, kSpBs / 32), nsm * kSpCtas), kSpBs, 0, c.stream>>>(a);
+    SM_LAUNCH_CHECK();
     int *pre = c.arena.get<int>(tag + ".pre", (size_t)m + 1);
     scan_excl(c, flag, pre, (long long)m + 1, tag + ".os", false);
     k_sp_out<<<nblocks(m, 256), 256, 0, c.stream>>>(flag, pre, m, vaccA, outIds, ioi);

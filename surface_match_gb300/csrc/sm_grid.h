@@ -42,11 +42,18 @@ SM_HD float thin_cell(float step, const float ext[3]) {
 
 // Cell side of a dense acceleration grid for searches within `step` (the reference-order
 // sampler's cell lists): slightly larger than the step, doubled until the dense grid fits
-// the cap.
-SM_HD float sample_cell(float step, const float ext[3]) {
+// `cap` cells and no axis passes 2^13 of them (the rounding of a cell coordinate then stays
+// below the cell's margin over the step).
+SM_HD float sample_cell(float step, const float ext[3], long long cap) {
     float g = step * (1.0f + 1.0f / 1024.0f);
-    while (cells_of(ext, g) > kMaxCells)
+    if (!(g > 1e-30f))
+        g = 1e-30f;
+    for (int it = 0; it < 256; it++) {
+        if (smm::fdiv(ext[0], g) < 8191.0f && smm::fdiv(ext[1], g) < 8191.0f &&
+            smm::fdiv(ext[2], g) < 8191.0f && cells_of(ext, g) <= cap)
+            break;
         g = g * 2.0f;
+    }
     return g;
 }
 

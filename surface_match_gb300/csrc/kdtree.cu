@@ -23,9 +23,8 @@
 // radius search found it, visiting points in tree position order (util.cpp:107-139). Each
 // point's fate depends only on the earlier points within the step: it is dropped once a
 // kept one reaches it, and kept once all of them are decided and none of the kept ones
-// reaches it. The GPU counts those earlier points per point (neighbourhoods from grid cells
-// of side >= step, each cell's points in tree order), then decides points as their counts
-// run out, through a device queue: every point is handled exactly once, and decisions
+// reaches it. The GPU decides them through a device queue of grid cells, each waiting for the
+// open point that blocks its first one (below, k_sp_run), so decisions
 // travel along the dependency chains of the greedy order. "Reaches" is the reference's
 // radius search membership: squared distance below step^2 and not pruned by the search
 // above the point's leaf - decided by walking the point's root-to-leaf path
@@ -557,7 +556,13 @@ __global__ void k_kd_finish(int4 *__restrict__ nd, const int *__restrict__ paren
 constexpr int       kSpBs     = 256;
 constexpr long long kSpIdle   = 1ll << 22; // polls of an unwritten queue slot before giving up
 constexpr int       kSpUnroll = 4;         // neighbourhood entries in flight per lane
-constexpr int       kSpCtas   = 4;         // CTAs per SM: the warps that hold cells at once
+// CTAs per SM (2 measured best of 1, 2 and 4 beside the voting stage: the warps that hold cells
+// at once), nanoseconds between two looks at a queue slot, and words between two control words
+// (on one line, with every waiting warp reading it at each look, a decision took 40 us instead
+// of 10: the large scene's two long samplings 3.3 + 4.4 ms instead of 1.2 + 1.6 ms)
+constexpr int       kSpCtas   = 2;
+constexpr int       kSpSleep  = 100;
+constexpr int       kSpCtl    = 32;
 constexpr long long kSpCells  = 1ll << 25; // most cells of the dense table (128 MB)
 
 struct SampleArgs {
@@ -748,13 +753,16 @@ __device__ __forceinline__ int sp_take(const SampleArgs &a) {
             if (c >= 0)
                 return c;
         }
-        if (ld_vol(a.open) <= 0 || ld_vol(a.err))
-            return -1;
-        if (it > kSpIdle) {
-            atomicExch(a.err, 1);
-            return -1;
+        // (thousands of warps may wait here: the shared words are read now and then only)
+        if ((it & 15) == 15) {
+            if (ld_vol(a.open) <= 0 || ld_vol(a.err))
+                return -1;
+            if (it > kSpIdle) {
+                atomicExch(a.err, 1);
+                return -1;
+            }
         }
-        __nanosleep(64);
+        __nanosleep(kSpSleep);
     }
 }
 
@@ -1279,7 +1287,7 @@ int kd_sample(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
     float4   *ent   = c.arena.get<float4>(tag + ".ent", m);
     float    *ex    = c.arena.get<float>(tag + ".ex", m);
     int      *flag  = c.arena.get<int>(tag + ".flag", (size_t)m + 1);
-    int      *ctl   = c.arena.get<int>(tag + ".ctl", 4); // head, tail, open cells, error
+    int      *ctl   = c.arena.get<int>(tag + ".ctl", 4 * kSpCtl); // head, tail, open cells, error
     SampleArgs a{};
     a.t = T.view(vaccA, pos);
     for (int d = 0; d < 3; d++)
@@ -1296,12 +1304,12 @@ int kd_sample(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
     a.ring     = c.arena.get<int>(tag + ".ring", ring);
     a.ringMask = ring - 1;
     a.head     = ctl;
-    a.tail     = ctl + 1;
-    a.open     = ctl + 2;
+    a.tail     = ctl + kSpCtl;
+    a.open     = ctl + 2 * kSpCtl;
     a.r2       = step * step;
     a.safe2    = (double)a.r2 * (1.0 - 1e-4);
     a.keptFlag = flag;
-    a.err      = ctl + 3;
+    a.err      = ctl + 3 * kSpCtl;
     k_sp_keys<<<nblocks(m, 256), 256, 0, c.stream>>>(vaccA, pos, m, gp, noCell, key, val);
     SM_LAUNCH_CHECK();
     radix_sort_pairs(c, key, val, m, bits, tag);
@@ -1310,7 +1318,7 @@ int kd_sample(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
     scan_excl(c, head, rank, (long long)m + 1, tag + ".hs", false);
     SM_CUDA(cudaMemsetAsync(cRank, 0xff, (size_t)nc * 4, c.stream));
     SM_CUDA(cudaMemsetAsync(flag, 0, ((size_t)m + 1) * 4, c.stream));
-    SM_CUDA(cudaMemsetAsync(ctl, 0, 4 * sizeof(int), c.stream));
+    SM_CUDA(cudaMemsetAsync(ctl, 0, 4 * kSpCtl * sizeof(int), c.stream));
     SM_CUDA(cudaMemsetAsync(a.ring, 0xff, (size_t)ring * 4, c.stream));
     k_sp_cells<<<nblocks(m, 256), 256, 0, c.stream>>>(key, val, m, noCell, head, rank, T.box,
                                                      T.leafOf, cRank, cList, cEnd, ent, ex, a);
@@ -1324,7 +1332,7 @@ int kd_sample(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
     k_sp_out<<<nblocks(m, 256), 256, 0, c.stream>>>(flag, pre, m, vaccA, outIds, ioi);
     SM_LAUNCH_CHECK();
     SM_CUDA(cudaMemcpyAsync(c.hostCounts, pre + m, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-    SM_CUDA(cudaMemcpyAsync(c.hostCounts + 1, ctl + 3, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+    SM_CUDA(cudaMemcpyAsync(c.hostCounts + 1, a.err, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
     c.sync_checked();
     if (c.hostCounts[1])
         throw Error(SM_ERR_RUNTIME, "tree-order sampler: a bounded wait expired");

@@ -249,21 +249,35 @@ __global__ void k_bucket_fill(const uint32_t *__restrict__ ck, const uint32_t *_
 // by compare-and-swap, so placement depends on timing but every key sits after an unbroken
 // run of occupied slots from its home slot, which is all a probe needs). The slot's last
 // word is the bucket's largest number of entries of one reference point: entries are in
-// pair order, so a reference point's entries are consecutive.
+// pair order, so a reference point's entries are consecutive. A warp per bucket: buckets are
+// very uneven (a planar face's pairs share one key, thousands of entries), and the longest one
+// walked by a single thread set the kernel's time (154 us for the gear at 0.04, 495 us for the
+// bracket at 0.03; the whole training and its download 1063 -> 947 and 3767 -> 3323 us).
 __global__ void k_bucket_insert(const uint32_t *__restrict__ dkeys, const uint32_t *__restrict__ doffs,
                                 const uint2 *__restrict__ ent, int nkeys, uint32_t mask,
                                 int *__restrict__ claim, uint4 *__restrict__ tab) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    const int b    = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
     if (b >= nkeys)
         return;
     const uint32_t k = dkeys[b], o0 = doffs[b], o1 = doffs[b + 1];
-    uint32_t       best = 0, run = 0, prev = 0xffffffffu;
-    for (uint32_t e = o0; e < o1; e++) {
-        const uint32_t r = ent[e].x;
-        run              = r == prev ? run + 1 : 1;
-        prev             = r;
-        best             = run > best ? run : best;
+    uint32_t       best = 0, carry = 0, prev = 0xffffffffu; // carry: length of the run at the edge
+    for (uint32_t e0 = o0; e0 < o1; e0 += 32) {
+        const uint32_t e  = e0 + lane;
+        const uint32_t r  = e < o1 ? ent[e].x : 0xffffffffu;
+        const uint32_t up = __shfl_up_sync(0xffffffffu, r, 1);
+        // heads of runs among the lanes up to this one; without any the run came in from before
+        const unsigned heads =
+            __ballot_sync(0xffffffffu, r != (lane == 0 ? prev : up)) & (0xffffffffu >> (31 - lane));
+        const uint32_t run = heads ? lane - (31 - __clz(heads)) + 1 : carry + lane + 1;
+        if (e < o1)
+            best = run > best ? run : best;
+        carry = __shfl_sync(0xffffffffu, run, 31);
+        prev  = __shfl_sync(0xffffffffu, r, 31);
     }
+    best = __reduce_max_sync(0xffffffffu, best);
+    if (lane != 0)
+        return;
     uint32_t i = k & mask;
     for (uint32_t n = 0; n <= mask; n++) {
         if (atomicCAS(&claim[i], -1, b) == -1) {
@@ -320,7 +334,7 @@ void build_model_table(Ctx &c, Model &m, const uint32_t *keys, const float *alph
     SM_CUDA(cudaMemsetAsync(claim, 0xff, (size_t)size * 4, c.stream));
     SM_CUDA(cudaMemsetAsync(m.hkeys, 0, (size_t)size * sizeof(uint4), c.stream));
     if (nkeys > 0) {
-        k_bucket_insert<<<nblocks(nkeys, 128), 128, 0, c.stream>>>(m.dkeys, m.doffs, m.entries, nkeys,
+        k_bucket_insert<<<nblocks((long long)nkeys * 32, 128), 128, 0, c.stream>>>(m.dkeys, m.doffs, m.entries, nkeys,
                                                                   m.hmask, claim, (uint4 *)m.hkeys);
         SM_LAUNCH_CHECK();
     }

@@ -43,12 +43,12 @@ struct Cand {
     smi::Pose34 M, keep, step;
     float       Pm[3], Qm[3];
     float       resMse, mse, score;
-    int         cnt, iterations, converged, stop, status, active, inl, pad;
+    int         cnt, iterations, converged, status, active, inl;
 };
 
 struct Stage {
     const float4 *src, *srcN; // model points / normals
-    int           n, nb;      // points, CTAs per candidate
+    int           n;          // points
     HGridView     G;          // scene subset grid (pts.w = subset rank)
     const float4 *dPos, *dNrm; // the subset's positions / normals by rank
     int           nDst;
@@ -77,14 +77,27 @@ struct Work {
     int                 maxSrc, maxDst;
     float              *trace;  // ncand x kTraceFloats (nullable)
     unsigned long long *live;   // (candidate, source point) searches of K1 (nullable: not counted)
+    // the candidates of each step of a stage (any order): iteration it refines those in
+    // list[it * ncand ..], cnt[it] of them; step `iters` holds those the stage leaves active
+    int                *cnt, *list;
+    int                 ncand;
 };
+
+// The candidates of step `it`: their number and the k-th.
+__device__ __forceinline__ int  step_count(const Work &w, int it) { return w.cnt[it]; }
+__device__ __forceinline__ int  step_cand(const Work &w, int it, int k) { return w.list[it * w.ncand + k]; }
+// Candidate and source point of item k of the step's candidates times n source points.
+__device__ __forceinline__ void step_item(const Work &w, int it, long long k, int n, int &ci, int &i) {
+    const int c = k < (1ll << 31) ? (int)((unsigned)k / (unsigned)n) : (int)(k / n);
+    ci          = step_cand(w, it, c);
+    i           = (int)(k - (long long)c * n);
+}
+__device__ __forceinline__ void step_add(const Work &w, int it, int ci) {
+    w.list[it * w.ncand + atomicAdd(&w.cnt[it], 1)] = ci;
+}
 
 __device__ __forceinline__ unsigned long long win_key(float d, int i) {
     return ((unsigned long long)__float_as_uint(d) << 32) | (unsigned)i;
-}
-
-__device__ __forceinline__ bool cand_live(const Cand &c, const Stage &s) {
-    return c.active && !c.stop && c.iterations < s.iters;
 }
 
 // The nearest point of the stage's subset to (x, y, z) by a warp, exact where its squared
@@ -99,34 +112,30 @@ __device__ __forceinline__ int stage_nearest(const Stage &s, float x, float y, f
     return warp_nn_walk(s.G, x, y, z, lim, d);
 }
 
-// K1: correspondences, one warp per source point (warp-cooperative grid search). In reference
-// order (TREE) a pair is what findClosestPoint (util.cpp:603-626) returns: a one-nearest search
-// of the reduced k-d tree with the tree's pruning; one beyond the rejection distance is
-// dropped, so the search is needed up to that distance only.
+// K1: correspondences, one warp per (candidate, source point) of the step's candidates
+// (warp-cooperative grid search; the grid of CTAs is one resident wave, so that the launches
+// after the last candidate stopped cost next to nothing: 9 us for a CTA per 8 points of every
+// candidate, 2.5 us now). In reference order (TREE) a pair is what findClosestPoint
+// (util.cpp:603-626) returns: a one-nearest search of the reduced k-d tree with the tree's
+// pruning; one beyond the rejection distance is dropped, so the search is needed up to that
+// distance only.
 template <bool TREE>
-__global__ void __launch_bounds__(kT, TREE ? 3 : 4) k_corr(Work w, Stage s, int usePrev) {
+__global__ void __launch_bounds__(kT, TREE ? 3 : 4) k_corr(Work w, Stage s, int it) {
     chain_enter(); // launched chained
-    const int ci   = blockIdx.y;
-    const int lane = threadIdx.x & 31;
-    int       i    = blockIdx.x * kW + (threadIdx.x >> 5);
-    // the first source point is read together with the candidate's state
-    float4 sp = i < s.n ? s.src[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 sn = i < s.n ? s.srcN[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const Cand &C = w.cand[ci];
-    if (!cand_live(C, s))
-        return; // (a candidate that is not live has no nearest points of this stage)
+    const int       lane  = threadIdx.x & 31;
+    const long long items = (long long)step_count(w, it) * s.n;
     if (w.live && blockIdx.x == 0 && threadIdx.x == 0)
-        atomicAdd(w.live, (unsigned long long)s.n);
-    for (; i < s.n; i += gridDim.x * kW) {
-        const size_t o = (size_t)ci * w.maxSrc + i;
+        atomicAdd(w.live, (unsigned long long)items);
+    for (long long k = blockIdx.x * kW + (threadIdx.x >> 5); k < items; k += gridDim.x * kW) {
+        int          ci, i;
+        step_item(w, it, k, s.n, ci, i);
+        const size_t o  = (size_t)ci * w.maxSrc + i;
+        const Cand  &C  = w.cand[ci];
+        const float4 sp = s.src[i], sn = s.srcN[i];
         float4       x, y;
-        if (i != blockIdx.x * kW + (threadIdx.x >> 5)) {
-            sp = s.src[i];
-            sn = s.srcN[i];
-        }
-        // written by this candidate's previous iteration of this stage (usePrev: not the
-        // first iteration), a rank of this stage's subset or -1
-        const int jp = usePrev ? w.nnPrev[o] : -1;
+        // written by this candidate's previous iteration of this stage (not in the first), a
+        // rank of this stage's subset or -1
+        const int jp = it > 0 ? w.nnPrev[o] : -1;
         float4    qp = make_float4(0.f, 0.f, 0.f, 0.f);
         if (jp >= 0 && jp < s.nDst)
             qp = s.dPos[jp];
@@ -161,37 +170,74 @@ __global__ void __launch_bounds__(kT, TREE ? 3 : 4) k_corr(Work w, Stage s, int 
 // memory; rank 0 reads the kRC partials through distributed shared memory and merges them
 // by the block tree (offsets kRC/2..1). No global fence or counter between CTAs, and the
 // centroids, the normal equations and the solve share one launch.
-template <int W> __device__ void block_tree(smi::KahanF (&v)[W], float (*red)[W][2]) {
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+//
+// The warp tree of many sums: at each offset a lane takes only half of the sums it still holds
+// (the lower half in the lower lanes), so 32 sums take 31 merges a lane instead of 160; the
+// merges and their operands are those of the plain tree. The tree over the warps and the one
+// over the CTAs run a lane per sum, serially in registers. (27 sums by the plain trees, every
+// lane merging all of them, made a third of the launch.)
+__device__ __forceinline__ smi::KahanF shfl_xor(const smi::KahanF &v, int off) {
+    smi::KahanF o;
+    o.s = __shfl_xor_sync(0xffffffffu, v.s, off);
+    o.c = __shfl_xor_sync(0xffffffffu, v.c, off);
+    return o;
+}
+
+// W <= 32 sums padded to P = 2^k: the tree's root of sum l * P / 32 ends on lane l (for P < 32
+// on the first of 32 / P lanes).
+template <int P, int OFF> __device__ __forceinline__ void warp_tree(smi::KahanF (&v)[P]) {
+    const bool high = (threadIdx.x & OFF) != 0;
+    if constexpr (P > 1) {
+        smi::KahanF h[P / 2];
 #pragma unroll
-    for (int off = 16; off >= 1; off >>= 1)
-        for (int k = 0; k < W; k++) {
-            smi::KahanF o;
-            o.s = __shfl_down_sync(0xffffffffu, v[k].s, off);
-            o.c = __shfl_down_sync(0xffffffffu, v[k].c, off);
-            v[k].merge(o);
+        for (int k = 0; k < P / 2; k++) {
+            const smi::KahanF keep = high ? v[P / 2 + k] : v[k];
+            const smi::KahanF got  = shfl_xor(high ? v[k] : v[P / 2 + k], OFF);
+            h[k]                   = high ? got : keep;  // the lower lane's partial
+            h[k].merge(high ? keep : got);
         }
-    if (lane == 0)
-        for (int k = 0; k < W; k++) {
-            red[wp][k][0] = v[k].s;
-            red[wp][k][1] = v[k].c;
-        }
+        if constexpr (OFF > 1)
+            warp_tree<P / 2, OFF / 2>(h);
+        v[0] = h[0];
+    } else {
+        const smi::KahanF got = shfl_xor(v[0], OFF);
+        smi::KahanF       r   = high ? got : v[0];
+        r.merge(high ? v[0] : got);
+        v[0] = r;
+        if constexpr (OFF > 1)
+            warp_tree<1, OFF / 2>(v);
+    }
+}
+
+// The block's totals of W sums (v: padded to P): lane k < W of warp 0 returns the k-th.
+template <int W, int P>
+__device__ __forceinline__ smi::KahanF block_tree(smi::KahanF (&v)[P], float (*red)[W][2]) {
+    constexpr int G = 32 / P; // lanes per sum after the warp tree
+    const int     lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    warp_tree<P, 16>(v);
+    if (lane % G == 0 && lane / G < W) {
+        red[wp][lane / G][0] = v[0].s;
+        red[wp][lane / G][1] = v[0].c;
+    }
     __syncthreads();
-    if (wp == 0) {
-        for (int k = 0; k < W; k++) {
-            v[k].s = lane < kRW ? red[lane][k][0] : 0.f;
-            v[k].c = lane < kRW ? red[lane][k][1] : 0.f;
+    smi::KahanF t;
+    t.init();
+    if (wp == 0 && lane < W) {
+        smi::KahanF p[kRW];
+#pragma unroll
+        for (int r = 0; r < kRW; r++) {
+            p[r].s = red[r][lane][0];
+            p[r].c = red[r][lane][1];
         }
 #pragma unroll
         for (int off = kRW / 2; off >= 1; off >>= 1)
-            for (int k = 0; k < W; k++) {
-                smi::KahanF o;
-                o.s = __shfl_down_sync(0xffffffffu, v[k].s, off);
-                o.c = __shfl_down_sync(0xffffffffu, v[k].c, off);
-                v[k].merge(o);
-            }
+#pragma unroll
+            for (int r = 0; r < off; r++)
+                p[r].merge(p[r + off]);
+        t = p[0];
     }
     __syncthreads(); // red may be reused
+    return t;
 }
 
 __device__ __forceinline__ int block_sum_int(int x, int *red) {
@@ -206,34 +252,32 @@ __device__ __forceinline__ int block_sum_int(int x, int *red) {
     return t;
 }
 
-// Rank 0's warp 0: the cluster's kRC published partials (lane r < kRC reads CTA r's through
-// distributed shared memory), merged by the block tree; lane 0 ends with the totals.
+// Rank 0's warp 0: lane k < W merges the cluster's kRC published partials of sum k (read through
+// distributed shared memory) by the block tree.
 template <int W>
-__device__ void cluster_merge(cg::cluster_group &cl, float (*part)[2], smi::KahanF (&v)[W]) {
-    const int lane = threadIdx.x & 31;
-    for (int k = 0; k < W; k++) {
-        float ps = 0.f, pc = 0.f;
-        if (lane < kRC) {
-            const float *rp = cl.map_shared_rank(&part[k][0], (unsigned)lane);
-            ps              = rp[0];
-            pc              = rp[1];
+__device__ __forceinline__ smi::KahanF cluster_merge(cg::cluster_group &cl, float (*part)[2]) {
+    const int   lane = threadIdx.x & 31;
+    smi::KahanF p[kRC];
+#pragma unroll
+    for (int r = 0; r < kRC; r++) {
+        p[r].init();
+        if (lane < W) {
+            const float *rp = cl.map_shared_rank(&part[lane][0], (unsigned)r);
+            p[r].s          = rp[0];
+            p[r].c          = rp[1];
         }
-        v[k].s = ps;
-        v[k].c = pc;
     }
 #pragma unroll
     for (int off = kRC / 2; off >= 1; off >>= 1)
-        for (int k = 0; k < W; k++) {
-            smi::KahanF o;
-            o.s = __shfl_down_sync(0xffffffffu, v[k].s, off);
-            o.c = __shfl_down_sync(0xffffffffu, v[k].c, off);
-            v[k].merge(o);
-        }
+#pragma unroll
+        for (int r = 0; r < off; r++)
+            p[r].merge(p[r + off]);
+    return p[0];
 }
 
 // K2: pair selection (the closest source point per scene point: the atomicMin winner), pair
 // count and centroids, then the normal-equation terms of the pairs and the FP64 solve.
-__global__ void __cluster_dims__(kRC, 1, 1) __launch_bounds__(kR) k_fit(Work w, Stage s) {
+__global__ void __cluster_dims__(kRC, 1, 1) __launch_bounds__(kR) k_fit(Work w, Stage s, int it) {
     chain_enter(); // launched chained
     __shared__ float red[kRW][smi::kNumSystem][2];
     __shared__ float part[smi::kNumSystem][2]; // this CTA's totals, read by rank 0
@@ -243,17 +287,17 @@ __global__ void __cluster_dims__(kRC, 1, 1) __launch_bounds__(kR) k_fit(Work w, 
     __shared__ int   sTotal;
     cg::cluster_group cl = cg::this_cluster();
     const int         rk = (int)cl.block_rank();
-    const int         ci = blockIdx.x / kRC;
-    Cand             &C  = w.cand[ci];
-    if (!cand_live(C, s))
+    if ((int)(blockIdx.x / kRC) >= step_count(w, it))
         return; // (the whole cluster: one candidate)
+    const int     ci   = step_cand(w, it, blockIdx.x / kRC);
+    Cand         &C    = w.cand[ci];
     int          *nnId = w.nnId + (size_t)ci * w.maxSrc;
     const int    *nnR  = w.nnR + (size_t)ci * w.maxSrc;
     const float4 *x4   = w.x4 + (size_t)ci * w.maxSrc;
     const float4 *n4   = w.n4 + (size_t)ci * w.maxSrc;
     const int     slot = rk * kR + threadIdx.x;
-    smi::KahanF   m[6];
-    for (int k = 0; k < 6; k++)
+    smi::KahanF   m[8]; // 6 sums
+    for (int k = 0; k < 8; k++)
         m[k].init();
     // a thread's pairs i = slot, slot + kIcpSlots, ... in ascending order, kFitU of them
     // loaded at once (their loads are independent; the sums still take them in order)
@@ -295,29 +339,28 @@ __global__ void __cluster_dims__(kRC, 1, 1) __launch_bounds__(kR) k_fit(Work w, 
         }
     }
     const int cntB = block_sum_int(cnt, ired);
-    block_tree<6>(m, reinterpret_cast<float (*)[6][2]>(&red[0][0][0]));
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < 6; k++) {
-            part[k][0] = m[k].s;
-            part[k][1] = m[k].c;
-        }
-        pcnt = cntB;
+    const smi::KahanF mt = block_tree<6>(m, reinterpret_cast<float (*)[6][2]>(&red[0][0][0]));
+    if (threadIdx.x < 6) {
+        part[threadIdx.x][0] = mt.s;
+        part[threadIdx.x][1] = mt.c;
     }
+    if (threadIdx.x == 0)
+        pcnt = cntB;
     cl.sync(); // the partials are published
     if (rk == 0 && threadIdx.x < 32) {
-        smi::KahanF mm[6];
-        cluster_merge<6>(cl, part, mm);
+        const smi::KahanF mm    = cluster_merge<6>(cl, part);
+        int               total = 0;
+        for (int r = 0; r < kRC; r++)
+            total += *cl.map_shared_rank(&pcnt, (unsigned)r);
+        if (threadIdx.x < 6) {
+            const float c      = smm::fdiv(mm.value(), (float)total);
+            sPQ[threadIdx.x]   = c;
+            if (threadIdx.x < 3)
+                C.Pm[threadIdx.x] = c;
+            else
+                C.Qm[threadIdx.x - 3] = c;
+        }
         if (threadIdx.x == 0) {
-            int total = 0;
-            for (int r = 0; r < kRC; r++)
-                total += *cl.map_shared_rank(&pcnt, (unsigned)r);
-            const float fc = (float)total;
-            for (int k = 0; k < 3; k++) {
-                C.Pm[k]    = smm::fdiv(mm[k].value(), fc);
-                C.Qm[k]    = smm::fdiv(mm[3 + k].value(), fc);
-                sPQ[k]     = C.Pm[k];
-                sPQ[3 + k] = C.Qm[k];
-            }
             C.cnt  = total;
             sTotal = total;
         }
@@ -330,8 +373,8 @@ __global__ void __cluster_dims__(kRC, 1, 1) __launch_bounds__(kR) k_fit(Work w, 
     cl.sync(); // every CTA has read rank 0's centroids (rank 0 may leave after this)
     if (total < 6)
         return;
-    smi::KahanF v[smi::kNumSystem];
-    for (int k = 0; k < smi::kNumSystem; k++)
+    smi::KahanF v[32]; // kNumSystem sums
+    for (int k = 0; k < 32; k++)
         v[k].init();
     for (int base = slot; base < s.n; base += 2 * smi::kIcpSlots) {
         int    id[2];
@@ -362,24 +405,21 @@ __global__ void __cluster_dims__(kRC, 1, 1) __launch_bounds__(kR) k_fit(Work w, 
                 v[k].add(t[k]);
         }
     }
-    block_tree<smi::kNumSystem>(v, red);
-    if (threadIdx.x == 0)
-        for (int k = 0; k < smi::kNumSystem; k++) {
-            part[k][0] = v[k].s;
-            part[k][1] = v[k].c;
-        }
+    const smi::KahanF vt = block_tree<smi::kNumSystem>(v, red);
+    if (threadIdx.x < smi::kNumSystem) {
+        part[threadIdx.x][0] = vt.s;
+        part[threadIdx.x][1] = vt.c;
+    }
     cl.sync(); // the partials are published
     if (rk == 0 && threadIdx.x < 32) {
-        cluster_merge<smi::kNumSystem>(cl, part, v);
+        const float tot = cluster_merge<smi::kNumSystem>(cl, part).value();
         cl.sync(); // (rank 0 has read every partial: the others may leave)
-        // the totals are on lane 0; warp 0 solves with one row of the system per lane
         float sys[smi::kNumSystem];
+#pragma unroll
         for (int k = 0; k < smi::kNumSystem; k++)
-            sys[k] = __shfl_sync(0xffffffffu, v[k].value(), 0);
-        const float       pm[3] = {Pm0, Pm1, Pm2}, qm[3] = {Qm0, Qm1, Qm2};
-        const smi::Pose34 st    = smi::solve_step_warp(sys, pm, qm);
-        if (threadIdx.x == 0)
-            C.step = st;
+            sys[k] = __shfl_sync(0xffffffffu, tot, k);
+        const float pm[3] = {Pm0, Pm1, Pm2}, qm[3] = {Qm0, Qm1, Qm2};
+        smi::solve_step_warp(sys, pm, qm, C.step.m);
     } else {
         cl.sync();
     }
@@ -387,41 +427,48 @@ __global__ void __cluster_dims__(kRC, 1, 1) __launch_bounds__(kR) k_fit(Work w, 
 
 // K4: residual distance of each pair after the step, one warp per pair
 template <bool TREE>
-__global__ void __launch_bounds__(kT, TREE ? 3 : 5) k_resid(Work w, Stage s) {
+__global__ void __launch_bounds__(kT, TREE ? 3 : 5) k_resid(Work w, Stage s, int it) {
     chain_enter(); // launched chained
-    const int   ci = blockIdx.y;
-    const Cand &C  = w.cand[ci];
-    if (!cand_live(C, s) || C.cnt < 6)
-        return;
-    for (int i = blockIdx.x * kW + (threadIdx.x >> 5); i < s.n; i += gridDim.x * kW) {
-        const size_t o = (size_t)ci * w.maxSrc + i;
-        if (w.nnId[o] < 0)
+    const long long items = (long long)step_count(w, it) * s.n;
+    for (long long k = blockIdx.x * kW + (threadIdx.x >> 5); k < items; k += gridDim.x * kW) {
+        int          ci, i;
+        step_item(w, it, k, s.n, ci, i);
+        const size_t o  = (size_t)ci * w.maxSrc + i;
+        const Cand  &C  = w.cand[ci];
+        const int    j  = w.nnId[o];
+        const float4 x  = w.x4[o];
+        if (C.cnt < 6 || j < 0)
             continue;
-        const float4 x = w.x4[o];
-        const float4 q = s.dPos[w.nnId[o]];
+        const float4 q = s.dPos[j];
         float        y0, y1, y2, d;
         smi::pose_apply(C.step, x.x, x.y, x.z, y0, y1, y2);
         // the pair's scene point bounds the search exactly
         stage_nearest<TREE>(s, y0, y1, y2, smm::dist2(y0, y1, y2, q.x, q.y, q.z), d);
         if ((threadIdx.x & 31) == 0)
-            w.resid[(size_t)ci * w.maxSrc + i] = smm::fsqrt(d);
+            w.resid[o] = smm::fsqrt(d);
     }
 }
 
 // K5: mean residual, the regist loop logic (icp.cpp:233-272), winner reset; one cluster per
-// candidate (the same layout as K2), rank 0's thread 0 runs the logic
-__global__ void __cluster_dims__(kRC, 1, 1) __launch_bounds__(kR) k_update(Work w, Stage s) {
+// candidate (the same layout as K2), rank 0's warp 0 runs the logic and lists the candidate for
+// the next iteration if it goes on
+__global__ void __cluster_dims__(kRC, 1, 1) __launch_bounds__(kR) k_update(Work w, Stage s, int it) {
     chain_enter(); // launched chained
     __shared__ float red[kRW][1][2];
     __shared__ float part[1][2];
     cg::cluster_group cl = cg::this_cluster();
     const int         rk = (int)cl.block_rank();
-    const int         ci = blockIdx.x / kRC;
-    Cand             &C  = w.cand[ci];
-    if (!cand_live(C, s))
+    if ((int)(blockIdx.x / kRC) >= step_count(w, it))
         return;
+    const int  ci   = step_cand(w, it, blockIdx.x / kRC);
+    Cand      &C    = w.cand[ci];
     const int  slot = rk * kR + threadIdx.x;
+    const int  lane = threadIdx.x & 31;
     const int *nnR  = w.nnR + (size_t)ci * w.maxSrc;
+    // the step's product with the pose, an entry per lane (used below if the step is taken)
+    float moved = 0.0f;
+    if (rk == 0 && threadIdx.x < 12)
+        moved = smi::pose_mul_entry(C.step.m, C.M.m, lane);
     for (int i = slot; i < s.n; i += smi::kIcpSlots)
         if (nnR[i] >= 0)
             w.win[(size_t)ci * w.maxDst + nnR[i]] = ~0ull;
@@ -446,53 +493,62 @@ __global__ void __cluster_dims__(kRC, 1, 1) __launch_bounds__(kR) k_update(Work 
                 if (id[u] >= 0)
                     v[0].add(d[u]);
         }
-        block_tree<1>(v, red);
+        const smi::KahanF vt = block_tree<1>(v, red);
         if (threadIdx.x == 0) {
-            part[0][0] = v[0].s;
-            part[0][1] = v[0].c;
+            part[0][0] = vt.s;
+            part[0][1] = vt.c;
         }
         cl.sync(); // the partials are published
-        if (rk == 0 && threadIdx.x < 32) {
-            cluster_merge<1>(cl, part, v);
-            if (threadIdx.x == 0)
-                mse = smm::fdiv(v[0].value(), (float)cnt);
-        }
+        if (rk == 0 && threadIdx.x < 32)
+            mse = __shfl_sync(0xffffffffu, smm::fdiv(cluster_merge<1>(cl, part).value(), (float)cnt), 0);
         cl.sync(); // rank 0 has read every partial: the others may leave
     }
-    if (rk != 0 || threadIdx.x != 0)
+    if (rk != 0 || threadIdx.x >= 32)
         return;
-    if (w.trace && C.iterations < kTraceIters) {
-        float *t = w.trace + (size_t)ci * kTraceFloats + (s.traceOff * kTraceIters + C.iterations) * 4;
+    const int   done   = C.iterations;
+    const float resMse = C.resMse;
+    __syncwarp();
+    if (lane == 0 && w.trace && done < kTraceIters) {
+        float *t = w.trace + (size_t)ci * kTraceFloats + (s.traceOff * kTraceIters + done) * 4;
         t[0]     = (float)cnt;
         t[1]     = mse;
         t[2]     = cnt >= 6 ? C.Pm[0] : -1.0f;
         t[3]     = cnt >= 6 ? C.step.m[3] : 0.0f;
     }
-    if (cnt > 6 && mse < s.mseMax)
-        C.converged = 1;
-    int stop = 0;
+    int  stop = 0;
+    bool take = false;
     if (cnt < 6) {
         stop = 1;
     } else {
         if (mse < s.mseMin)
             stop = 1;
-        const float rate = smm::fdiv(C.resMse - mse, C.resMse);
+        const float rate = smm::fdiv(resMse - mse, resMse);
         if (rate < 0.05f)
             stop = 1;
-        if (C.iterations++ >= s.iters)
+        if (done >= s.iters)
             stop = 1;
-        if (rate > 0.0f) {
-            C.resMse = mse;
-            C.M      = smi::pose_mul(C.step, C.M);
-        }
+        take = rate > 0.0f;
     }
-    C.stop = stop;
+    if (take && lane < 12)
+        C.M.m[lane] = moved;
+    if (lane == 0) {
+        if (cnt > 6 && mse < s.mseMax)
+            C.converged = 1;
+        if (take)
+            C.resMse = mse;
+        if (cnt >= 6)
+            C.iterations = done + 1;
+        if (!stop && done + 1 < s.iters)
+            step_add(w, it + 1, ci);
+    }
 }
 
-__global__ void k_init(Work w, const float *__restrict__ cands, int ncand, float voteThreshold,
-                       int sparse) {
+__global__ void k_init(Work w, const float *__restrict__ cands, float voteThreshold, int sparse,
+                       int steps) {
     const int ci = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ci >= ncand)
+    for (int k = ci; k < steps; k += gridDim.x * blockDim.x)
+        w.cnt[k] = 0; // the candidate counts of every step of both stages
+    if (ci >= w.ncand)
         return;
     Cand        &C = w.cand[ci];
     const float *P = cands + (size_t)ci * smi::kPoseFloats;
@@ -507,24 +563,26 @@ __global__ void k_init(Work w, const float *__restrict__ cands, int ncand, float
             w.trace[(size_t)ci * kTraceFloats + e] = -1.0f;
 }
 
-__global__ void k_stage_begin(Work w, int ncand) {
+__global__ void k_stage_begin(Work w, int iters) {
     chain_enter(); // launched chained
     const int ci = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ci >= ncand)
+    if (ci >= w.ncand)
         return;
     Cand &C      = w.cand[ci];
     C.resMse     = FLT_MAX;
     C.iterations = 0;
     C.converged  = 0;
-    C.stop       = 0;
     C.inl        = 0;
+    if (C.active && iters > 0)
+        step_add(w, 0, ci);
 }
 
-// After a refinement: failed candidates get their status; converged ones keep the pose.
-__global__ void k_stage_end(Work w, int ncand, int failStatus) {
+// After a refinement: failed candidates get their status; converged ones keep the pose and are
+// listed for the scoring.
+__global__ void k_stage_end(Work w, int last, int failStatus) {
     chain_enter(); // launched chained
     const int ci = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ci >= ncand)
+    if (ci >= w.ncand)
         return;
     Cand &C = w.cand[ci];
     if (!C.active)
@@ -534,27 +592,37 @@ __global__ void k_stage_end(Work w, int ncand, int failStatus) {
         C.active = 0;
     } else {
         C.keep = C.M;
+        step_add(w, last, ci);
     }
 }
 
-// Inliers of each candidate: source points with a scene point closer than the scoring
-// distance, one warp per point (warp_any_within); with TREE the scene point that the
-// reference's search of the whole tree returns (inliner, util.cpp:628-641).
+// Inliers of each candidate left (step `last`): source points with a scene point closer than the
+// scoring distance, one warp per point (warp_any_within); with TREE the scene point that the
+// reference's search of the whole tree returns (inliner, util.cpp:628-641). A warp takes
+// consecutive points, so that it adds to a candidate's count once or twice.
 template <bool TREE>
 __global__ void __launch_bounds__(kT, TREE ? 3 : 6)
-    k_inliers(Work w, const float4 *__restrict__ src, int n, HGridView F, float r2, smk::KdView t,
-              int treeM, const int *__restrict__ treePos, const float *__restrict__ exc) {
+    k_inliers(Work w, const float4 *__restrict__ src, int n, int last, HGridView F, float r2,
+              smk::KdView t, int treeM, const int *__restrict__ treePos,
+              const float *__restrict__ exc) {
     chain_enter(); // launched chained
-    __shared__ int sc[kW];
-    const int      ci = blockIdx.y;
-    const Cand    &C  = w.cand[ci];
-    if (!C.active)
-        return;
-    const int lane = threadIdx.x & 31;
-    int       c    = 0;
-    for (int i = blockIdx.x * kW + (threadIdx.x >> 5); i < n; i += gridDim.x * kW) {
-        float x, y, z;
-        smi::pose_apply(C.M, src[i].x, src[i].y, src[i].z, x, y, z);
+    const long long items = (long long)step_count(w, last) * n;
+    const long long warps = (long long)gridDim.x * kW, per = (items + warps - 1) / warps;
+    long long       k   = (blockIdx.x * (long long)kW + (threadIdx.x >> 5)) * per;
+    const long long end = k + per < items ? k + per : items;
+    int             c = 0, at = -1;
+    for (; k < end; k++) {
+        int ci, i;
+        step_item(w, last, k, n, ci, i);
+        if (ci != at) {
+            if (c && (threadIdx.x & 31) == 0)
+                atomicAdd(&w.cand[at].inl, c);
+            at = ci;
+            c  = 0;
+        }
+        float        x, y, z;
+        const float4 p = src[i];
+        smi::pose_apply(w.cand[ci].M, p.x, p.y, p.z, x, y, z);
         if (TREE) {
             float     d;
             const int j =
@@ -564,16 +632,8 @@ __global__ void __launch_bounds__(kT, TREE ? 3 : 6)
             c += warp_any_within(F, x, y, z, r2) ? 1 : 0;
         }
     }
-    if (lane == 0)
-        sc[threadIdx.x >> 5] = c;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int t2 = 0;
-        for (int k = 0; k < kW; k++)
-            t2 += sc[k];
-        if (t2)
-            atomicAdd(&w.cand[ci].inl, t2);
-    }
+    if (c && (threadIdx.x & 31) == 0)
+        atomicAdd(&w.cand[at].inl, c);
 }
 
 __global__ void k_score(Work w, int ncand, int n, float minScore, int failStatus, int slot) {
@@ -609,29 +669,38 @@ __global__ void k_finish(Work w, int ncand, int refine, float minScore, int *sta
 }
 
 
-void run_stage(Ctx &c, Work &w, const Stage &s, int ncand) {
-    const dim3 gc(ncand * kRC);                               // reductions: a cluster per candidate
-    const dim3 gw(std::max(1, nblocks(s.n, kW)), ncand); // searches: a warp per point
-    const bool tree = s.tree.nd != nullptr;
-    launch_chained(c, k_stage_begin, nblocks(ncand, 128), 128, 0, w, ncand);
+// CTAs of a launch over `items` warps' worth of work: at most one resident wave (perSm CTAs of kT
+// threads, the kernels' launch bounds).
+int wave(const Ctx &c, long long items, int perSm) {
+    int nsm = 0;
+    SM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device));
+    return (int)std::max<long long>(1, std::min<long long>((items + kW - 1) / kW, (long long)nsm * perSm));
+}
+
+void run_stage(Ctx &c, const Work &w, const Stage &s) {
+    const int       gc   = w.ncand * kRC; // reductions: a cluster per candidate
+    const bool      tree = s.tree.nd != nullptr;
+    const long long all  = (long long)w.ncand * s.n;
+    const int gCorr = wave(c, all, tree ? 3 : 4), gResid = wave(c, all, tree ? 3 : 5);
+    launch_chained(c, k_stage_begin, nblocks(w.ncand, 128), 128, 0, w, s.iters);
     for (int it = 0; it < s.iters; it++) {
         cudaEvent_t t0 = c.clock.begin(c.stream);
         if (tree)
-            launch_chained(c, k_corr<true>, gw, kT, 0, w, s, it > 0 ? 1 : 0);
+            launch_chained(c, k_corr<true>, gCorr, kT, 0, w, s, it);
         else
-            launch_chained(c, k_corr<false>, gw, kT, 0, w, s, it > 0 ? 1 : 0);
+            launch_chained(c, k_corr<false>, gCorr, kT, 0, w, s, it);
         c.clock.end(c.stream, t0, KernelClock::kCorr, 0.0); // bytes from the live count
         t0 = c.clock.begin(c.stream);
-        launch_chained(c, k_fit, gc, kR, 0, w, s);
+        launch_chained(c, k_fit, gc, kR, 0, w, s, it);
         c.clock.end(c.stream, t0, KernelClock::kFit, 0.0);
         t0 = c.clock.begin(c.stream);
         if (tree)
-            launch_chained(c, k_resid<true>, gw, kT, 0, w, s);
+            launch_chained(c, k_resid<true>, gResid, kT, 0, w, s, it);
         else
-            launch_chained(c, k_resid<false>, gw, kT, 0, w, s);
+            launch_chained(c, k_resid<false>, gResid, kT, 0, w, s, it);
         c.clock.end(c.stream, t0, KernelClock::kResid, 0.0);
         t0 = c.clock.begin(c.stream);
-        launch_chained(c, k_update, gc, kR, 0, w, s);
+        launch_chained(c, k_update, gc, kR, 0, w, s, it);
         c.clock.end(c.stream, t0, KernelClock::kUpdate, 0.0);
     }
 }
@@ -661,24 +730,31 @@ void icp_all(Ctx &c, const Model &m, const IcpScene &sc, const IcpParams &p, con
         w.live = c.arena.get<unsigned long long>("icp.live", 1);
         SM_CUDA(cudaMemsetAsync(w.live, 0, sizeof(unsigned long long), c.stream));
     }
+    // steps of the sparse stage (5 iterations and the scoring), then of the dense one
+    constexpr int sparseIters = 5;
+    const int     sparseLast = sparseIters, denseLast = std::max(p.denseSteps, 0);
+    const int     steps = sparseLast + 1 + denseLast + 1;
+    w.ncand = ncand;
+    w.cnt   = c.arena.get<int>("icp.cnt", steps);
+    w.list  = c.arena.get<int>("icp.list", (size_t)steps * ncand);
     SM_CUDA(cudaMemsetAsync(w.win, 0xff, (size_t)ncand * w.maxDst * 8, c.stream));
-    k_init<<<nblocks(ncand, 128), 128, 0, c.stream>>>(w, cands, ncand, p.voteThreshold, p.sparse);
+    k_init<<<nblocks(ncand, 128), 128, 0, c.stream>>>(w, cands, p.voteThreshold, p.sparse, steps);
     SM_LAUNCH_CHECK();
     const float rej2 = p.rejectDist * p.rejectDist;
     const float sc2  = p.scoreDist * p.scoreDist;
     const bool tree = sc.tree != nullptr;
-    auto inliers = [&](const float4 *src, int n) {
-        const dim3 g(std::max(1, nblocks(n, kW)), ncand);
+    auto inliers = [&](const float4 *src, int n, int last) {
+        const int g = wave(c, (long long)ncand * n, tree ? 3 : 6);
         if (tree)
-            launch_chained(c, k_inliers<true>, g, kT, 0, w, src, n, sc.full.view(), sc2,
+            launch_chained(c, k_inliers<true>, g, kT, 0, w, src, n, last, sc.full.view(), sc2,
                            sc.tree->view(nullptr, sc.pos, nullptr, sc.tpF), sc.tree->m,
                            (const int *)sc.tree->treePos, sc.exc + 2);
         else
-            launch_chained(c, k_inliers<false>, g, kT, 0, w, src, n, sc.full.view(), sc2,
+            launch_chained(c, k_inliers<false>, g, kT, 0, w, src, n, last, sc.full.view(), sc2,
                            smk::KdView{}, 0, (const int *)nullptr, (const float *)nullptr);
     };
     if (p.sparse) {
-        Stage s{m.sp, m.sn, m.ns, nblocks(m.ns, kT), sc.sampled.view(), sc.posS, sc.nrmS, sc.sampled.m, 5,
+        Stage s{m.sp, m.sn, m.ns, sc.sampled.view(), sc.posS, sc.nrmS, sc.sampled.m, sparseIters,
                 p.sampleStep * 0.5f, p.sampleStep, rej2, 0};
         if (tree) {
             s.tree   = sc.tree->view(sc.ioiS, sc.pos, sc.neS, sc.tpS);
@@ -687,14 +763,14 @@ void icp_all(Ctx &c, const Model &m, const IcpScene &sc, const IcpParams &p, con
             s.tposOf = sc.tposS;
             s.exc    = sc.exc;
         }
-        run_stage(c, w, s, ncand);
-        launch_chained(c, k_stage_end, nblocks(ncand, 128), 128, 0, w, ncand, 2);
-        inliers(m.sp, m.ns);
+        run_stage(c, w, s);
+        launch_chained(c, k_stage_end, nblocks(ncand, 128), 128, 0, w, sparseLast, 2);
+        inliers(m.sp, m.ns, sparseLast);
         launch_chained(c, k_score, nblocks(ncand, 128), 128, 0, w, ncand, m.ns, p.minScore, 3,
                        0);
         if (p.dense) {
-            Stage d{m.rp, m.rn, m.nr, nblocks(m.nr, kT), sc.resampled.view(), sc.posR, sc.nrmR,
-                    sc.resampled.m, p.denseSteps, p.reSampleStep * 0.5f, p.sampleStep, rej2, 1};
+            Stage d{m.rp, m.rn, m.nr, sc.resampled.view(), sc.posR, sc.nrmR, sc.resampled.m,
+                    p.denseSteps, p.reSampleStep * 0.5f, p.sampleStep, rej2, 1};
             if (tree) {
                 d.tree   = sc.tree->view(sc.ioiR, sc.pos, sc.neR, sc.tpR);
                 d.treeM  = sc.tree->m;
@@ -702,9 +778,11 @@ void icp_all(Ctx &c, const Model &m, const IcpScene &sc, const IcpParams &p, con
                 d.tposOf = sc.tposR;
                 d.exc    = sc.exc + 1;
             }
-            run_stage(c, w, d, ncand);
-            launch_chained(c, k_stage_end, nblocks(ncand, 128), 128, 0, w, ncand, 4);
-            inliers(m.rp, m.nr);
+            w.cnt += sparseLast + 1;
+            w.list += (size_t)(sparseLast + 1) * ncand;
+            run_stage(c, w, d);
+            launch_chained(c, k_stage_end, nblocks(ncand, 128), 128, 0, w, denseLast, 4);
+            inliers(m.rp, m.nr, denseLast);
             launch_chained(c, k_score, nblocks(ncand, 128), 128, 0, w, ncand, m.nr, p.minScore,
                            5, 1);
         }

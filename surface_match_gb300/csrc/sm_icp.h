@@ -139,22 +139,6 @@ SM_HD Pose34 solve_step(const float sys[kNumSystem], const float Pm[3], const fl
     return step_pose(u, Pm, Qm);
 }
 
-#if defined(__CUDACC__)
-// solve_step by one warp (every lane calls it and gets the pose): the Cholesky factorisation
-// runs one row per lane (sml::cholesky6_warp); identical results.
-__device__ __forceinline__ Pose34 solve_step_warp(const float sys[kNumSystem], const float Pm[3],
-                                                  const float Qm[3]) {
-    double A[6][6], r[6], u[6];
-    system_matrix(sys, A, r);
-    if (!sml::cholesky6_warp(A, r, u)) {
-        double A2[6][6], r2[6];
-        system_matrix(sys, A2, r2);
-        sml::pinv6(A2, r2, u);
-    }
-    return step_pose(u, Pm, Qm);
-}
-#endif
-
 SM_HD Pose34 step_pose(const double u[6], const float Pm[3], const float Qm[3]) {
     const double an = sml::dsqrt(u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
     const double h  = sml::dsqrt(1.0 + an * an);
@@ -198,6 +182,72 @@ SM_HD Pose34 step_pose(const double u[6], const float Pm[3], const float Qm[3]) 
     }
     return o;
 }
+
+#if defined(__CUDACC__)
+// solve_step by one warp (every lane calls it), the pose written to out[12]: the Cholesky
+// factorisation runs one row per lane (sml::cholesky6_warp), the rotation one entry per lane
+// and the translation one row per lane. An FP64 warp instruction costs the same for one lane as
+// for 32, so 18 entries one after the other by every lane cost 18 times as much. Identical
+// results.
+__device__ __forceinline__ void solve_step_warp(const float sys[kNumSystem], const float Pm[3],
+                                                const float Qm[3], float *out) {
+    const int lane = threadIdx.x & 31;
+    double    A[6][6], r[6], u[6];
+    system_matrix(sys, A, r);
+    if (!sml::cholesky6_warp(A, r, u)) {
+        double A2[6][6], r2[6];
+        system_matrix(sys, A2, r2);
+        sml::pinv6(A2, r2, u);
+    }
+    const double an = sml::dsqrt(u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
+    const double h  = sml::dsqrt(1.0 + an * an);
+    const double cs = 1.0 / h, sn = an * cs;
+    double       a[3] = {0.0, 0.0, 0.0};
+    if (an > 0.0) {
+        const double ia = 1.0 / an;
+        a[0]            = u[0] * ia;
+        a[1]            = u[1] * ia;
+        a[2]            = u[2] * ia;
+    }
+    const double aa = a[0] * a[0] + a[1] * a[1] + a[2] * a[2];
+    const double s1 = sn, c1 = 1.0 - cs, s2 = 2.0 * sn * cs, c2 = 2.0 * sn * sn;
+    // lane e < 9: entry (i, j) of R_i and R as in step_pose
+    const int    e  = lane < 9 ? lane : 0;
+    const int    i = e / 3, j = e % 3;
+    const double ai = i == 0 ? a[0] : i == 1 ? a[1] : a[2];
+    const double aj = j == 0 ? a[0] : j == 1 ? a[1] : a[2];
+    // W = [a]x: +-a[k] for the third axis k, + where (i, j) follows (k) cyclically backwards
+    const int    k  = 3 - i - j;
+    const double ak = k == 0 ? a[0] : k == 1 ? a[1] : a[2];
+    const double W  = i == j ? 0.0 : ((j - i == 1 || j - i == -2) ? -ak : ak);
+    const double w2 = ai * aj - (i == j ? aa : 0.0);
+    const double id = i == j ? 1.0 : 0.0;
+    const double Ri = id + s1 * W + c1 * w2;
+    const double R  = id + s2 * W + c2 * w2;
+    if (lane < 9)
+        out[i * 4 + j] = (float)R;
+    // lane l < 3: row l of the translation
+    const int l = lane < 3 ? lane : 0;
+    double    t = 0.0;
+    for (int m = 0; m < 3; m++) {
+        const double Rm  = __shfl_sync(0xffffffffu, R, 3 * l + m);
+        const double Rim = __shfl_sync(0xffffffffu, Ri, 3 * l + m);
+        t += Rm * (-(double)Pm[m]) + Rim * (cs * u[3 + m]);
+    }
+    t += l == 0 ? (double)Qm[0] : l == 1 ? (double)Qm[1] : (double)Qm[2];
+    if (lane < 3)
+        out[l * 4 + 3] = (float)t;
+}
+
+// Entry e < 12 of pose_mul(a, b).
+__device__ __forceinline__ float pose_mul_entry(const float *a, const float *b, int e) {
+    const int i = e / 4, j = e % 4;
+    double    s = (j == 3) ? (double)a[i * 4 + 3] : 0.0;
+    for (int k = 0; k < 3; k++)
+        s += (double)a[i * 4 + k] * (double)b[k * 4 + j];
+    return (float)s;
+}
+#endif
 
 // Pose record of one voting candidate: T (3x4), quaternion (w,x,y,z), rotation angle,
 // votes -- 18 floats, the layout of the pose list.

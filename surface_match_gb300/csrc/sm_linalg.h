@@ -418,66 +418,73 @@ SML_HD bool cholesky6(const double A[6][6], const double r[6], double u[6]) {
 
 #if defined(__CUDACC__)
 // cholesky6 by one warp, one row per lane (lanes 0-5; every lane calls it): per column the
-// pivot's square root, then all rows' updates and divisions at once; the triangular solves
-// column by column. Each element sees the same operations in the same order as cholesky6,
-// so the results are identical; every lane gets u. Returns false where cholesky6 does.
+// pivot's square root and reciprocal, the column, and at once its products out of all later
+// columns of the row (an element sees the same operations in the same order as in cholesky6,
+// so the results are identical, but the subtractions of a pivot are not left for the moment
+// it is needed). Each lane also keeps its column of L (the broadcasts of the update), so that
+// the back substitution needs no transpose. Every lane gets u. Returns false where cholesky6
+// does.
 __device__ __forceinline__ bool cholesky6_warp(const double A[6][6], const double r[6], double u[6]) {
     const int lane = threadIdx.x & 31;
     const int row  = lane < 6 ? lane : 5;
-    double    Lr[6]; // row `row` of L
-    double    inv  = 0.0; // 1 / L[row][row]
+    double    a[6], Lr[6], Lc[6]; // what is left of row `row` of A; row and column `row` of L
+    double    inv  = 0.0;         // 1 / L[row][row]
     double    dmax = 0.0;
     SML_UNROLL
-    for (int i = 0; i < 6; i++)
+    for (int i = 0; i < 6; i++) {
         dmax = A[i][i] > dmax ? A[i][i] : dmax;
+        Lc[i] = 0.0;
+    }
     if (!(dmax > 0.0))
         return false;
     SML_UNROLL
     for (int j = 0; j < 6; j++) {
-        // the pivot row j: s = A[j][j] - sum_k L[j][k]^2 (lane j), broadcast
-        double s = A[j][j];
+        double v = A[0][j];
         SML_UNROLL
-        for (int k = 0; k < j; k++) {
-            const double ljk = __shfl_sync(0xffffffffu, Lr[k], j);
-            s -= ljk * ljk;
-        }
+        for (int i = 1; i < 6; i++)
+            v = row == i ? A[i][j] : v;
+        a[j] = v;
+    }
+    SML_UNROLL
+    for (int j = 0; j < 6; j++) {
+        const double s = __shfl_sync(0xffffffffu, a[j], j);
         if (!(s > dmax * 1e-13))
             return false;
         const double ljj  = dsqrt(s);
         const double invj = 1.0 / ljj;
         if (row == j)
             inv = invj;
-        // rows i > j: t = A[i][j] - sum_k L[i][k] L[j][k], L[i][j] = t * (1 / L[j][j])
-        double t = A[row][j];
+        const double l = row == j ? ljj : (row > j ? a[j] * invj : 0.0);
+        Lr[j]          = l;
         SML_UNROLL
-        for (int k = 0; k < j; k++)
-            t -= Lr[k] * __shfl_sync(0xffffffffu, Lr[k], j);
-        Lr[j] = row == j ? ljj : (row > j ? t * invj : 0.0);
+        for (int i = j + 1; i < 6; i++) {
+            const double lij = __shfl_sync(0xffffffffu, l, i);
+            a[i] -= l * lij;
+            if (row == j)
+                Lc[i] = lij;
+        }
     }
     // forward: y_i = (r_i - sum_{k<i} L[i][k] y_k) * (1 / L[i][i]), column by column
-    double ti = r[row], y[6];
+    double ti = r[0], yr = 0.0;
+    SML_UNROLL
+    for (int i = 1; i < 6; i++)
+        ti = row == i ? r[i] : ti;
     SML_UNROLL
     for (int k = 0; k < 6; k++) {
         const double yk = __shfl_sync(0xffffffffu, ti * inv, k);
-        y[k]            = yk;
+        if (row == k)
+            yr = yk;
         if (row > k)
             ti -= Lr[k] * yk;
     }
-    // back: u_i = (y_i - sum_{k>i, descending} L[k][i] u_k) * (1 / L[i][i]); L[k][i] is row k's
-    double tb = y[row];
+    // back: u_i = (y_i - sum_{k>i, descending} L[k][i] u_k) * (1 / L[i][i])
+    double tb = yr;
     SML_UNROLL
     for (int k = 5; k >= 0; k--) {
-        const double uk  = __shfl_sync(0xffffffffu, tb * inv, k);
-        u[k]             = uk;
-        double lki = 0.0; // L[k][row] held by lane k
-        SML_UNROLL
-        for (int i = 0; i < 6; i++) {
-            const double v = __shfl_sync(0xffffffffu, Lr[i], k);
-            if (i == row)
-                lki = v;
-        }
+        const double uk = __shfl_sync(0xffffffffu, tb * inv, k);
+        u[k]            = uk;
         if (row < k)
-            tb -= lki * uk;
+            tb -= Lc[k] * uk;
     }
     return true;
 }

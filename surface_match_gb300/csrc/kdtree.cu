@@ -954,41 +954,38 @@ __global__ void k_kd_knn(KdView t, const float4 *__restrict__ qpos, const int *_
     kd_knn_query(t, q, k, nbr + (size_t)i * k, dist + (size_t)i * k, nullptr, err);
 }
 
-// One query per warp, the point list[t], answered on the grid of the tree's points
-// (sm_kdgrid.cuh). With smoothing, neighbours that still need a normal are marked.
+// One query per warp over part `part` of a normal estimation's list, answered on the grid of the
+// tree's points (sm_kdgrid.cuh); as k_knn (prep.cu).
 constexpr int kKnnBs = 256;
 __global__ void __launch_bounds__(kKnnBs)
-    k_kd_knn_grid(KdView t, int m, HGridView g, const int *__restrict__ treePos,
-                  const int *__restrict__ list, const int *__restrict__ nq, int k,
-                  int *__restrict__ nbr, int *__restrict__ cnt, int *__restrict__ err,
-                  const float4 *__restrict__ nrm, int *__restrict__ need) {
+    k_kd_knn_grid(KdView t, int m, HGridView g, const int *__restrict__ treePos, NormalList L,
+                  int part, int k, bool grow, int *__restrict__ err,
+                  const float4 *__restrict__ nrm) {
     const int lane = threadIdx.x & 31;
-    const int i    = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (i >= *nq)
+    const int i    = L.begin(part) +
+                  (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (i >= L.end(part))
         return;
-    const float4 p = t.pos[list[i]];
+    const float4 p = t.pos[L.list[i]];
     int          id;
-    int          n = smk::warp_kd_knearest(t, m, g, treePos, p.x, p.y, p.z, k, &id);
-    int         *L = nbr + (size_t)i * k;
+    int          n   = smk::warp_kd_knearest(t, m, g, treePos, p.x, p.y, p.z, k, &id);
+    int         *out = L.nbr + (size_t)i * k;
     if (n < 0) {
         if (lane == 0) {
             const float q[3] = {p.x, p.y, p.z};
-            kd_knn_query(t, q, k, L, nullptr, cnt + i, err);
+            kd_knn_query(t, q, k, out, nullptr, L.nbrCnt + i, err);
         }
         __syncwarp();
-        n  = cnt[i];
-        id = lane < n ? L[lane] : -1;
+        n  = L.nbrCnt[i];
+        id = lane < n ? out[lane] : -1;
     } else {
         if (lane < k)
-            L[lane] = lane < n ? id : -1;
+            out[lane] = lane < n ? id : -1;
         if (lane == 0)
-            cnt[i] = n;
+            L.nbrCnt[i] = n;
     }
-    if (need && lane < n && need[id] == 0) {
-        const float4 v = nrm[id];
-        if (!(isfinite(v.x) && isfinite(v.y) && isfinite(v.z)))
-            need[id] = 1;
-    }
+    if (grow)
+        L.add_neighbour(lane < n, id, nrm);
 }
 
 // ---- the voting stage's radius searches (ppf.cpp:273-276) -------------------------------
@@ -1354,15 +1351,15 @@ void kd_knn(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
     SM_LAUNCH_CHECK();
 }
 
-void kd_knn_points(Ctx &c, const KdTree &T, const HGrid &g, const float4 *pos, const int *list,
-                   const int *nq, int nqMax, int k, int *nbr, int *cnt, const float4 *nrm,
-                   int *need) {
+void kd_knn_points(Ctx &c, const KdTree &T, const HGrid &g, const float4 *pos,
+                   const smd::NormalList &L, int part, int nqMax, int k, bool grow,
+                   const float4 *nrm) {
     if (nqMax <= 0 || T.m <= 0)
         return;
     int *err = c.arena.get<int>("kd.knn.err", 1);
     SM_CUDA(cudaMemsetAsync(err, 0, sizeof(int), c.stream));
     k_kd_knn_grid<<<nblocks((long long)nqMax * 32, kKnnBs), kKnnBs, 0, c.stream>>>(
-        T.view(nullptr, pos), T.m, g.view(), T.treePos, list, nq, k, nbr, cnt, err, nrm, need);
+        T.view(nullptr, pos), T.m, g.view(), T.treePos, L, part, k, grow, err, nrm);
     SM_LAUNCH_CHECK();
 }
 

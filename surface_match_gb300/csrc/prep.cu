@@ -695,48 +695,42 @@ __global__ void __launch_bounds__(kSpWarps * 32)
 
 // ---------------------------------------------------------------------------------------
 __global__ void k_mark_todo(const int *__restrict__ ids, int m, const float4 *__restrict__ nrm,
-                            int *__restrict__ need) {
+                            NormalList L) {
     chain_enter(); // launched chained
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m)
-        return;
-    const int id = ids[i];
-    if (!finite3(nrm[id].x, nrm[id].y, nrm[id].z))
-        need[id] = 2;
+    const int i   = blockIdx.x * blockDim.x + threadIdx.x;
+    const int id  = i < m ? ids[i] : 0;
+    bool      add = false;
+    if (i < m) {
+        const float4 n = nrm[id];
+        add            = !finite3(n.x, n.y, n.z);
+        if (add)
+            atomicOr(&L.seen[id >> 5], 1u << (id & 31));
+    }
+    warp_append(add, id, L.list, L.count);
 }
 
-// One warp per query (exact k nearest neighbours, sm_device.cuh warp_knn_sorted); lane j
-// writes the j-th neighbour, and with smoothing marks it when it still needs a normal.
+// One warp per query (exact k nearest neighbours, sm_device.cuh warp_knn_sorted) of part `part`
+// of the list; lane j writes the j-th neighbour, and with `grow` lists it when it still needs a
+// normal.
 __global__ void __launch_bounds__(256, 6)
-    k_knn(const int *__restrict__ list, const int *__restrict__ nlp, HGridView G, const float4 *__restrict__ pos,
-                      int k, int *__restrict__ nbr, int *__restrict__ nbrCnt, int markNeighbours,
-                      const float4 *__restrict__ nrm, int *__restrict__ need) {
+    k_knn(NormalList L, int part, HGridView G, const float4 *__restrict__ pos, int k, bool grow,
+          const float4 *__restrict__ nrm) {
     chain_enter(); // launched chained
-    const int nl = *nlp; // device-side count of the list
     const int lane = threadIdx.x & 31;
-    const int t    = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (t >= nl)
+    const int t    = L.begin(part) +
+                  (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (t >= L.end(part))
         return;
-    const float4 q = pos[list[t]];
+    const float4 q = pos[L.list[t]];
     int          id;
     float        d;
     const int    n = warp_knn_sorted(G, q.x, q.y, q.z, k, &id, &d);
     if (lane < k)
-        nbr[(size_t)t * k + lane] = lane < n ? id : -1;
+        L.nbr[(size_t)t * k + lane] = lane < n ? id : -1;
     if (lane == 0)
-        nbrCnt[t] = n;
-    if (markNeighbours && lane < n && need[id] == 0 && !finite3(nrm[id].x, nrm[id].y, nrm[id].z))
-        need[id] = 1;
-}
-
-// list[0 .. *nlp) on the device; nlMax bounds it for the launch.
-void launch_knn(const Ctx &c, const int *list, const int *nlp, int nlMax, const HGridView &G,
-                const float4 *pos, int k, int *nbr, int *cnt, int mark, const float4 *nrm,
-                int *need) {
-    if (nlMax <= 0)
-        return;
-    launch_chained(c, k_knn, nblocks((long long)nlMax * 32, 256), 256, 0, list, nlp, G, pos, k, nbr,
-                   cnt, mark, nrm, need);
+        L.nbrCnt[t] = n;
+    if (grow)
+        L.add_neighbour(lane < n, id, nrm);
 }
 
 // ---- hashed grid build -----------------------------------------------------------------
@@ -812,16 +806,7 @@ __global__ void k_hg_pack_from_start(const unsigned long long *__restrict__ keys
         dense[k] = make_int2(start[t], (int)cnt);
 }
 
-// Query lists in the query grid's cell order: a warp then searches 32 neighbouring queries
-// (similar cells, shared cache lines, little divergence). flags[k] = need[gids[k]] == eq.
-__global__ void k_flags_grid_order(const int *__restrict__ gids, int m, const int *__restrict__ need,
-                                   int eq, int *__restrict__ flags) {
-    chain_enter(); // launched chained
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < m)
-        flags[i] = need[gids[i]] == eq ? 1 : 0;
-}
-
+// out[pre[i]] = gids[i] where flags[i] != 0
 __global__ void k_scatter_ids(const int *__restrict__ flags, const int *__restrict__ pre, int n,
                               const int *__restrict__ gids, int *__restrict__ out) {
     chain_enter(); // launched chained
@@ -830,17 +815,16 @@ __global__ void k_scatter_ids(const int *__restrict__ flags, const int *__restri
         out[pre[i]] = gids[i];
 }
 
-// Phase A: centroid and FP32-Kahan covariance of the neighbourhood, FP64 eigensolve.
-__global__ void k_pca(const int *__restrict__ list, const int *__restrict__ nlp, const int *__restrict__ nbr,
-                      const int *__restrict__ nbrCnt, int k, const float4 *__restrict__ pos,
-                      float4 *__restrict__ cen, float4 *__restrict__ nout) {
+// Phase A: centroid and FP32-Kahan covariance of the neighbourhood, FP64 eigensolve, for the
+// whole list.
+__global__ void k_pca(NormalList L, int k, const float4 *__restrict__ pos, float4 *__restrict__ cen,
+                      float4 *__restrict__ nout) {
     chain_enter(); // launched chained
-    const int nl = *nlp; // device-side count of the list
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nl)
+    if (t >= L.end(1))
         return;
-    const int  m = nbrCnt[t];
-    const int *L = nbr + (size_t)t * k;
+    const int  m = L.nbrCnt[t];
+    const int *N = L.nbr + (size_t)t * k;
     if (m < 3) {
         cen[t]  = make_float4(0.f, 0.f, 0.f, -1.0f); // w < 0: no estimate
         nout[t] = make_float4(0.f, 0.f, 0.f, -1.0f);
@@ -851,7 +835,7 @@ __global__ void k_pca(const int *__restrict__ list, const int *__restrict__ nlp,
     sy.init();
     sz.init();
     for (int j = 0; j < m; j++) {
-        const float4 p = pos[L[j]];
+        const float4 p = pos[N[j]];
         sx.add(p.x);
         sy.add(p.y);
         sz.add(p.z);
@@ -862,7 +846,7 @@ __global__ void k_pca(const int *__restrict__ list, const int *__restrict__ nlp,
     for (int e = 0; e < 6; e++)
         a[e].init();
     for (int j = 0; j < m; j++) {
-        const float4 p  = pos[L[j]];
+        const float4 p  = pos[N[j]];
         const float  dx = p.x - cx, dy = p.y - cy, dz = p.z - cz;
         a[0].add(dx * dx);
         a[1].add(dx * dy);
@@ -880,37 +864,35 @@ __global__ void k_pca(const int *__restrict__ list, const int *__restrict__ nlp,
     nout[t] = make_float4(n3[0], n3[1], n3[2], 1.0f);
 }
 
-__global__ void k_pca_write(const int *__restrict__ list, const int *__restrict__ nlp, const float4 *__restrict__ cen,
+__global__ void k_pca_write(NormalList L, const float4 *__restrict__ cen,
                             const float4 *__restrict__ nin, float4 *__restrict__ pos,
                             float4 *__restrict__ nrm) {
     chain_enter(); // launched chained
-    const int nl = *nlp; // device-side count of the list
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nl || cen[t].w < 0.0f)
+    if (t >= L.end(1) || cen[t].w < 0.0f)
         return;
-    const int id = list[t];
+    const int id = L.list[t];
     pos[id]      = make_float4(cen[t].x, cen[t].y, cen[t].z, 0.0f);
     nrm[id]      = make_float4(nin[t].x, nin[t].y, nin[t].z, 0.0f);
 }
 
-// Phase B: sign-aligned sum of the raw neighbourhood normals (util.cpp:292-306).
-__global__ void k_smooth(const int *__restrict__ list, const int *__restrict__ nlp, const int *__restrict__ nbr,
-                         const int *__restrict__ nbrCnt, int k, const float4 *__restrict__ nrm,
+// Phase B: sign-aligned sum of the raw neighbourhood normals (util.cpp:292-306) of the points
+// to estimate.
+__global__ void k_smooth(NormalList L, int k, const float4 *__restrict__ nrm,
                          float4 *__restrict__ out) {
     chain_enter(); // launched chained
-    const int nl = *nlp; // device-side count of the list
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nl)
+    if (t >= L.end(0))
         return;
-    const int m = nbrCnt[t];
+    const int m = L.nbrCnt[t];
     if (m < 3) {
         out[t] = make_float4(0.f, 0.f, 0.f, -1.0f);
         return;
     }
-    const float4 n0 = nrm[list[t]];
+    const float4 n0 = nrm[L.list[t]];
     float        sx = 0.f, sy = 0.f, sz = 0.f;
     for (int j = 0; j < m; j++) {
-        const float4 n = nrm[nbr[(size_t)t * k + j]];
+        const float4 n = nrm[L.nbr[(size_t)t * k + j]];
         const float  d = n.x * n0.x + (n.y * n0.y + n.z * n0.z);
         if (d > 0.0f) {
             sx = sx + n.x;
@@ -932,14 +914,13 @@ __global__ void k_smooth(const int *__restrict__ list, const int *__restrict__ n
     out[t] = make_float4(sx, sy, sz, 1.0f);
 }
 
-__global__ void k_smooth_write(const int *__restrict__ list, const int *__restrict__ nlp, const float4 *__restrict__ sm,
+__global__ void k_smooth_write(NormalList L, const float4 *__restrict__ sm,
                                float4 *__restrict__ nrm) {
     chain_enter(); // launched chained
-    const int nl = *nlp; // device-side count of the list
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nl || sm[t].w < 0.0f)
+    if (t >= L.end(0) || sm[t].w < 0.0f)
         return;
-    nrm[list[t]] = make_float4(sm[t].x, sm[t].y, sm[t].z, 0.0f);
+    nrm[L.list[t]] = make_float4(sm[t].x, sm[t].y, sm[t].z, 0.0f);
 }
 
 // Phase C: orientation toward the viewpoint, or +z (util.cpp:309-333).
@@ -1075,24 +1056,6 @@ void compact_known(Ctx &c, const int *flags, int n, int *outIds, const std::stri
     int *pre = c.arena.get<int>(tag + ".pre", n);
     scan_impl(c, flags, pre, n, kNoEq, tag, false);
     launch_chained(c, k_scatter_flags, nblocks(n, 256), 256, 0, flags, pre, n, kNoEq, outIds);
-}
-
-// The points p of grid H with need[p] == eq, in H's cell order, into out; returns the device
-// address of their count (no host round trip).
-static int *compact_grid_order(Ctx &c, const HGrid &H, const int *need, int eq, int *out,
-                               const std::string &tag) {
-    int *flags = c.arena.get<int>(tag + ".gf", std::max(H.m, 1));
-    int *pre   = c.arena.get<int>(tag + ".gp", std::max(H.m, 1));
-    if (H.m <= 0) {
-        int *z = c.arena.get<int>(tag + ".gz", 1);
-        SM_CUDA(cudaMemsetAsync(z, 0, sizeof(int), c.stream));
-        return z;
-    }
-    launch_chained(c, k_flags_grid_order, nblocks(H.m, 256), 256, 0, H.ids, H.m, need, eq,
-                   flags);
-    int *total = scan_flags_total(c, flags, pre, H.m, tag + ".gc");
-    launch_chained(c, k_scatter_ids, nblocks(H.m, 256), 256, 0, flags, pre, H.m, H.ids, out);
-    return total;
 }
 
 void build_hgrid(Ctx &c, const float4 *pos, const int *ids, int m, const Box &box, float g,
@@ -1273,52 +1236,38 @@ void estimate_normals(Ctx &c, float4 *pos, float4 *nrm, int npoints, const int *
         k = 3;
     if (k > kMaxKnn)
         throw Error(SM_ERR_RANGE, "knnNormal larger than " + std::to_string(kMaxKnn) + " is not supported");
-    int *need = c.arena.get<int>(tag + ".need", npoints);
-    FillSet clear;
-    clear.add(need, (size_t)npoints * sizeof(int), 0u);
-    fill(c, clear);
-    launch_chained(c, k_mark_todo, nblocks(m, 256), 256, 0, ids, m, nrm, need);
-    // the query lists and their counts stay on the device; launches are sized by bounds
-    int       *todo   = c.arena.get<int>(tag + ".todo", std::max(m, 1));
-    const int *ntodo  = compact_grid_order(c, query, need, 2, todo, tag + ".ct");
-    int       *nbrT   = c.arena.get<int>(tag + ".nbrT", (size_t)m * k);
-    int       *cntT   = c.arena.get<int>(tag + ".cntT", m);
-    if (tree)
-        kd_knn_points(c, *tree, query, pos, todo, ntodo, m, k, nbrT, cntT, nrm,
-                      smooth ? need : nullptr);
-    else
-        launch_knn(c, todo, ntodo, m, query.view(), pos, k, nbrT, cntT, smooth ? 1 : 0, nrm, need);
+    // the list and its counts stay on the device; launches are sized by bounds
     const int  extraMax = smooth ? (int)std::min<long long>(npoints, (long long)m * k) : 0;
-    int       *extra = nullptr, *nbrE = nullptr, *cntE = nullptr;
-    const int *nextra = nullptr;
-    if (extraMax > 0) {
-        extra  = c.arena.get<int>(tag + ".extra", std::max(extraMax, 1));
-        nextra = compact_grid_order(c, query, need, 1, extra, tag + ".ce");
-        nbrE   = c.arena.get<int>(tag + ".nbrE", (size_t)extraMax * k);
-        cntE   = c.arena.get<int>(tag + ".cntE", extraMax);
+    const long long most = (long long)m + extraMax;
+    NormalList L;
+    L.list   = c.arena.get<int>(tag + ".list", (size_t)most);
+    L.seen   = c.arena.get<uint32_t>(tag + ".seen", ((size_t)npoints + 31) / 32);
+    L.count  = c.arena.get<int>(tag + ".count", 2);
+    L.nbr    = c.arena.get<int>(tag + ".nbr", (size_t)most * k);
+    L.nbrCnt = c.arena.get<int>(tag + ".nbrCnt", (size_t)most);
+    FillSet clear;
+    clear.add(L.seen, ((size_t)npoints + 31) / 32 * 4, 0u);
+    clear.add(L.count, 2 * sizeof(int), 0u);
+    fill(c, clear);
+    launch_chained(c, k_mark_todo, nblocks(m, 256), 256, 0, ids, m, nrm, L);
+    // with the reference's k-d tree the k nearest are those its depth-first search finds
+    // (ties: first found)
+    for (int part = 0; part < (extraMax > 0 ? 2 : 1); part++) {
+        const int  nq   = part ? extraMax : m;
+        const bool grow = part == 0 && smooth;
         if (tree)
-            kd_knn_points(c, *tree, query, pos, extra, nextra, extraMax, k, nbrE, cntE, nrm, nullptr);
+            kd_knn_points(c, *tree, query, pos, L, part, nq, k, grow, nrm);
         else
-            launch_knn(c, extra, nextra, extraMax, query.view(), pos, k, nbrE, cntE, 0, nrm, need);
+            launch_chained(c, k_knn, nblocks((long long)nq * 32, 256), 256, 0, L, part,
+                           query.view(), pos, k, grow, nrm);
     }
-    const int nmax = std::max(m, extraMax);
-    float4   *cen  = c.arena.get<float4>(tag + ".cen", 2 * (size_t)nmax);
-    float4   *nn   = c.arena.get<float4>(tag + ".nn", 2 * (size_t)nmax);
-    launch_chained(c, k_pca, nblocks(m, 128), 128, 0, todo, ntodo, nbrT, cntT, k, pos, cen,
-                   nn);
-    if (extraMax > 0) {
-        launch_chained(c, k_pca, nblocks(extraMax, 128), 128, 0, extra, nextra, nbrE, cntE, k,
-                       pos, cen + nmax, nn + nmax);
-    }
-    launch_chained(c, k_pca_write, nblocks(m, 256), 256, 0, todo, ntodo, cen, nn, pos, nrm);
-    if (extraMax > 0) {
-        launch_chained(c, k_pca_write, nblocks(extraMax, 256), 256, 0, extra, nextra,
-                       cen + nmax, nn + nmax, pos, nrm);
-    }
+    float4 *cen = c.arena.get<float4>(tag + ".cen", (size_t)most);
+    float4 *nn  = c.arena.get<float4>(tag + ".nn", (size_t)most);
+    launch_chained(c, k_pca, nblocks(most, 128), 128, 0, L, k, pos, cen, nn);
+    launch_chained(c, k_pca_write, nblocks(most, 256), 256, 0, L, cen, nn, pos, nrm);
     if (smooth) {
-        launch_chained(c, k_smooth, nblocks(m, 256), 256, 0, todo, ntodo, nbrT, cntT, k, nrm,
-                       cen);
-        launch_chained(c, k_smooth_write, nblocks(m, 256), 256, 0, todo, ntodo, cen, nrm);
+        launch_chained(c, k_smooth, nblocks(m, 256), 256, 0, L, k, nrm, cen);
+        launch_chained(c, k_smooth_write, nblocks(m, 256), 256, 0, L, cen, nrm);
     }
     const bool hasVp = vp && std::isfinite(vp[0]) && std::isfinite(vp[1]) && std::isfinite(vp[2]);
     launch_chained(c, k_orient, nblocks(m, 256), 256, 0, ids, m, pos, nrm, hasVp ? 1 : 0,

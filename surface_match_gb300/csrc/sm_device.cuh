@@ -95,6 +95,45 @@ __device__ __forceinline__ int warp_incl_scan(int v) {
     return v;
 }
 
+// list[*count ..] += v for the lanes with add set, a warp's at once (any order between warps).
+__device__ __forceinline__ void warp_append(bool add, int v, int *__restrict__ list,
+                                            int *__restrict__ count) {
+    const unsigned m = __ballot_sync(0xffffffffu, add);
+    if (!m)
+        return;
+    const int lane = threadIdx.x & 31;
+    int       base = 0;
+    if (lane == 0)
+        base = atomicAdd(count, __popc(m));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (add)
+        list[base + __popc(m & ((1u << lane) - 1u))] = v;
+}
+
+// The query list of a normal estimation: part 0, the points to estimate, then (with smoothing)
+// part 1, their neighbours without a normal. Points are appended as they are found; the order
+// within a part does not matter, as every result belongs to one point. `seen` holds a bit per
+// listed point. (Flags over all points with a scan and a scatter per part, in grid order, took
+// six launches and 56 us of the 470 us that the large scene's first normals and sampling took.)
+struct NormalList {
+    int      *list, *count; // count[p]: points of part p
+    uint32_t *seen;
+    int      *nbr, *nbrCnt; // per listed point: its k nearest (-1 beyond their count)
+    __device__ __forceinline__ int begin(int part) const { return part ? count[0] : 0; }
+    __device__ __forceinline__ int end(int part) const { return part ? count[0] + count[1] : count[0]; }
+    // a warp of part 0: lists neighbour `id` of each lane in part 1 if it has no normal yet
+    __device__ __forceinline__ void add_neighbour(bool valid, int id,
+                                                  const float4 *__restrict__ nrm) const {
+        bool add = false;
+        if (valid && !((*(const volatile uint32_t *)&seen[id >> 5] >> (id & 31)) & 1u)) {
+            const float4 n = nrm[id];
+            if (!(isfinite(n.x) && isfinite(n.y) && isfinite(n.z)))
+                add = !((atomicOr(&seen[id >> 5], 1u << (id & 31)) >> (id & 31)) & 1u);
+        }
+        warp_append(add, id, list + count[0], count + 1);
+    }
+};
+
 // Warp minimum of a 64-bit key: the high words' minimum, then the low words' minimum among
 // the lanes that hold it (two single-instruction warp reductions).
 __device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long v) {

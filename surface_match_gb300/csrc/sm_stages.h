@@ -314,11 +314,12 @@ int kd_sample(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
 // its j-th nearest.
 void kd_knn(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
             const float4 *qpos, const int *nq, int nqMax, int k, int *nbr, float *dist);
-// The same for the points list[t] of the whole tree, given a grid of its points at their live
-// positions `pos`; need (nullable): neighbours without a finite normal are marked 1 where 0.
-void kd_knn_points(Ctx &c, const KdTree &T, const HGrid &g, const float4 *pos, const int *list,
-                   const int *nq, int nqMax, int k, int *nbr, int *cnt, const float4 *nrm,
-                   int *need);
+// The same for part `part` (at most nqMax points) of a normal estimation's list, given a grid of
+// the tree's points at their live positions `pos`; grow: neighbours without a finite normal are
+// listed.
+void kd_knn_points(Ctx &c, const KdTree &T, const HGrid &g, const float4 *pos,
+                   const smd::NormalList &L, int part, int nqMax, int k, bool grow,
+                   const float4 *nrm);
 // flags[v] = 1 when node v's subtree holds a position whose vaccActive entry is >= 0
 // (the searches of a reduce()d tree skip the others).
 void kd_mark_nonempty(Ctx &c, const KdTree &T, const int *vaccActive, int *flags);

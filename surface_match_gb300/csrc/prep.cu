@@ -743,8 +743,8 @@ __device__ __forceinline__ unsigned long long hkey(const float4 &p, const GridPa
 }
 
 __global__ void k_hg_insert(const float4 *__restrict__ pos, const int *__restrict__ ids, int m,
-                            GridParams gp, unsigned long long *__restrict__ keys, uint32_t mask,
-                            int *__restrict__ slotOf, int *__restrict__ cnt) {
+                            GridParams gp, uint4 *__restrict__ slot, uint32_t mask,
+                            int2 *__restrict__ place) {
     chain_enter(); // launched chained
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m)
@@ -752,10 +752,11 @@ __global__ void k_hg_insert(const float4 *__restrict__ pos, const int *__restric
     const unsigned long long key = hkey(pos[ids[i]], gp);
     uint32_t                 h   = (uint32_t)smm::mix64(key) & mask;
     for (uint32_t p = 0; p <= mask; p++) {
-        const unsigned long long prev = atomicCAS(&keys[h], ~0ull, key);
+        unsigned long long      *k    = reinterpret_cast<unsigned long long *>(&slot[h]);
+        const unsigned long long prev = atomicCAS(k, ~0ull, key);
         if (prev == ~0ull || prev == key) {
-            slotOf[i] = (int)h;
-            atomicAdd(&cnt[h], 1);
+            // (the count starts at all ones: the first point takes place 0)
+            place[i] = make_int2((int)h, (int)(atomicAdd(&slot[h].w, 1u) + 1u));
             return;
         }
         h = (h + 1) & mask;
@@ -763,17 +764,16 @@ __global__ void k_hg_insert(const float4 *__restrict__ pos, const int *__restric
 }
 
 __global__ void k_hg_scatter(const float4 *__restrict__ pos, const int *__restrict__ ids,
-                             const int *__restrict__ slotOf, int m, int *__restrict__ fill,
-                             int *__restrict__ gids, float4 *__restrict__ pts, int wIsRank) {
+                             const uint4 *__restrict__ slot, const int2 *__restrict__ place, int m,
+                             float4 *__restrict__ pts, int wIsRank) {
     chain_enter(); // launched chained
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m)
         return;
     const int    id = ids[i];
     const float4 p  = pos[id];
-    const int    k  = atomicAdd(&fill[slotOf[i]], 1);
-    gids[k]         = id;
-    pts[k]          = make_float4(p.x, p.y, p.z, __int_as_float(wIsRank ? i : id));
+    const int2   at = place[i];
+    pts[slot[at.x].z + at.y] = make_float4(p.x, p.y, p.z, __int_as_float(wIsRank ? i : id));
 }
 
 // Rank-ordered copies of a subset's positions and normals: out[r] = in[ids[r]].
@@ -789,23 +789,6 @@ __global__ void k_gather_subset(const float4 *__restrict__ pos, const float4 *__
     subNrm[r]    = nrm[id];
 }
 
-__global__ void k_hg_pack_from_start(const unsigned long long *__restrict__ keys,
-                                     const int *__restrict__ start, uint32_t T,
-                                     uint4 *__restrict__ slot, uint32_t *__restrict__ occ,
-                                     int2 *__restrict__ dense) {
-    chain_enter(); // launched chained
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= T)
-        return;
-    const unsigned long long k   = keys[t];
-    const uint32_t           cnt = (uint32_t)(start[t + 1] - start[t]);
-    slot[t] = make_uint4((uint32_t)k, (uint32_t)(k >> 32), (uint32_t)start[t], cnt);
-    if (occ && cnt)
-        atomicOr(&occ[k >> 5], 1u << (k & 31));
-    if (dense && cnt)
-        dense[k] = make_int2(start[t], (int)cnt);
-}
-
 // out[pre[i]] = gids[i] where flags[i] != 0
 __global__ void k_scatter_ids(const int *__restrict__ flags, const int *__restrict__ pre, int n,
                               const int *__restrict__ gids, int *__restrict__ out) {
@@ -816,6 +799,34 @@ __global__ void k_scatter_ids(const int *__restrict__ flags, const int *__restri
 }
 
 // Phase A: centroid and FP32-Kahan covariance of the neighbourhood, FP64 eigensolve, for the
+// Ranges of the occupied cells, their occupancy bits and direct-table entries.
+__global__ void __launch_bounds__(256)
+    k_hg_ranges(uint4 *__restrict__ slot, uint32_t T, int *__restrict__ next,
+                uint32_t *__restrict__ occ, int2 *__restrict__ dense) {
+    chain_enter(); // launched chained
+    __shared__ int sh[33];
+    __shared__ int sBase;
+    const uint32_t t   = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint4    v   = t < T ? slot[t] : make_uint4(~0u, ~0u, ~0u, ~0u);
+    const int      cnt = (int)(v.w + 1u);
+    int            tot;
+    const int      ex = block_excl_scan(cnt, sh, &tot);
+    if (tot == 0)
+        return; // (uniform)
+    if (threadIdx.x == 0)
+        sBase = atomicAdd(next, tot);
+    __syncthreads();
+    if (cnt == 0)
+        return;
+    const int                first = sBase + ex;
+    const unsigned long long k     = ((unsigned long long)v.y << 32) | v.x;
+    slot[t].z                      = (uint32_t)first;
+    if (occ)
+        atomicOr(&occ[k >> 5], 1u << (k & 31));
+    if (dense)
+        dense[k] = make_int2(first, cnt);
+}
+
 // whole list.
 __global__ void k_pca(NormalList L, int k, const float4 *__restrict__ pos, float4 *__restrict__ cen,
                       float4 *__restrict__ nout) {
@@ -1077,43 +1088,32 @@ void build_hgrid(Ctx &c, const float4 *pos, const int *ids, int m, const Box &bo
         T <<= 1;
     H.mask = T - 1;
     H.m    = m;
-    auto *keys   = c.arena.get<unsigned long long>(tag + ".keys", T);
-    int  *cnt    = c.arena.get<int>(tag + ".cnt", T + 1);
-    int  *start  = c.arena.get<int>(tag + ".start", T + 1);
-    int  *slotOf = c.arena.get<int>(tag + ".slotOf", std::max(m, 1));
-    H.ids        = c.arena.get<int>(tag + ".ids", std::max(m, 1));
-    H.pts        = c.arena.get<float4>(tag + ".pts", std::max(m, 1));
-    H.slot       = c.arena.get<uint4>(tag + ".slot", T);
+    int  *next  = c.arena.get<int>(tag + ".next", 1);
+    int2 *place = c.arena.get<int2>(tag + ".place", std::max(m, 1));
+    H.pts       = c.arena.get<float4>(tag + ".pts", std::max(m, 1));
+    H.slot      = c.arena.get<uint4>(tag + ".slot", T);
     // occupancy bits over the cell box, when it has at most 2^28 cells (32 MB), and a direct
     // {first, count} table too when it has at most 2^22 cells (32 MB); all cleared with the
-    // key and count tables in one launch
+    // slots and the counter in one launch
     const unsigned long long ncell = (unsigned long long)H.dim[0] * H.dim[1] * H.dim[2];
     const size_t             words = (size_t)((ncell + 31) / 32);
     H.occ   = ncell <= (1ull << 28) ? c.arena.get<uint32_t>(tag + ".occ", words) : nullptr;
     H.dense = ncell <= (1ull << 22) ? c.arena.get<int2>(tag + ".dense", (size_t)ncell) : nullptr;
     FillSet clear;
-    clear.add(keys, (size_t)T * 8, 0xffffffffu);
-    clear.add(cnt, (size_t)(T + 1) * 4, 0u);
+    clear.add(H.slot, (size_t)T * sizeof(uint4), 0xffffffffu);
+    clear.add(next, sizeof(int), 0u);
     if (H.occ)
         clear.add(H.occ, words * 4, 0u);
     if (H.dense)
         clear.add(H.dense, (size_t)ncell * sizeof(int2), 0u);
     fill(c, clear);
-    GridParams gp = grid_params(box, g, H.dim);
-    if (m > 0) {
-        launch_chained(c, k_hg_insert, nblocks(m, 256), 256, 0, pos, ids, m, gp, keys, H.mask,
-                       slotOf, cnt);
-    }
-    scan_excl(c, cnt, start, (long long)T + 1, tag, false);
-    int *fill = cnt;
-    SM_CUDA(cudaMemcpyAsync(fill, start, (size_t)T * 4, cudaMemcpyDeviceToDevice, c.stream));
-    if (m > 0) {
-        launch_chained(c, k_hg_scatter, nblocks(m, 256), 256, 0, pos, ids, slotOf, m, fill,
-                       H.ids, H.pts, wIsRank ? 1 : 0);
-    }
-    // counts again for the packed table: start[t+1] - start[t]
-    launch_chained(c, k_hg_pack_from_start, nblocks(T, 256), 256, 0, keys, start, T, H.slot,
-                   H.occ, H.dense);
+    if (m <= 0)
+        return;
+    const GridParams gp = grid_params(box, g, H.dim);
+    launch_chained(c, k_hg_insert, nblocks(m, 256), 256, 0, pos, ids, m, gp, H.slot, H.mask, place);
+    launch_chained(c, k_hg_ranges, nblocks(T, 256), 256, 0, H.slot, T, next, H.occ, H.dense);
+    launch_chained(c, k_hg_scatter, nblocks(m, 256), 256, 0, pos, ids, H.slot, place, m, H.pts,
+                   wIsRank ? 1 : 0);
 }
 
 void gather_subset(Ctx &c, const float4 *pos, const float4 *nrm, const int *ids, int m,

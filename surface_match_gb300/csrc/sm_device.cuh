@@ -16,8 +16,8 @@ constexpr int kMaxKnn      = 32; // largest supported knnNormal
 constexpr int kKnnMaxShell = 24; // shells a k-nearest walk visits before it scans every point
 
 // Device view of a hashed uniform grid: only occupied cells are stored, in an
-// open-addressed table of uint4 {key low, key high, first point, point count} (count 0 =
-// empty slot), so cells can be as fine as the queries want whatever the scene's extent,
+// open-addressed table of uint4 {key low, key high, first point, point count - 1} (all ones in
+// an empty slot), so cells can be as fine as the queries want whatever the scene's extent,
 // and the table stays small enough to live in L2. The points of a cell are contiguous in
 // `pts` (position, point index in w), so a search reads them without an indirection, and
 // an occupancy bitmap over the cell box lets searches skip empty cells without a probe.
@@ -28,7 +28,6 @@ struct HGridView {
     int           dim[3];
     const uint4  *slot;
     uint32_t      mask;
-    const int    *ids;
     const float4 *pts;
     const uint32_t *occ;   // one bit per cell of the dim box (nullptr: not built)
     const int2     *dense; // {first, count} per cell of the dim box (nullptr: not built)
@@ -42,11 +41,11 @@ struct HGridView {
         uint32_t h = (uint32_t)smm::mix64(key) & mask;
         for (uint32_t p = 0; p <= mask; p++) {
             const uint4 v = slot[h];
-            if (v.w == 0u)
+            if (v.w == 0xffffffffu)
                 break;
             if (v.x == (uint32_t)key && v.y == (uint32_t)(key >> 32)) {
                 s = (int)v.z;
-                e = (int)(v.z + v.w);
+                e = (int)(v.z + v.w + 1u);
                 return;
             }
             h = (h + 1) & mask;

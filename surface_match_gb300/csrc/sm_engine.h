@@ -116,7 +116,6 @@ struct HGrid {
     int       dim[3] = {1, 1, 1};
     uint4    *slot   = nullptr;
     uint32_t  mask   = 0;
-    int      *ids    = nullptr;
     float4   *pts    = nullptr; // positions in cell order, point index in w (bit pattern)
     uint32_t *occ    = nullptr; // occupancy bit per cell (nullptr when the cell box is too large)
     int2     *dense  = nullptr; // {first, count} per cell (nullptr unless the cell box is small)
@@ -130,7 +129,6 @@ struct HGrid {
         v.g    = g;
         v.slot = slot;
         v.mask = mask;
-        v.ids  = ids;
         v.pts  = pts;
         v.occ   = occ;
         v.dense = dense;

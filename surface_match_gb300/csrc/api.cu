@@ -315,7 +315,7 @@ void train(Ctx &c, Model &m, const float *xyzIn, const float *nrmIn, int64_t n64
     if (nvalid == 0)
         throw Error(SM_ERR_RUNTIME, "Invalid Input: empty model in trainModel");
     int *valid = c.arena.get<int>("t.vids", n);
-    compact_known(c, val, n, valid, "t.cv");
+    compact_known(c, val, n, nvalid, valid);
     const float diam         = box.diameter();
     const float sampleStep   = diam * sdRel;
     const float reSampleStep = diam * tp.poseRefRelSamplingDistance;
@@ -471,7 +471,7 @@ void match(Ctx &c, const Model &m, const float *xyzIn, const float *nrmIn, int64
     Box          box;
     const int    nvalid = prep_points(c, xyz, nin, n, pos, nrm, val, box);
     int         *valid  = c.arena.get<int>("m.vids", n);
-    compact_known(c, val, n, valid, "m.cv"); // nvalid points
+    compact_known(c, val, n, nvalid, valid); // nvalid points
     record(c, 1);
     if (nvalid == 0) {
         // no finite point: the reference's search structures are empty and it returns no
@@ -1077,7 +1077,7 @@ SM_API int sm_estimate_normals_mls(sm_context ctx, const float *xyzIn, const flo
         const int nvalid = prep_points(c, xyz, nullptr, n, pos, nrm, val, box);
         if (nvalid > 0 && !ids.empty()) {
             int *valid = c.arena.get<int>("l.vids", n);
-            compact_known(c, val, n, valid, "l.cv");
+            compact_known(c, val, n, nvalid, valid);
             int *dids = c.arena.get<int>("l.ids", ids.size());
             SM_CUDA(cudaMemcpyAsync(dids, ids.data(), ids.size() * 4, cudaMemcpyHostToDevice,
                                     c.stream));
@@ -1113,7 +1113,7 @@ SM_API int sm_kdtree_probe(sm_context ctx, const float *xyzIn, int64_t n64, floa
         Box          box;
         const int    nvalid = prep_points(c, xyz, nullptr, n, pos, nrm, val, box);
         int         *valid  = c.arena.get<int>("kp.vids", n);
-        compact_known(c, val, n, valid, "kp.cv");
+        compact_known(c, val, n, nvalid, valid);
         KdTree T;
         build_kdtree(c, pos, n, valid, nvalid, box, T, "kp.tree");
         if (outVacc) {

@@ -20,7 +20,6 @@ namespace {
 constexpr int kScanBs   = 512;
 constexpr int kScanIpt  = 8;
 constexpr int kScanTile = kScanBs * kScanIpt;
-constexpr int kNoEq     = INT_MIN; // scan raw values instead of (value == eq)
 
 struct GridParams {
     float org[3], g;
@@ -47,9 +46,32 @@ __device__ __forceinline__ bool finite3(float x, float y, float z) {
 }
 
 // ---------------------------------------------------------------------------------------
-__global__ void k_prep(const float *__restrict__ xyz, const float *__restrict__ nin, int n,
-                       float4 *__restrict__ pos, float4 *__restrict__ nrm, int *__restrict__ valid,
-                       int *__restrict__ bbox, int *__restrict__ nvalid) {
+// Three floats of each of the four points 4 g .. 4 g + 3 (below n): three 16-byte loads where the
+// array is aligned to them, else one by one.
+__device__ __forceinline__ void load_points4(const float *__restrict__ a, int g, int n, float v[12]) {
+    const size_t o = 12 * (size_t)g;
+    if (((uintptr_t)a & 15) == 0 && 4 * g + 3 < n) {
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const float4 q = reinterpret_cast<const float4 *>(a + o)[k];
+            v[4 * k]       = q.x;
+            v[4 * k + 1]   = q.y;
+            v[4 * k + 2]   = q.z;
+            v[4 * k + 3]   = q.w;
+        }
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < 12; k++)
+        v[k] = 4 * g + k / 3 < n ? a[o + k] : 0.0f;
+}
+
+// A thread takes four points (0.92 M points: 27.5 us with a point per thread, its three floats
+// loaded one by one, and 2432 CTAs adding to the box).
+__global__ void __launch_bounds__(256)
+    k_prep(const float *__restrict__ xyz, const float *__restrict__ nin, int n,
+           float4 *__restrict__ pos, float4 *__restrict__ nrm, int *__restrict__ valid,
+           int *__restrict__ bbox, int *__restrict__ nvalid) {
     __shared__ int smn[3], smx[3], scnt;
     if (threadIdx.x < 3) {
         smn[threadIdx.x] = INT_MAX;
@@ -59,32 +81,43 @@ __global__ void k_prep(const float *__restrict__ xyz, const float *__restrict__ 
         scnt = 0;
     __syncthreads();
     int lmn[3] = {INT_MAX, INT_MAX, INT_MAX}, lmx[3] = {INT_MIN, INT_MIN, INT_MIN}, lc = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float x = xyz[3 * (size_t)i], y = xyz[3 * (size_t)i + 1], z = xyz[3 * (size_t)i + 2];
-        bool        ok = finite3(x, y, z);
-        float4      nn = nan4();
-        if (nin) {
-            float a = nin[3 * (size_t)i], b = nin[3 * (size_t)i + 1], c = nin[3 * (size_t)i + 2];
-            ok      = ok && finite3(a, b, c);
-            const float sq = a * a + (b * b + c * c);
-            if (sq > 0.0f) {
-                const float s = smm::fsqrt(sq);
-                a             = smm::fdiv(a, s);
-                b             = smm::fdiv(b, s);
-                c             = smm::fdiv(c, s);
+    const int groups = (n + 3) / 4;
+    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < groups; g += gridDim.x * blockDim.x) {
+        float p[12], q[12];
+        load_points4(xyz, g, n, p);
+        if (nin)
+            load_points4(nin, g, n, q);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int i = 4 * g + k;
+            if (i >= n)
+                break;
+            const float x = p[3 * k], y = p[3 * k + 1], z = p[3 * k + 2];
+            bool        ok = finite3(x, y, z);
+            float4      nn = nan4();
+            if (nin) {
+                float a = q[3 * k], b = q[3 * k + 1], c = q[3 * k + 2];
+                ok      = ok && finite3(a, b, c);
+                const float sq = a * a + (b * b + c * c);
+                if (sq > 0.0f) {
+                    const float s = smm::fsqrt(sq);
+                    a             = smm::fdiv(a, s);
+                    b             = smm::fdiv(b, s);
+                    c             = smm::fdiv(c, s);
+                }
+                nn = make_float4(a, b, c, 0.0f);
             }
-            nn = make_float4(a, b, c, 0.0f);
-        }
-        pos[i]   = make_float4(x, y, z, 0.0f);
-        nrm[i]   = nn;
-        valid[i] = ok ? 1 : 0;
-        if (ok) {
-            const int o[3] = {f2ord(x), f2ord(y), f2ord(z)};
-            for (int a = 0; a < 3; a++) {
-                lmn[a] = min(lmn[a], o[a]);
-                lmx[a] = max(lmx[a], o[a]);
+            pos[i]   = make_float4(x, y, z, 0.0f);
+            nrm[i]   = nn;
+            valid[i] = ok ? 1 : 0;
+            if (ok) {
+                const int o[3] = {f2ord(x), f2ord(y), f2ord(z)};
+                for (int a = 0; a < 3; a++) {
+                    lmn[a] = min(lmn[a], o[a]);
+                    lmx[a] = max(lmx[a], o[a]);
+                }
+                lc++;
             }
-            lc++;
         }
     }
     for (int a = 0; a < 3; a++) {
@@ -165,13 +198,6 @@ static void fill(Ctx &c, const FillSet &f) {
 }
 
 // ---------------------------------------------------------------------------------------
-__device__ __forceinline__ int scan_val(const int *in, long long i, long long n, int eq) {
-    if (i >= n)
-        return 0;
-    const int v = in[i];
-    return eq == kNoEq ? v : (v == eq ? 1 : 0);
-}
-
 // Single-pass exclusive scan with decoupled look-back (Merrill & Garland, "Single-pass
 // Parallel Prefix Scan with Decoupled Look-back", 2016). Tiles of kScanTile values take a
 // ticket in launch order; a tile publishes its aggregate, then warp 0 walks back over the
@@ -191,10 +217,18 @@ __device__ __forceinline__ void st_relaxed_u64(unsigned long long *p, unsigned l
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
+// What a scan writes: kPrefix, out[i] = sum of the values before i; kSelect (0/1 flags), the
+// places i of set flags packed into out; kSelectIds, ids[i] for these. A thread's eight values
+// are two 16-byte loads (and stores of prefixes) where the arrays are aligned to them. (One by
+// one, and with the selected places written by a second kernel from the stored prefixes, 0.92 M
+// flags took 11 + 7 us, a table of 2 M counts 20 us.)
+enum ScanOut { kPrefix, kSelect, kSelectIds };
+
+template <ScanOut MODE>
 __global__ void __launch_bounds__(kScanBs)
-    k_scan_lookback(const int *__restrict__ in, int *__restrict__ out, long long n, int eq,
-                    unsigned long long *__restrict__ status, int *__restrict__ ticket,
-                    int nparts, unsigned epoch, int *__restrict__ total) {
+    k_scan_lookback(const int *__restrict__ in, int *__restrict__ out, long long n,
+                    const int *__restrict__ ids, unsigned long long *__restrict__ status,
+                    int *__restrict__ ticket, int nparts, unsigned epoch, int *__restrict__ total) {
     chain_enter(); // launched chained
     __shared__ int sh[33];
     __shared__ int sTile, sExcl;
@@ -207,12 +241,20 @@ __global__ void __launch_bounds__(kScanBs)
     __syncthreads();
     const int       tile = sTile;
     const long long base = (long long)tile * kScanTile + (long long)threadIdx.x * kScanIpt;
-    int             v[kScanIpt], s = 0;
+    alignas(16) int v[kScanIpt];
+    int             s = 0;
+    const bool      whole = base + kScanIpt <= n;
+    if (whole && ((uintptr_t)in & 15) == 0) {
+        *reinterpret_cast<int4 *>(&v[0]) = *reinterpret_cast<const int4 *>(in + base);
+        *reinterpret_cast<int4 *>(&v[4]) = *reinterpret_cast<const int4 *>(in + base + 4);
+    } else {
 #pragma unroll
-    for (int k = 0; k < kScanIpt; k++) {
-        v[k] = scan_val(in, base + k, n, eq);
-        s += v[k];
+        for (int k = 0; k < kScanIpt; k++)
+            v[k] = base + k < n ? in[base + k] : 0;
     }
+#pragma unroll
+    for (int k = 0; k < kScanIpt; k++)
+        s += v[k];
     int       agg;
     const int ex  = block_excl_scan(s, sh, &agg);
     const unsigned long long tag = (unsigned long long)epoch << 34;
@@ -263,23 +305,35 @@ __global__ void __launch_bounds__(kScanBs)
     }
     __syncthreads();
     int o = ex + sExcl;
+    if (MODE != kPrefix) {
+#pragma unroll
+        for (int k = 0; k < kScanIpt; k++)
+            if (v[k]) // (0 past the end)
+                out[o++] = MODE == kSelectIds ? ids[base + k] : (int)(base + k);
+        return;
+    }
+    alignas(16) int w[kScanIpt];
 #pragma unroll
     for (int k = 0; k < kScanIpt; k++) {
-        if (base + k < n)
-            out[base + k] = o;
+        w[k] = o;
         o += v[k];
+    }
+    if (whole && ((uintptr_t)out & 15) == 0) {
+        *reinterpret_cast<int4 *>(out + base)     = *reinterpret_cast<int4 *>(&w[0]);
+        *reinterpret_cast<int4 *>(out + base + 4) = *reinterpret_cast<int4 *>(&w[4]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < kScanIpt; k++)
+            if (base + k < n)
+                out[base + k] = w[k];
     }
 }
 
-__global__ void k_scatter_flags(const int *__restrict__ flags, const int *__restrict__ pre, int n,
-                                int eq, int *__restrict__ out) {
+__global__ void k_iota(int *__restrict__ out, int n) {
     chain_enter(); // launched chained
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n)
-        return;
-    const int v = flags[i];
-    if (eq == kNoEq ? v != 0 : v == eq)
-        out[pre[i]] = i;
+    if (i < n)
+        out[i] = i;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -379,14 +433,14 @@ __global__ void k_thin_scatter(const float4 *__restrict__ pos, const int *__rest
                                const unsigned long long *__restrict__ keys, int dim0, int dim1,
                                float4 *__restrict__ pts, int *__restrict__ ph,
                                int *__restrict__ lists, int2 *__restrict__ rankCnt,
-                               int *__restrict__ keptFlag) {
+                               int *__restrict__ keptFlag, int *__restrict__ overflow) {
     chain_enter(); // launched chained
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m)
         return;
-    keptFlag[i] = 0; // the phases' kept flags (and, at m, the overflow word) start clear
+    keptFlag[i] = 0; // the phases' kept flags and the overflow word start clear
     if (i == 0)
-        keptFlag[m] = 0;
+        *overflow = 0;
     const int    h = slotOf[i];
     const int    k = sub[i];
     const float4 p = pos[ids[i]];
@@ -742,6 +796,12 @@ __device__ __forceinline__ unsigned long long hkey(const float4 &p, const GridPa
            (unsigned)cx;
 }
 
+// Hashed grid, three passes over one table of uint4 {key low, key high, first point, points - 1},
+// all ones where empty (so that one fill clears it): points claim their cell's slot by its
+// 64-bit key and take a place in the cell, then every occupied cell takes its points' range from
+// a counter (a CTA's at once; the cells' order in the point arrays does not matter), then the
+// points go to their places. (A key table, a count table, their scan, a copy of the scan and a
+// pack into the slots moved twice the bytes: 81 us a grid of 0.92 M points against 57 us now.)
 __global__ void k_hg_insert(const float4 *__restrict__ pos, const int *__restrict__ ids, int m,
                             GridParams gp, uint4 *__restrict__ slot, uint32_t mask,
                             int2 *__restrict__ place) {
@@ -763,42 +823,6 @@ __global__ void k_hg_insert(const float4 *__restrict__ pos, const int *__restric
     }
 }
 
-__global__ void k_hg_scatter(const float4 *__restrict__ pos, const int *__restrict__ ids,
-                             const uint4 *__restrict__ slot, const int2 *__restrict__ place, int m,
-                             float4 *__restrict__ pts, int wIsRank) {
-    chain_enter(); // launched chained
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m)
-        return;
-    const int    id = ids[i];
-    const float4 p  = pos[id];
-    const int2   at = place[i];
-    pts[slot[at.x].z + at.y] = make_float4(p.x, p.y, p.z, __int_as_float(wIsRank ? i : id));
-}
-
-// Rank-ordered copies of a subset's positions and normals: out[r] = in[ids[r]].
-__global__ void k_gather_subset(const float4 *__restrict__ pos, const float4 *__restrict__ nrm,
-                                const int *__restrict__ ids, int m, float4 *__restrict__ subPos,
-                                float4 *__restrict__ subNrm) {
-    chain_enter(); // launched chained
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= m)
-        return;
-    const int id = ids[r];
-    subPos[r]    = pos[id];
-    subNrm[r]    = nrm[id];
-}
-
-// out[pre[i]] = gids[i] where flags[i] != 0
-__global__ void k_scatter_ids(const int *__restrict__ flags, const int *__restrict__ pre, int n,
-                              const int *__restrict__ gids, int *__restrict__ out) {
-    chain_enter(); // launched chained
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && flags[i])
-        out[pre[i]] = gids[i];
-}
-
-// Phase A: centroid and FP32-Kahan covariance of the neighbourhood, FP64 eigensolve, for the
 // Ranges of the occupied cells, their occupancy bits and direct-table entries.
 __global__ void __launch_bounds__(256)
     k_hg_ranges(uint4 *__restrict__ slot, uint32_t T, int *__restrict__ next,
@@ -827,6 +851,33 @@ __global__ void __launch_bounds__(256)
         dense[k] = make_int2(first, cnt);
 }
 
+__global__ void k_hg_scatter(const float4 *__restrict__ pos, const int *__restrict__ ids,
+                             const uint4 *__restrict__ slot, const int2 *__restrict__ place, int m,
+                             float4 *__restrict__ pts, int wIsRank) {
+    chain_enter(); // launched chained
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m)
+        return;
+    const int    id = ids[i];
+    const float4 p  = pos[id];
+    const int2   at = place[i];
+    pts[slot[at.x].z + at.y] = make_float4(p.x, p.y, p.z, __int_as_float(wIsRank ? i : id));
+}
+
+// Rank-ordered copies of a subset's positions and normals: out[r] = in[ids[r]].
+__global__ void k_gather_subset(const float4 *__restrict__ pos, const float4 *__restrict__ nrm,
+                                const int *__restrict__ ids, int m, float4 *__restrict__ subPos,
+                                float4 *__restrict__ subNrm) {
+    chain_enter(); // launched chained
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= m)
+        return;
+    const int id = ids[r];
+    subPos[r]    = pos[id];
+    subNrm[r]    = nrm[id];
+}
+
+// Phase A: centroid and FP32-Kahan covariance of the neighbourhood, FP64 eigensolve, for the
 // whole list.
 __global__ void k_pca(NormalList L, int k, const float4 *__restrict__ pos, float4 *__restrict__ cen,
                       float4 *__restrict__ nout) {
@@ -979,9 +1030,7 @@ int prep_points(Ctx &c, const float *xyz, const float *nin, int n, float4 *pos, 
     k_init_bbox<<<1, 32, 0, c.stream>>>(dev, dev + 6);
     SM_LAUNCH_CHECK();
     const int bs = 256;
-    int       nb = std::min(nblocks(n, bs), 152 * 16);
-    if (nb < 1)
-        nb = 1;
+    const int nb = std::max(1, std::min(nblocks(nblocks(n, 4), bs), 152 * 8));
     k_prep<<<nb, bs, 0, c.stream>>>(xyz, nin, n, pos, nrm, validFlag, dev, dev + 6);
     SM_LAUNCH_CHECK();
     SM_CUDA(cudaMemcpyAsync(c.hostCounts, dev, 7 * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
@@ -1009,9 +1058,9 @@ static unsigned scan_state(Ctx &c, int nparts) {
     return ++S.epoch;
 }
 
-// Exclusive scan of n values (or of value == eq flags) into out; the total goes to *total
-// (device) when given.
-static void scan_into(Ctx &c, const int *in, int *out, long long n, int eq, int *total) {
+// A scan of n values (see ScanOut); the total goes to *total (device) when given.
+template <ScanOut MODE>
+static void scan_launch(Ctx &c, const int *in, int *out, long long n, const int *ids, int *total) {
     const int nparts = (int)((n + kScanTile - 1) / kScanTile);
     if (nparts == 0) {
         if (total)
@@ -1020,53 +1069,39 @@ static void scan_into(Ctx &c, const int *in, int *out, long long n, int eq, int 
     }
     const unsigned epoch = scan_state(c, nparts);
     cudaEvent_t    t0    = c.clock.begin(c.stream);
-    launch_chained(c, k_scan_lookback, nparts, kScanBs, 0, in, out, n, eq, c.scan.status,
+    launch_chained(c, k_scan_lookback<MODE>, nparts, kScanBs, 0, in, out, n, ids, c.scan.status,
                    c.scan.ticket, nparts, epoch, total);
     c.clock.end(c.stream, t0, KernelClock::kScan, 8.0 * (double)n); // 4-byte value in, 4 out
 }
 
-static int scan_impl(Ctx &c, const int *in, int *out, long long n, int eq, const std::string &tag,
-                     bool wantTotal) {
-    int *total = c.arena.get<int>(tag + ".scantot", 1);
-    scan_into(c, in, out, n, eq, total);
-    if (!wantTotal)
-        return -1;
+// *total (device) to the host.
+static int read_total(Ctx &c, const int *total) {
     SM_CUDA(cudaMemcpyAsync(c.hostCounts, total, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
     c.sync_checked();
     return c.hostCounts[0];
 }
 
-// Exclusive scan of 0/1 flags without a host round trip; returns the device address of the
-// total.
-static int *scan_flags_total(Ctx &c, const int *flags, int *pre, int n, const std::string &tag) {
-    int *total = c.arena.get<int>(tag + ".scantot", 1);
-    scan_into(c, flags, pre, n, kNoEq, total);
-    return total;
-}
-
 int scan_excl(Ctx &c, const int *in, int *out, long long n, const std::string &tag, bool wantTotal) {
-    return scan_impl(c, in, out, n, kNoEq, tag, wantTotal);
-}
-
-static int compact_eq(Ctx &c, const int *flags, int n, int eq, int *outIds, const std::string &tag) {
-    if (n <= 0)
-        return 0;
-    int      *pre   = c.arena.get<int>(tag + ".pre", n);
-    const int total = scan_impl(c, flags, pre, n, eq, tag, true);
-    launch_chained(c, k_scatter_flags, nblocks(n, 256), 256, 0, flags, pre, n, eq, outIds);
-    return total;
+    int *total = c.arena.get<int>(tag + ".scantot", 1);
+    scan_launch<kPrefix>(c, in, out, n, nullptr, total);
+    return wantTotal ? read_total(c, total) : -1;
 }
 
 int compact(Ctx &c, const int *flags, int n, int *outIds, const std::string &tag) {
-    return compact_eq(c, flags, n, kNoEq, outIds, tag);
+    if (n <= 0)
+        return 0;
+    int *total = c.arena.get<int>(tag + ".scantot", 1);
+    scan_launch<kSelect>(c, flags, outIds, n, nullptr, total);
+    return read_total(c, total);
 }
 
-void compact_known(Ctx &c, const int *flags, int n, int *outIds, const std::string &tag) {
+void compact_known(Ctx &c, const int *flags, int n, int count, int *outIds) {
     if (n <= 0)
         return;
-    int *pre = c.arena.get<int>(tag + ".pre", n);
-    scan_impl(c, flags, pre, n, kNoEq, tag, false);
-    launch_chained(c, k_scatter_flags, nblocks(n, 256), 256, 0, flags, pre, n, kNoEq, outIds);
+    if (count == n) // every flag is set
+        launch_chained(c, k_iota, nblocks(n, 256), 256, 0, outIds, n);
+    else
+        scan_launch<kSelect>(c, flags, outIds, n, nullptr, nullptr);
 }
 
 void build_hgrid(Ctx &c, const float4 *pos, const int *ids, int m, const Box &box, float g,
@@ -1163,8 +1198,9 @@ int sample_points(Ctx &c, const float4 *pos, int npoints, const int *ids, int m,
     int   *ph      = c.arena.get<int>(tag + ".ph", kSpPh);
     int2  *rankCnt = c.arena.get<int2>(tag + ".rank", T);
     int   *lists   = c.arena.get<int>(tag + ".phl", maxOcc);
-    int   *keptFlag = c.arena.get<int>(tag + ".kf", (size_t)m + 1); // over the list places
-    int   *overflow = keptFlag + m;
+    int   *keptFlag = c.arena.get<int>(tag + ".kf", m); // over the list places
+    int   *result   = c.arena.get<int>(tag + ".res", 2); // points kept, overflow
+    int   *overflow = result + 1;
     FillSet clear;
     if (!dense)
         clear.add(keys, (size_t)T * 8, 0xffffffffu);
@@ -1177,7 +1213,7 @@ int sample_points(Ctx &c, const float4 *pos, int npoints, const int *ids, int m,
     scan_excl(c, cnt, start, (long long)T + 1, tag + ".g", false);
     launch_chained(c, k_phase_offsets, 1, 32, 0, ph);
     launch_chained(c, k_thin_scatter, nblocks(m, 256), 256, 0, pos, ids, m, slotOf, sub,
-                   start, keys, dim[0], dim[1], pts, ph, lists, rankCnt, keptFlag);
+                   start, keys, dim[0], dim[1], pts, ph, lists, rankCnt, keptFlag, overflow);
     ThinView V;
     for (int a = 0; a < 3; a++) {
         V.org[a] = box.mn[a];
@@ -1215,12 +1251,9 @@ int sample_points(Ctx &c, const float4 *pos, int npoints, const int *ids, int m,
         // once (16 + 4 bytes), spread over the 8 phases
         c.clock.end(c.stream, t0, KernelClock::kSamplePhase, 20.0 * (double)m / 8.0);
     }
-    // the kept points in index order (list order), and the overflow flag, in one round trip
-    int *pre   = c.arena.get<int>(tag + ".out.pre", std::max(m, 1));
-    int *total = scan_flags_total(c, keptFlag, pre, m, tag + ".out");
-    launch_chained(c, k_scatter_ids, nblocks(m, 256), 256, 0, keptFlag, pre, m, ids, outIds);
-    SM_CUDA(cudaMemcpyAsync(c.hostCounts, total, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-    SM_CUDA(cudaMemcpyAsync(c.hostCounts + 1, overflow, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+    // the kept points in index order (list order), their number and the overflow flag
+    scan_launch<kSelectIds>(c, keptFlag, outIds, m, ids, result);
+    SM_CUDA(cudaMemcpyAsync(c.hostCounts, result, 2 * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
     c.sync();
     if (c.hostCounts[1])
         throw Error(SM_ERR_CAPACITY, "sampler: kept-point capacity per cell exceeded");

@@ -246,7 +246,7 @@ int scan_excl(Ctx &c, const int *in, int *out, long long n, const std::string &t
 // Ascending indices i with flags[i] != 0; returns the count (synchronises).
 int compact(Ctx &c, const int *flags, int n, int *outIds, const std::string &tag);
 // The same when the count is known already (no host round trip).
-void compact_known(Ctx &c, const int *flags, int n, int *outIds, const std::string &tag);
+void compact_known(Ctx &c, const int *flags, int n, int count, int *outIds);
 // Hashed grid over points ids[0..m) with cell side g (fine cells at any scene extent).
 void build_hgrid(Ctx &c, const float4 *pos, const int *ids, int m, const Box &box, float g,
                  HGrid &H, const std::string &tag, bool wIsRank = false);

@@ -305,27 +305,27 @@ __global__ void __launch_bounds__(kScanBs)
     }
     __syncthreads();
     int o = ex + sExcl;
-    if (MODE != kPrefix) {
+    if constexpr (MODE != kPrefix) {
 #pragma unroll
         for (int k = 0; k < kScanIpt; k++)
             if (v[k]) // (0 past the end)
                 out[o++] = MODE == kSelectIds ? ids[base + k] : (int)(base + k);
-        return;
-    }
-    alignas(16) int w[kScanIpt];
-#pragma unroll
-    for (int k = 0; k < kScanIpt; k++) {
-        w[k] = o;
-        o += v[k];
-    }
-    if (whole && ((uintptr_t)out & 15) == 0) {
-        *reinterpret_cast<int4 *>(out + base)     = *reinterpret_cast<int4 *>(&w[0]);
-        *reinterpret_cast<int4 *>(out + base + 4) = *reinterpret_cast<int4 *>(&w[4]);
     } else {
+        alignas(16) int w[kScanIpt];
 #pragma unroll
-        for (int k = 0; k < kScanIpt; k++)
-            if (base + k < n)
-                out[base + k] = w[k];
+        for (int k = 0; k < kScanIpt; k++) {
+            w[k] = o;
+            o += v[k];
+        }
+        if (whole && ((uintptr_t)out & 15) == 0) {
+            *reinterpret_cast<int4 *>(out + base)     = *reinterpret_cast<int4 *>(&w[0]);
+            *reinterpret_cast<int4 *>(out + base + 4) = *reinterpret_cast<int4 *>(&w[4]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < kScanIpt; k++)
+                if (base + k < n)
+                    out[base + k] = w[k];
+        }
     }
 }
 
@@ -337,38 +337,67 @@ __global__ void k_iota(int *__restrict__ out, int n) {
 }
 
 // ---------------------------------------------------------------------------------------
-constexpr int kSpHeavy = 128; // sampler cells with more points are taken by a whole CTA
+// Sampler cells by how many points they hold: up to kSpSmall a group of eight lanes takes the
+// cell, up to kSpHeavy a warp, above a CTA. (A warp for every cell up to 128 points left most
+// lanes idle at the refinement's step, whose cells hold six points: 20 us a phase of 0.92 M
+// points' 154,000 cells, 16 us now.) Where a phase has no more small cells than the launch has
+// warps, a warp takes each: 6.5 us a phase of the 13,000-point scene against 10.5 us by groups.
+constexpr int kSpSmall = 32;
+constexpr int kSpHeavy = 128;
+constexpr int kSpBs    = 1024; // threads of the table passes: few CTAs add to the phase counters
 
 // The sampler's cells keep their side just above the step whatever the scene's extent
 // (the work per point is then bounded by the packing of kept points, not by how coarse a
 // capped grid would have to be). Their table is dense (slot = cell key) when the cell box is
 // small against the points (see sample_points), else hashed: keys[slot] holds the cell key
-// (open addressing, ~0 = empty), so only occupied cells are stored. A cell's points are
-// contiguous in pts from start[slot] (an empty dense slot has start[slot + 1] == start[slot]);
-// rankCnt[slot] = {the cell's kept-point record (its place in the phase lists), kept count},
+// (open addressing, ~0 = empty), so only occupied cells are stored. cnt[slot] = the cell's
+// points (0: empty); info[slot] = {first, kept}: a cell's points are contiguous in pts from
+// `first`, its kept points' positions in keptPos from there too, `kept` of them so far. info is
 // written for occupied cells only.
 struct ThinView {
-    float                     org[3];
-    float                     g;
     int                       dim[3];
     const unsigned long long *keys; // nullptr: dense table
     uint32_t                  mask;
-    const int                *start; // table slots + 1
+    const int                *cnt;
+    int2                     *info;
     const float4             *pts;
-    // the table slot of the cell with key `key`, -1 when the cell holds no point
-    __device__ __forceinline__ int find(unsigned long long key) const {
-        if (!keys)
-            return start[key + 1] > start[key] ? (int)key : -1;
-        uint32_t h = (uint32_t)smm::mix64(key) & mask;
-        for (uint32_t p = 0; p <= mask; p++) {
-            const unsigned long long k = keys[h];
-            if (k == key)
-                return (int)h;
-            if (k == ~0ull)
-                return -1;
-            h = (h + 1) & mask;
+    float4                   *keptPos;
+    int                       m; // points
+    // {first, kept} of the K cells with keys key[] where want[] is set, {0, 0} for a cell
+    // without points: the loads of all K in flight together
+    template <int K>
+    __device__ __forceinline__ void find(const unsigned long long (&key)[K], const bool (&want)[K],
+                                         int2 (&v)[K]) const {
+        if (!keys) {
+            int n[K];
+#pragma unroll
+            for (int r = 0; r < K; r++) {
+                const unsigned long long t = want[r] ? key[r] : 0ull;
+                v[r]                       = info[t];
+                n[r]                       = cnt[t];
+            }
+#pragma unroll
+            for (int r = 0; r < K; r++)
+                if (!want[r] || n[r] == 0)
+                    v[r] = make_int2(0, 0);
+            return;
         }
-        return -1;
+        uint32_t           h[K];
+        unsigned long long k[K];
+#pragma unroll
+        for (int r = 0; r < K; r++) {
+            h[r] = (uint32_t)smm::mix64(key[r]) & mask;
+            k[r] = want[r] ? keys[h[r]] : ~0ull;
+        }
+#pragma unroll
+        for (int r = 0; r < K; r++)
+            while (k[r] != key[r] && k[r] != ~0ull) { // (a free slot ends every probe)
+                h[r] = (h[r] + 1) & mask;
+                k[r] = keys[h[r]];
+            }
+#pragma unroll
+        for (int r = 0; r < K; r++)
+            v[r] = k[r] != ~0ull ? info[h[r]] : make_int2(0, 0);
     }
 };
 
@@ -376,374 +405,517 @@ __device__ __forceinline__ unsigned long long cell_key(int x, int y, int z, int 
     return ((unsigned long long)z * (unsigned)dim1 + (unsigned)y) * (unsigned)dim0 + (unsigned)x;
 }
 
-// Counting pass: the point's cell enters the table (slotOf) and the point takes its place
-// within the cell (sub); the point that opens a cell also counts the cell in its phase
-// (ph[0..7]). A hashed table has at least twice as many slots as points, so every cell
-// finds one; a dense one (keys == nullptr) files the cell under its key.
-__global__ void k_thin_insert(const float4 *__restrict__ pos, const int *__restrict__ ids, int m,
-                              GridParams gp, unsigned long long *__restrict__ keys, uint32_t mask,
-                              int *__restrict__ slotOf, int *__restrict__ sub,
-                              int *__restrict__ cnt, int *__restrict__ ph) {
+__device__ __forceinline__ void cell_coords(unsigned long long key, int dim0, int dim1, int c[3]) {
+    if (key >> 32) {
+        c[0] = (int)(key % (unsigned)dim0);
+        c[1] = (int)((key / (unsigned)dim0) % (unsigned)dim1);
+        c[2] = (int)(key / ((unsigned long long)dim0 * (unsigned)dim1));
+    } else {
+        const unsigned k = (unsigned)key, r = k / (unsigned)dim0;
+        c[0] = (int)(k - r * (unsigned)dim0);
+        c[2] = (int)(r / (unsigned)dim1);
+        c[1] = (int)(r - (unsigned)c[2] * (unsigned)dim1);
+    }
+}
+
+// The phases' counters: occupied cells, then the cells listed so far per class, then the heavy
+// cells taken.
+enum { kPhCells = 0, kPhSmall = 8, kPhMedium = 16, kPhHeavy = 24, kPhTaken = 32, kPhNext = 40, kPhWords = 41 };
+
+// Counting pass: the point's cell enters the table and the point takes its place within the
+// cell (place = {slot, place}); the point that opens a cell also counts the cell in its phase,
+// in shared memory first (a global counter per phase took one update per cell: 67 us of the
+// refinement's sampling). A hashed table has at least twice as many slots as points, so every
+// cell finds one; a dense one (keys == nullptr) files the cell under its key.
+__global__ void __launch_bounds__(kSpBs)
+    k_thin_insert(const float4 *__restrict__ pos, const int *__restrict__ ids, int m, GridParams gp,
+                  unsigned long long *__restrict__ keys, uint32_t mask, int2 *__restrict__ place,
+                  int *__restrict__ cnt, int *__restrict__ ph) {
     chain_enter(); // launched chained
+    __shared__ int h[8];
+    if (threadIdx.x < 8)
+        h[threadIdx.x] = 0;
+    __syncthreads();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m)
-        return;
-    const float4             p   = pos[ids[i]];
-    const int                cx  = smg::coord(p.x, gp.org[0], gp.g, gp.dim[0]);
-    const int                cy  = smg::coord(p.y, gp.org[1], gp.g, gp.dim[1]);
-    const int                cz  = smg::coord(p.z, gp.org[2], gp.g, gp.dim[2]);
-    const unsigned long long key = cell_key(cx, cy, cz, gp.dim[0], gp.dim[1]);
-    uint32_t                 h   = keys ? (uint32_t)smm::mix64(key) & mask : (uint32_t)key;
-    for (uint32_t q = 0; q <= mask; q++) {
-        const unsigned long long prev = keys ? atomicCAS(&keys[h], ~0ull, key) : key;
-        if (prev == ~0ull || prev == key) {
-            slotOf[i]   = (int)h;
-            const int k = atomicAdd(&cnt[h], 1);
-            sub[i]      = k;
-            if (k == 0)
-                atomicAdd(&ph[smg::phase_of(cx, cy, cz)], 1);
-            return;
+    if (i < m) {
+        const float4             p   = pos[ids[i]];
+        const int                cx  = smg::coord(p.x, gp.org[0], gp.g, gp.dim[0]);
+        const int                cy  = smg::coord(p.y, gp.org[1], gp.g, gp.dim[1]);
+        const int                cz  = smg::coord(p.z, gp.org[2], gp.g, gp.dim[2]);
+        const unsigned long long key = cell_key(cx, cy, cz, gp.dim[0], gp.dim[1]);
+        uint32_t                 t   = keys ? (uint32_t)smm::mix64(key) & mask : (uint32_t)key;
+        for (uint32_t q = 0; q <= mask; q++) {
+            const unsigned long long prev = keys ? atomicCAS(&keys[t], ~0ull, key) : key;
+            if (prev == ~0ull || prev == key) {
+                const int k = atomicAdd(&cnt[t], 1);
+                place[i]    = make_int2((int)t, k);
+                if (k == 0)
+                    atomicAdd(&h[smg::phase_of(cx, cy, cz)], 1);
+                break;
+            }
+            t = (t + 1) & mask;
         }
-        h = (h + 1) & mask;
     }
+    __syncthreads();
+    if (threadIdx.x < 8 && h[threadIdx.x])
+        atomicAdd(&ph[kPhCells + threadIdx.x], h[threadIdx.x]);
 }
 
-// ph[0..7] = occupied cells per phase; this sets ph[8..15] = the phases' list offsets and
-// ph[16..23] = their front fill pointers (ph[24..31] count heavy cells placed from the
-// back, ph[32..39] hand heavy cells to CTAs; both start at 0).
-__global__ void k_phase_offsets(int *__restrict__ ph) {
-    chain_enter(); // launched chained
-    if (threadIdx.x != 0)
-        return;
+// First list place of phase p.
+__device__ __forceinline__ int phase_off(const int *__restrict__ ph, int p) {
     int o = 0;
-    for (int p = 0; p < 8; p++) {
-        ph[8 + p]  = o;
-        ph[16 + p] = o;
-        o += ph[p];
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+        o += q < p ? ph[kPhCells + q] : 0;
+    return o;
+}
+
+// Occupied cells take their points' range from a counter (a CTA's at once; the cells' order does
+// not matter) and enter their phase's lists (any order: cells of one phase do not interact):
+// entries {slot, first, key}, small cells in one list, in the other medium ones from the front
+// and heavy ones from the back. Four slots a thread.
+__global__ void __launch_bounds__(kSpBs)
+    k_thin_cells(ThinView G, uint32_t T, int *__restrict__ ph, int4 *__restrict__ small,
+                 int4 *__restrict__ large) {
+    chain_enter(); // launched chained
+    __shared__ int sh[33], h[24], base[24], sBase;
+    if (threadIdx.x < 24)
+        h[threadIdx.x] = 0;
+    const uint32_t t0 = 4u * (blockIdx.x * blockDim.x + threadIdx.x);
+    int            n[4], s = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        n[j] = t0 + j < T ? G.cnt[t0 + j] : 0;
+        s += n[j];
+    }
+    int       tot;
+    const int ex = block_excl_scan(s, sh, &tot); // (its barriers cover h)
+    if (tot == 0)
+        return; // (uniform)
+    if (threadIdx.x == 0)
+        sBase = atomicAdd(&ph[kPhNext], tot);
+    int                cls[4], at[4];
+    unsigned long long key[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        cls[j] = -1;
+        if (n[j] > 0) {
+            int c[3];
+            key[j] = G.keys ? G.keys[t0 + j] : (unsigned long long)(t0 + j);
+            cell_coords(key[j], G.dim[0], G.dim[1], c);
+            cls[j] = smg::phase_of(c[0], c[1], c[2]) +
+                     (n[j] <= kSpSmall ? 0 : n[j] <= kSpHeavy ? 8 : 16);
+            at[j] = atomicAdd(&h[cls[j]], 1);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 24) {
+        const int p   = threadIdx.x & 7;
+        const int off = phase_off(ph, p);
+        const int b   = h[threadIdx.x] ? atomicAdd(&ph[kPhSmall + threadIdx.x], h[threadIdx.x]) : 0;
+        base[threadIdx.x] = threadIdx.x < 16 ? off + b : off + ph[kPhCells + p] - 1 - b;
+    }
+    __syncthreads();
+    int first = sBase + ex;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        if (cls[j] < 0)
+            continue;
+        const int4 e = make_int4((int)(t0 + j), first, (int)(uint32_t)key[j],
+                                 (int)(uint32_t)(key[j] >> 32));
+        G.info[t0 + j] = make_int2(first, 0);
+        if (cls[j] < 8)
+            small[base[cls[j]] + at[j]] = e;
+        else
+            large[base[cls[j]] + (cls[j] < 16 ? at[j] : -at[j])] = e;
+        first += n[j];
     }
 }
 
-// Placing pass: the point's position (its place i in the ascending id list in w: list order
-// is index order) at its place in the cell; the point with place 0 lists the cell's slot in
-// its phase (any order: cells of one phase do not interact) and records
-// rankCnt[slot] = {its list place (the index of the cell's kept-point record), 0 kept}.
+// Placing pass: the point's position (its place i in the ascending id list in w: list order is
+// index order) at its place in the cell; its kept flag starts clear.
 __global__ void k_thin_scatter(const float4 *__restrict__ pos, const int *__restrict__ ids, int m,
-                               const int *__restrict__ slotOf, const int *__restrict__ sub,
-                               const int *__restrict__ start,
-                               const unsigned long long *__restrict__ keys, int dim0, int dim1,
-                               float4 *__restrict__ pts, int *__restrict__ ph,
-                               int *__restrict__ lists, int2 *__restrict__ rankCnt,
-                               int *__restrict__ keptFlag, int *__restrict__ overflow) {
+                               const int2 *__restrict__ place, const int2 *__restrict__ info,
+                               float4 *__restrict__ pts, int *__restrict__ keptFlag) {
     chain_enter(); // launched chained
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m)
         return;
-    keptFlag[i] = 0; // the phases' kept flags and the overflow word start clear
-    if (i == 0)
-        *overflow = 0;
-    const int    h = slotOf[i];
-    const int    k = sub[i];
-    const float4 p = pos[ids[i]];
-    pts[start[h] + k] = make_float4(p.x, p.y, p.z, __int_as_float(i));
-    if (k == 0) {
-        const unsigned long long key = keys ? keys[h] : (unsigned long long)h;
-        const unsigned long long xy  = (unsigned long long)dim0 * (unsigned)dim1;
-        const int cx = (int)(key % (unsigned)dim0), cy = (int)((key / (unsigned)dim0) % (unsigned)dim1);
-        const int cz    = (int)(key / xy);
-        const int phase = smg::phase_of(cx, cy, cz);
-        // light cells fill the phase's list region from the front, heavy ones (more than
-        // kSpHeavy points, taken by whole CTAs) from the back
-        const int slot = start[h + 1] - start[h] > kSpHeavy
-                             ? ph[8 + phase] + ph[phase] - 1 - atomicAdd(&ph[24 + phase], 1)
-                             : atomicAdd(&ph[16 + phase], 1);
-        lists[slot]    = h;
-        rankCnt[h]     = make_int2(slot, 0);
-    }
+    const int2   at = place[i];
+    const float4 p  = pos[ids[i]];
+    pts[info[at.x].x + at.y] = make_float4(p.x, p.y, p.z, __int_as_float(i));
+    keptFlag[i]              = 0;
 }
 
 // ---------------------------------------------------------------------------------------
-constexpr int kSpWarps  = 8;   // warps per CTA of the phase kernel (a warp per light cell)
-constexpr int kSpReg    = kSpHeavy / 32; // light cell: points per lane, held in registers
-constexpr int kSpHStage = 448; // heavy cell: neighbours' kept points staged (26 x 16 + 32)
-constexpr int kSpStage  = 128; // light cell: neighbours' kept points staged per warp
+constexpr int kSpWarps  = 8;   // warps per CTA of the phase kernel
+constexpr int kSpReg    = kSpHeavy / 32; // medium cell: points per lane, held in registers
+constexpr int kSpHStage = 448; // heavy cell: neighbours' kept points staged
+constexpr int kSpStage  = 128; // medium cell: neighbours' kept points staged per warp
+constexpr int kSpGStage = 32;  // small cell: the same per group of eight lanes
 constexpr int kSpBuf    = kSpWarps * kSpStage > kSpHStage ? kSpWarps * kSpStage : kSpHStage;
-constexpr int kSpPh     = 40;  // ph[]: counts, offsets, light fill, heavy fill, heavy take
+static_assert(kSpSmall == 32 && kSpStage == 4 * kSpGStage, "a small cell is four points a lane");
 
-// The 26 neighbours of cell (cx, cy, cz) without its centre, lane l < 26 taking one:
-// the neighbour's kept-point record and kept count (cells of later phases have none yet,
-// empty cells have no record: -1, 0).
-__device__ __forceinline__ void sp_neighbour(const ThinView &G, const int2 *__restrict__ rankCnt,
-                                             int cx, int cy, int cz, int l, int &nr, int &cnt) {
-    nr  = -1;
-    cnt = 0;
-    const int o = l < 13 ? l : l + 1;
-    const int x = cx + o % 3 - 1, y = cy + (o / 3) % 3 - 1, z = cz + o / 9 - 1;
-    if (x >= 0 && y >= 0 && z >= 0 && x < G.dim[0] && y < G.dim[1] && z < G.dim[2]) {
-        const int t = G.find(cell_key(x, y, z, G.dim[0], G.dim[1]));
-        if (t >= 0) {
-            const int2 v = rankCnt[t];
-            nr           = v.x;
-            cnt          = nr >= 0 ? v.y : 0;
+// Neighbours l, l + 32 / K, ... < 26 of cell c (the centre left out; none unless live): {first,
+// kept}; cells of later phases have kept nothing yet, empty cells give {0, 0}.
+template <int K>
+__device__ __forceinline__ void sp_neighbours(const ThinView &G, const int c[3], int l, bool live,
+                                              int2 (&nb)[K]) {
+    unsigned long long key[K];
+    bool               want[K];
+#pragma unroll
+    for (int r = 0; r < K; r++) {
+        const int i = l + r * (32 / K), o = i < 13 ? i : i + 1;
+        const int x = c[0] + o % 3 - 1, y = c[1] + (o / 3) % 3 - 1, z = c[2] + o / 9 - 1;
+        want[r] = live && i < 26 && x >= 0 && y >= 0 && z >= 0 && x < G.dim[0] && y < G.dim[1] &&
+                  z < G.dim[2];
+        key[r] = cell_key(x, y, z, G.dim[0], G.dim[1]);
+    }
+    G.find(key, want, nb);
+}
+
+__device__ __forceinline__ unsigned long long entry_key(const int4 &e) {
+    return ((unsigned long long)(uint32_t)e.w << 32) | (uint32_t)e.z;
+}
+
+__device__ __forceinline__ bool sp_near(const float4 &o, const float4 &q, float r2) {
+    return smm::dist2(o.x, o.y, o.z, q.x, q.y, q.z) < r2;
+}
+
+// The sequential greedy visits a cell's points by ascending index and keeps a point unless a
+// kept point lies within the step; the kept points of the 26 neighbour cells (earlier phases)
+// are fixed, so the cell first drops every point within the step of one of them (order-free),
+// then repeats "keep the smallest surviving index, drop the survivors within the step of it" -
+// the same kept set as the sequential visit, at (kept points x cell size / threads) work and
+// without sorting. Points are named by their place in the ascending id list (same order as the
+// index), and keptFlag is over those places.
+
+// A heavy cell by the whole CTA: neighbours' kept points staged in shared memory when they fit,
+// survivors flagged in alive.
+__device__ void sp_heavy(const ThinView &G, const int4 &e, float r2, int *__restrict__ keptFlag,
+                         int *__restrict__ alive, float4 *stage) {
+    __shared__ int    sFirst[26], sPre[27], sMin[kSpWarps];
+    __shared__ float4 sKeep;
+    const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
+    const int s = e.y, n = G.cnt[e.x];
+    alive += s;
+    if (wl == 0) {
+        int c[3];
+        cell_coords(entry_key(e), G.dim[0], G.dim[1], c);
+        int2 nb[1];
+        sp_neighbours(G, c, lane, true, nb);
+        const int incl = warp_incl_scan(nb[0].y);
+        if (lane < 26) {
+            sFirst[lane] = nb[0].x;
+            sPre[lane]   = incl - nb[0].y;
+        }
+        if (lane == 31)
+            sPre[26] = incl;
+    }
+    __syncthreads();
+    const int  NK      = sPre[26];
+    const bool stageNb = NK <= kSpHStage;
+    if (stageNb) {
+        for (int t = tid; t < NK; t += kSpWarps * 32) {
+            int j = 0;
+            while (sPre[j + 1] <= t)
+                j++;
+            stage[t] = G.keptPos[sFirst[j] + (t - sPre[j])];
         }
     }
+    __syncthreads();
+    for (int i = tid; i < n; i += kSpWarps * 32) {
+        const float4 q  = G.pts[s + i];
+        bool         ok = true;
+        if (stageNb) {
+            for (int k = 0; k < NK && ok; k++)
+                ok = !sp_near(stage[k], q, r2);
+        } else {
+            for (int j = 0; j < 26 && ok; j++)
+                for (int k = 0; k < sPre[j + 1] - sPre[j] && ok; k++)
+                    ok = !sp_near(G.keptPos[sFirst[j] + k], q, r2);
+        }
+        alive[i] = ok ? 1 : 0;
+    }
+    __syncthreads();
+    int nk = 0;
+    for (;;) {
+        int    myMin = INT_MAX;
+        float4 myP   = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int i = tid; i < n; i += kSpWarps * 32)
+            if (alive[i]) {
+                const float4 q  = G.pts[s + i];
+                const int    id = __float_as_int(q.w);
+                if (id < myMin) {
+                    myMin = id;
+                    myP   = q;
+                }
+            }
+        const int wm = __reduce_min_sync(0xffffffffu, myMin);
+        if (lane == 0)
+            sMin[wl] = wm;
+        __syncthreads();
+        int m = INT_MAX;
+        for (int k = 0; k < kSpWarps; k++)
+            m = min(m, sMin[k]);
+        if (m == INT_MAX)
+            break; // (uniform: every thread read the same minima)
+        if (myMin == m)
+            sKeep = myP; // the unique holder
+        __syncthreads();
+        const float4 kp = sKeep;
+        if (tid == 0) {
+            keptFlag[m]          = 1;
+            G.keptPos[s + nk]    = kp;
+        }
+        nk++;
+        for (int i = tid; i < n; i += kSpWarps * 32) {
+            if (!alive[i])
+                continue;
+            const float4 q = G.pts[s + i];
+            if (__float_as_int(q.w) == m || sp_near(kp, q, r2))
+                alive[i] = 0;
+        }
+        __syncthreads(); // drops done and sMin / sKeep read before the next round
+    }
+    if (tid == 0)
+        G.info[e.x].y = nk;
+    __syncthreads(); // the buffers are reused by the next cell
 }
 
-__device__ __forceinline__ void cell_coords(const ThinView &G, int cell, int &cx, int &cy, int &cz) {
-    const unsigned long long key = G.keys ? G.keys[cell] : (unsigned long long)cell;
-    cx = (int)(key % (unsigned)G.dim[0]);
-    cy = (int)((key / (unsigned)G.dim[0]) % (unsigned)G.dim[1]);
-    cz = (int)(key / ((unsigned long long)G.dim[0] * (unsigned)G.dim[1]));
+// A medium cell by a warp: its points in registers (kSpReg per lane), the neighbours' kept points
+// staged in shared memory by the whole warp at once when they fit, else read one by one (a
+// broadcast each).
+__device__ __forceinline__ void sp_medium(const ThinView &G, const int4 &e, float r2,
+                                          int *__restrict__ keptFlag, float4 *stage) {
+    const int lane = threadIdx.x & 31;
+    const int s = e.y, n = G.cnt[e.x]; // n <= kSpHeavy
+    float4    q[kSpReg];
+#pragma unroll
+    for (int j = 0; j < kSpReg; j++) // (whatever follows the cell's points is masked below)
+        q[j] = G.pts[min(s + lane + 32 * j, G.m - 1)];
+    int c[3];
+    cell_coords(entry_key(e), G.dim[0], G.dim[1], c);
+    int2 nb1[1];
+    sp_neighbours(G, c, lane, true, nb1);
+    const int2 nb    = nb1[0];
+    unsigned   alive = 0u; // bit j: point lane + 32 j is still a candidate
+#pragma unroll
+    for (int j = 0; j < kSpReg; j++)
+        alive |= (lane + 32 * j < n ? 1u : 0u) << j;
+    auto drop = [&](const float4 &o) {
+#pragma unroll
+        for (int j = 0; j < kSpReg; j++)
+            if (sp_near(o, q[j], r2))
+                alive &= ~(1u << j);
+    };
+    const int incl = warp_incl_scan(nb.y);
+    const int excl = incl - nb.y;
+    const int NK   = __shfl_sync(0xffffffffu, incl, 31);
+    if (NK <= kSpStage) {
+        for (int base = 0; base < NK; base += 32) {
+            const int t  = base + lane;
+            int       lo = 0; // the neighbour holding kept point t: last with excl <= t
+#pragma unroll
+            for (int step = 16; step >= 1; step >>= 1) {
+                const int mid = lo + step;
+                const int ev  = __shfl_sync(0xffffffffu, excl, mid & 31);
+                if (mid < 26 && ev <= t)
+                    lo = mid;
+            }
+            const int fj = __shfl_sync(0xffffffffu, nb.x, lo);
+            const int ej = __shfl_sync(0xffffffffu, excl, lo);
+            if (t < NK)
+                stage[t] = G.keptPos[fj + (t - ej)];
+        }
+        __syncwarp();
+        for (int k = 0; k < NK; k++)
+            drop(stage[k]);
+        __syncwarp(); // the slice is refilled by the warp's next cell
+    } else {
+        for (int j = 0; j < 26; j++) {
+            const int fj = __shfl_sync(0xffffffffu, nb.x, j);
+            const int cj = __shfl_sync(0xffffffffu, nb.y, j);
+            for (int k = 0; k < cj; k++)
+                drop(G.keptPos[fj + k]);
+        }
+    }
+    // keep the smallest surviving index, drop the survivors within the step, repeat; the lane
+    // that holds the kept point hands its position to the warp
+    int nk = 0;
+    for (;;) {
+        int    myMin = INT_MAX;
+        float4 myP   = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < kSpReg; j++) {
+            const int id = __float_as_int(q[j].w);
+            if (((alive >> j) & 1u) && id < myMin) {
+                myMin = id;
+                myP   = q[j];
+            }
+        }
+        const int m = __reduce_min_sync(0xffffffffu, myMin);
+        if (m == INT_MAX)
+            break;
+        const int    src = __ffs(__ballot_sync(0xffffffffu, myMin == m)) - 1;
+        const float4 kp  = make_float4(__shfl_sync(0xffffffffu, myP.x, src),
+                                       __shfl_sync(0xffffffffu, myP.y, src),
+                                       __shfl_sync(0xffffffffu, myP.z, src), 0.0f);
+        if (lane == 0) {
+            keptFlag[m]       = 1;
+            G.keptPos[s + nk] = kp;
+        }
+        nk++;
+#pragma unroll
+        for (int j = 0; j < kSpReg; j++)
+            if (__float_as_int(q[j].w) == m || sp_near(kp, q[j], r2))
+                alive &= ~(1u << j);
+    }
+    if (lane == 0)
+        G.info[e.x].y = nk;
 }
 
-// One warp per light cell, one CTA per heavy cell of the current phase. The sequential
-// greedy visits the cell's points by ascending index and keeps a point unless a kept point
-// lies within the step; the kept points of the 26 neighbour cells (earlier phases) are
-// fixed, so the cell first drops every point within the step of one of them (order-free),
-// then repeats "keep the smallest surviving index, drop the survivors within the step of
-// it" - the same kept set as the sequential visit, at (kept points x cell size / threads)
-// work and without sorting. Kept points are recorded as positions (keptPos, `cap` per cell)
-// and their number in rankCnt[slot].y, next to the cell's record index (one load per
-// neighbour). Points are named by their place in the ascending id list (same order as the
-// index), and keptFlag is over those places. A light cell's points sit in its warp's
-// registers (kSpReg per lane) and the neighbours' kept points are read once each by the
-// warp; heavy cells (more than kSpHeavy points) spread each step over the CTA, which takes
-// them first, one at a time from a per-phase counter (neighbours' kept points staged in
-// shared memory when they fit, `alive` flags in aliveTmp).
-__global__ void __launch_bounds__(kSpWarps * 32)
-    k_sample_phase(ThinView G, const int *__restrict__ lists, int *__restrict__ ph, int phase,
-                   int2 *__restrict__ rankCnt, float4 *__restrict__ keptPos, int cap, float r2,
-                   int *__restrict__ keptFlag, int *__restrict__ overflow,
+// Four small cells by a warp, eight lanes each (live: this group has one): four points a lane, and
+// up to four neighbours a lane, whose kept points the lanes stage in parallel.
+__device__ __forceinline__ void sp_small(const ThinView &G, const int4 &e, bool live, float r2,
+                                         int *__restrict__ keptFlag, float4 *stage) {
+    const int lane = threadIdx.x & 31, gl = lane & 7, g0 = lane & 24;
+    const int s    = e.y;
+    float4    q[4];
+    int2      nb[4];
+    const int n = live ? G.cnt[e.x] : 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        q[j] = G.pts[min(s + gl + 8 * j, G.m - 1)];
+    int c[3];
+    cell_coords(entry_key(e), G.dim[0], G.dim[1], c);
+    sp_neighbours(G, c, gl, live, nb);
+    const int mine = nb[0].y + nb[1].y + nb[2].y + nb[3].y;
+    unsigned alive = 0u; // bit j: point gl + 8 j is still a candidate
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        alive |= (gl + 8 * j < n ? 1u : 0u) << j;
+    auto drop = [&](const float4 &o) {
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (sp_near(o, q[j], r2))
+                alive &= ~(1u << j);
+    };
+    int incl = mine; // inclusive prefix over the group
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o, 8);
+        if (gl >= o)
+            incl += t;
+    }
+    const int NK   = __shfl_sync(0xffffffffu, incl, 7, 8);
+    const int most = __reduce_max_sync(0xffffffffu, NK);
+    if (most <= kSpGStage) {
+        float4 kp[4]; // most neighbours have kept one point: these loads in flight together
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+            if (nb[r].y > 0)
+                kp[r] = G.keptPos[nb[r].x];
+        int at = incl - mine;
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            if (nb[r].y > 0)
+                stage[at] = kp[r];
+            for (int k = 1; k < nb[r].y; k++)
+                stage[at + k] = G.keptPos[nb[r].x + k];
+            at += nb[r].y;
+        }
+        __syncwarp();
+        for (int k = 0; k < most; k++)
+            if (k < NK)
+                drop(stage[k]);
+        __syncwarp(); // the slice is refilled by the group's next cell
+    } else {
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+            for (int l = 0; l < 8; l++) {
+                const int f  = __shfl_sync(0xffffffffu, nb[r].x, l, 8);
+                const int cj = __shfl_sync(0xffffffffu, nb[r].y, l, 8);
+                for (int k = 0; k < cj; k++)
+                    drop(G.keptPos[f + k]);
+            }
+    }
+    int nk = 0;
+    for (;;) {
+        int    myMin = INT_MAX;
+        float4 myP   = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int id = __float_as_int(q[j].w);
+            if (((alive >> j) & 1u) && id < myMin) {
+                myMin = id;
+                myP   = q[j];
+            }
+        }
+        int m = myMin;
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1)
+            m = min(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (__all_sync(0xffffffffu, m == INT_MAX))
+            break; // no group has a survivor
+        const unsigned who = __ballot_sync(0xffffffffu, myMin == m && m != INT_MAX) & (0xffu << g0);
+        const int      src = who ? __ffs(who) - 1 : lane;
+        const float4   kp  = make_float4(__shfl_sync(0xffffffffu, myP.x, src),
+                                         __shfl_sync(0xffffffffu, myP.y, src),
+                                         __shfl_sync(0xffffffffu, myP.z, src), 0.0f);
+        if (m == INT_MAX)
+            continue; // (the group waits for the others)
+        if (gl == 0) {
+            keptFlag[m]       = 1;
+            G.keptPos[s + nk] = kp;
+        }
+        nk++;
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (__float_as_int(q[j].w) == m || sp_near(kp, q[j], r2))
+                alive &= ~(1u << j);
+    }
+    if (live && gl == 0)
+        G.info[e.x].y = nk;
+}
+
+// The cells of the current phase: heavy ones first, one at a time from a counter, then medium and
+// small ones by stride.
+__global__ void __launch_bounds__(kSpWarps * 32, 4)
+    k_sample_phase(ThinView G, const int4 *__restrict__ small, const int4 *__restrict__ large,
+                   int *__restrict__ ph, int phase, float r2, int *__restrict__ keptFlag,
                    int *__restrict__ aliveTmp) {
-    smd::chain_enter(); // phases are chained launches: the previous phase's flags are final
-    __shared__ float4 stageBuf[kSpBuf]; // heavy cell: [0, kSpHStage); light warp w: its slice
-    __shared__ int    snr[26], scnt[26];
-    __shared__ int    sCell, sMin[kSpWarps];
-    __shared__ float4 sKeep;
-    const int  wl    = threadIdx.x >> 5;
-    const int  lane  = threadIdx.x & 31;
-    const int  tid   = threadIdx.x;
-    const int  off   = ph[8 + phase];
-    const int  total = ph[phase];
-    const int  nl    = ph[16 + phase] - off; // light cells: list front
-    const int  nh    = ph[24 + phase];       // heavy cells: list back
-    const int *cells = lists + off;
-
-    // ---- heavy cells: the whole CTA on one cell
-    for (; nh > 0;) {
-        if (tid == 0)
-            sCell = atomicAdd(&ph[32 + phase], 1);
+    smd::chain_enter(); // phases are chained launches: the previous phase's cells are final
+    __shared__ float4 stageBuf[kSpBuf]; // heavy cell: [0, kSpHStage); warp w: its slice
+    __shared__ int    sCell;
+    const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int off = phase_off(ph, phase);
+    const int nS = ph[kPhSmall + phase], nM = ph[kPhMedium + phase], nH = ph[kPhHeavy + phase];
+    while (nH > 0) {
+        if (threadIdx.x == 0)
+            sCell = atomicAdd(&ph[kPhTaken + phase], 1);
         __syncthreads();
         const int hc = sCell;
         __syncthreads(); // every thread has read sCell before it is taken again
-        if (hc >= nh)
+        if (hc >= nH)
             break;
-        const int cell = cells[total - 1 - hc];
-        const int rk   = rankCnt[cell].x;
-        int       cx, cy, cz;
-        cell_coords(G, cell, cx, cy, cz);
-        const int s = G.start[cell], n = G.start[cell + 1] - s;
-        if (wl == 0) {
-            int nr = -1, cnt = 0;
-            if (lane < 26)
-                sp_neighbour(G, rankCnt, cx, cy, cz, lane, nr, cnt);
-            const int incl = warp_incl_scan(cnt);
-            if (lane < 26) {
-                snr[lane]  = nr;
-                scnt[lane] = incl - cnt; // exclusive prefix
-            }
-            if (lane == 31)
-                sMin[0] = incl; // NK
-        }
-        __syncthreads();
-        const int  NK      = sMin[0];
-        const bool stageNb = NK <= kSpHStage;
-        if (stageNb) {
-            for (int t = tid; t < NK; t += kSpWarps * 32) {
-                int j = 0;
-                while (j < 25 && scnt[j + 1] <= t)
-                    j++;
-                stageBuf[t] = keptPos[(size_t)snr[j] * cap + (t - scnt[j])];
-            }
-        }
-        __syncthreads();
-        int *alive = aliveTmp + s;
-        for (int i = tid; i < n; i += kSpWarps * 32) {
-            const float4 q  = G.pts[s + i];
-            bool         ok = true;
-            if (stageNb) {
-                for (int k = 0; k < NK && ok; k++) {
-                    const float4 o = stageBuf[k];
-                    if (smm::dist2(o.x, o.y, o.z, q.x, q.y, q.z) < r2)
-                        ok = false;
-                }
-            } else {
-                for (int j = 0; j < 26 && ok; j++) {
-                    const int nj = snr[j];
-                    const int cj = (j < 25 ? scnt[j + 1] : NK) - scnt[j];
-                    for (int k = 0; k < cj && ok; k++) {
-                        const float4 o = keptPos[(size_t)nj * cap + k];
-                        if (smm::dist2(o.x, o.y, o.z, q.x, q.y, q.z) < r2)
-                            ok = false;
-                    }
-                }
-            }
-            alive[i] = ok ? 1 : 0;
-        }
-        __syncthreads();
-        float4 *mine = keptPos + (size_t)rk * cap;
-        int     nk   = 0;
-        for (;;) {
-            int    myMin = INT_MAX;
-            float4 myP   = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int i = tid; i < n; i += kSpWarps * 32)
-                if (alive[i]) {
-                    const float4 q  = G.pts[s + i];
-                    const int    id = __float_as_int(q.w);
-                    if (id < myMin) {
-                        myMin = id;
-                        myP   = q;
-                    }
-                }
-            const int wm = __reduce_min_sync(0xffffffffu, myMin);
-            if (lane == 0)
-                sMin[wl] = wm;
-            __syncthreads();
-            int m = INT_MAX;
-            for (int k = 0; k < kSpWarps; k++)
-                m = min(m, sMin[k]);
-            if (m == INT_MAX)
-                break; // (uniform: every thread read the same minima)
-            if (myMin == m)
-                sKeep = make_float4(myP.x, myP.y, myP.z, 0.0f); // the unique holder
-            __syncthreads();
-            const float4 kp = sKeep;
-            if (tid == 0) {
-                keptFlag[m] = 1;
-                if (nk < cap)
-                    mine[nk] = kp;
-                else
-                    atomicExch(overflow, 1);
-            }
-            nk = min(nk + 1, cap);
-            for (int i = tid; i < n; i += kSpWarps * 32) {
-                if (!alive[i])
-                    continue;
-                const float4 q = G.pts[s + i];
-                if (__float_as_int(q.w) == m || smm::dist2(kp.x, kp.y, kp.z, q.x, q.y, q.z) < r2)
-                    alive[i] = 0;
-            }
-            __syncthreads(); // drops done and sMin / sKeep read before the next round
-        }
-        if (tid == 0)
-            rankCnt[cell].y = nk;
-        __syncthreads(); // the buffers are reused by the next cell
+        sp_heavy(G, large[off + ph[kPhCells + phase] - 1 - hc], r2, keptFlag, aliveTmp, stageBuf);
     }
-
-    // ---- light cells: a warp each, the cell's points in registers (kSpReg per lane)
-    for (int w = blockIdx.x * kSpWarps + wl; w < nl; w += gridDim.x * kSpWarps) {
-        const int cell = cells[w];
-        const int rk   = rankCnt[cell].x;
-        int       cx, cy, cz;
-        cell_coords(G, cell, cx, cy, cz);
-        const int s = G.start[cell], n = G.start[cell + 1] - s; // n <= kSpHeavy
-        float4    q[kSpReg];
-        unsigned  alive = 0u; // bit j: point lane + 32 j is still a candidate
-#pragma unroll
-        for (int j = 0; j < kSpReg; j++) {
-            const int i = lane + 32 * j;
-            q[j]        = i < n ? G.pts[s + i] : make_float4(0.f, 0.f, 0.f, 0.f);
-            alive |= (i < n ? 1u : 0u) << j;
-        }
-        int nr = -1, cnt = 0;
-        if (lane < 26)
-            sp_neighbour(G, rankCnt, cx, cy, cz, lane, nr, cnt);
-        // survivors of the neighbours' kept points, each tested against every point the lane
-        // holds: staged in shared memory by the whole warp at once when they fit, else the
-        // neighbours one by one, each kept point read once by the warp (a broadcast)
-        const int incl = warp_incl_scan(cnt);
-        const int excl = incl - cnt;
-        const int NK   = __shfl_sync(0xffffffffu, incl, 31);
-        unsigned  nz   = __ballot_sync(0xffffffffu, cnt > 0);
-        if (NK <= kSpStage) {
-            float4 *st = stageBuf + wl * kSpStage;
-            for (int base = 0; base < NK; base += 32) {
-                const int t  = base + lane;
-                int       lo = 0; // the neighbour holding kept point t: last with excl <= t
-#pragma unroll
-                for (int step = 16; step >= 1; step >>= 1) {
-                    const int mid = lo + step;
-                    const int ev  = __shfl_sync(0xffffffffu, excl, mid & 31);
-                    if (mid < 26 && ev <= t)
-                        lo = mid;
-                }
-                const int nj = __shfl_sync(0xffffffffu, nr, lo);
-                const int ej = __shfl_sync(0xffffffffu, excl, lo);
-                if (t < NK)
-                    st[t] = keptPos[(size_t)nj * cap + (t - ej)];
-            }
-            __syncwarp();
-            for (int kk = 0; kk < NK; kk++) {
-                const float4 o = st[kk];
-#pragma unroll
-                for (int j = 0; j < kSpReg; j++)
-                    if (smm::dist2(o.x, o.y, o.z, q[j].x, q[j].y, q[j].z) < r2)
-                        alive &= ~(1u << j);
-            }
-            __syncwarp(); // the slice is refilled by the warp's next cell
-            nz = 0u;
-        }
-        while (nz && __any_sync(0xffffffffu, alive != 0u)) {
-            const int jn = __ffs(nz) - 1;
-            nz &= nz - 1u;
-            const int     nj = __shfl_sync(0xffffffffu, nr, jn);
-            const int     cj = __shfl_sync(0xffffffffu, cnt, jn);
-            const float4 *kn = keptPos + (size_t)nj * cap;
-            for (int k = 0; k < cj; k++) {
-                const float4 o = kn[k];
-#pragma unroll
-                for (int j = 0; j < kSpReg; j++)
-                    if (smm::dist2(o.x, o.y, o.z, q[j].x, q[j].y, q[j].z) < r2)
-                        alive &= ~(1u << j);
-            }
-        }
-        // keep the smallest surviving index, drop the survivors within the step, repeat; the
-        // lane that holds the kept point hands its position to the warp
-        float4 *mine = keptPos + (size_t)rk * cap;
-        int     nk   = 0;
-        for (;;) {
-            int    myMin = INT_MAX;
-            float4 myP   = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int j = 0; j < kSpReg; j++) {
-                const int id = __float_as_int(q[j].w);
-                if (((alive >> j) & 1u) && id < myMin) {
-                    myMin = id;
-                    myP   = q[j];
-                }
-            }
-            const int m = __reduce_min_sync(0xffffffffu, myMin);
-            if (m == INT_MAX)
-                break;
-            const int    src = __ffs(__ballot_sync(0xffffffffu, myMin == m)) - 1;
-            const float4 kp  = make_float4(__shfl_sync(0xffffffffu, myP.x, src),
-                                           __shfl_sync(0xffffffffu, myP.y, src),
-                                           __shfl_sync(0xffffffffu, myP.z, src), 0.0f);
-            if (lane == 0) {
-                keptFlag[m] = 1;
-                if (nk < cap)
-                    mine[nk] = kp;
-                else
-                    atomicExch(overflow, 1);
-            }
-            nk = min(nk + 1, cap);
-#pragma unroll
-            for (int j = 0; j < kSpReg; j++)
-                if (__float_as_int(q[j].w) == m ||
-                    smm::dist2(kp.x, kp.y, kp.z, q[j].x, q[j].y, q[j].z) < r2)
-                    alive &= ~(1u << j);
-        }
-        if (lane == 0)
-            rankCnt[cell].y = nk;
+    float4   *stage = stageBuf + wl * kSpStage;
+    const int w0    = blockIdx.x * kSpWarps + wl, nw = gridDim.x * kSpWarps;
+    for (int w = w0; w < nM; w += nw)
+        sp_medium(G, large[off + w], r2, keptFlag, stage);
+    // (from the other end of the grid: the warps without a medium cell start)
+    if (nS <= nw) { // a warp for each: the shortest chain where there are warps enough
+        for (int w = nw - 1 - w0; w < nS; w += nw)
+            sp_medium(G, small[off + w], r2, keptFlag, stage);
+        return;
+    }
+    for (int w = nw - 1 - w0; 4 * w < nS; w += nw) {
+        const int  k    = 4 * w + (lane >> 3);
+        const bool live = k < nS;
+        sp_small(G, live ? small[off + k] : make_int4(0, 0, 0, 0), live, r2, keptFlag,
+                 stage + (lane >> 3) * kSpGStage);
     }
 }
 
@@ -1188,50 +1360,39 @@ int sample_points(Ctx &c, const float4 *pos, int npoints, const int *ids, int m,
     const bool               dense = ncell <= std::min<unsigned long long>(dmax, 1ull << 27);
     if (dense)
         T = (uint32_t)ncell;
-    const long long maxOcc = m;
-    auto *keys = dense ? nullptr : c.arena.get<unsigned long long>(tag + ".g.keys", T);
-    int   *cnt     = c.arena.get<int>(tag + ".g.cnt", (size_t)T + 1);
-    int   *start   = c.arena.get<int>(tag + ".g.start", (size_t)T + 1);
-    float4 *pts    = c.arena.get<float4>(tag + ".g.pts", m);
-    int   *slotOf  = c.arena.get<int>(tag + ".g.slotOf", m);
-    int   *sub     = c.arena.get<int>(tag + ".g.sub", m);
-    int   *ph      = c.arena.get<int>(tag + ".ph", kSpPh);
-    int2  *rankCnt = c.arena.get<int2>(tag + ".rank", T);
-    int   *lists   = c.arena.get<int>(tag + ".phl", maxOcc);
-    int   *keptFlag = c.arena.get<int>(tag + ".kf", m); // over the list places
-    int   *result   = c.arena.get<int>(tag + ".res", 2); // points kept, overflow
-    int   *overflow = result + 1;
+    ThinView V;
+    for (int a = 0; a < 3; a++)
+        V.dim[a] = dim[a];
+    auto *keys  = dense ? nullptr : c.arena.get<unsigned long long>(tag + ".g.keys", T);
+    int  *cnt   = c.arena.get<int>(tag + ".g.cnt", T);
+    auto *pts   = c.arena.get<float4>(tag + ".g.pts", m);
+    V.keys      = keys;
+    V.mask      = dense ? 0u : T - 1;
+    V.cnt       = cnt;
+    V.info      = c.arena.get<int2>(tag + ".g.info", T);
+    V.pts       = pts;
+    V.keptPos   = c.arena.get<float4>(tag + ".kp", m);
+    V.m         = m;
+    int2 *place = c.arena.get<int2>(tag + ".g.place", m);
+    int  *ph    = c.arena.get<int>(tag + ".ph", kPhWords);
+    int4 *small = c.arena.get<int4>(tag + ".phs", m); // (at most a cell per point)
+    int4 *large = c.arena.get<int4>(tag + ".phl", m);
+    int  *keptFlag = c.arena.get<int>(tag + ".kf", m); // over the list places
+    int  *aliveTmp = c.arena.get<int>(tag + ".al", m);
     FillSet clear;
     if (!dense)
         clear.add(keys, (size_t)T * 8, 0xffffffffu);
-    clear.add(cnt, ((size_t)T + 1) * sizeof(int), 0u);
-    clear.add(ph, kSpPh * sizeof(int), 0u);
+    clear.add(cnt, (size_t)T * sizeof(int), 0u);
+    clear.add(ph, kPhWords * sizeof(int), 0u);
     fill(c, clear);
     const GridParams gpar = grid_params(box, g, dim);
-    launch_chained(c, k_thin_insert, nblocks(m, 256), 256, 0, pos, ids, m, gpar, keys,
-                   dense ? 0u : T - 1, slotOf, sub, cnt, ph);
-    scan_excl(c, cnt, start, (long long)T + 1, tag + ".g", false);
-    launch_chained(c, k_phase_offsets, 1, 32, 0, ph);
-    launch_chained(c, k_thin_scatter, nblocks(m, 256), 256, 0, pos, ids, m, slotOf, sub,
-                   start, keys, dim[0], dim[1], pts, ph, lists, rankCnt, keptFlag, overflow);
-    ThinView V;
-    for (int a = 0; a < 3; a++) {
-        V.org[a] = box.mn[a];
-        V.dim[a] = dim[a];
-    }
-    V.g     = g;
-    V.keys  = keys;
-    V.mask  = dense ? 0u : T - 1;
-    V.start = start;
-    V.pts   = pts;
-    // kept-list capacity: points at pairwise distance >= step inside a cube of side g fit
-    // disjoint balls of radius step/2 inside the cube grown by step/2.
-    const double s   = (double)g / (double)step;
-    const int    cap = (int)std::floor((s + 1.0) * (s + 1.0) * (s + 1.0) / (3.14159265358979 / 6.0)) + 1;
-    float4 *keptPos  = c.arena.get<float4>(tag + ".kp", (size_t)maxOcc * cap);
-    int    *aliveTmp = c.arena.get<int>(tag + ".al", std::max(m, 1));
+    launch_chained(c, k_thin_insert, nblocks(m, kSpBs), kSpBs, 0, pos, ids, m, gpar, keys, V.mask,
+                   place, cnt, ph);
+    launch_chained(c, k_thin_cells, nblocks(T, 4 * kSpBs), kSpBs, 0, V, T, ph, small, large);
+    launch_chained(c, k_thin_scatter, nblocks(m, 256), 256, 0, pos, ids, m, place, V.info, pts,
+                   keptFlag);
     const float r2 = step * step;
-    // one resident wave: heavy cells are handed out by a counter, light cells by stride
+    // one resident wave: heavy cells are handed out by a counter, the others by stride
     static std::atomic<int> resident[64];
     const int               dev = c.device >= 0 && c.device < 64 ? c.device : 0;
     int                     per = resident[dev].load();
@@ -1242,21 +1403,20 @@ int sample_points(Ctx &c, const float4 *pos, int npoints, const int *ids, int m,
     }
     int nsm = 0;
     SM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device));
-    const int gp = (int)std::min<long long>((maxOcc + kSpWarps - 1) / kSpWarps, (long long)nsm * per);
+    const int gp = (int)std::min<long long>((m + kSpWarps - 1) / kSpWarps, (long long)nsm * per);
     for (int p = 0; p < 8; p++) {
         cudaEvent_t t0 = c.clock.begin(c.stream);
-        launch_chained(c, k_sample_phase, gp, kSpWarps * 32, 0, V, lists, ph, p, rankCnt,
-                       keptPos, cap, r2, keptFlag, overflow, aliveTmp);
+        launch_chained(c, k_sample_phase, gp, kSpWarps * 32, 0, V, small, large, ph, p, r2, keptFlag,
+                       aliveTmp);
         // algorithmic bytes of a sampling: each point's position read and its flag written
         // once (16 + 4 bytes), spread over the 8 phases
         c.clock.end(c.stream, t0, KernelClock::kSamplePhase, 20.0 * (double)m / 8.0);
     }
-    // the kept points in index order (list order), their number and the overflow flag
-    scan_launch<kSelectIds>(c, keptFlag, outIds, m, ids, result);
-    SM_CUDA(cudaMemcpyAsync(c.hostCounts, result, 2 * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+    // the kept points in index order (list order) and their number
+    int *total = c.arena.get<int>(tag + ".res", 1);
+    scan_launch<kSelectIds>(c, keptFlag, outIds, m, ids, total);
+    SM_CUDA(cudaMemcpyAsync(c.hostCounts, total, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
     c.sync();
-    if (c.hostCounts[1])
-        throw Error(SM_ERR_CAPACITY, "sampler: kept-point capacity per cell exceeded");
     return c.hostCounts[0];
 }
 

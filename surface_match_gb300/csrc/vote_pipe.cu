@@ -1,19 +1,20 @@
 // vote_pipe.cu - the voting stage of matchScene (ppf.cpp:247-409) as a pipeline of
 // kernels, each shaped for what it spends its time on.
 //
-//  1. k_kp_radius / k_kp_csr: per keypoint its neighbour count, its rows (neighbours other
-//     than itself) and the list position of its first "tail" row - the reference computes
-//     a keypoint's rows in 8-lane blocks and the last (rows mod 8) one by one, with
-//     different float rounding. In radius mode (all candidates within the model diameter,
-//     in ascending order) the rows are kept as a bitmask over the candidate list, computed
-//     from candidate tiles staged in shared memory and shared by eight keypoints.
-//  2. A prefix sum over the rows gives every keypoint a segment of the row list.
-//  3. k_rows_fill writes (keypoint, point, lane rule) per row into its segment.
-//  4. k_ppf: one thread per row at full occupancy - quantised PPF key, scene alpha, model
-//     table probe; a hit (bucket, count, alpha) is appended to the keypoint's segment.
-//  5. k_lpt: keypoints ordered by their vote count, largest first, so the heaviest
+//  1. k_kp_radius + k_kp_info, or k_kp_csr + k_rows_count: per keypoint its neighbour count, its
+//     rows (neighbours other than itself) and the list position of its first "tail" row - the
+//     reference computes a keypoint's rows in 8-lane blocks and the last (rows mod 8) one by
+//     one, with different float rounding. In radius mode (all candidates within the model
+//     diameter, in ascending order) the rows are kept as a bitmask over the candidate list,
+//     computed from candidate tiles staged in shared memory and shared by 32 keypoints.
+//  2. A prefix sum over the rows gives every keypoint a segment of the hit list.
+//  3. k_ppf: a CTA per keypoint (several where keypoints are few), each warp packing rows from
+//     its share of the candidates until it has 32: quantised PPF key and model table probe by a
+//     lane per row; the hits, packed again, pay for the scene alpha; a hit (bucket, count,
+//     alpha) is appended to the keypoint's segment.
+//  4. k_lpt: keypoints ordered by their vote count, largest first, so the heaviest
 //     accumulators start first and the tail of the next kernel stays short.
-//  6. k_vote_acc: one CTA per keypoint votes its hits into a shared-memory (reference
+//  5. k_vote_acc: one CTA per keypoint votes its hits into a shared-memory (reference
 //     point x angle bin) accumulator - 16-bit counters when the keypoint's vote count
 //     allows - then extracts peaks, the top three candidates and their poses.
 #include <atomic>
@@ -32,8 +33,10 @@ void fill_vote_model(const Model &m, float minScore, VoteArgs &a);
 
 namespace {
 
-constexpr int kKpWarps   = 8;    // keypoints per CTA of the radius kernel
+constexpr int kKpWarps   = 8;    // warps per CTA of the radius kernel
+constexpr int kKpPer     = 4;    // keypoints per warp of it
 constexpr int kTile      = 1024; // candidates per shared-memory tile
+constexpr int kPpfBs     = 256;
 // vote accumulation launch shapes the launch tuner chooses between - CTA size, and one CTA per
 // keypoint or a persistent grid that takes keypoints from a device counter in LPT order;
 // every one computes the same accumulators, peaks and candidates
@@ -47,8 +50,9 @@ struct PipeBufs {
     smm::RT            *rt;      // K: transform of the keypoint
     uint32_t           *mask;    // K x words: row bits over the candidate list (radius mode)
     int                 words;
+    int                 splits;  // radius mode: parts of the candidate list
+    int2               *part;    // splits x K: {neighbours, rows} in the part
     int                *rowOff;  // K + 1
-    int2               *rows;    // rows: {keypoint, point * 2 + block lane}
     int4               *hits;    // per row segment: {bucket offset, count, alpha bits, 0}
     int                *hitCnt;  // K
     unsigned long long *votes;   // K
@@ -103,58 +107,91 @@ __device__ __forceinline__ int tail_from_mask(const uint32_t *m, int nw, int nee
     return found;
 }
 
-// Radius mode: eight keypoints per CTA, one per warp, over shared-memory tiles of the
-// candidates' positions.
-__global__ void __launch_bounds__(kKpWarps * 32) k_kp_radius(VoteArgs a, PipeBufs b) {
+// Radius mode, part blockIdx.y of the candidates: kKpPer keypoints per warp over shared-memory
+// tiles of the candidates' positions (id in w). The parts make CTAs enough: with one CTA per
+// eight keypoints over all candidates, 2390 keypoints x 18,069 candidates took 145 us, now 54 us.
+__global__ void __launch_bounds__(kKpWarps * 32) k_kp_radius(VoteArgs a, PipeBufs b, int per) {
     smd::chain_enter(); // launched chained
     __shared__ float4 tp[kTile];
-    __shared__ int    tid_[kTile];
-    const int   lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int   c    = blockIdx.x * kKpWarps + w;
-    const bool  live = c < a.K;
-    const int   pid  = live ? a.kp[c] : -1;
-    float4      p1   = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (live)
-        p1 = a.pos[pid];
-    uint32_t *mrow = b.mask + (size_t)(live ? c : 0) * b.words;
-    int       S = 0, R = 0;
-    for (int t0 = 0; t0 < a.ncand; t0 += kTile) {
-        const int tn = min(kTile, a.ncand - t0);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int c0   = (blockIdx.x * kKpWarps + w) * kKpPer;
+    const int i0 = blockIdx.y * per, i1 = min(a.ncand, i0 + per);
+    int       pid[kKpPer], S[kKpPer], R[kKpPer];
+    float     x[kKpPer], y[kKpPer], z[kKpPer];
+#pragma unroll
+    for (int k = 0; k < kKpPer; k++) {
+        pid[k]         = c0 + k < a.K ? a.kp[c0 + k] : -1;
+        const float4 p = pid[k] >= 0 ? a.pos[pid[k]] : make_float4(0.f, 0.f, 0.f, 0.f);
+        x[k]           = p.x;
+        y[k]           = p.y;
+        z[k]           = p.z;
+        S[k] = R[k] = 0;
+    }
+    for (int t0 = i0; t0 < i1; t0 += kTile) {
+        const int tn = min(kTile, i1 - t0);
         __syncthreads();
         for (int i = threadIdx.x; i < tn; i += blockDim.x) {
-            const int id = a.cand[t0 + i];
-            tid_[i]      = id;
-            tp[i]        = a.pos[id];
+            const int    id = a.cand[t0 + i];
+            const float4 q  = a.pos[id];
+            tp[i]           = make_float4(q.x, q.y, q.z, __int_as_float(id));
         }
         __syncthreads();
-        if (!live)
+        if (pid[0] < 0)
             continue;
         for (int j = 0; j < tn; j += 32) {
-            const int  i   = j + lane;
-            bool       in  = false;
-            bool       row = false;
-            if (i < tn) {
-                const float4 q = tp[i];
-                in             = smm::dist2(p1.x, p1.y, p1.z, q.x, q.y, q.z) < a.sqDiam;
-                row            = in && tid_[i] != pid;
+            const bool   ok = j + lane < tn;
+            const float4 q  = tp[ok ? j + lane : 0];
+            uint32_t     word = 0;
+#pragma unroll
+            for (int k = 0; k < kKpPer; k++) {
+                const bool in = ok && smm::dist2(x[k], y[k], z[k], q.x, q.y, q.z) < a.sqDiam;
+                S[k] += __popc(__ballot_sync(0xffffffffu, in));
+                const uint32_t row =
+                    __ballot_sync(0xffffffffu, in && __float_as_int(q.w) != pid[k]);
+                R[k] += __popc(row);
+                word = lane == k ? row : word;
             }
-            const uint32_t bi = __ballot_sync(0xffffffffu, in);
-            const uint32_t br = __ballot_sync(0xffffffffu, row);
-            S += __popc(bi);
-            R += __popc(br);
-            if (lane == 0)
-                mrow[(t0 + j) >> 5] = br;
+            if (lane < kKpPer && c0 + lane < a.K)
+                b.mask[(size_t)(c0 + lane) * b.words + ((t0 + j) >> 5)] = word;
         }
     }
-    if (!live)
+#pragma unroll
+    for (int k = 0; k < kKpPer; k++)
+        if (lane == k && c0 + k < a.K)
+            b.part[(size_t)blockIdx.y * a.K + c0 + k] = make_int2(S[k], R[k]);
+}
+
+// Radius mode, a warp per keypoint: its counts over the parts, its first tail row, its transform;
+// the row counts (cnt[K] = 0 closes the scan's input), and the per-keypoint hit counters and
+// vote totals cleared for k_ppf.
+__global__ void k_kp_info(VoteArgs a, PipeBufs b, int *__restrict__ cnt) {
+    smd::chain_enter(); // launched chained
+    const int lane = threadIdx.x & 31;
+    const int c    = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (c >= a.K)
         return;
-    __syncwarp();
-    const int tail = tail_from_mask(mrow, b.words, R % smm::kLanes, a.ncand);
-    if (lane == 0) {
-        const float4 n1 = a.nrm[pid];
-        b.info[c]       = kp_info(a, S, R, tail, n1);
-        b.rt[c]         = smm::transform_rt(p1.x, p1.y, p1.z, n1.x, n1.y, n1.z);
+    int S = 0, R = 0;
+    for (int s = lane; s < b.splits; s += 32) {
+        const int2 v = b.part[(size_t)s * a.K + c];
+        S += v.x;
+        R += v.y;
     }
+    S = __reduce_add_sync(0xffffffffu, S);
+    R = __reduce_add_sync(0xffffffffu, R);
+    const int tail = tail_from_mask(b.mask + (size_t)c * b.words, b.words, R % smm::kLanes, a.ncand);
+    if (lane != 0)
+        return;
+    const int    pid = a.kp[c];
+    const float4 p1 = a.pos[pid], n1 = a.nrm[pid];
+    const int4   info = kp_info(a, S, R, tail, n1);
+    b.info[c]         = info;
+    b.rt[c]           = smm::transform_rt(p1.x, p1.y, p1.z, n1.x, n1.y, n1.z);
+    cnt[c]            = info.y;
+    b.hitCnt[c]       = 0;
+    b.votes[c]        = 0ull;
+    b.bound[c]        = 0ull;
+    if (c == 0)
+        cnt[a.K] = 0;
 }
 
 // CSR mode: one warp per keypoint over its list.
@@ -210,79 +247,122 @@ __global__ void k_rows_count(const int4 *__restrict__ info, int K, int *__restri
     }
 }
 
-// The rows of keypoint blockIdx.x into its segment (any order within it).
-__global__ void k_rows_fill(VoteArgs a, PipeBufs b, int csr) {
+// Keypoint blockIdx.x; its 8 x gridDim.y warps take its candidates (CSR: list entries) 128 at a
+// time in turn. A warp packs the rows it finds into its queue (a few of 32 candidates are rows:
+// a lane per candidate would idle) and takes 32 at a time, a lane each, for the PPF key and the
+// table probe; the few hits wait in a second queue for the scene alpha. No barriers: the warps of
+// a CTA share nothing. (8.4 M rows: through a row list in global memory, with the alpha of every
+// row, 51 + 248 us; packed by the whole CTA between barriers 532 us; now 267 us, mostly the
+// issue of the keys' arithmetic, some 700 instructions a row with its divisions and arc tangents.)
+template <bool CSR>
+__global__ void __launch_bounds__(kPpfBs) k_ppf(VoteArgs a, PipeBufs b) {
     smd::chain_enter(); // launched chained
-    __shared__ int sN;
+    constexpr int W = kPpfBs / 32;
+    __shared__ int  rowQ[W][160]; // point * 2 + block lane
+    __shared__ int4 hitQ[W][64];  // {row, bucket offset, count, multiplicity}
     const int  c    = blockIdx.x;
     const int4 info = b.info[c];
     if (info.y == 0)
         return;
-    if (threadIdx.x == 0)
-        sN = 0;
-    __syncthreads();
-    int2     *out  = b.rows + b.rowOff[c];
-    const int pid  = a.kp[c];
-    const int lane = threadIdx.x & 31;
-    if (!csr) {
-        const uint32_t *m = b.mask + (size_t)c * b.words;
-        for (int wi = threadIdx.x; wi < b.words; wi += blockDim.x) {
-            uint32_t wv = m[wi];
-            if (!wv)
-                continue;
-            int p = atomicAdd(&sN, __popc(wv));
-            while (wv) {
-                const int bit = __ffs(wv) - 1;
-                wv &= wv - 1;
-                const int i = wi * 32 + bit;
-                out[p++]    = make_int2(c, a.cand[i] * 2 + (i < info.z ? 1 : 0));
-            }
-        }
-        return;
-    }
-    const int  beg = a.nbrOff[c], len = a.nbrOff[c + 1] - beg;
-    const int *L   = a.nbrIds + beg;
-    for (int i0 = 0; i0 < len; i0 += blockDim.x) {
-        const int      i     = i0 + threadIdx.x;
-        const int      id    = i < len ? L[i] : -1;
-        const bool     row   = i < len && id != pid;
-        const uint32_t m     = __ballot_sync(0xffffffffu, row);
-        int            wbase = 0;
-        if (lane == 0 && m)
-            wbase = atomicAdd(&sN, __popc(m));
-        wbase = __shfl_sync(0xffffffffu, wbase, 0);
-        if (row)
-            out[wbase + __popc(m & ((1u << lane) - 1u))] = make_int2(c, id * 2 + (i < info.z ? 1 : 0));
-    }
-}
+    const int       lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t  below = (1u << lane) - 1u;
+    const int       pid   = a.kp[c];
+    const float4    p1 = a.pos[pid], n1 = a.nrm[pid];
+    const int       beg = CSR ? a.nbrOff[c] : 0;
+    const int       len = CSR ? a.nbrOff[c + 1] - beg : a.ncand;
+    const uint32_t *mask = CSR ? nullptr : b.mask + (size_t)c * b.words;
+    int            *rq   = rowQ[w];
+    int4           *hq   = hitQ[w];
+    int             nr = 0, nh = 0;
+    unsigned long long votes = 0, bound = 0;
 
-// One thread per row: PPF key and scene alpha with the row's lane rule, then the model
-// table probe; hits go to the keypoint's segment.
-__global__ void k_ppf(VoteArgs a, PipeBufs b, const int *__restrict__ total) {
-    smd::chain_enter(); // launched chained
-    const int n = *total;
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-        const int2     row = b.rows[r];
-        const int      c   = row.x;
-        const int      id  = row.y >> 1;
-        const bool     blk = (row.y & 1) != 0;
-        const int      pid = a.kp[c];
-        const float4   p1 = a.pos[pid], n1 = a.nrm[pid];
-        const float4   q = a.pos[id], n2 = a.nrm[id];
-        const smm::RT  rt  = b.rt[c];
-        const uint32_t key = smm::ppf_key(blk, p1.x, p1.y, p1.z, n1.x, n1.y, n1.z, q.x, q.y, q.z,
-                                          n2.x, n2.y, n2.z, a.angleStep, a.distStep);
-        const float as = smm::alpha_of(blk, rt, q.x, q.y, q.z);
-        if (smm::fisnan(as))
-            continue;
-        uint32_t  off = 0, mult = 0;
-        const int cnt = (int)probe(a.htab, a.hmask, key, off, mult);
-        if (cnt > 0) {
-            const int slot               = atomicAdd(&b.hitCnt[c], 1);
-            b.hits[b.rowOff[c] + slot]   = make_int4((int)off, cnt, __float_as_int(as), 0);
-            atomicAdd(&b.votes[c], (unsigned long long)cnt);
-            atomicAdd(&b.bound[c], (unsigned long long)mult);
+    auto take_hits = [&](int n) { // the queue's last n <= 32 hits
+        const int4 v  = lane < n ? hq[nh - n + lane] : make_int4(0, 0, 0, 0);
+        float      as = 0.0f;
+        bool       ok = lane < n;
+        if (ok) {
+            const float4  q  = a.pos[v.x >> 1];
+            const smm::RT rt = b.rt[c];
+            as               = smm::alpha_of((v.x & 1) != 0, rt, q.x, q.y, q.z);
+            ok               = !smm::fisnan(as);
         }
+        nh -= n;
+        const uint32_t m    = __ballot_sync(0xffffffffu, ok);
+        int            base = 0;
+        if (lane == 0 && m)
+            base = atomicAdd(&b.hitCnt[c], __popc(m));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (ok) {
+            b.hits[b.rowOff[c] + base + __popc(m & below)] =
+                make_int4(v.y, v.z, __float_as_int(as), 0);
+            votes += (unsigned)v.z;
+            bound += (unsigned)v.w;
+        }
+    };
+    auto take_rows = [&](int n) { // the queue's last n <= 32 rows
+        uint32_t off = 0, mult = 0;
+        int      cnt = 0, row = 0;
+        if (lane < n) {
+            row                = rq[nr - n + lane];
+            const float4   p2 = a.pos[row >> 1], n2 = a.nrm[row >> 1];
+            const uint32_t key =
+                smm::ppf_key((row & 1) != 0, p1.x, p1.y, p1.z, n1.x, n1.y, n1.z, p2.x, p2.y, p2.z,
+                             n2.x, n2.y, n2.z, a.angleStep, a.distStep);
+            cnt = (int)probe(a.htab, a.hmask, key, off, mult);
+        }
+        nr -= n;
+        const uint32_t m = __ballot_sync(0xffffffffu, cnt > 0);
+        if (cnt > 0)
+            hq[nh + __popc(m & below)] = make_int4(row, (int)off, cnt, (int)mult);
+        nh += __popc(m); // (below 32 before: 64 entries hold it)
+        __syncwarp();
+        if (nh >= 32)
+            take_hits(32);
+        __syncwarp(); // (the queues' places are written again after their reads)
+    };
+
+    const int step = gridDim.y * W * 128;
+    for (int i0 = (blockIdx.y * W + w) * 128; i0 < len; i0 += step) {
+        uint32_t m[4];
+        int      id[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) { // the loads of 128 candidates in flight
+            const int i = i0 + k * 32 + lane;
+            if (CSR)
+                id[k] = i < len ? a.nbrIds[beg + i] : pid;
+            else
+                m[k] = i0 + k * 32 < len ? mask[(i0 >> 5) + k] : 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (CSR)
+                m[k] = __ballot_sync(0xffffffffu, id[k] != pid);
+            else if ((m[k] >> lane) & 1u)
+                id[k] = a.cand[i0 + k * 32 + lane];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if ((m[k] >> lane) & 1u)
+                rq[nr + __popc(m[k] & below)] =
+                    id[k] * 2 + (i0 + k * 32 + lane < info.z ? 1 : 0);
+            nr += __popc(m[k]); // (below 32 before: 160 entries hold 128 more)
+        }
+        __syncwarp();
+        while (nr >= 32)
+            take_rows(32);
+    }
+    if (nr > 0)
+        take_rows(nr);
+    if (nh > 0)
+        take_hits(nh);
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+        votes += __shfl_xor_sync(0xffffffffu, votes, o);
+        bound += __shfl_xor_sync(0xffffffffu, bound, o);
+    }
+    if (lane == 0 && votes) {
+        atomicAdd(&b.votes[c], votes);
+        atomicAdd(&b.bound[c], bound);
     }
 }
 
@@ -544,19 +624,34 @@ void vote(Ctx &c, const Model &m, const float4 *pos, const float4 *nrm, const in
     b.order  = c.arena.get<int>("v.order", K);
     b.next   = c.arena.get<int>("v.next", 1);
     int *cnt = c.arena.get<int>("v.rowcnt", (size_t)K + 1);
-    if (csr)
+    int  nsm = 0;
+    SM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device));
+    if (csr) {
         launch_chained(c, k_kp_csr, nblocks((long long)K * 32, 256), 256, 0, a, b);
-    else
-        launch_chained(c, k_kp_radius, nblocks(K, kKpWarps), kKpWarps * 32, 0, a, b);
-    launch_chained(c, k_rows_count, nblocks(K, 256), 256, 0, b.info, K, cnt, b);
+        launch_chained(c, k_rows_count, nblocks(K, 256), 256, 0, b.info, K, cnt, b);
+    } else {
+        // parts of the candidate list (whole mask words, 256 candidates at least) so that some
+        // four CTAs per SM run
+        const int gx   = nblocks(K, kKpPer * kKpWarps);
+        const int want = std::max(1, std::min(nblocks(ncand, 256), nblocks(4LL * nsm, gx)));
+        const int per  = nblocks(nblocks(ncand, want), 32) * 32;
+        b.splits       = std::max(1, nblocks(ncand, per));
+        b.part         = c.arena.get<int2>("v.part", (size_t)b.splits * K);
+        launch_chained(c, k_kp_radius, dim3(gx, b.splits), kKpWarps * 32, 0, a, b, per);
+        launch_chained(c, k_kp_info, nblocks((long long)K * 32, 256), 256, 0, a, b, cnt);
+    }
     const int rtot = scan_excl(c, cnt, b.rowOff, (long long)K + 1, "v.scan", true);
-    b.rows = c.arena.get<int2>("v.rows", std::max(rtot, 1));
     b.hits = c.arena.get<int4>("v.hits", std::max(rtot, 1));
-    launch_chained(c, k_rows_fill, K, 256, 0, a, b, csr ? 1 : 0);
     SM_CUDA(cudaEventRecord(c.ev[10], c.stream));
     if (rtot > 0) {
-        const int g = (int)std::min<long long>(nblocks(rtot, 256), 152LL * 8);
-        launch_chained(c, k_ppf, g, 256, 0, a, b, b.rowOff + K);
+        // several CTAs per keypoint where the keypoints would not fill the SMs (for CSR lists as
+        // far as the rows could need them)
+        const int most = nblocks(csr ? rtot : ncand, 128 * (kPpfBs / 32));
+        const int gy   = std::max(1, std::min(most, nblocks(4LL * nsm, K)));
+        if (csr)
+            launch_chained(c, k_ppf<true>, dim3(K, gy), kPpfBs, 0, a, b);
+        else
+            launch_chained(c, k_ppf<false>, dim3(K, gy), kPpfBs, 0, a, b);
     }
     SM_CUDA(cudaEventRecord(c.ev[11], c.stream));
     launch_chained(c, k_lpt, 1, 1024, 0, b.votes, K, b.order, b.next);

@@ -116,6 +116,50 @@ __global__ void k_gather_poses(const float *__restrict__ poses, const int *__res
         out[(size_t)i * smi::kPoseFloats + e] = poses[(size_t)s * smi::kPoseFloats + e];
 }
 
+// What the host reads of a match, in one buffer: {pairs, hits, votes} (int64) over the keypoints'
+// statistics rows, then per candidate its status, score and pose (14 words).
+constexpr int kResultHead = 6; // 32-bit words
+constexpr int kResultCand = 14;
+
+__global__ void __launch_bounds__(256)
+    k_pack_result(const long long *__restrict__ kst, int K, const int *__restrict__ status,
+                  const float *__restrict__ score, const float *__restrict__ pose, int ncand,
+                  int *__restrict__ out) {
+    smd::chain_enter(); // launched chained
+    if (blockIdx.x > 0) {
+        const int t = (blockIdx.x - 1) * blockDim.x + threadIdx.x;
+        if (t >= ncand * kResultCand)
+            return;
+        const int ci = t / kResultCand, e = t % kResultCand;
+        out[kResultHead + t] = e == 0   ? status[ci]
+                               : e == 1 ? __float_as_int(score[ci])
+                                        : __float_as_int(pose[(size_t)ci * 12 + e - 2]);
+        return;
+    }
+    __shared__ unsigned long long sum[3];
+    if (threadIdx.x < 3)
+        sum[threadIdx.x] = 0ull;
+    __syncthreads();
+    unsigned long long v[3] = {0, 0, 0};
+    for (int k = threadIdx.x; k < K; k += blockDim.x) {
+        const long long *st = kst + (size_t)k * 8;
+        if (st[1] == 0)
+            v[0] += (unsigned long long)(st[0] - 1);
+        v[1] += (unsigned long long)st[2];
+        v[2] += (unsigned long long)st[3];
+    }
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1)
+        for (int e = 0; e < 3; e++)
+            v[e] += __shfl_xor_sync(0xffffffffu, v[e], o);
+    if ((threadIdx.x & 31) == 0)
+        for (int e = 0; e < 3; e++)
+            atomicAdd(&sum[e], v[e]);
+    __syncthreads();
+    if (threadIdx.x < 3)
+        reinterpret_cast<unsigned long long *>(out)[threadIdx.x] = sum[threadIdx.x];
+}
+
 __global__ void k_rank_of(const int *__restrict__ ids, int m, const int *__restrict__ treePos,
                           int *__restrict__ rank, int *__restrict__ tpos) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
@@ -409,7 +453,7 @@ Ctx &aux_ctx(Ctx &c) {
         SM_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
         SM_CUDA(cudaStreamCreateWithPriority(&a->stream, cudaStreamNonBlocking, greatest));
         a->ownStream = true;
-        SM_CUDA(cudaMallocHost((void **)&a->hostCounts, 64 * sizeof(int)));
+        SM_CUDA(cudaMallocHost((void **)&a->hostCounts, kHostInts * sizeof(int)));
         for (auto &e : a->ev)
             SM_CUDA(cudaEventCreate(&e));
         a->arena.set_stream(a->stream, c.device);
@@ -709,13 +753,20 @@ void match(Ctx &c, const Model &m, const float *xyzIn, const float *nrmIn, int64
     float *cpose  = c.arena.get<float>("m.cpose", (size_t)std::max(ncand, 1) * 12);
     float *ctrace = c.arena.get<float>("m.ctrace", (size_t)std::max(ncand, 1) * kIcpTraceFloats);
     icp_all(c, m, s, ip, cands, ncand, cstat, cscore, cpose, ctrace);
-    std::vector<int>   hs(ncand);
-    std::vector<float> hsc(ncand), hp((size_t)ncand * 12);
-    if (ncand) {
-        SM_CUDA(cudaMemcpyAsync(hs.data(), cstat, ncand * 4, cudaMemcpyDeviceToHost, c.stream));
-        SM_CUDA(cudaMemcpyAsync(hsc.data(), cscore, ncand * 4, cudaMemcpyDeviceToHost, c.stream));
-        SM_CUDA(cudaMemcpyAsync(hp.data(), cpose, (size_t)ncand * 48, cudaMemcpyDeviceToHost, c.stream));
+    // one copy of everything the host needs, to page-locked memory where it fits (a copy to
+    // pageable memory waits for the stream by itself: three of them and the statistics rows,
+    // read after the last wait, took some 40 us a call)
+    const size_t words = kResultHead + (size_t)ncand * kResultCand;
+    int         *dres  = c.arena.get<int>("m.result", words);
+    launch_chained(c, k_pack_result, 1 + nblocks((long long)ncand * kResultCand, 256), 256, 0,
+                   vo.stats, K, cstat, cscore, cpose, ncand, dres);
+    std::vector<int> big;
+    int             *hres = c.hostCounts + kHostResult;
+    if (words > kHostInts - kHostResult) {
+        big.resize(words);
+        hres = big.data();
     }
+    SM_CUDA(cudaMemcpyAsync(hres, dres, words * 4, cudaMemcpyDeviceToHost, c.stream));
     record(c, 7);
     c.sync_checked();
     if (c.clock.on) {
@@ -733,20 +784,28 @@ void match(Ctx &c, const Model &m, const float *xyzIn, const float *nrmIn, int64
             c.aux->clock.resolve();
     }
     // selection walk (ppf.cpp:439-495) and ordering by score (ppf.cpp:498-507)
+    auto             cand = [&](int i) { return hres + kResultHead + (size_t)i * kResultCand; };
+    auto             hsc  = [&](int i) {
+        float v;
+        memcpy(&v, cand(i) + 1, 4);
+        return v;
+    };
     std::vector<int> acc;
     for (int i = 0; i < ncand; i++) {
-        if (hs[i] != 0)
+        if (cand(i)[0] != 0)
             continue;
         acc.push_back(i);
         if ((int)acc.size() >= mp.numMatches)
             break;
     }
-    std::stable_sort(acc.begin(), acc.end(), [&](int a, int b) { return hsc[a] > hsc[b]; });
+    std::stable_sort(acc.begin(), acc.end(), [&](int a, int b) { return hsc(a) > hsc(b); });
     res.pose.clear();
     res.score.clear();
     for (int i : acc) {
-        res.pose.insert(res.pose.end(), hp.begin() + (size_t)i * 12, hp.begin() + (size_t)i * 12 + 12);
-        res.score.push_back(hsc[i]);
+        float p[12];
+        memcpy(p, cand(i) + 2, sizeof(p));
+        res.pose.insert(res.pose.end(), p, p + 12);
+        res.score.push_back(hsc(i));
     }
     c.last.n     = n;
     c.last.ns    = ns;
@@ -765,15 +824,11 @@ void match(Ctx &c, const Model &m, const float *xyzIn, const float *nrmIn, int64
         stats->n_resampled = nres;
         stats->n_poses     = np;
         stats->n_clusters  = ncand;
-        std::vector<long long> st((size_t)K * 8);
-        if (K)
-            SM_CUDA(cudaMemcpy(st.data(), vo.stats, (size_t)K * 64, cudaMemcpyDeviceToHost));
-        for (int k = 0; k < K; k++) {
-            if (st[(size_t)k * 8 + 1] == 0)
-                stats->n_pairs += st[(size_t)k * 8] - 1;
-            stats->n_hits += st[(size_t)k * 8 + 2];
-            stats->n_votes += st[(size_t)k * 8 + 3];
-        }
+        long long sums[3];
+        memcpy(sums, hres, sizeof(sums));
+        stats->n_pairs = sums[0];
+        stats->n_hits  = sums[1];
+        stats->n_votes = sums[2];
         const int stage[8][2] = {{0, 1}, {1, 2}, {2, 3}, {8, 9}, {4, 5}, {5, 6}, {6, 7}, {0, 7}};
         for (int i = 0; i < 8; i++)
             SM_CUDA(cudaEventElapsedTime(&stats->ms[i], c.ev[stage[i][0]], c.ev[stage[i][1]]));
@@ -949,7 +1004,7 @@ SM_API int sm_context_create(int device, void *stream, sm_context *out) {
             SM_CUDA(cudaStreamCreateWithFlags(&c->ctx.stream, cudaStreamNonBlocking));
             c->ctx.ownStream = true;
         }
-        SM_CUDA(cudaMallocHost((void **)&c->ctx.hostCounts, 64 * sizeof(int)));
+        SM_CUDA(cudaMallocHost((void **)&c->ctx.hostCounts, kHostInts * sizeof(int)));
         for (auto &e : c->ctx.ev)
             SM_CUDA(cudaEventCreate(&e));
         c->ctx.arena.set_stream(c->ctx.stream, device);

@@ -43,7 +43,7 @@ std::unique_ptr<Ctx> acquire_worker(int device) {
     SM_CUDA(cudaSetDevice(device));
     SM_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     c->ownStream = true;
-    SM_CUDA(cudaMallocHost((void **)&c->hostCounts, 64 * sizeof(int)));
+    SM_CUDA(cudaMallocHost((void **)&c->hostCounts, kHostInts * sizeof(int)));
     for (auto &e : c->ev)
         SM_CUDA(cudaEventCreate(&e));
     c->arena.set_stream(c->stream, device);

@@ -166,6 +166,11 @@ struct KernelClock {
     }
 };
 
+// A context's page-locked scratch, in ints: counts first, from kHostResult on a match's results
+// (some 1100 candidates).
+constexpr int kHostResult = 64;
+constexpr int kHostInts   = kHostResult + 16384;
+
 struct Ctx {
     int          device    = 0;
     cudaStream_t stream    = nullptr;

@@ -543,14 +543,15 @@ void match(Ctx &c, const Model &m, const float *xyzIn, const float *nrmIn, int64
     // reference order: the scene's k-d tree (ppf.cpp:197) over the valid points; `ioi` is
     // its reduce() array of the sampled points (ppf.cpp:201-213)
     KdTree      T;
-    int        *ioi = nullptr;
-    int         ns  = 0;
+    int        *ioi    = nullptr;
+    const int  *before = nullptr; // sampled points below each tree position
+    int         ns     = 0;
     HGrid       q;
     float       gq  = 0.0f;
     if (ref) {
         build_kdtree(c, pos, n, valid, nvalid, box, T, "m.tree");
         ioi = c.arena.get<int>("m.ioi", std::max(nvalid, 1));
-        ns  = kd_sample(c, T, nullptr, pos, sampleStep, box, sampled, ioi, "m.s1");
+        ns  = kd_sample(c, T, nullptr, pos, sampleStep, box, sampled, ioi, "m.s1", &before);
     } else {
         ns = sample_points(c, pos, n, valid, nvalid, box, sampleStep, sampled, "m.s1");
     }
@@ -708,11 +709,11 @@ void match(Ctx &c, const Model &m, const float *xyzIn, const float *nrmIn, int64
     vo.acc    = nullptr;
     record(c, 8);
     if (ref) {
-        // the keypoints' radius searches in the reduced tree, tail rows last (ppf.cpp:273-299)
-        int        *off = nullptr, *ids = nullptr;
-        const float dm  = m.box.diameter();
-        kd_vote_lists(c, T, ioi, pos, kp, K, sampled, ns, dm * dm, &off, &ids, "m.rl");
-        vote(c, m, pos, nrm, kp, K, off, ids, nullptr, 0, minScore, vo, 0);
+        // the keypoints' radius searches in the reduced tree (ppf.cpp:273-299)
+        VoteTree    vt;
+        const float dm = m.box.diameter();
+        kd_vote_tree(c, T, ioi, pos, sampled, ns, before, dm * dm, vt, "m.vt");
+        vote(c, m, pos, nrm, kp, K, nullptr, nullptr, sampled, ns, minScore, vo, 0, &vt);
     } else {
         vote(c, m, pos, nrm, kp, K, nullptr, nullptr, sampled, ns, minScore, vo, 0);
     }

@@ -988,139 +988,22 @@ __global__ void __launch_bounds__(kKnnBs)
         L.add_neighbour(lane < n, id, nrm);
 }
 
-// ---- the voting stage's radius searches (ppf.cpp:273-276) -------------------------------
-constexpr int kRlBs  = 256;
-constexpr int kTailN = 7; // rows % 8 < 8
-
-struct TailKey {
-    uint64_t key;
-    int                pos, cand; // tree position, candidate index
-};
-__device__ __forceinline__ bool tail_after(const TailKey &a, const TailKey &b) {
-    return a.key > b.key || (a.key == b.key && a.pos > b.pos);
-}
-
-// One CTA per keypoint over the candidates (the sampled points): membership of the radius
-// search of radius^2 r2 in the reduced tree (distance and the search's pruning), as a
-// bitmask over the candidate list; the member count; and the candidates of the last
-// (rows mod 8) rows other than the keypoint itself in the search's depth-first order -
-// the rows the reference evaluates one by one after its 8-lane blocks.
-__global__ void __launch_bounds__(kRlBs)
-    k_kd_radius(KdView t, const int *__restrict__ treePos, const int *__restrict__ kp, int K,
-                const int *__restrict__ cand, int ncand, float r2, uint32_t *__restrict__ mask,
-                int words, int *__restrict__ count, int *__restrict__ tail) {
-    __shared__ TailKey sk[kRlBs];
-    __shared__ int     sh[33];
-    const int c = blockIdx.x;
-    if (c >= K)
+// ---- the voting stage's candidates (ppf.cpp:273-276) --------------------------------------
+// Candidate r (id cand[r], the reduced tree's r-th point): its tree position, and the squared
+// distance below which a radius search of radius^2 r2 surely reaches it: the search's bound
+// above the point's leaf is at most (distance + excursion)^2 (as in `reaches`).
+__global__ void k_kd_cands(const int *__restrict__ cand, int n, const int *__restrict__ treePos,
+                           const float4 *__restrict__ pos, const float *__restrict__ nodeBox,
+                           const int *__restrict__ leafOf, float r2, int *__restrict__ posOf,
+                           float *__restrict__ sure) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= n)
         return;
-    const int    pid  = kp[c];
-    const float4 p    = t.pos[pid];
-    const float  q[3] = {p.x, p.y, p.z};
-    TailKey      top[kTailN];
-    for (int k = 0; k < kTailN; k++)
-        top[k] = TailKey{0ull, -1, -1};
-    int       nTop = 0, S = 0;
-    bool      self = false;
-    uint32_t *mrow = mask + (size_t)c * words;
-    for (int j0 = 0; j0 < ncand; j0 += kRlBs) {
-        const int j   = j0 + threadIdx.x;
-        bool      mem = false;
-        if (j < ncand) {
-            const int id = cand[j];
-            const float d = smk::eval_metric(q, t.pos[id]);
-            if (d < r2) {
-                const int ip = treePos[id];
-                uint64_t  key;
-                mem = smk::kd_reaches(t, q, ip, r2, &key);
-                self = self || (mem && id == pid);
-                if (mem && id != pid) {
-                    TailKey e{key, ip, j};
-                    // keep the kTailN latest in search order, sorted latest first
-                    int at = nTop < kTailN ? nTop : kTailN;
-                    while (at > 0 && tail_after(e, top[at - 1]))
-                        at--;
-                    if (at < kTailN) {
-                        for (int k = (nTop < kTailN ? nTop : kTailN - 1); k > at; k--)
-                            top[k] = top[k - 1];
-                        top[at] = e;
-                        if (nTop < kTailN)
-                            nTop++;
-                    }
-                }
-            }
-        }
-        const uint32_t b = __ballot_sync(0xffffffffu, mem);
-        if ((threadIdx.x & 31) == 0 && ((j0 + threadIdx.x) >> 5) < words)
-            mrow[(j0 + threadIdx.x) >> 5] = b;
-        S += mem ? 1 : 0;
-    }
-    int tot;
-    block_excl_scan(S, sh, &tot);
-    // rows = the members other than the keypoint (which its own search finds)
-    const int rows = tot - (__syncthreads_or(self ? 1 : 0) ? 1 : 0);
-    const int need = rows % 8;
-    // the `need` latest rows: rounds of a block-wide maximum over the threads' lists
-    int head = 0;
-    for (int r = 0; r < need; r++) {
-        sk[threadIdx.x] = head < nTop ? top[head] : TailKey{0ull, -1, -1};
-        __syncthreads();
-        for (int o = kRlBs / 2; o > 0; o >>= 1) {
-            if (threadIdx.x < o && tail_after(sk[threadIdx.x + o], sk[threadIdx.x]))
-                sk[threadIdx.x] = sk[threadIdx.x + o];
-            __syncthreads();
-        }
-        const TailKey w = sk[0];
-        if (head < nTop && top[head].pos == w.pos && top[head].cand == w.cand)
-            head++;
-        if (threadIdx.x == 0)
-            tail[(size_t)c * kTailN + r] = w.cand;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        count[c] = tot;
-        for (int r = need; r < kTailN; r++)
-            tail[(size_t)c * kTailN + r] = -1;
-    }
-}
-
-// The CSR list of keypoint blockIdx.x: its members in candidate order except the tail
-// rows, then the tail rows (the voting stage marks the last rows % 8 rows of a list as the
-// reference's one-by-one rows).
-__global__ void __launch_bounds__(kRlBs)
-    k_kd_fill(const uint32_t *__restrict__ mask, int words, const int *__restrict__ cand,
-              int ncand, const int *__restrict__ off, const int *__restrict__ tail,
-              int *__restrict__ ids) {
-    __shared__ int sh[33];
-    __shared__ int sT[kTailN];
-    const int c = blockIdx.x;
-    if (threadIdx.x < kTailN)
-        sT[threadIdx.x] = tail[(size_t)c * kTailN + threadIdx.x];
-    __syncthreads();
-    int nt = 0;
-    for (int k = 0; k < kTailN; k++)
-        nt += sT[k] >= 0 ? 1 : 0;
-    const uint32_t *mrow = mask + (size_t)c * words;
-    int            *out  = ids + off[c];
-    const int       len  = off[c + 1] - off[c];
-    int             base = 0;
-    for (int j0 = 0; j0 < ncand; j0 += kRlBs) {
-        const int j  = j0 + threadIdx.x;
-        bool      in = j < ncand && ((mrow[j >> 5] >> (j & 31)) & 1u);
-        if (in)
-            for (int k = 0; k < kTailN; k++)
-                if (sT[k] == j)
-                    in = false;
-        int       tot;
-        const int ex = block_excl_scan(in ? 1 : 0, sh, &tot);
-        if (in)
-            out[base + ex] = cand[j];
-        base += tot;
-    }
-    // the tail rows last, in search order (earliest first)
-    if (threadIdx.x == 0)
-        for (int k = nt - 1, o = len - nt; k >= 0; k--, o++)
-            out[o] = cand[sT[k]];
+    const int    id = cand[r], ip = treePos[id];
+    const double s = sqrt((double)r2 * (1.0 - 1e-4)) -
+                     excursion(nodeBox + 6 * (size_t)leafOf[ip], pos[id]);
+    posOf[r]       = ip;
+    sure[r]        = s > 0.0 ? (float)(s * s * (1.0 - 1e-6)) : 0.0f;
 }
 
 // Leaves holding an active position flag themselves and their ancestors (a walk stops at
@@ -1253,7 +1136,7 @@ void build_kdtree(Ctx &c, const float4 *pos, int npoints, const int *ids, int m,
 }
 
 int kd_sample(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos, float step,
-              const Box &box, int *outIds, int *ioi, const std::string &tag) {
+              const Box &box, int *outIds, int *ioi, const std::string &tag, const int **before) {
     const int m = T.m;
     if (m <= 0)
         return 0;
@@ -1326,6 +1209,8 @@ int kd_sample(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
     SM_LAUNCH_CHECK();
     int *pre = c.arena.get<int>(tag + ".pre", (size_t)m + 1);
     scan_excl(c, flag, pre, (long long)m + 1, tag + ".os", false);
+    if (before)
+        *before = pre;
     k_sp_out<<<nblocks(m, 256), 256, 0, c.stream>>>(flag, pre, m, vaccA, outIds, ioi);
     SM_LAUNCH_CHECK();
     SM_CUDA(cudaMemcpyAsync(c.hostCounts, pre + m, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
@@ -1363,30 +1248,22 @@ void kd_knn_points(Ctx &c, const KdTree &T, const HGrid &g, const float4 *pos,
     SM_LAUNCH_CHECK();
 }
 
-int kd_vote_lists(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
-                  const int *kp, int K, const int *cand, int ncand, float r2, int **offOut,
-                  int **idsOut, const std::string &tag) {
-    int *off = c.arena.get<int>(tag + ".off", (size_t)K + 1);
-    *offOut  = off;
-    if (K <= 0) {
-        *idsOut = c.arena.get<int>(tag + ".ids", 1);
-        return 0;
-    }
-    const int words = std::max((ncand + 31) / 32, 1);
-    uint32_t *mask  = c.arena.get<uint32_t>(tag + ".mask", (size_t)K * words);
-    int      *cnt   = c.arena.get<int>(tag + ".cnt", (size_t)K + 1);
-    int      *tail  = c.arena.get<int>(tag + ".tail", (size_t)K * kTailN);
-    SM_CUDA(cudaMemsetAsync(mask, 0, (size_t)K * words * 4, c.stream));
-    SM_CUDA(cudaMemsetAsync(cnt + K, 0, sizeof(int), c.stream));
-    k_kd_radius<<<K, kRlBs, 0, c.stream>>>(T.view(vaccActive, pos), T.treePos, kp, K, cand, ncand,
-                                            r2, mask, words, cnt, tail);
+void kd_vote_tree(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
+                  const int *cand, int ncand, const int *before, float r2, VoteTree &V,
+                  const std::string &tag) {
+    int   *posOf = c.arena.get<int>(tag + ".pos", std::max(ncand, 1));
+    float *sure  = c.arena.get<float>(tag + ".sure", std::max(ncand, 1));
+    V.view       = T.view(vaccActive, pos);
+    V.m          = T.m;
+    V.treePos    = T.treePos;
+    V.posOf      = posOf;
+    V.before     = before;
+    V.sure       = sure;
+    if (ncand <= 0)
+        return;
+    k_kd_cands<<<nblocks(ncand, 256), 256, 0, c.stream>>>(cand, ncand, T.treePos, pos, T.box,
+                                                          T.leafOf, r2, posOf, sure);
     SM_LAUNCH_CHECK();
-    const int total = scan_excl(c, cnt, off, (long long)K + 1, tag + ".scan", true);
-    int      *ids   = c.arena.get<int>(tag + ".ids", std::max(total, 1));
-    *idsOut         = ids;
-    k_kd_fill<<<K, kRlBs, 0, c.stream>>>(mask, words, cand, ncand, off, tail, ids);
-    SM_LAUNCH_CHECK();
-    return total;
 }
 
 void kd_mark_nonempty(Ctx &c, const KdTree &T, const int *vaccActive, int *flags) {

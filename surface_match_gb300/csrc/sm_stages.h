@@ -309,11 +309,13 @@ void build_kdtree(Ctx &c, const float4 *pos, int npoints, const int *ids, int m,
 // samplePointCloud (util.cpp:107-139) on the tree: greedy thinning at `step` in tree
 // position order over the positions whose vaccActive entry is >= 0 (the reduce()d tree),
 // distances on the live positions `pos`. Writes the kept ids in tree order to outIds and,
-// when ioi is given, the reduce() array (kept point id per tree position, else -1).
+// when ioi is given, the reduce() array (kept point id per tree position, else -1); *before
+// (nullable): how many are kept below each tree position (T.m + 1 values, in the workspace).
 // Returns the number kept. `box` bounds the grid that buckets the points (points outside
 // are clamped into its border cells).
 int kd_sample(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos, float step,
-              const Box &box, int *outIds, int *ioi, const std::string &tag);
+              const Box &box, int *outIds, int *ioi, const std::string &tag,
+              const int **before = nullptr);
 // KNNResultSet searches (nanoflann findNeighbors) on the tree, one per query: query t at
 // qpos[t] for t < *nq (a device count, nqMax bounds the launch); nbr[t*k + j] / dist[t*k + j]
 // its j-th nearest.
@@ -334,14 +336,20 @@ void kd_mark_nonempty(Ctx &c, const KdTree &T, const int *vaccActive, int *flags
 // build-time boxes (smk::nn_bound).
 void kd_tree_positions(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
                        float4 *tpos, float *excMax = nullptr);
-// The voting stage's radius searches (ppf.cpp:273-276) in the reduced tree: for each of the
-// K keypoints the candidates (cand[0..ncand), the sampled points) its search of radius^2 r2
-// returns, as CSR lists (*offOut: K + 1 offsets, *idsOut: ids) whose last (rows mod 8) rows
-// other than the keypoint are the search's last ones in depth-first order (the reference's
-// scalar-tail rows); the rest in candidate order. Returns the total list length.
-int kd_vote_lists(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
-                  const int *kp, int K, const int *cand, int ncand, float r2, int **offOut,
-                  int **idsOut, const std::string &tag);
+// The reduced tree over the voting stage's candidates (cand[0..ncand), the points of vaccActive
+// in tree order; before[i] of them at tree positions below i, T.m + 1 values), for radius
+// searches of radius^2 r2.
+struct VoteTree {
+    smk::KdView  view;
+    int          m       = 0;       // tree positions
+    const int   *treePos = nullptr; // per point id: its tree position
+    const int   *posOf   = nullptr; // per candidate: its tree position
+    const int   *before  = nullptr;
+    const float *sure    = nullptr; // per candidate: closer than this (squared), a search reaches it
+};
+void kd_vote_tree(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
+                  const int *cand, int ncand, const int *before, float r2, VoteTree &V,
+                  const std::string &tag);
 
 // ---- mls.cu ---------------------------------------------------------------------------
 constexpr int kMlsMaxOrder = 4; // largest polynomial order of the MLS fit
@@ -364,10 +372,11 @@ struct VoteOut {
 };
 // Voting for K keypoints with neighbours either given as CSR lists (nbrOff/nbrIds) or, when
 // nbrOff == nullptr, all points of `cand[0..ncand)` within the model diameter in ascending
-// order.
+// order; with `tree`, those that its radius searches of that radius find, the last ones in its
+// depth-first order taking the scalar tail's place.
 void vote(Ctx &c, const Model &m, const float4 *pos, const float4 *nrm, const int *kp, int K,
           const int *nbrOff, const int *nbrIds, const int *cand, int ncand, float minScore,
-          const VoteOut &out, int dumpK);
+          const VoteOut &out, int dumpK, const VoteTree *tree = nullptr);
 // The same from CSR lists in a single kernel that needs no workspace (same results).
 void vote_fused(Ctx &c, const Model &m, const float4 *pos, const float4 *nrm, const int *kp,
                 int K, const int *nbrOff, const int *nbrIds, float minScore, const VoteOut &out,

@@ -6,7 +6,9 @@
 //     reference computes a keypoint's rows in 8-lane blocks and the last (rows mod 8) one by
 //     one, with different float rounding. In radius mode (all candidates within the model
 //     diameter, in ascending order) the rows are kept as a bitmask over the candidate list,
-//     computed from candidate tiles staged in shared memory and shared by 32 keypoints.
+//     computed from candidate tiles staged in shared memory and shared by 32 keypoints. In
+//     reference order a candidate is a neighbour when the k-d tree's radius search reaches it,
+//     and the tail rows are the last ones in the search's depth-first order.
 //  2. A prefix sum over the rows gives every keypoint a segment of the hit list.
 //  3. k_ppf: a CTA per keypoint (several where keypoints are few), each warp packing rows from
 //     its share of the candidates until it has 32: quantised PPF key and model table probe by a
@@ -22,6 +24,7 @@
 #include <cstring>
 #include <mutex>
 
+#include "sm_kdtree.cuh"
 #include "sm_stages.h"
 #include "sm_vote.cuh"
 
@@ -52,6 +55,8 @@ struct PipeBufs {
     int                 words;
     int                 splits;  // radius mode: parts of the candidate list
     int2               *part;    // splits x K: {neighbours, rows} in the part
+    VoteTree            tree;    // reference order
+    int                *tail;    // reference order: K x 8, the tail rows' candidates (else -1)
     int                *rowOff;  // K + 1
     int4               *hits;    // per row segment: {bucket offset, count, alpha bits, 0}
     int                *hitCnt;  // K
@@ -108,24 +113,39 @@ __device__ __forceinline__ int tail_from_mask(const uint32_t *m, int nw, int nee
 }
 
 // Radius mode, part blockIdx.y of the candidates: kKpPer keypoints per warp over shared-memory
-// tiles of the candidates' positions (id in w). The parts make CTAs enough: with one CTA per
-// eight keypoints over all candidates, 2390 keypoints x 18,069 candidates took 145 us, now 54 us.
+// tiles of the candidates' positions. The parts make CTAs enough: with one CTA per eight
+// keypoints over all candidates, 2390 keypoints x 18,069 candidates took 145 us, now 54 us.
+//
+// TREE: a candidate nearer than its `sure` distance is reached; one between that and the radius
+// waits in the warp's queue for the walk down its root path (smk::kd_reaches), a lane each 32 at
+// a time. (A CTA per keypoint walking the path of every candidate within the radius took 1470 us
+// for 2489 keypoints x 18,248 candidates, and the neighbour lists made from it another 170 us.)
+template <bool TREE>
 __global__ void __launch_bounds__(kKpWarps * 32) k_kp_radius(VoteArgs a, PipeBufs b, int per) {
     smd::chain_enter(); // launched chained
-    __shared__ float4 tp[kTile];
+    __shared__ float4   tp[kTile]; // w: candidate id, TREE: its sure distance
+    __shared__ uint32_t words[kKpWarps][kKpPer][TREE ? kTile / 32 : 1];
+    __shared__ int      queue[kKpWarps][TREE ? 32 * kKpPer + 32 : 1]; // keypoint << 16 | place
+    __shared__ float    kx[kKpWarps][kKpPer][3];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int c0   = (blockIdx.x * kKpWarps + w) * kKpPer;
     const int i0 = blockIdx.y * per, i1 = min(a.ncand, i0 + per);
-    int       pid[kKpPer], S[kKpPer], R[kKpPer];
+    int       self[kKpPer], S[kKpPer], R[kKpPer]; // self: the keypoint's id, TREE: its candidate
     float     x[kKpPer], y[kKpPer], z[kKpPer];
 #pragma unroll
     for (int k = 0; k < kKpPer; k++) {
-        pid[k]         = c0 + k < a.K ? a.kp[c0 + k] : -1;
-        const float4 p = pid[k] >= 0 ? a.pos[pid[k]] : make_float4(0.f, 0.f, 0.f, 0.f);
-        x[k]           = p.x;
-        y[k]           = p.y;
-        z[k]           = p.z;
+        const int    pid = c0 + k < a.K ? a.kp[c0 + k] : -1;
+        const float4 p   = pid >= 0 ? a.pos[pid] : make_float4(0.f, 0.f, 0.f, 0.f);
+        self[k]          = TREE && pid >= 0 ? b.tree.before[b.tree.treePos[pid]] : pid;
+        x[k]             = p.x;
+        y[k]             = p.y;
+        z[k]             = p.z;
         S[k] = R[k] = 0;
+        if (TREE && lane == 0) {
+            kx[w][k][0] = p.x;
+            kx[w][k][1] = p.y;
+            kx[w][k][2] = p.z;
+        }
     }
     for (int t0 = i0; t0 < i1; t0 += kTile) {
         const int tn = min(kTile, i1 - t0);
@@ -133,38 +153,160 @@ __global__ void __launch_bounds__(kKpWarps * 32) k_kp_radius(VoteArgs a, PipeBuf
         for (int i = threadIdx.x; i < tn; i += blockDim.x) {
             const int    id = a.cand[t0 + i];
             const float4 q  = a.pos[id];
-            tp[i]           = make_float4(q.x, q.y, q.z, __int_as_float(id));
+            tp[i] = make_float4(q.x, q.y, q.z, TREE ? b.tree.sure[t0 + i] : __int_as_float(id));
         }
         __syncthreads();
-        if (pid[0] < 0)
+        if (c0 >= a.K)
             continue;
+        int  nq   = 0;
+        auto walk = [&](int n) { // the queue's last n <= 32 pairs
+            if (lane < n) {
+                const int e = queue[w][nq - n + lane], k = e >> 16, j = e & 0xffff;
+                uint64_t  key;
+                if (smk::kd_reaches(b.tree.view, kx[w][k], b.tree.posOf[t0 + j], a.sqDiam, &key))
+                    atomicOr(&words[w][k][j >> 5], 1u << (j & 31));
+            }
+            nq -= n;
+            __syncwarp();
+        };
         for (int j = 0; j < tn; j += 32) {
             const bool   ok = j + lane < tn;
             const float4 q  = tp[ok ? j + lane : 0];
             uint32_t     word = 0;
 #pragma unroll
             for (int k = 0; k < kKpPer; k++) {
-                const bool in = ok && smm::dist2(x[k], y[k], z[k], q.x, q.y, q.z) < a.sqDiam;
-                S[k] += __popc(__ballot_sync(0xffffffffu, in));
-                const uint32_t row =
-                    __ballot_sync(0xffffffffu, in && __float_as_int(q.w) != pid[k]);
-                R[k] += __popc(row);
-                word = lane == k ? row : word;
+                const float d  = smm::dist2(x[k], y[k], z[k], q.x, q.y, q.z);
+                const bool  in = ok && d < a.sqDiam;
+                if (TREE) {
+                    const bool     sure = in && d < q.w;
+                    const uint32_t row  = __ballot_sync(0xffffffffu, sure);
+                    const uint32_t ask  = __ballot_sync(0xffffffffu, in && !sure && c0 + k < a.K);
+                    if (in && !sure && c0 + k < a.K)
+                        queue[w][nq + __popc(ask & ((1u << lane) - 1u))] = (k << 16) | (j + lane);
+                    nq += __popc(ask); // (below 32 before the round)
+                    word = lane == k ? row : word;
+                } else {
+                    S[k] += __popc(__ballot_sync(0xffffffffu, in));
+                    const uint32_t row =
+                        __ballot_sync(0xffffffffu, in && __float_as_int(q.w) != self[k]);
+                    R[k] += __popc(row);
+                    word = lane == k ? row : word;
+                }
             }
-            if (lane < kKpPer && c0 + lane < a.K)
+            if (TREE) {
+                if (lane < kKpPer)
+                    words[w][lane][j >> 5] = word;
+                __syncwarp();
+                while (nq >= 32)
+                    walk(32);
+            } else if (lane < kKpPer && c0 + lane < a.K) {
                 b.mask[(size_t)(c0 + lane) * b.words + ((t0 + j) >> 5)] = word;
+            }
+        }
+        if (TREE) {
+            if (nq > 0)
+                walk(nq);
+#pragma unroll
+            for (int k = 0; k < kKpPer; k++) { // a word per lane: counts, the keypoint taken out
+                if (c0 + k >= a.K || lane * 32 >= tn)
+                    continue;
+                uint32_t m = words[w][k][lane];
+                S[k] += __popc(m);
+                if ((self[k] - t0) >> 5 == lane)
+                    m &= ~(1u << ((self[k] - t0) & 31));
+                R[k] += __popc(m);
+                b.mask[(size_t)(c0 + k) * b.words + (t0 >> 5) + lane] = m;
+            }
+            __syncwarp();
         }
     }
 #pragma unroll
-    for (int k = 0; k < kKpPer; k++)
+    for (int k = 0; k < kKpPer; k++) {
+        if (TREE) {
+            S[k] = __reduce_add_sync(0xffffffffu, S[k]);
+            R[k] = __reduce_add_sync(0xffffffffu, R[k]);
+        }
         if (lane == k && c0 + k < a.K)
             b.part[(size_t)blockIdx.y * a.K + c0 + k] = make_int2(S[k], R[k]);
+    }
 }
 
-// Radius mode, a warp per keypoint: its counts over the parts, its first tail row, its transform;
-// the row counts (cnt[K] = 0 closes the scan's input), and the per-keypoint hit counters and
-// vote totals cleared for k_ppf.
-__global__ void k_kp_info(VoteArgs a, PipeBufs b, int *__restrict__ cnt) {
+// Set bits of the mask row in [l, r), by a warp.
+__device__ __forceinline__ int mask_count(const uint32_t *mask, int l, int r) {
+    int n = 0;
+    if (l < r)
+        for (int w = (l >> 5) + (int)(threadIdx.x & 31); w <= (r - 1) >> 5; w += 32) {
+            uint32_t m = mask[w];
+            if (w == l >> 5)
+                m &= ~0u << (l & 31);
+            if (w == (r - 1) >> 5)
+                m &= ~0u >> (31 - ((r - 1) & 31));
+            n += __popc(m);
+        }
+    return __reduce_add_sync(0xffffffffu, n);
+}
+
+// The last n set bits of the mask row in [l, r) (at least n are set), to out[0..n), by a warp.
+__device__ __forceinline__ void mask_last(const uint32_t *mask, int l, int r, int n, int *out) {
+    const int lane = threadIdx.x & 31;
+    int       at   = 0;
+    for (int w1 = (r - 1) >> 5; at < n && w1 >= l >> 5; w1 -= 32) {
+        const int w = w1 - lane; // lane 0: the last word
+        uint32_t  m = w >= l >> 5 ? mask[w] : 0u;
+        if (w == l >> 5)
+            m &= ~0u << (l & 31);
+        if (w == (r - 1) >> 5)
+            m &= ~0u >> (31 - ((r - 1) & 31));
+        const int incl = warp_incl_scan(__popc(m));
+        int       k    = at + incl - __popc(m);
+        while (m && k < n) {
+            const int bit = 31 - __clz(m);
+            m ^= 1u << bit;
+            out[k++] = w * 32 + bit;
+        }
+        at += __shfl_sync(0xffffffffu, incl, 31);
+    }
+}
+
+// The last `need` of a keypoint's rows in the depth-first order of its radius search (nearer
+// child first): from the root, a far child that holds as many is where they lie, one that holds
+// fewer gives all of its own. Rows of a subtree are a range of the mask, as the candidates are
+// in tree order.
+__device__ __forceinline__ void tree_tail(const VoteTree &T, const uint32_t *mask, const float q[3],
+                                          int need, int *out) {
+    int v = 0, l = 0, r = T.m;
+    while (need > 0) {
+        const int4 n = T.view.nd[v];
+        if (smk::is_leaf(n)) {
+            mask_last(mask, T.before[n.x], T.before[n.y], need, out);
+            return;
+        }
+        const int   f     = smk::divfeat_of(n);
+        const float val   = f == 0 ? q[0] : f == 1 ? q[1] : q[2];
+        const bool  near1 = ((val - __int_as_float(n.x)) + (val - __int_as_float(n.y))) < 0.0f;
+        const int   fl = near1 ? n.w : l, fr = near1 ? r : n.w; // the far child's positions
+        const int   cl = T.before[fl], cr = T.before[fr];
+        const int   c  = mask_count(mask, cl, cr);
+        const int   c1 = smk::child1_of(n);
+        if (c >= need) {
+            v = near1 ? c1 + 1 : c1;
+            l = fl;
+            r = fr;
+            continue;
+        }
+        mask_last(mask, cl, cr, c, out);
+        out += c;
+        need -= c;
+        v = near1 ? c1 : c1 + 1;
+        l = near1 ? l : n.w;
+        r = near1 ? n.w : r;
+    }
+}
+
+// Radius mode, a warp per keypoint: its counts over the parts, its tail rows, its transform; the
+// row counts (cnt[K] = 0 closes the scan's input), and the per-keypoint hit counters and vote
+// totals cleared for k_ppf.
+template <bool TREE> __global__ void k_kp_info(VoteArgs a, PipeBufs b, int *__restrict__ cnt) {
     smd::chain_enter(); // launched chained
     const int lane = threadIdx.x & 31;
     const int c    = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -178,11 +320,22 @@ __global__ void k_kp_info(VoteArgs a, PipeBufs b, int *__restrict__ cnt) {
     }
     S = __reduce_add_sync(0xffffffffu, S);
     R = __reduce_add_sync(0xffffffffu, R);
-    const int tail = tail_from_mask(b.mask + (size_t)c * b.words, b.words, R % smm::kLanes, a.ncand);
+    const int       pid  = a.kp[c];
+    const float4    p1   = a.pos[pid];
+    const uint32_t *mask = b.mask + (size_t)c * b.words;
+    int             tail = 0;
+    if (TREE) {
+        const float q[3] = {p1.x, p1.y, p1.z};
+        if (lane < 8)
+            b.tail[(size_t)c * 8 + lane] = -1;
+        __syncwarp();
+        tree_tail(b.tree, mask, q, R % smm::kLanes, b.tail + (size_t)c * 8);
+    } else {
+        tail = tail_from_mask(mask, b.words, R % smm::kLanes, a.ncand);
+    }
     if (lane != 0)
         return;
-    const int    pid = a.kp[c];
-    const float4 p1 = a.pos[pid], n1 = a.nrm[pid];
+    const float4 n1   = a.nrm[pid];
     const int4   info = kp_info(a, S, R, tail, n1);
     b.info[c]         = info;
     b.rt[c]           = smm::transform_rt(p1.x, p1.y, p1.z, n1.x, n1.y, n1.z);
@@ -254,10 +407,13 @@ __global__ void k_rows_count(const int4 *__restrict__ info, int K, int *__restri
 // a CTA share nothing. (8.4 M rows: through a row list in global memory, with the alpha of every
 // row, 51 + 248 us; packed by the whole CTA between barriers 532 us; now 267 us, mostly the
 // issue of the keys' arithmetic, some 700 instructions a row with its divisions and arc tangents.)
-template <bool CSR>
-__global__ void __launch_bounds__(kPpfBs) k_ppf(VoteArgs a, PipeBufs b) {
+enum RowSource { kRowsMask, kRowsTree, kRowsCsr }; // tree: a mask with listed tail rows
+
+template <RowSource SRC>
+__global__ void __launch_bounds__(kPpfBs, 5) k_ppf(VoteArgs a, PipeBufs b) {
     smd::chain_enter(); // launched chained
-    constexpr int W = kPpfBs / 32;
+    constexpr int  W   = kPpfBs / 32;
+    constexpr bool CSR = SRC == kRowsCsr;
     __shared__ int  rowQ[W][160]; // point * 2 + block lane
     __shared__ int4 hitQ[W][64];  // {row, bucket offset, count, multiplicity}
     const int  c    = blockIdx.x;
@@ -321,6 +477,7 @@ __global__ void __launch_bounds__(kPpfBs) k_ppf(VoteArgs a, PipeBufs b) {
         __syncwarp(); // (the queues' places are written again after their reads)
     };
 
+    const int tail = SRC == kRowsTree ? b.tail[(size_t)c * 8 + (lane & 7)] : -1;
     const int step = gridDim.y * W * 128;
     for (int i0 = (blockIdx.y * W + w) * 128; i0 < len; i0 += step) {
         uint32_t m[4];
@@ -340,11 +497,23 @@ __global__ void __launch_bounds__(kPpfBs) k_ppf(VoteArgs a, PipeBufs b) {
             else if ((m[k] >> lane) & 1u)
                 id[k] = a.cand[i0 + k * 32 + lane];
         }
+        // the lane's rows that the reference computes one by one
+        unsigned single = 0u;
+        if (SRC == kRowsTree) {
+            uint32_t here = __ballot_sync(0xffffffffu, lane < 8 && tail >= 0 && (tail ^ i0) < 128);
+            while (here) {
+                const int t = __shfl_sync(0xffffffffu, tail, __ffs(here) - 1) - i0;
+                here &= here - 1u;
+                if ((t & 31) == lane)
+                    single |= 1u << (t >> 5);
+            }
+        }
 #pragma unroll
         for (int k = 0; k < 4; k++) {
+            const bool block =
+                SRC == kRowsTree ? !((single >> k) & 1u) : i0 + k * 32 + lane < info.z;
             if ((m[k] >> lane) & 1u)
-                rq[nr + __popc(m[k] & below)] =
-                    id[k] * 2 + (i0 + k * 32 + lane < info.z ? 1 : 0);
+                rq[nr + __popc(m[k] & below)] = id[k] * 2 + (block ? 1 : 0);
             nr += __popc(m[k]); // (below 32 before: 160 entries hold 128 more)
         }
         __syncwarp();
@@ -569,12 +738,12 @@ int vote_tuned_shape(int device, int *persistent) {
 
 void vote(Ctx &c, const Model &m, const float4 *pos, const float4 *nrm, const int *kp, int K,
           const int *nbrOff, const int *nbrIds, const int *cand, int ncand, float minScore,
-          const VoteOut &out, int dumpK) {
+          const VoteOut &out, int dumpK, const VoteTree *tree) {
     if (K <= 0)
         return;
     // rows (keypoint, neighbour) are counted and offset in 32-bit ints: at most K x ncand in
     // radius mode (every candidate a neighbour of every keypoint)
-    if (!nbrOff && (long long)K * (long long)ncand > 0x7fffffffll)
+    if (!nbrOff && !tree && (long long)K * (long long)ncand > 0x7fffffffll)
         throw Error(SM_ERR_CAPACITY, "too many keypoint x sampled point pairs for one call");
     VoteArgs a{};
     fill_vote_model(m, minScore, a);
@@ -637,8 +806,16 @@ void vote(Ctx &c, const Model &m, const float4 *pos, const float4 *nrm, const in
         const int per  = nblocks(nblocks(ncand, want), 32) * 32;
         b.splits       = std::max(1, nblocks(ncand, per));
         b.part         = c.arena.get<int2>("v.part", (size_t)b.splits * K);
-        launch_chained(c, k_kp_radius, dim3(gx, b.splits), kKpWarps * 32, 0, a, b, per);
-        launch_chained(c, k_kp_info, nblocks((long long)K * 32, 256), 256, 0, a, b, cnt);
+        const int gi   = nblocks((long long)K * 32, 256);
+        if (tree) {
+            b.tree = *tree;
+            b.tail = c.arena.get<int>("v.tail", (size_t)K * 8);
+            launch_chained(c, k_kp_radius<true>, dim3(gx, b.splits), kKpWarps * 32, 0, a, b, per);
+            launch_chained(c, k_kp_info<true>, gi, 256, 0, a, b, cnt);
+        } else {
+            launch_chained(c, k_kp_radius<false>, dim3(gx, b.splits), kKpWarps * 32, 0, a, b, per);
+            launch_chained(c, k_kp_info<false>, gi, 256, 0, a, b, cnt);
+        }
     }
     const int rtot = scan_excl(c, cnt, b.rowOff, (long long)K + 1, "v.scan", true);
     b.hits = c.arena.get<int4>("v.hits", std::max(rtot, 1));
@@ -649,9 +826,11 @@ void vote(Ctx &c, const Model &m, const float4 *pos, const float4 *nrm, const in
         const int most = nblocks(csr ? rtot : ncand, 128 * (kPpfBs / 32));
         const int gy   = std::max(1, std::min(most, nblocks(4LL * nsm, K)));
         if (csr)
-            launch_chained(c, k_ppf<true>, dim3(K, gy), kPpfBs, 0, a, b);
+            launch_chained(c, k_ppf<kRowsCsr>, dim3(K, gy), kPpfBs, 0, a, b);
+        else if (tree)
+            launch_chained(c, k_ppf<kRowsTree>, dim3(K, gy), kPpfBs, 0, a, b);
         else
-            launch_chained(c, k_ppf<false>, dim3(K, gy), kPpfBs, 0, a, b);
+            launch_chained(c, k_ppf<kRowsMask>, dim3(K, gy), kPpfBs, 0, a, b);
     }
     SM_CUDA(cudaEventRecord(c.ev[11], c.stream));
     launch_chained(c, k_lpt, 1, 1024, 0, b.votes, K, b.order, b.next);

@@ -23,7 +23,7 @@ CU_SOURCES = ["sort.cu", "kdtree.cu", "prep.cu", "vote.cu", "vote_pipe.cu", "clu
               "probe.cu", "mls.cu"]
 CPP_SOURCES: list = []
 HEADERS = ["sm_math.h", "sm_linalg.h", "sm_icp.h", "sm_grid.h", "sm_device.cuh", "sm_vote.cuh",
-           "sm_kdtree.cuh", "sm_kdgrid.cuh",
+           "sm_kdtree.cuh", "sm_kdgrid.cuh", "sm_scan.cuh",
            "sm_engine.h", "sm_stages.h"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--fmad=false", "-prec-div=true",

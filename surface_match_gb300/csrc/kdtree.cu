@@ -35,6 +35,7 @@
 
 #include "sm_kdgrid.cuh"
 #include "sm_kdtree.cuh"
+#include "sm_scan.cuh"
 #include "sm_stages.h"
 
 namespace sm {
@@ -91,6 +92,44 @@ __device__ __forceinline__ void add_bounds(S *seg, int s, const float4 &p) {
         }
 }
 
+// The same by a whole CTA: where every thread with a point names one range, the CTA adds once
+// (at the first levels every warp of the launch would add to the same few words: 95 us a level).
+template <class S>
+__device__ __forceinline__ void add_bounds_block(S *seg, int s, const float4 &p) {
+    __shared__ int sOne, lo[3], hi[3];
+    if (threadIdx.x == 0)
+        sOne = -1;
+    if (threadIdx.x < 3) {
+        lo[threadIdx.x] = INT_MAX;
+        hi[threadIdx.x] = INT_MIN;
+    }
+    __syncthreads();
+    if (s >= 0)
+        sOne = s; // (any one of them)
+    __syncthreads();
+    const int one = sOne;
+    if (!__syncthreads_and(s < 0 || s == one)) {
+        add_bounds(seg, s, p);
+        return;
+    }
+    if (one < 0)
+        return;
+    const int o[3] = {f2ord(p.x), f2ord(p.y), f2ord(p.z)};
+    for (int a = 0; a < 3; a++) {
+        const int l = __reduce_min_sync(0xffffffffu, s >= 0 ? o[a] : INT_MAX);
+        const int h = __reduce_max_sync(0xffffffffu, s >= 0 ? o[a] : INT_MIN);
+        if ((threadIdx.x & 31) == 0) {
+            atomicMin(&lo[a], l);
+            atomicMax(&hi[a], h);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        atomicMin(&seg[one].mn[threadIdx.x], lo[threadIdx.x]);
+        atomicMax(&seg[one].mx[threadIdx.x], hi[threadIdx.x]);
+    }
+}
+
 __device__ __forceinline__ float coord_of(const float4 &p, int a) {
     return a == 0 ? p.x : (a == 1 ? p.y : p.z);
 }
@@ -141,7 +180,16 @@ __device__ __forceinline__ int split_index(int count, int lim1, int lim2) {
 __device__ __forceinline__ int4 leaf_node(int l, int r) { return make_int4(l, r, -1, 0); }
 
 // ---- top levels: one kernel per step over the whole position array -------------------
-__global__ void k_kd_root(Seg *seg, Seg *small, int m, Box box, int4 *nd, int *parent, int *cnt) {
+// Control words: nodes, small ranges, error, then per level its open ranges and whether a
+// point lies on a cut (else the second pass has nothing to do). The levels' launches are chained
+// and sized by bounds; the host looks at the counts every kKdLevels levels only. (One round trip,
+// two counter copies, a flag kernel per pass and ordinary launches a level: 3.3 ms for 0.92 M
+// points, now 1.9 ms.)
+enum { kKdNodes = 0, kKdSmallN = 1, kKdErr = 2, kKdOpen = 8, kKdOnCut = 8 + 2 * smk::kMaxDepth };
+constexpr int kKdCtl    = kKdOnCut + 2 * smk::kMaxDepth;
+constexpr int kKdLevels = 4;
+
+__global__ void k_kd_root(Seg *seg, Seg *small, int m, Box box, int4 *nd, int *parent, int *ctl) {
     Seg s{};
     s.left  = 0;
     s.right = m;
@@ -154,15 +202,15 @@ __global__ void k_kd_root(Seg *seg, Seg *small, int m, Box box, int4 *nd, int *p
         s.mx[a] = INT_MIN;
     }
     s.child[0] = s.child[1] = -1;
-    seg[0]     = s;
-    parent[0]  = -1;
-    cnt[0]     = 1;                    // nodes
-    cnt[4]     = m > kSmall ? 1 : 0;  // open ranges of the first level
+    seg[0]        = s;
+    parent[0]     = -1;
+    ctl[kKdNodes] = 1;
+    ctl[kKdOpen]  = m > kSmall ? 1 : 0; // open ranges of the first level
     if (m <= smk::kLeafMax) {
         nd[0] = leaf_node(0, m);
     } else if (m <= kSmall) {
-        small[0] = s;                  // the whole cloud is one small range
-        cnt[2]   = 1;
+        small[0]       = s; // the whole cloud is one small range
+        ctl[kKdSmallN] = 1;
     }
 }
 
@@ -176,10 +224,11 @@ __global__ void k_kd_init(const float4 *__restrict__ pos, const int *__restrict_
         rec[i]       = make_float4(p.x, p.y, p.z, __int_as_float(id));
         segOf[i]     = 0;
     }
-    add_bounds(seg, i < m ? 0 : -1, p);
+    add_bounds_block(seg, i < m ? 0 : -1, p);
 }
 
 __global__ void k_kd_cut(Seg *__restrict__ seg, const int *__restrict__ nseg) {
+    chain_enter(); // launched chained
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= *nseg)
         return;
@@ -192,63 +241,87 @@ __device__ __forceinline__ int pass_start(const Seg &S, int pass, const int *g1)
     return pass == 1 ? S.left : S.left + (g1[S.right] - g1[S.left]);
 }
 
-__global__ void k_kd_flags(const float4 *__restrict__ rec, const int *__restrict__ segOf, int m,
-                           const Seg *__restrict__ seg, int pass, const int *__restrict__ g1,
-                           int *__restrict__ flag) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > m)
-        return;
-    int f = 0;
-    if (i < m) {
-        const int s = segOf[i];
-        if (s >= 0) {
-            const Seg &S = seg[s];
-            if (i >= pass_start(S, pass, g1)) {
-                const float x = coord_of(rec[i], S.cutfeat);
-                f             = pass == 1 ? (x < S.cutval) : (x <= S.cutval);
+// A pass's flags as the values of a scan (the flag of position i is then g[i + 1] - g[i]),
+// evaluated in position order and handed over as bits. Pass 1 notes points on a cut; without any
+// pass 2 is skipped.
+struct KdFlags {
+    const float4 *rec;
+    const int    *segOf;
+    const Seg    *seg;
+    const int    *nseg, *g1;
+    int          *onCut;
+    int           pass, m;
+    __device__ __forceinline__ bool skip() const { return *nseg == 0 || (pass == 2 && *onCut == 0); }
+    __device__ __forceinline__ void load(long long tile, long long, int (&v)[kScanIpt]) const {
+        __shared__ uint32_t bits[kScanTile / 32];
+        bool                on = false;
+#pragma unroll
+        for (int k = 0; k < kScanIpt; k++) {
+            const int j = k * kScanBs + threadIdx.x, i = (int)tile + j;
+            bool      f = false;
+            const int s = i < m ? segOf[i] : -1;
+            if (s >= 0) {
+                const Seg &S = seg[s];
+                if (pass == 1 || i >= pass_start(S, 2, g1)) {
+                    const float x = coord_of(rec[i], S.cutfeat);
+                    f             = pass == 1 ? x < S.cutval : x <= S.cutval;
+                    on            = on || x == S.cutval;
+                }
             }
+            const uint32_t b = __ballot_sync(0xffffffffu, f);
+            if ((threadIdx.x & 31) == 0)
+                bits[j >> 5] = b;
         }
+        if (pass == 1 && on)
+            *onCut = 1;
+        __syncthreads();
+        const uint32_t b = bits[threadIdx.x / 4] >> ((threadIdx.x & 3) * 8);
+#pragma unroll
+        for (int k = 0; k < kScanIpt; k++)
+            v[k] = (b >> k) & 1u;
     }
-    flag[i] = f;
+};
+
+// The open range of position i in a pass: its start there, false when i takes no part.
+__device__ __forceinline__ bool kd_part(const KdFlags &F, int i, int &a, int &right) {
+    if (i >= F.m)
+        return false;
+    const int s = F.segOf[i];
+    if (s < 0)
+        return false;
+    const Seg &S = F.seg[s];
+    a            = pass_start(S, F.pass, F.g1);
+    right        = S.right;
+    return i >= a;
 }
 
 // The back part's misplaced elements record their positions by rank from the back.
-__global__ void k_kd_rank(const int *__restrict__ segOf, int m, const Seg *__restrict__ seg,
-                          int pass, const int *__restrict__ g1, const int *__restrict__ flag,
-                          const int *__restrict__ g, int *__restrict__ badR) {
+__global__ void k_kd_rank(KdFlags F, const int *__restrict__ g, int *__restrict__ badR) {
+    chain_enter(); // launched chained
+    if (F.skip())
+        return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m || !flag[i])
+    int       a, right;
+    if (!kd_part(F, i, a, right))
         return;
-    const int s = segOf[i];
-    if (s < 0)
-        return;
-    const Seg &S = seg[s];
-    const int  a = pass_start(S, pass, g1);
-    if (i < a)
-        return;
-    const int T = g[S.right] - g[a], lt = g[i] - g[a];
-    if (i - a >= T)
-        badR[a + (T - lt - 1)] = i;
+    const int ga = g[a], gi = g[i], T = g[right] - ga;
+    if (i - a >= T && g[i + 1] != gi)
+        badR[a + (T - (gi - ga) - 1)] = i;
 }
 
 // The front part's misplaced elements swap with their partners (disjoint pairs).
-__global__ void k_kd_swap(float4 *__restrict__ rec, const int *__restrict__ segOf, int m,
-                          const Seg *__restrict__ seg, int pass, const int *__restrict__ g1,
-                          const int *__restrict__ flag, const int *__restrict__ g,
+__global__ void k_kd_swap(KdFlags F, float4 *__restrict__ rec, const int *__restrict__ g,
                           const int *__restrict__ badR) {
+    chain_enter(); // launched chained
+    if (F.skip())
+        return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m || flag[i])
+    int       a, right;
+    if (!kd_part(F, i, a, right))
         return;
-    const int s = segOf[i];
-    if (s < 0)
-        return;
-    const Seg &S = seg[s];
-    const int  a = pass_start(S, pass, g1);
-    if (i < a)
-        return;
-    const int T = g[S.right] - g[a], lt = g[i] - g[a];
-    if (i - a < T) {
-        const int    p = badR[a + (i - a - lt)];
+    const int ga = g[a], gi = g[i], T = g[right] - ga;
+    if (i - a < T && g[i + 1] == gi) {
+        const int    p = badR[a + (i - a - (gi - ga))];
         const float4 x = rec[i];
         rec[i]         = rec[p];
         rec[p]         = x;
@@ -257,24 +330,25 @@ __global__ void k_kd_swap(float4 *__restrict__ rec, const int *__restrict__ segO
 
 // Children of every open range: nodes, leaves, small ranges and next-level ranges.
 __global__ void k_kd_children(Seg *__restrict__ seg, const int *__restrict__ nseg,
-                              const int *__restrict__ g1, const int *__restrict__ g2,
-                              int4 *__restrict__ nd, int *__restrict__ parent,
-                              int *__restrict__ nodeCount, Seg *__restrict__ next,
-                              int *__restrict__ nnext, Seg *__restrict__ small,
-                              int *__restrict__ nsmall, int *__restrict__ depthErr) {
+                              const int *__restrict__ onCut, const int *__restrict__ g1,
+                              const int *__restrict__ g2, int4 *__restrict__ nd,
+                              int *__restrict__ parent, int *__restrict__ ctl,
+                              Seg *__restrict__ next, int *__restrict__ nnext,
+                              Seg *__restrict__ small) {
+    chain_enter(); // launched chained
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= *nseg)
         return;
     Seg      &S     = seg[s];
     const int count = S.right - S.left;
     const int lim1  = g1[S.right] - g1[S.left];
-    const int lim2  = lim1 + (g2[S.right] - g2[S.left + lim1]);
+    const int lim2  = *onCut ? lim1 + (g2[S.right] - g2[S.left + lim1]) : lim1;
     const int index = split_index(count, lim1, lim2);
     S.index         = index;
-    const int c1    = atomicAdd(nodeCount, 2);
+    const int c1    = atomicAdd(&ctl[kKdNodes], 2);
     nd[S.node]      = make_int4(0, 0, c1 | (S.cutfeat << 30), S.left + index);
     if (S.depth + 1 >= smk::kMaxDepth)
-        atomicExch(depthErr, 1);
+        atomicExch(&ctl[kKdErr], 1);
     for (int k = 0; k < 2; k++) {
         const int l = k == 0 ? S.left : S.left + index;
         const int r = k == 0 ? S.left + index : S.right;
@@ -299,7 +373,7 @@ __global__ void k_kd_children(Seg *__restrict__ seg, const int *__restrict__ nse
         if (r - l <= smk::kLeafMax) {
             nd[c1 + k] = leaf_node(l, r);
         } else if (r - l <= kSmall) {
-            small[atomicAdd(nsmall, 1)] = C;
+            small[atomicAdd(&ctl[kKdSmallN], 1)] = C;
         } else {
             const int id = atomicAdd(nnext, 1);
             next[id]     = C;
@@ -310,7 +384,11 @@ __global__ void k_kd_children(Seg *__restrict__ seg, const int *__restrict__ nse
 
 // Next-level segment of every position, and the next level's point bounds.
 __global__ void k_kd_advance(const float4 *__restrict__ rec, int *__restrict__ segOf, int m,
-                             const Seg *__restrict__ seg, Seg *__restrict__ next) {
+                             const Seg *__restrict__ seg, const int *__restrict__ nseg,
+                             Seg *__restrict__ next) {
+    chain_enter(); // launched chained
+    if (*nseg == 0)
+        return;
     const int i  = blockIdx.x * blockDim.x + threadIdx.x;
     int       ns = -1;
     float4    p  = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -323,7 +401,7 @@ __global__ void k_kd_advance(const float4 *__restrict__ rec, int *__restrict__ s
             p            = rec[i];
         }
     }
-    add_bounds(next, ns, p);
+    add_bounds_block(next, ns, p);
 }
 
 // ---- small ranges: one CTA of 1024 threads, one position per thread -------------------
@@ -1066,72 +1144,73 @@ void build_kdtree(Ctx &c, const float4 *pos, int npoints, const int *ids, int m,
     int *parent  = c.arena.get<int>(tag + ".par", cap);
     T.parent     = parent;
     int *arrive  = c.arena.get<int>(tag + ".arr", cap);
-    int *cnt     = c.arena.get<int>(tag + ".cnt", 8); // nodes, nnext, nsmall, err
+    int *ctl     = c.arena.get<int>(tag + ".ctl", kKdCtl);
     int *segOf   = c.arena.get<int>(tag + ".segof", std::max(m, 1));
-    int *flag    = c.arena.get<int>(tag + ".flag", (size_t)m + 1);
     int *g1      = c.arena.get<int>(tag + ".g1", (size_t)m + 1);
     int *g2      = c.arena.get<int>(tag + ".g2", (size_t)m + 1);
     int *badR    = c.arena.get<int>(tag + ".badr", std::max(m, 1));
     const int maxSeg = std::max(m / (smk::kLeafMax + 1) + 2, 2);
-    Seg *segA  = c.arena.get<Seg>(tag + ".segA", maxSeg);
-    Seg *segB  = c.arena.get<Seg>(tag + ".segB", maxSeg);
-    Seg *small = c.arena.get<Seg>(tag + ".small", maxSeg);
-    SM_CUDA(cudaMemsetAsync(cnt, 0, 8 * sizeof(int), c.stream));
+    const int maxOpen = m / (kSmall + 1) + 1; // open ranges of a level: above kSmall points each
+    Seg *segs[2] = {c.arena.get<Seg>(tag + ".segA", maxSeg), c.arena.get<Seg>(tag + ".segB", maxSeg)};
+    Seg *small   = c.arena.get<Seg>(tag + ".small", maxSeg);
+    SM_CUDA(cudaMemsetAsync(ctl, 0, kKdCtl * sizeof(int), c.stream));
     SM_CUDA(cudaMemsetAsync(T.treePos, 0xff, (size_t)std::max(npoints, 1) * 4, c.stream));
     if (m == 0)
         return;
-    int *nseg = cnt + 4; // open ranges of the current level (device)
-    k_kd_root<<<1, 1, 0, c.stream>>>(segA, small, m, box, T.nd, parent, cnt);
+    k_kd_root<<<1, 1, 0, c.stream>>>(segs[0], small, m, box, T.nd, parent, ctl);
     SM_LAUNCH_CHECK();
-    k_kd_init<<<nblocks(m, 256), 256, 0, c.stream>>>(pos, ids, m, T.rec, segOf, segA);
+    k_kd_init<<<nblocks(m, 256), 256, 0, c.stream>>>(pos, ids, m, T.rec, segOf, segs[0]);
     SM_LAUNCH_CHECK();
-    int hostSeg = m > kSmall ? 1 : 0;
-    Seg *cur = segA, *nxt = segB;
-    const int gm = nblocks((long long)m + 1, 256);
-    while (hostSeg > 0) {
-        k_kd_cut<<<nblocks(hostSeg, 128), 128, 0, c.stream>>>(cur, nseg);
-        SM_LAUNCH_CHECK();
-        for (int pass = 1; pass <= 2; pass++) {
-            int *g = pass == 1 ? g1 : g2;
-            k_kd_flags<<<gm, 256, 0, c.stream>>>(T.rec, segOf, m, cur, pass, g1, flag);
-            SM_LAUNCH_CHECK();
-            scan_excl(c, flag, g, (long long)m + 1, tag + ".scan", false);
-            k_kd_rank<<<gm, 256, 0, c.stream>>>(segOf, m, cur, pass, g1, flag, g, badR);
-            SM_LAUNCH_CHECK();
-            k_kd_swap<<<gm, 256, 0, c.stream>>>(T.rec, segOf, m, cur, pass, g1, flag, g, badR);
-            SM_LAUNCH_CHECK();
-        }
-        SM_CUDA(cudaMemsetAsync(cnt + 1, 0, sizeof(int), c.stream));
-        k_kd_children<<<nblocks(hostSeg, 128), 128, 0, c.stream>>>(
-            cur, nseg, g1, g2, T.nd, parent, cnt, nxt, cnt + 1, small, cnt + 2, cnt + 3);
-        SM_LAUNCH_CHECK();
-        k_kd_advance<<<nblocks(m, 256), 256, 0, c.stream>>>(T.rec, segOf, m, cur, nxt);
-        SM_LAUNCH_CHECK();
-        SM_CUDA(cudaMemcpyAsync(nseg, cnt + 1, sizeof(int), cudaMemcpyDeviceToDevice, c.stream));
-        SM_CUDA(cudaMemcpyAsync(c.hostCounts, cnt, 4 * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+    const int       gm    = nblocks(m, 256), go = nblocks(maxOpen, 128);
+    const long long n1    = (long long)m + 1;
+    const int       parts = (int)((n1 + kScanTile - 1) / kScanTile);
+    auto            read  = [&](int first, int n) { // control words to the host
+        SM_CUDA(cudaMemcpyAsync(c.hostCounts, ctl + first, n * sizeof(int), cudaMemcpyDeviceToHost,
+                                c.stream));
         c.sync_checked();
-        hostSeg = c.hostCounts[1];
-        std::swap(cur, nxt);
-        if (c.hostCounts[3])
-            throw Error(SM_ERR_CAPACITY, "k-d tree deeper than " + std::to_string(smk::kMaxDepth));
+    };
+    // (a level above kMaxDepth has no open range: its parents set the error and the host stops)
+    bool open = m > kSmall;
+    for (int level = 0; open; level++) {
+        Seg *cur = segs[level & 1], *nxt = segs[(level + 1) & 1];
+        int *nseg = ctl + kKdOpen + level, *onCut = ctl + kKdOnCut + level;
+        launch_chained(c, k_kd_cut, go, 128, 0, cur, nseg);
+        for (int pass = 1; pass <= 2; pass++) {
+            int    *g = pass == 1 ? g1 : g2;
+            KdFlags F{T.rec, segOf, cur, nseg, g1, onCut, pass, m};
+            const unsigned epoch = scan_state(c, parts);
+            launch_chained(c, k_scan_lookback<KdFlags, kPrefix>, parts, kScanBs, 0, F, g, n1,
+                           (const int *)nullptr, c.scan.status, c.scan.ticket, parts, epoch,
+                           (int *)nullptr);
+            launch_chained(c, k_kd_rank, gm, 256, 0, F, g, badR);
+            launch_chained(c, k_kd_swap, gm, 256, 0, F, T.rec, g, badR);
+        }
+        launch_chained(c, k_kd_children, go, 128, 0, cur, nseg, onCut, g1, g2, T.nd, parent, ctl, nxt,
+                       nseg + 1, small);
+        launch_chained(c, k_kd_advance, gm, 256, 0, T.rec, segOf, m, cur, nseg, nxt);
+        if ((level + 1) % kKdLevels == 0) {
+            read(0, kKdOpen + level + 2);
+            open = c.hostCounts[kKdOpen + level + 1] > 0;
+            if (c.hostCounts[kKdErr])
+                throw Error(SM_ERR_CAPACITY, "k-d tree deeper than " + std::to_string(smk::kMaxDepth));
+        }
     }
-    SM_CUDA(cudaMemcpyAsync(c.hostCounts, cnt, 4 * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-    c.sync_checked();
-    const int nsmall = c.hostCounts[2];
+    read(0, kKdOpen);
+    const int nsmall = c.hostCounts[kKdSmallN];
     if (nsmall > 0) {
-        k_kd_small<<<nsmall, kSmall, 0, c.stream>>>(small, T.rec, T.nd, parent, cnt, cnt + 3);
+        k_kd_small<<<nsmall, kSmall, 0, c.stream>>>(small, T.rec, T.nd, parent, ctl + kKdNodes,
+                                                    ctl + kKdErr);
         SM_LAUNCH_CHECK();
     }
     SM_CUDA(cudaMemsetAsync(arrive, 0, (size_t)cap * 4, c.stream));
-    k_kd_finish<<<nblocks(cap, 256), 256, 0, c.stream>>>(T.nd, parent, cnt, T.rec, T.box, arrive,
-                                                         T.vacc, T.leafOf, T.treePos);
+    k_kd_finish<<<nblocks(cap, 256), 256, 0, c.stream>>>(T.nd, parent, ctl + kKdNodes, T.rec, T.box,
+                                                         arrive, T.vacc, T.leafOf, T.treePos);
     SM_LAUNCH_CHECK();
-    SM_CUDA(cudaMemcpyAsync(c.hostCounts, cnt, 4 * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-    c.sync_checked();
-    T.nnodes = c.hostCounts[0];
-    if (c.hostCounts[3] == 1)
+    read(0, kKdOpen);
+    T.nnodes = c.hostCounts[kKdNodes];
+    if (c.hostCounts[kKdErr] == 1)
         throw Error(SM_ERR_CAPACITY, "k-d tree deeper than " + std::to_string(smk::kMaxDepth));
-    if (c.hostCounts[3] == 2)
+    if (c.hostCounts[kKdErr] == 2)
         throw Error(SM_ERR_CAPACITY, "k-d tree build: too many open ranges in a small range");
 }
 

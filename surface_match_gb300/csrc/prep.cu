@@ -10,6 +10,7 @@
 
 #include "sm_icp.h"
 #include "sm_linalg.h"
+#include "sm_scan.cuh"
 #include "sm_stages.h"
 
 namespace sm {
@@ -17,9 +18,6 @@ using namespace smd;
 
 namespace {
 
-constexpr int kScanBs   = 512;
-constexpr int kScanIpt  = 8;
-constexpr int kScanTile = kScanBs * kScanIpt;
 
 struct GridParams {
     float org[3], g;
@@ -198,137 +196,6 @@ static void fill(Ctx &c, const FillSet &f) {
 }
 
 // ---------------------------------------------------------------------------------------
-// Single-pass exclusive scan with decoupled look-back (Merrill & Garland, "Single-pass
-// Parallel Prefix Scan with Decoupled Look-back", 2016). Tiles of kScanTile values take a
-// ticket in launch order; a tile publishes its aggregate, then warp 0 walks back over the
-// tiles before it, 32 at a time, summing aggregates until it meets a tile whose inclusive
-// prefix is published, and publishes its own inclusive prefix. A tile waits only on tiles
-// that took earlier tickets (already running or done), so every wait ends; each is bounded
-// all the same and sets *err when its limit passes. Status words: epoch (30 bits, new per
-// scan, so the array needs no reset) | flag (2 bits: 1 aggregate, 2 inclusive) | value.
-constexpr unsigned long long kLbAgg = 1ull << 32, kLbIncl = 2ull << 32;
-
-__device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long *p) {
-    unsigned long long v;
-    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_relaxed_u64(unsigned long long *p, unsigned long long v) {
-    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-
-// What a scan writes: kPrefix, out[i] = sum of the values before i; kSelect (0/1 flags), the
-// places i of set flags packed into out; kSelectIds, ids[i] for these. A thread's eight values
-// are two 16-byte loads (and stores of prefixes) where the arrays are aligned to them. (One by
-// one, and with the selected places written by a second kernel from the stored prefixes, 0.92 M
-// flags took 11 + 7 us, a table of 2 M counts 20 us.)
-enum ScanOut { kPrefix, kSelect, kSelectIds };
-
-template <ScanOut MODE>
-__global__ void __launch_bounds__(kScanBs)
-    k_scan_lookback(const int *__restrict__ in, int *__restrict__ out, long long n,
-                    const int *__restrict__ ids, unsigned long long *__restrict__ status,
-                    int *__restrict__ ticket, int nparts, unsigned epoch, int *__restrict__ total) {
-    chain_enter(); // launched chained
-    __shared__ int sh[33];
-    __shared__ int sTile, sExcl;
-    if (threadIdx.x == 0) {
-        const int t = atomicAdd(ticket, 1);
-        if (t == nparts - 1)
-            ticket[0] = 0; // every ticket of this launch is taken: ready for the next scan
-        sTile = t;
-    }
-    __syncthreads();
-    const int       tile = sTile;
-    const long long base = (long long)tile * kScanTile + (long long)threadIdx.x * kScanIpt;
-    alignas(16) int v[kScanIpt];
-    int             s = 0;
-    const bool      whole = base + kScanIpt <= n;
-    if (whole && ((uintptr_t)in & 15) == 0) {
-        *reinterpret_cast<int4 *>(&v[0]) = *reinterpret_cast<const int4 *>(in + base);
-        *reinterpret_cast<int4 *>(&v[4]) = *reinterpret_cast<const int4 *>(in + base + 4);
-    } else {
-#pragma unroll
-        for (int k = 0; k < kScanIpt; k++)
-            v[k] = base + k < n ? in[base + k] : 0;
-    }
-#pragma unroll
-    for (int k = 0; k < kScanIpt; k++)
-        s += v[k];
-    int       agg;
-    const int ex  = block_excl_scan(s, sh, &agg);
-    const unsigned long long tag = (unsigned long long)epoch << 34;
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        int       excl = 0;
-        if (tile == 0) {
-            if (lane == 0)
-                st_relaxed_u64(&status[0], tag | kLbIncl | (unsigned)agg);
-        } else {
-            if (lane == 0)
-                st_relaxed_u64(&status[tile], tag | kLbAgg | (unsigned)agg);
-            for (int top = tile - 1;; top -= 32) {
-                const int          p = top - lane; // lane 0: the nearest predecessor
-                unsigned long long w = tag | kLbIncl; // lanes before tile 0: inclusive 0
-                for (int it = 0;; it++) {
-                    if (p >= 0)
-                        w = ld_relaxed_u64(&status[p]);
-                    const bool ready = (w >> 34) == epoch && ((w >> 32) & 3ull) != 0;
-                    if (__all_sync(0xffffffffu, ready))
-                        break;
-                    if (it > (1 << 22)) {
-                        if (lane == 0)
-                            atomicExch(ticket + 1, 1);
-                        w = tag | kLbIncl;
-                        break;
-                    }
-                    __nanosleep(32);
-                }
-                const bool     isIncl = ((w >> 32) & 3ull) == 2ull;
-                const unsigned incl   = __ballot_sync(0xffffffffu, isIncl);
-                int            val    = (int)(unsigned)(w & 0xffffffffull);
-                if (incl) {
-                    const int first = __ffs(incl) - 1;
-                    excl += __reduce_add_sync(0xffffffffu, lane <= first ? val : 0);
-                    break;
-                }
-                excl += __reduce_add_sync(0xffffffffu, val);
-            }
-            if (lane == 0)
-                st_relaxed_u64(&status[tile], tag | kLbIncl | (unsigned)(excl + agg));
-        }
-        if (lane == 0) {
-            sExcl = excl;
-            if (tile == nparts - 1 && total)
-                *total = excl + agg;
-        }
-    }
-    __syncthreads();
-    int o = ex + sExcl;
-    if constexpr (MODE != kPrefix) {
-#pragma unroll
-        for (int k = 0; k < kScanIpt; k++)
-            if (v[k]) // (0 past the end)
-                out[o++] = MODE == kSelectIds ? ids[base + k] : (int)(base + k);
-    } else {
-        alignas(16) int w[kScanIpt];
-#pragma unroll
-        for (int k = 0; k < kScanIpt; k++) {
-            w[k] = o;
-            o += v[k];
-        }
-        if (whole && ((uintptr_t)out & 15) == 0) {
-            *reinterpret_cast<int4 *>(out + base)     = *reinterpret_cast<int4 *>(&w[0]);
-            *reinterpret_cast<int4 *>(out + base + 4) = *reinterpret_cast<int4 *>(&w[4]);
-        } else {
-#pragma unroll
-            for (int k = 0; k < kScanIpt; k++)
-                if (base + k < n)
-                    out[base + k] = w[k];
-        }
-    }
-}
-
 __global__ void k_iota(int *__restrict__ out, int n) {
     chain_enter(); // launched chained
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1216,7 +1083,7 @@ int prep_points(Ctx &c, const float *xyz, const float *nin, int n, float4 *pos, 
 
 // The context's look-back state, grown to at least nparts tiles (zeroed when allocated);
 // returns the next scan epoch.
-static unsigned scan_state(Ctx &c, int nparts) {
+unsigned scan_state(Ctx &c, int nparts) {
     Ctx::ScanState &S = c.scan;
     if (nparts > S.cap || S.epoch >= (1u << 30) - 1) {
         const int cap = std::max(nparts, std::max(S.cap, 1024));
@@ -1241,8 +1108,8 @@ static void scan_launch(Ctx &c, const int *in, int *out, long long n, const int 
     }
     const unsigned epoch = scan_state(c, nparts);
     cudaEvent_t    t0    = c.clock.begin(c.stream);
-    launch_chained(c, k_scan_lookback<MODE>, nparts, kScanBs, 0, in, out, n, ids, c.scan.status,
-                   c.scan.ticket, nparts, epoch, total);
+    launch_chained(c, k_scan_lookback<ScanInts, MODE>, nparts, kScanBs, 0, ScanInts{in}, out, n, ids,
+                   c.scan.status, c.scan.ticket, nparts, epoch, total);
     c.clock.end(c.stream, t0, KernelClock::kScan, 8.0 * (double)n); // 4-byte value in, 4 out
 }
 

@@ -248,6 +248,9 @@ int prep_points(Ctx &c, const float *xyz, const float *nrm, int n, float4 *pos, 
 // wantTotal).
 int scan_excl(Ctx &c, const int *in, int *out, long long n, const std::string &tag,
               bool wantTotal = true);
+// The context's look-back state (sm_scan.cuh), grown to at least nparts tiles; returns the next
+// scan epoch.
+unsigned scan_state(Ctx &c, int nparts);
 // Ascending indices i with flags[i] != 0; returns the count (synchronises).
 int compact(Ctx &c, const int *flags, int n, int *outIds, const std::string &tag);
 // The same when the count is known already (no host round trip).

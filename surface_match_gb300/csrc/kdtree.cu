@@ -647,7 +647,7 @@ struct SampleArgs {
     KdView          t;
     int             dim[3];
     const float4   *ent;      // cell runs: {x, y, z, tree position bits}, tree order in a run
-    const float    *ex;       // the entries' excursions from their leaves' build-time boxes
+    const float    *sure;     // the entries' sure_reach
     const int      *cellRank; // dense cell -> occupied rank (-1: empty)
     const int      *cellList; // occupied rank -> dense cell
     const int      *cellEnd;  // occupied rank -> end of its run of the entries
@@ -660,7 +660,6 @@ struct SampleArgs {
     int            *head, *tail;
     int            *open;     // cells with points not yet decided
     float           r2;
-    double          safe2;
     int            *keptFlag; // per tree position
     int            *err;      // a bounded wait expired
 };
@@ -679,19 +678,26 @@ __device__ __forceinline__ double excursion(const float *box, const float4 &p) {
     return sqrt(s);
 }
 
+// Squared distance below which a radius search of radius^2 r2 surely reaches a point that lies
+// `e` outside its leaf's build-time box: the search's lower bound at any node above the leaf is at
+// most (distance + e)^2 (the margins cover the float rounding of the search's running bound and
+// of the result). Computed once per point in FP64, so that a test is a float comparison: a test
+// with the square root in FP64 waited a microsecond for that pipe.
+__device__ __forceinline__ float sure_reach(float r2, double e) {
+    const double s = sqrt((double)r2 * (1.0 - 1e-4)) - e;
+    return s > 0.0 ? (float)(s * s * (1.0 - 1e-6)) : 0.0f;
+}
+
 // Whether the radius search from kept point q reaches the point p at tree position ip
-// (radiusSearch membership, nanoflann.hpp:1736-1749): distance first; the search's
-// lower bound at any node above p's leaf is at most (|q - p| + excursion)^2, so the path
-// walk is needed only near the radius or for points that left their leaf's box. The
-// margin covers the float rounding of the search's running bound.
+// (radiusSearch membership, nanoflann.hpp:1736-1749): distance first; the walk down the path only
+// near the radius or for points that left their leaf's box.
 __device__ __forceinline__ bool reaches(const SampleArgs &a, const float4 &q, const float4 &p,
-                                        int ip, double e) {
+                                        int ip, float sure) {
     const float qq[3] = {q.x, q.y, q.z};
     const float d     = smk::eval_metric(qq, p);
     if (!(d < a.r2))
         return false;
-    const double b = sqrt((double)d) + e;
-    if (b * b < a.safe2)
+    if (d < sure)
         return true;
     uint64_t key;
     return smk::kd_reaches(a.t, qq, ip, a.r2, &key);
@@ -726,14 +732,13 @@ __global__ void k_sp_heads(const uint32_t *__restrict__ key, int m, uint32_t noC
 }
 
 // The cells' runs (every occupied cell queued, in run order), and the runs' points in run
-// order: {x, y, z, tree position bits}, with the point's excursion from its leaf's build-time
-// box.
+// order: {x, y, z, tree position bits}, with the distance a search surely reaches it at.
 __global__ void k_sp_cells(const uint32_t *__restrict__ key, const uint32_t *__restrict__ sortPos,
                            int m, uint32_t noCell, const int *__restrict__ head,
                            const int *__restrict__ rank, const float *__restrict__ nodeBox,
                            const int *__restrict__ leafOf, int *__restrict__ cellRank,
                            int *__restrict__ cellList, int *__restrict__ cellEnd,
-                           float4 *__restrict__ ent, float *__restrict__ ex, SampleArgs a) {
+                           float4 *__restrict__ ent, float *__restrict__ sure, SampleArgs a) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= m || key[k] == noCell)
         return;
@@ -753,7 +758,7 @@ __global__ void k_sp_cells(const uint32_t *__restrict__ key, const uint32_t *__r
     const int    ip = (int)sortPos[k];
     const float4 p  = a.t.pos[a.t.vacc[ip]];
     ent[k]          = make_float4(p.x, p.y, p.z, __int_as_float(ip));
-    ex[k]           = (float)excursion(nodeBox + 6 * (size_t)leafOf[ip], p);
+    sure[k]         = sure_reach(a.r2, excursion(nodeBox + 6 * (size_t)leafOf[ip], p));
     a.dec[k]        = 0;
     a.filed[k]      = -1;
 }
@@ -888,21 +893,23 @@ __device__ __forceinline__ void sp_drop(const SampleArgs &a, int r, int k, const
     const int   excl = nb_runs(a, r, k + 1, -1, nb, tot);
     for (int base = 0; base < tot; base += 32 * kSpUnroll) {
         int    kp[kSpUnroll], dec[kSpUnroll];
+        float  sure[kSpUnroll];
         float4 p[kSpUnroll];
 #pragma unroll
         for (int u = 0; u < kSpUnroll; u++)
             kp[u] = nb_entry(min(base + u * 32 + lane, tot - 1), excl, nb);
 #pragma unroll
         for (int u = 0; u < kSpUnroll; u++) {
-            p[u]   = a.ent[kp[u]];
-            dec[u] = ld_vol(&a.dec[kp[u]]);
+            p[u]    = a.ent[kp[u]];
+            sure[u] = a.sure[kp[u]];
+            dec[u]  = ld_vol(&a.dec[kp[u]]);
         }
         bool gone[kSpUnroll], any = false;
 #pragma unroll
         for (int u = 0; u < kSpUnroll; u++) {
             gone[u] = base + u * 32 + lane < tot && dec[u] == 0 && __float_as_int(p[u].w) > iq &&
                       smk::eval_metric(qq, p[u]) < a.r2 &&
-                      reaches(a, q, p[u], __float_as_int(p[u].w), (double)a.ex[kp[u]]);
+                      reaches(a, q, p[u], __float_as_int(p[u].w), sure[u]);
             if (gone[u]) {
                 *(volatile int *)&a.dec[kp[u]] = 2;
                 any                            = true;
@@ -1078,10 +1085,8 @@ __global__ void k_kd_cands(const int *__restrict__ cand, int n, const int *__res
     if (r >= n)
         return;
     const int    id = cand[r], ip = treePos[id];
-    const double s = sqrt((double)r2 * (1.0 - 1e-4)) -
-                     excursion(nodeBox + 6 * (size_t)leafOf[ip], pos[id]);
-    posOf[r]       = ip;
-    sure[r]        = s > 0.0 ? (float)(s * s * (1.0 - 1e-6)) : 0.0f;
+    posOf[r] = ip;
+    sure[r]  = sure_reach(r2, excursion(nodeBox + 6 * (size_t)leafOf[ip], pos[id]));
 }
 
 // Leaves holding an active position flag themselves and their ancestors (a walk stops at
@@ -1244,7 +1249,7 @@ int kd_sample(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
     int      *cList = c.arena.get<int>(tag + ".clist", m); // at most a cell per point
     int      *cEnd  = c.arena.get<int>(tag + ".cend", m);
     float4   *ent   = c.arena.get<float4>(tag + ".ent", m);
-    float    *ex    = c.arena.get<float>(tag + ".ex", m);
+    float    *sure  = c.arena.get<float>(tag + ".sure", m);
     int      *flag  = c.arena.get<int>(tag + ".flag", (size_t)m + 1);
     int      *ctl   = c.arena.get<int>(tag + ".ctl", 4 * kSpCtl); // head, tail, open cells, error
     SampleArgs a{};
@@ -1252,7 +1257,7 @@ int kd_sample(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
     for (int d = 0; d < 3; d++)
         a.dim[d] = gp.dim[d];
     a.ent      = ent;
-    a.ex       = ex;
+    a.sure     = sure;
     a.cellRank = cRank;
     a.cellList = cList;
     a.cellEnd  = cEnd;
@@ -1266,7 +1271,6 @@ int kd_sample(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
     a.tail     = ctl + kSpCtl;
     a.open     = ctl + 2 * kSpCtl;
     a.r2       = step * step;
-    a.safe2    = (double)a.r2 * (1.0 - 1e-4);
     a.keptFlag = flag;
     a.err      = ctl + 3 * kSpCtl;
     k_sp_keys<<<nblocks(m, 256), 256, 0, c.stream>>>(vaccA, pos, m, gp, noCell, key, val);
@@ -1280,7 +1284,7 @@ int kd_sample(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
     SM_CUDA(cudaMemsetAsync(ctl, 0, 4 * kSpCtl * sizeof(int), c.stream));
     SM_CUDA(cudaMemsetAsync(a.ring, 0xff, (size_t)ring * 4, c.stream));
     k_sp_cells<<<nblocks(m, 256), 256, 0, c.stream>>>(key, val, m, noCell, head, rank, T.box,
-                                                     T.leafOf, cRank, cList, cEnd, ent, ex, a);
+                                                     T.leafOf, cRank, cList, cEnd, ent, sure, a);
     SM_LAUNCH_CHECK();
     int nsm = 0;
     SM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device));

@@ -630,7 +630,8 @@ __global__ void k_kd_finish(int4 *__restrict__ nd, const int *__restrict__ paren
 // blocker, so there is always a cell to go on with, and a warp waits for queue slots only.
 // (Handling every point through the queue, with a neighbourhood pass per point to count its
 // earlier neighbours and one when it was decided, took 7.8 + 7.3 ms for the large scene's
-// 0.92 M points at steps 4.3 and 1.4 mm, where 7,000 and 56,000 are kept.)
+// 0.92 M points at steps 4.3 and 1.4 mm, where 7,000 and 56,000 are kept; now 1.26 + 1.35 ms.
+// The rest is the chain: about 150 decisions of 8 us in a row at the larger step.)
 constexpr int       kSpBs     = 256;
 constexpr long long kSpIdle   = 1ll << 22; // polls of an unwritten queue slot before giving up
 constexpr int       kSpUnroll = 4;         // neighbourhood entries in flight per lane
@@ -638,10 +639,11 @@ constexpr int       kSpUnroll = 4;         // neighbourhood entries in flight pe
 // at once), nanoseconds between two looks at a queue slot, and words between two control words
 // (on one line, with every waiting warp reading it at each look, a decision took 40 us instead
 // of 10: the large scene's two long samplings 3.3 + 4.4 ms instead of 1.2 + 1.6 ms)
-constexpr int       kSpCtas   = 2;
-constexpr int       kSpSleep  = 100;
-constexpr int       kSpCtl    = 32;
-constexpr long long kSpCells  = 1ll << 25; // most cells of the dense table (128 MB)
+constexpr int       kSpCtas     = 2;
+constexpr int       kSpSleep    = 100;
+constexpr int       kSpCtl      = 32;
+constexpr int       kSpUnlinked = -2;      // a filed cell's link until it is stored
+constexpr long long kSpCells    = 1ll << 25; // most cells of the dense table (128 MB)
 
 struct SampleArgs {
     KdView          t;
@@ -651,11 +653,12 @@ struct SampleArgs {
     const int      *cellRank; // dense cell -> occupied rank (-1: empty)
     const int      *cellList; // occupied rank -> dense cell
     const int      *cellEnd;  // occupied rank -> end of its run of the entries
-    int            *cur;      // occupied rank -> no entry of its run before this one is open
+    // occupied rank -> an entry of its run that no open one comes before, and its tree position
+    unsigned long long *cur;
     int            *dec;      // per entry: 0 open, 1 kept, 2 dropped
     int            *filed;    // per entry: first cell filed under it (-1: none)
     int            *nextCell; // per occupied rank: the next cell filed under the same entry
-    int            *ring;     // queue of cells (-1: slot not written)
+    int            *ring;     // queue of dense cells (-1: slot not written)
     unsigned        ringMask;
     int            *head, *tail;
     int            *open;     // cells with points not yet decided
@@ -663,6 +666,9 @@ struct SampleArgs {
     int            *keptFlag; // per tree position
     int            *err;      // a bounded wait expired
 };
+__device__ __forceinline__ unsigned long long sp_cur(int k, int pos) {
+    return (unsigned long long)(unsigned)pos << 32 | (unsigned)k;
+}
 
 __device__ __forceinline__ int ld_vol(const int *p) { return *(const volatile int *)p; }
 
@@ -731,8 +737,7 @@ __global__ void k_sp_heads(const uint32_t *__restrict__ key, int m, uint32_t noC
     head[k] = (k < m && key[k] != noCell && (k == 0 || key[k - 1] != key[k])) ? 1 : 0;
 }
 
-// The cells' runs (every occupied cell queued, in run order), and the runs' points in run
-// order: {x, y, z, tree position bits}, with the distance a search surely reaches it at.
+// The cells' runs, and the runs' points in run order: {x, y, z, tree position bits}, with the distance a search surely reaches it at.
 __global__ void k_sp_cells(const uint32_t *__restrict__ key, const uint32_t *__restrict__ sortPos,
                            int m, uint32_t noCell, const int *__restrict__ head,
                            const int *__restrict__ rank, const float *__restrict__ nodeBox,
@@ -746,49 +751,18 @@ __global__ void k_sp_cells(const uint32_t *__restrict__ key, const uint32_t *__r
     if (head[k]) {
         cellRank[key[k]] = r;
         cellList[r]      = (int)key[k];
-        a.cur[r]         = k;
-        a.ring[r]        = r;
+        a.cur[r]         = sp_cur(k, (int)sortPos[k]);
     }
     if (k == m - 1 || key[k + 1] != key[k])
         cellEnd[r] = k + 1;
-    if (k == m - 1 || key[k + 1] == noCell) { // (the active entries sort first)
-        *a.tail = r + 1;
+    if (k == m - 1 || key[k + 1] == noCell) // (the active entries sort first)
         *a.open = r + 1;
-    }
     const int    ip = (int)sortPos[k];
     const float4 p  = a.t.pos[a.t.vacc[ip]];
     ent[k]          = make_float4(p.x, p.y, p.z, __int_as_float(ip));
     sure[k]         = sure_reach(a.r2, excursion(nodeBox + 6 * (size_t)leafOf[ip], p));
     a.dec[k]        = 0;
     a.filed[k]      = -1;
-}
-
-// The 27 cells around cell r: lane l < 27 gets the first open entry (or one before it) of
-// neighbour l's run, own cell from entry `own`; returns the lane's exclusive prefix of the
-// runs' lengths and writes their total to tot. With before >= 0, runs whose first open
-// point's tree position is above it count as empty.
-__device__ __forceinline__ int nb_runs(const SampleArgs &a, int r, int own, int before, int &nb,
-                                       int &tot) {
-    const int lane = threadIdx.x & 31;
-    const int cid  = a.cellList[r];
-    const int cx = cid % a.dim[0], cy = (cid / a.dim[0]) % a.dim[1], cz = cid / (a.dim[0] * a.dim[1]);
-    nb      = 0;
-    int len = 0;
-    if (lane < 27) {
-        const int x = cx + lane % 3 - 1, y = cy + (lane / 3) % 3 - 1, z = cz + lane / 9 - 1;
-        if (x >= 0 && y >= 0 && z >= 0 && x < a.dim[0] && y < a.dim[1] && z < a.dim[2]) {
-            const int nr = a.cellRank[(z * a.dim[1] + y) * a.dim[0] + x];
-            if (nr >= 0) {
-                nb  = nr == r ? own : ld_vol(&a.cur[nr]);
-                len = a.cellEnd[nr] - nb;
-                if (len > 0 && before >= 0 && __float_as_int(a.ent[nb].w) > before)
-                    len = 0;
-            }
-        }
-    }
-    const int incl = warp_incl_scan(len);
-    tot            = __shfl_sync(0xffffffffu, incl, 31);
-    return incl - len;
 }
 
 // Entry of flattened neighbourhood index t: binary search over the lanes' prefixes.
@@ -804,21 +778,42 @@ __device__ __forceinline__ int nb_entry(int t, int excl, int nb) {
     return __shfl_sync(0xffffffffu, nb, lo) + (t - __shfl_sync(0xffffffffu, excl, lo));
 }
 
-// (store; fence; load of the other's word) on both sides of a filing: whichever of the filing
-// warp and the deciding one comes second sees the other
+// Memory order. A cell moves between warps through the ring: pushed after a fence, taken by an
+// acquire. Filing stores the link and then looks at the entry's decision, deciding stores the
+// decision and then looks at the entry's list, each with a sequentially consistent fence
+// between: whichever comes second sees the other.
 __device__ __forceinline__ void fence_sc() { asm volatile("fence.sc.gpu;" ::: "memory"); }
-
+__device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+__device__ __forceinline__ int  exch_acquire(int *p, int v) {
+    int o;
+    asm volatile("atom.acquire.gpu.global.exch.b32 %0, [%1], %2;" : "=r"(o) : "l"(p), "r"(v) : "memory");
+    return o;
+}
+__device__ __forceinline__ int exch_release(int *p, int v) {
+    int o;
+    asm volatile("atom.release.gpu.global.exch.b32 %0, [%1], %2;" : "=r"(o) : "l"(p), "r"(v) : "memory");
+    return o;
+}
 // Queues the cells filed under entry j. A slot is written once its last reader has emptied it:
 // at most every cell is queued, and the ring holds twice as many.
 __device__ __forceinline__ void sp_wake(const SampleArgs &a, int j) {
-    int c = atomicExch(&a.filed[j], -1);
+    int c = exch_acquire(&a.filed[j], -1);
     if (c < 0)
         return;
-    __threadfence();
+    fence_acq_rel();
     while (c >= 0) {
-        const int nx = ld_vol(&a.nextCell[c]); // (its holder may file it anew once it is queued)
-        int      *s  = &a.ring[(unsigned)atomicAdd(a.tail, 1) & a.ringMask];
-        for (long long it = 0; atomicCAS(s, -1, c) != -1; it++)
+        // (a cell enters the list before its link is stored)
+        int nx = ld_vol(&a.nextCell[c]);
+        for (long long it = 0; nx == kSpUnlinked; it++) {
+            if (it > kSpIdle) {
+                atomicExch(a.err, 1);
+                return;
+            }
+            nx = ld_vol(&a.nextCell[c]);
+        }
+        const int cid = a.cellList[c];
+        int      *s   = &a.ring[(unsigned)atomicAdd(a.tail, 1) & a.ringMask];
+        for (long long it = 0; atomicCAS(s, -1, cid) != -1; it++)
             if (it > kSpIdle) {
                 atomicExch(a.err, 1);
                 return;
@@ -832,7 +827,7 @@ __device__ __forceinline__ int sp_take(const SampleArgs &a) {
     int *s = &a.ring[(unsigned)atomicAdd(a.head, 1) & a.ringMask];
     for (long long it = 0;; it++) {
         if (ld_vol(s) >= 0) {
-            const int c = atomicExch(s, -1);
+            const int c = exch_acquire(s, -1);
             if (c >= 0)
                 return c;
         }
@@ -849,31 +844,69 @@ __device__ __forceinline__ int sp_take(const SampleArgs &a) {
     }
 }
 
+// The runs around a cell, a neighbour per lane (-1: none, lane kSpOwn: the cell itself). A take
+// is a chain of dependent loads, so what a later step needs is read with the one before it.
+constexpr int kSpOwn = 13;
+struct SpRuns {
+    int nr, nend;      // occupied rank, end of its run
+    int from, pos;     // its first open entry (or one before it) and that one's tree position
+    int nb, excl, tot; // this pass's begin, exclusive prefix of the lengths and their sum
+    __device__ __forceinline__ void find(const SampleArgs &a, int cid) {
+        const int lane = threadIdx.x & 31;
+        const int cx = cid % a.dim[0], cy = (cid / a.dim[0]) % a.dim[1],
+                  cz = cid / (a.dim[0] * a.dim[1]);
+        const int x = cx + lane % 3 - 1, y = cy + (lane / 3) % 3 - 1, z = cz + lane / 9 - 1;
+        nr   = -1;
+        nend = from = pos = 0;
+        if (lane < 27 && x >= 0 && y >= 0 && z >= 0 && x < a.dim[0] && y < a.dim[1] && z < a.dim[2])
+            nr = a.cellRank[(z * a.dim[1] + y) * a.dim[0] + x];
+        if (nr >= 0)
+            nend = a.cellEnd[nr];
+        look(a);
+    }
+    __device__ __forceinline__ void look(const SampleArgs &a) {
+        if (nr < 0)
+            return;
+        const unsigned long long w = *(const volatile unsigned long long *)&a.cur[nr];
+        from = (int)(unsigned)w;
+        pos  = (int)(w >> 32);
+    }
+    // each run from its first open entry, the cell's own from entry `own`; with before >= 0 runs
+    // whose first open point's tree position is above it count as empty
+    __device__ __forceinline__ void begin(int own, int before) {
+        const bool self = (threadIdx.x & 31) == kSpOwn;
+        nb              = self ? own : from;
+        const int len   = nr < 0 || (before >= 0 && !self && pos > before) ? 0 : nend - nb;
+        const int incl  = warp_incl_scan(len);
+        tot             = __shfl_sync(0xffffffffu, incl, 31);
+        excl            = incl - len;
+    }
+    __device__ __forceinline__ int entry(int t) const { return nb_entry(min(t, tot - 1), excl, nb); }
+};
+
 // An open entry with tree position below ip within the step of p: -1 when there is none.
-__device__ __forceinline__ int sp_blocker(const SampleArgs &a, int r, int k, const float4 &p,
+__device__ __forceinline__ int sp_blocker(const SampleArgs &a, SpRuns &R, int k, const float4 &p,
                                           int ip) {
-    const int lane = threadIdx.x & 31;
-    int       nb, tot;
-    const int excl = nb_runs(a, r, k, ip - 1, nb, tot);
-    for (int base = 0; base < tot; base += 32 * kSpUnroll) {
+    const int   lane = threadIdx.x & 31;
+    const float q[3] = {p.x, p.y, p.z};
+    R.begin(k, ip - 1);
+    for (int base = 0; base < R.tot; base += 32 * kSpUnroll) {
         int    kb[kSpUnroll], dec[kSpUnroll];
         float4 b[kSpUnroll];
 #pragma unroll
         for (int u = 0; u < kSpUnroll; u++)
-            kb[u] = nb_entry(min(base + u * 32 + lane, tot - 1), excl, nb);
+            kb[u] = R.entry(base + u * 32 + lane);
 #pragma unroll
         for (int u = 0; u < kSpUnroll; u++) {
             b[u]   = a.ent[kb[u]];
             dec[u] = ld_vol(&a.dec[kb[u]]);
         }
-        int last = -1; // the lane's latest blocker: it waits longest, so it is the one to wait for
-        int at   = -1;
+        int last = -1, at = -1; // the lane's latest blocker waits longest: the one to wait for
 #pragma unroll
         for (int u = 0; u < kSpUnroll; u++) {
-            const int   ib    = __float_as_int(b[u].w);
-            const float bq[3] = {b[u].x, b[u].y, b[u].z};
-            if (base + u * 32 + lane < tot && dec[u] == 0 && ib < ip && ib > last &&
-                smk::eval_metric(bq, p) < a.r2) {
+            const int ib = __float_as_int(b[u].w);
+            if (base + u * 32 + lane < R.tot && dec[u] == 0 && ib < ip && ib > last &&
+                smk::eval_metric(q, b[u]) < a.r2) {
                 last = ib;
                 at   = kb[u];
             }
@@ -885,89 +918,135 @@ __device__ __forceinline__ int sp_blocker(const SampleArgs &a, int r, int k, con
     return -1;
 }
 
-// Drops the open later points that the search of kept point q (entry k of cell r) reaches.
-__device__ __forceinline__ void sp_drop(const SampleArgs &a, int r, int k, const float4 &q, int iq) {
-    const int   lane  = threadIdx.x & 31;
-    const float qq[3] = {q.x, q.y, q.z};
-    int         nb, tot;
-    const int   excl = nb_runs(a, r, k + 1, -1, nb, tot);
-    for (int base = 0; base < tot; base += 32 * kSpUnroll) {
-        int    kp[kSpUnroll], dec[kSpUnroll];
-        float  sure[kSpUnroll];
-        float4 p[kSpUnroll];
-#pragma unroll
-        for (int u = 0; u < kSpUnroll; u++)
-            kp[u] = nb_entry(min(base + u * 32 + lane, tot - 1), excl, nb);
-#pragma unroll
-        for (int u = 0; u < kSpUnroll; u++) {
-            p[u]    = a.ent[kp[u]];
-            sure[u] = a.sure[kp[u]];
-            dec[u]  = ld_vol(&a.dec[kp[u]]);
-        }
-        bool gone[kSpUnroll], any = false;
-#pragma unroll
-        for (int u = 0; u < kSpUnroll; u++) {
-            gone[u] = base + u * 32 + lane < tot && dec[u] == 0 && __float_as_int(p[u].w) > iq &&
-                      smk::eval_metric(qq, p[u]) < a.r2 &&
-                      reaches(a, q, p[u], __float_as_int(p[u].w), sure[u]);
-            if (gone[u]) {
-                *(volatile int *)&a.dec[kp[u]] = 2;
-                any                            = true;
-            }
-        }
-        if (!any)
+// Drops the open later points of kept point p's runs from the 1024th on that its search reaches and
+// queues the cells filed under them.
+__device__ __forceinline__ void sp_drop_far(const SampleArgs &a, const SpRuns &R, const float4 &p,
+                                            int ip) {
+    const int lane = threadIdx.x & 31;
+    for (int base = 1024; base < R.tot; base += 32) {
+        const int    kb = R.entry(base + lane);
+        const float4 b  = a.ent[kb];
+        const bool   go = base + lane < R.tot && __float_as_int(b.w) > ip && ld_vol(&a.dec[kb]) == 0 &&
+                        reaches(a, p, b, __float_as_int(b.w), a.sure[kb]);
+        if (go)
+            *(volatile int *)&a.dec[kb] = 2;
+        if (!__any_sync(0xffffffffu, go))
             continue;
         fence_sc();
+        if (go && ld_vol(&a.filed[kb]) >= 0)
+            sp_wake(a, kb);
+    }
+}
+
+// Drops the open later points that the search of kept point p (entry k) reaches: a bit of the
+// lane for each (bit j: entry 32 j + lane) of the first 1024, for the caller to wake after its
+// fence. Those from the 1024th on are woken here.
+__device__ __forceinline__ unsigned sp_drop(const SampleArgs &a, SpRuns &R, int k, const float4 &p,
+                                            int ip) {
+    const int   lane = threadIdx.x & 31;
+    const float q[3] = {p.x, p.y, p.z};
+    unsigned    drop = 0u;
+    R.begin(k + 1, -1);
+    for (int base = 0; base < min(R.tot, 1024); base += 32 * kSpUnroll) {
+        int    kb[kSpUnroll], dec[kSpUnroll];
+        float  sure[kSpUnroll];
+        float4 b[kSpUnroll];
 #pragma unroll
         for (int u = 0; u < kSpUnroll; u++)
-            if (gone[u] && ld_vol(&a.filed[kp[u]]) >= 0)
-                sp_wake(a, kp[u]);
+            kb[u] = R.entry(base + u * 32 + lane);
+#pragma unroll
+        for (int u = 0; u < kSpUnroll; u++) {
+            b[u]    = a.ent[kb[u]];
+            sure[u] = a.sure[kb[u]];
+            dec[u]  = ld_vol(&a.dec[kb[u]]);
+        }
+#pragma unroll
+        for (int u = 0; u < kSpUnroll; u++) {
+            const int ib = __float_as_int(b[u].w);
+            if (base + u * 32 + lane < R.tot && dec[u] == 0 && ib > ip &&
+                smk::eval_metric(q, b[u]) < a.r2 && reaches(a, p, b[u], ib, sure[u])) {
+                *(volatile int *)&a.dec[kb[u]] = 2;
+                drop |= 1u << (base / 32 + u);
+            }
+        }
+    }
+    if (R.tot > 1024)
+        sp_drop_far(a, R, p, ip);
+    return drop;
+}
+
+// Before the queue runs nothing is decided: a warp per cell files it under the first blocker of
+// its first point, or queues it. (Through the queue these are a third of its takes, each with the
+// queue's fences: the large scene's last sampling took 1.79 ms in k_sp_run alone, now 0.08 ms here
+// and 1.27 ms there.)
+__global__ void __launch_bounds__(kSpBs) k_sp_first(SampleArgs a) {
+    const int lane = threadIdx.x & 31;
+    const int n = *a.open, nw = gridDim.x * (kSpBs / 32);
+    for (int r = blockIdx.x * (kSpBs / 32) + (threadIdx.x >> 5); r < n; r += nw) {
+        SpRuns R;
+        const int cid = a.cellList[r];
+        R.find(a, cid);
+        const int    k = __shfl_sync(0xffffffffu, R.from, kSpOwn);
+        const float4 p = a.ent[k];
+        const int    j = sp_blocker(a, R, k, p, __float_as_int(p.w));
+        if (lane == 0) {
+            if (j >= 0)
+                a.nextCell[r] = atomicExch(&a.filed[j], r);
+            else
+                a.ring[(unsigned)atomicAdd(a.tail, 1) & a.ringMask] = cid;
+        }
     }
 }
 
 __global__ void __launch_bounds__(kSpBs) k_sp_run(SampleArgs a) {
     const int lane = threadIdx.x & 31;
     for (;;) {
-        const int r = __shfl_sync(0xffffffffu, lane == 0 ? sp_take(a) : 0, 0);
-        if (r < 0)
+        const int cid = __shfl_sync(0xffffffffu, lane == 0 ? sp_take(a) : 0, 0);
+        if (cid < 0)
             return;
-        __threadfence(); // the decisions before the cell was queued are visible
-        int       k = ld_vol(&a.cur[r]);
-        const int e = a.cellEnd[r];
-        for (;;) {
+        __syncwarp(); // (lane 0's acquire holds for the warp)
+        SpRuns R;
+        R.find(a, cid);
+        const int r = __shfl_sync(0xffffffffu, R.nr, kSpOwn);
+        const int e = __shfl_sync(0xffffffffu, R.nend, kSpOwn);
+        int       k = __shfl_sync(0xffffffffu, R.from, kSpOwn);
+        for (bool again = false;; again = true) {
+            if (again)
+                R.look(a);
             // the cell's first open entry
             unsigned open = 0u;
+            float4   p;
             for (; k < e; k += 32) {
-                open = __ballot_sync(0xffffffffu, k + lane < e && ld_vol(&a.dec[k + lane]) == 0);
+                const int  kl = min(k + lane, e - 1);
+                const bool un = ld_vol(&a.dec[kl]) == 0;
+                p             = a.ent[kl];
+                open          = __ballot_sync(0xffffffffu, un && k + lane < e);
                 if (open)
                     break;
             }
             if (!open) {
                 if (lane == 0) {
-                    *(volatile int *)&a.cur[r] = e;
+                    *(volatile unsigned long long *)&a.cur[r] = sp_cur(e, INT_MAX);
                     atomicSub(a.open, 1);
                 }
                 break;
             }
-            k += __ffs(open) - 1;
+            const int at = __ffs(open) - 1;
+            k += at;
+            p.x = __shfl_sync(0xffffffffu, p.x, at);
+            p.y = __shfl_sync(0xffffffffu, p.y, at);
+            p.z = __shfl_sync(0xffffffffu, p.z, at);
+            p.w = __shfl_sync(0xffffffffu, p.w, at);
+            const int ip = __float_as_int(p.w);
             if (lane == 0)
-                *(volatile int *)&a.cur[r] = k;
-            const float4 p  = a.ent[k];
-            const int    ip = __float_as_int(p.w);
-            const int    j  = sp_blocker(a, r, k, p, ip);
+                *(volatile unsigned long long *)&a.cur[r] = sp_cur(k, ip);
+            const int j = sp_blocker(a, R, k, p, ip);
             if (j >= 0) {
                 if (lane == 0) {
-                    // file the cell under j, unless j was decided meanwhile: then whoever takes
-                    // j's list (this warp or the one that decided j) queues it
-                    int old = ld_vol(&a.filed[j]);
-                    for (;;) {
-                        *(volatile int *)&a.nextCell[r] = old;
-                        __threadfence();
-                        const int seen = atomicCAS(&a.filed[j], old, r);
-                        if (seen == old)
-                            break;
-                        old = seen;
-                    }
+                    // file the cell under j; if j was decided meanwhile, whoever takes j's list
+                    // (this lane or the one that decided j) queues the cell
+                    *(volatile int *)&a.nextCell[r] = kSpUnlinked;
+                    *(volatile int *)&a.nextCell[r] = exch_release(&a.filed[j], r);
                     fence_sc();
                     if (ld_vol(&a.dec[j]) != 0)
                         sp_wake(a, j);
@@ -977,19 +1056,25 @@ __global__ void __launch_bounds__(kSpBs) k_sp_run(SampleArgs a) {
             }
             // no open earlier point within the step. A kept point drops before it counts as
             // decided, so p's own state is final now
-            __threadfence();
+            fence_acq_rel();
             if (__shfl_sync(0xffffffffu, lane == 0 ? ld_vol(&a.dec[k]) : 0, 0) != 0)
                 continue; // dropped meanwhile: on to the cell's next open entry
-            sp_drop(a, r, k, p, ip);
-            __threadfence();
+            const unsigned drop = sp_drop(a, R, k, p, ip);
+            const unsigned any  = __reduce_or_sync(0xffffffffu, drop);
+            fence_acq_rel();
             __syncwarp();
             if (lane == 0) {
-                a.keptFlag[ip]               = 1;
-                *(volatile int *)&a.dec[k]   = 1;
-                fence_sc();
-                if (ld_vol(&a.filed[k]) >= 0)
-                    sp_wake(a, k);
+                a.keptFlag[ip]             = 1;
+                *(volatile int *)&a.dec[k] = 1;
             }
+            fence_sc();
+            for (unsigned m = any; m; m &= m - 1u) {
+                const int jb = __ffs(m) - 1, kb = R.entry(jb * 32 + lane);
+                if (((drop >> jb) & 1u) && ld_vol(&a.filed[kb]) >= 0)
+                    sp_wake(a, kb);
+            }
+            if (lane == 0 && ld_vol(&a.filed[k]) >= 0)
+                sp_wake(a, k);
             __syncwarp();
         }
     }
@@ -1261,7 +1346,7 @@ int kd_sample(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
     a.cellRank = cRank;
     a.cellList = cList;
     a.cellEnd  = cEnd;
-    a.cur      = c.arena.get<int>(tag + ".cur", m);
+    a.cur      = c.arena.get<unsigned long long>(tag + ".cur", m);
     a.dec      = c.arena.get<int>(tag + ".dec", m);
     a.filed    = c.arena.get<int>(tag + ".filed", m);
     a.nextCell = c.arena.get<int>(tag + ".next", m);
@@ -1288,6 +1373,8 @@ int kd_sample(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
     SM_LAUNCH_CHECK();
     int nsm = 0;
     SM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device));
+    k_sp_first<<<std::min(nblocks(m, kSpBs / 32), nsm * 8), kSpBs, 0, c.stream>>>(a);
+    SM_LAUNCH_CHECK();
     k_sp_run<<<std::min(nblocks(m, kSpBs / 32), nsm * kSpCtas), kSpBs, 0, c.stream>>>(a);
     SM_LAUNCH_CHECK();
     int *pre = c.arena.get<int>(tag + ".pre", (size_t)m + 1);

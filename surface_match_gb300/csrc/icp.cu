@@ -100,22 +100,26 @@ __device__ __forceinline__ unsigned long long win_key(float d, int i) {
     return ((unsigned long long)__float_as_uint(d) << 32) | (unsigned)i;
 }
 
-// The nearest point of the stage's subset to (x, y, z) by a warp, exact where its squared
-// distance is at most lim: subset rank (-1: none found) and squared distance d. With TREE the
-// point that the reference's search finds (sm_kdgrid.cuh).
+// The nearest point of the stage's subset to each lane's (x, y, z) (`need`: it has one), exact
+// where its squared distance is at most lim: subset rank (-1: none found) and squared distance
+// d. With TREE the point that the reference's search finds (sm_kdgrid.cuh).
 template <bool TREE>
 __device__ __forceinline__ int stage_nearest(const Stage &s, float x, float y, float z, float lim,
-                                             float &d) {
+                                             bool need, float &d) {
     if (TREE)
-        return smk::warp_kd_nearest(s.tree, s.treeM, s.G, s.tposOf, s.rankOf, *s.exc, x, y, z, lim,
-                                    &d);
-    return warp_nn_walk(s.G, x, y, z, lim, d);
+        return smk::lanes_kd_nearest(s.tree, s.treeM, s.G, s.tposOf, s.rankOf, *s.exc, x, y, z, lim,
+                                     need, &d);
+    return lanes_nn_walk(s.G, x, y, z, lim, need, &d);
 }
 
-// K1: correspondences, one warp per (candidate, source point) of the step's candidates
-// (warp-cooperative grid search; the grid of CTAs is one resident wave, so that the launches
-// after the last candidate stopped cost next to nothing: 9 us for a CTA per 8 points of every
-// candidate, 2.5 us now). In reference order (TREE) a pair is what findClosestPoint
+// K1: correspondences of the (candidate, source point) items of the step's candidates. A warp
+// takes up to 32 items, spread over the launch so that the far-off points, whose searches are
+// the long ones, fall on many warps: it loads, moves and stores them a lane each and searches for
+// them one after the other. (What surrounds a search was a quarter of its instructions when the
+// whole warp did it for each item: ten launches of the large scene 219 -> 201 us; in reference
+// order, where the root paths are a lane's too, 705 -> 563 us.) The CTAs are one resident wave,
+// so that the launches after the last candidate stopped cost little: 9 us for a CTA per 8 points
+// of every candidate, 3 us now. In reference order (TREE) a pair is what findClosestPoint
 // (util.cpp:603-626) returns: a one-nearest search of the reduced k-d tree with the tree's
 // pruning; one beyond the rejection distance is dropped, so the search is needed up to that
 // distance only.
@@ -126,29 +130,37 @@ __global__ void __launch_bounds__(kT, TREE ? 3 : 4) k_corr(Work w, Stage s, int 
     const long long items = (long long)step_count(w, it) * s.n;
     if (w.live && blockIdx.x == 0 && threadIdx.x == 0)
         atomicAdd(w.live, (unsigned long long)items);
-    for (long long k = blockIdx.x * kW + (threadIdx.x >> 5); k < items; k += gridDim.x * kW) {
-        int          ci, i;
-        step_item(w, it, k, s.n, ci, i);
-        const size_t o  = (size_t)ci * w.maxSrc + i;
-        const Cand  &C  = w.cand[ci];
-        const float4 sp = s.src[i], sn = s.srcN[i];
-        float4       x, y;
-        // written by this candidate's previous iteration of this stage (not in the first), a
-        // rank of this stage's subset or -1
-        const int jp = it > 0 ? w.nnPrev[o] : -1;
-        float4    qp = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (jp >= 0 && jp < s.nDst)
-            qp = s.dPos[jp];
-        smi::pose_apply(C.M, sp.x, sp.y, sp.z, x.x, x.y, x.z);
-        smi::pose_rotate(C.M, sn.x, sn.y, sn.z, y.x, y.y, y.z);
-        // the last iteration's nearest point of this stage bounds the search exactly
-        float lim = s.rej2;
-        if (jp >= 0 && jp < s.nDst)
-            lim = fminf(lim, smm::dist2(x.x, x.y, x.z, qp.x, qp.y, qp.z));
-        float      d;
-        const int  j  = stage_nearest<TREE>(s, x.x, x.y, x.z, lim, d); // subset rank
-        const bool ok = j >= 0 && d <= s.rej2;
-        if (lane == 0) {
+    const long long warps = (long long)gridDim.x * kW;
+    for (long long base = blockIdx.x * kW + (threadIdx.x >> 5); base < items; base += 32 * warps) {
+        const long long k    = base + lane * warps;
+        const bool      have = k < items;
+        int             ci = 0, i = 0;
+        if (have)
+            step_item(w, it, k, s.n, ci, i);
+        const size_t o   = (size_t)ci * w.maxSrc + i;
+        const Cand  &C   = w.cand[ci];
+        float4       x   = make_float4(0.f, 0.f, 0.f, 0.f);
+        float        lim = s.rej2;
+        if (have) {
+            // written by this candidate's previous iteration of this stage (not in the first), a
+            // rank of this stage's subset or -1
+            const int    jp = it > 0 ? w.nnPrev[o] : -1;
+            const float4 sp = s.src[i];
+            float4       qp = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (jp >= 0 && jp < s.nDst)
+                qp = s.dPos[jp];
+            smi::pose_apply(C.M, sp.x, sp.y, sp.z, x.x, x.y, x.z);
+            // the last iteration's nearest point of this stage bounds the search exactly
+            if (jp >= 0 && jp < s.nDst)
+                lim = fminf(lim, smm::dist2(x.x, x.y, x.z, qp.x, qp.y, qp.z));
+        }
+        float     d;
+        const int j = stage_nearest<TREE>(s, x.x, x.y, x.z, lim, have, d); // subset rank
+        if (have) {
+            const bool   ok = j >= 0 && d <= s.rej2;
+            const float4 sn = s.srcN[i];
+            float4       y;
+            smi::pose_rotate(C.M, sn.x, sn.y, sn.z, y.x, y.y, y.z);
             w.nnPrev[o] = j;
             x.w         = d;
             y.w         = 0.0f;
@@ -425,26 +437,35 @@ __global__ void __cluster_dims__(kRC, 1, 1) __launch_bounds__(kR) k_fit(Work w, 
     }
 }
 
-// K4: residual distance of each pair after the step, one warp per pair
+// K4: residual distance of each pair after the step, items as in K1 (ten launches of the large
+// scene in reference order 528 -> 452 us)
 template <bool TREE>
 __global__ void __launch_bounds__(kT, TREE ? 3 : 5) k_resid(Work w, Stage s, int it) {
     chain_enter(); // launched chained
     const long long items = (long long)step_count(w, it) * s.n;
-    for (long long k = blockIdx.x * kW + (threadIdx.x >> 5); k < items; k += gridDim.x * kW) {
-        int          ci, i;
-        step_item(w, it, k, s.n, ci, i);
-        const size_t o  = (size_t)ci * w.maxSrc + i;
-        const Cand  &C  = w.cand[ci];
-        const int    j  = w.nnId[o];
-        const float4 x  = w.x4[o];
-        if (C.cnt < 6 || j < 0)
-            continue;
-        const float4 q = s.dPos[j];
-        float        y0, y1, y2, d;
-        smi::pose_apply(C.step, x.x, x.y, x.z, y0, y1, y2);
-        // the pair's scene point bounds the search exactly
-        stage_nearest<TREE>(s, y0, y1, y2, smm::dist2(y0, y1, y2, q.x, q.y, q.z), d);
-        if ((threadIdx.x & 31) == 0)
+    const long long warps = (long long)gridDim.x * kW;
+    for (long long base = blockIdx.x * kW + (threadIdx.x >> 5); base < items; base += 32 * warps) {
+        const long long k    = base + (threadIdx.x & 31) * warps;
+        bool            have = k < items;
+        int             ci = 0, i = 0;
+        if (have)
+            step_item(w, it, k, s.n, ci, i);
+        const size_t o = (size_t)ci * w.maxSrc + i;
+        float        y0 = 0.f, y1 = 0.f, y2 = 0.f, lim = 0.f, d;
+        if (have) {
+            const Cand  &C = w.cand[ci];
+            const int    j = w.nnId[o];
+            const float4 x = w.x4[o];
+            have           = C.cnt >= 6 && j >= 0;
+            if (have) {
+                const float4 q = s.dPos[j];
+                smi::pose_apply(C.step, x.x, x.y, x.z, y0, y1, y2);
+                // the pair's scene point bounds the search exactly
+                lim = smm::dist2(y0, y1, y2, q.x, q.y, q.z);
+            }
+        }
+        stage_nearest<TREE>(s, y0, y1, y2, lim, have, d);
+        if (have)
             w.resid[o] = smm::fsqrt(d);
     }
 }
@@ -597,9 +618,10 @@ __global__ void k_stage_end(Work w, int last, int failStatus) {
 }
 
 // Inliers of each candidate left (step `last`): source points with a scene point closer than the
-// scoring distance, one warp per point (warp_any_within); with TREE the scene point that the
-// reference's search of the whole tree returns (inliner, util.cpp:628-641). A warp takes
-// consecutive points, so that it adds to a candidate's count once or twice.
+// scoring distance (warp_any_within); with TREE the scene point that the reference's search of the
+// whole tree returns (inliner, util.cpp:628-641). A warp takes consecutive points, 32 at a time a
+// lane each, and adds to a candidate's count once per 32 (two launches of the large scene in
+// reference order 250 -> 158 us).
 template <bool TREE>
 __global__ void __launch_bounds__(kT, TREE ? 3 : 6)
     k_inliers(Work w, const float4 *__restrict__ src, int n, int last, HGridView F, float r2,
@@ -610,30 +632,36 @@ __global__ void __launch_bounds__(kT, TREE ? 3 : 6)
     const long long warps = (long long)gridDim.x * kW, per = (items + warps - 1) / warps;
     long long       k   = (blockIdx.x * (long long)kW + (threadIdx.x >> 5)) * per;
     const long long end = k + per < items ? k + per : items;
-    int             c = 0, at = -1;
-    for (; k < end; k++) {
-        int ci, i;
-        step_item(w, last, k, n, ci, i);
-        if (ci != at) {
-            if (c && (threadIdx.x & 31) == 0)
-                atomicAdd(&w.cand[at].inl, c);
-            at = ci;
-            c  = 0;
+    const int       lane = threadIdx.x & 31;
+    for (; k < end; k += 32) {
+        const bool have = k + lane < end;
+        int        ci = -1, i = 0;
+        float      x = 0.f, y = 0.f, z = 0.f;
+        if (have) {
+            step_item(w, last, k + lane, n, ci, i);
+            const float4 p = src[i];
+            smi::pose_apply(w.cand[ci].M, p.x, p.y, p.z, x, y, z);
         }
-        float        x, y, z;
-        const float4 p = src[i];
-        smi::pose_apply(w.cand[ci].M, p.x, p.y, p.z, x, y, z);
+        bool in = false;
         if (TREE) {
             float     d;
-            const int j =
-                smk::warp_kd_nearest(t, treeM, F, treePos, nullptr, *exc, x, y, z, r2, &d);
-            c += (j >= 0 && d < r2) ? 1 : 0;
+            const int j = smk::lanes_kd_nearest(t, treeM, F, treePos, nullptr, *exc, x, y, z, r2, have, &d);
+            in          = j >= 0 && d < r2;
         } else {
-            c += warp_any_within(F, x, y, z, r2) ? 1 : 0;
+            for (unsigned m = __ballot_sync(0xffffffffu, have); m; m &= m - 1u) {
+                const int  l = __ffs(m) - 1;
+                const bool h = warp_any_within(F, __shfl_sync(0xffffffffu, x, l), __shfl_sync(0xffffffffu, y, l),
+                                               __shfl_sync(0xffffffffu, z, l), r2);
+                if (lane == l)
+                    in = h;
+            }
         }
+        // a count per candidate of the 32 points
+        const unsigned same = __match_any_sync(0xffffffffu, ci);
+        const unsigned hits = __ballot_sync(0xffffffffu, in) & same;
+        if (hits && lane == __ffs(same) - 1)
+            atomicAdd(&w.cand[ci].inl, __popc(hits));
     }
-    if (c && (threadIdx.x & 31) == 0)
-        atomicAdd(&w.cand[at].inl, c);
 }
 
 __global__ void k_score(Work w, int ncand, int n, float minScore, int failStatus, int slot) {

@@ -581,6 +581,26 @@ __device__ __forceinline__ int warp_nn_walk(const HGridView &g, float qx, float 
     return (int)(unsigned)(best & 0xffffffffu);
 }
 
+// The same for up to 32 queries of a warp, a lane's own each (`need`: it has one), query after
+// query: what surrounds a search is done for 32 queries at once.
+__device__ __forceinline__ int lanes_nn_walk(const HGridView &g, float qx, float qy, float qz,
+                                             float limit2, bool need, float *d) {
+    int j = -1;
+    *d    = 3.402823466e+38f;
+    for (unsigned w = __ballot_sync(0xffffffffu, need); w; w &= w - 1u) {
+        const int src = __ffs(w) - 1;
+        float     dd;
+        const int r = warp_nn_walk(g, __shfl_sync(0xffffffffu, qx, src), __shfl_sync(0xffffffffu, qy, src),
+                                   __shfl_sync(0xffffffffu, qz, src),
+                                   __shfl_sync(0xffffffffu, limit2, src), dd);
+        if ((threadIdx.x & 31) == src) {
+            j  = r;
+            *d = dd;
+        }
+    }
+    return j;
+}
+
 // Whether any point lies closer than sqrt(r2) to q, by a warp: cells whose lower bound
 // reaches r2 are skipped, and the search ends at the first round with a hit or after the
 // ring whose bound reaches sqrt(r2).

@@ -319,6 +319,56 @@ __device__ __forceinline__ int warp_kd_nearest(const KdView &t, int m, const smd
     return __shfl_sync(0xffffffffu, id, 0);
 }
 
+// The same for up to 32 queries of a warp, a lane's own each (`need`: it has one): the nearest
+// points on the grid by the whole warp, query after query, then the root paths of those that
+// are the only ones at their distance by their lanes at once (a point that is reached even with
+// its own distance as the bound is the one that is returned), and the search above for the rest.
+// (A warp's restricted search per query took two thirds of the time of the reference order's
+// correspondences.)
+__device__ __forceinline__ int lanes_kd_nearest(const KdView &t, int m, const smd::HGridView &g,
+                                                const int *__restrict__ posOf,
+                                                const int *__restrict__ nameOf, float exc, float qx,
+                                                float qy, float qz, float limit2, bool need, float *d) {
+    const int lane = threadIdx.x & 31;
+    int       j    = -1;
+    bool      tied = false;
+    float     dd;
+    *d = 3.402823466e+38f;
+    // (no distance from a point that is not finite is below the search's start)
+    need = need && isfinite(qx) && isfinite(qy) && isfinite(qz);
+    for (unsigned w = __ballot_sync(0xffffffffu, need); w; w &= w - 1u) {
+        const int src = __ffs(w) - 1;
+        bool      tie;
+        const int r = warp_nn_tie(g, __shfl_sync(0xffffffffu, qx, src), __shfl_sync(0xffffffffu, qy, src),
+                                  __shfl_sync(0xffffffffu, qz, src),
+                                  __shfl_sync(0xffffffffu, limit2, src), dd, tie);
+        if (lane == src) {
+            j    = r;
+            *d   = dd;
+            tied = tie;
+        }
+    }
+    bool open = false;
+    if (j >= 0 && *d > limit2) {
+        j = -1; // the reference's result is no nearer
+    } else if (j >= 0) {
+        uint64_t    key;
+        const float q[3] = {qx, qy, qz};
+        open             = tied || !kd_reaches(t, q, posOf[j], *d, &key);
+    }
+    for (unsigned w = __ballot_sync(0xffffffffu, open); w; w &= w - 1u) {
+        const int src = __ffs(w) - 1;
+        const int r   = warp_kd_nearest(t, m, g, posOf, nameOf, exc, __shfl_sync(0xffffffffu, qx, src),
+                                        __shfl_sync(0xffffffffu, qy, src), __shfl_sync(0xffffffffu, qz, src),
+                                        __shfl_sync(0xffffffffu, limit2, src), &dd);
+        if (lane == src) {
+            j  = r;
+            *d = dd;
+        }
+    }
+    return j;
+}
+
 // The k nearest (k <= 32) that the reference's search of tree `t` (m positions; the points of
 // grid g) returns from q, in its order: lane j < the returned count gets the j-th point's id.
 // -1: not decided here (the caller runs the search itself).

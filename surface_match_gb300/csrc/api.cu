@@ -763,7 +763,7 @@ void match(Ctx &c, const Model &m, const float *xyzIn, const float *nrmIn, int64
                    vo.stats, K, cstat, cscore, cpose, ncand, dres);
     std::vector<int> big;
     int             *hres = c.hostCounts + kHostResult;
-    if (words > kHostInts - kHostResult) {
+    if (words > kHostStep - kHostResult) {
         big.resize(words);
         hres = big.data();
     }

@@ -81,6 +81,7 @@ struct Work {
     // list[it * ncand ..], cnt[it] of them; step `iters` holds those the stage leaves active
     int                *cnt, *list;
     int                 ncand;
+    unsigned long long *heard; // page-locked: {tag, candidates} of the last step begun
 };
 
 // The candidates of step `it`: their number and the k-th.
@@ -124,12 +125,17 @@ __device__ __forceinline__ int stage_nearest(const Stage &s, float x, float y, f
 // pruning; one beyond the rejection distance is dropped, so the search is needed up to that
 // distance only.
 template <bool TREE>
-__global__ void __launch_bounds__(kT, TREE ? 3 : 4) k_corr(Work w, Stage s, int it) {
+__global__ void __launch_bounds__(kT, TREE ? 3 : 4)
+    k_corr(Work w, Stage s, int it, unsigned tag) {
     chain_enter(); // launched chained
     const int       lane  = threadIdx.x & 31;
     const long long items = (long long)step_count(w, it) * s.n;
-    if (w.live && blockIdx.x == 0 && threadIdx.x == 0)
-        atomicAdd(w.live, (unsigned long long)items);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *(volatile unsigned long long *)w.heard =
+            ((unsigned long long)tag << 32) | (unsigned)step_count(w, it);
+        if (w.live)
+            atomicAdd(w.live, (unsigned long long)items);
+    }
     const long long warps = (long long)gridDim.x * kW;
     for (long long base = blockIdx.x * kW + (threadIdx.x >> 5); base < items; base += 32 * warps) {
         const long long k    = base + lane * warps;
@@ -705,6 +711,30 @@ int wave(const Ctx &c, long long items, int perSm) {
     return (int)std::max<long long>(1, std::min<long long>((items + kW - 1) / kW, (long long)nsm * perSm));
 }
 
+// The candidates of the refinement step of this tag, once it has begun: a poll of page-locked
+// memory, which ends with the stream's work (-1: not told, the caller goes on).
+int step_heard(Ctx &c, unsigned tag) {
+    const volatile unsigned long long *word =
+        reinterpret_cast<const volatile unsigned long long *>(c.hostCounts + kHostStep);
+    for (int spin = 1;; spin++) {
+        const unsigned long long v = *word;
+        if ((unsigned)(v >> 32) == tag)
+            return (int)(unsigned)v;
+        if (spin % 1024 == 0) {
+            const cudaError_t e = cudaStreamQuery(c.stream);
+            if (e == cudaErrorNotReady)
+                continue;
+            SM_CUDA(e);
+            const unsigned long long last = *word;
+            return (unsigned)(last >> 32) == tag ? (int)(unsigned)last : -1;
+        }
+    }
+}
+
+// Most stages end after two or three steps: their candidates converge, whatever the limit. A
+// step is launched while the one before it runs, and none after one that found no candidates left
+// (four empty launches otherwise for every step up to the limit: a refinement limited to 15
+// dense steps took 0.49 ms, 0.43 now).
 void run_stage(Ctx &c, const Work &w, const Stage &s) {
     const int       gc   = w.ncand * kRC; // reductions: a cluster per candidate
     const bool      tree = s.tree.nd != nullptr;
@@ -712,11 +742,14 @@ void run_stage(Ctx &c, const Work &w, const Stage &s) {
     const int gCorr = wave(c, all, tree ? 3 : 4), gResid = wave(c, all, tree ? 3 : 5);
     launch_chained(c, k_stage_begin, nblocks(w.ncand, 128), 128, 0, w, s.iters);
     for (int it = 0; it < s.iters; it++) {
-        cudaEvent_t t0 = c.clock.begin(c.stream);
+        if (it >= 2 && step_heard(c, c.stepTag) == 0)
+            break;
+        const unsigned tag = c.stepTag = std::max(c.stepTag + 1u, 1u);
+        cudaEvent_t    t0  = c.clock.begin(c.stream);
         if (tree)
-            launch_chained(c, k_corr<true>, gCorr, kT, 0, w, s, it);
+            launch_chained(c, k_corr<true>, gCorr, kT, 0, w, s, it, tag);
         else
-            launch_chained(c, k_corr<false>, gCorr, kT, 0, w, s, it);
+            launch_chained(c, k_corr<false>, gCorr, kT, 0, w, s, it, tag);
         c.clock.end(c.stream, t0, KernelClock::kCorr, 0.0); // bytes from the live count
         t0 = c.clock.begin(c.stream);
         launch_chained(c, k_fit, gc, kR, 0, w, s, it);
@@ -754,6 +787,8 @@ void icp_all(Ctx &c, const Model &m, const IcpScene &sc, const IcpParams &p, con
     w.win    = c.arena.get<unsigned long long>("icp.win", (size_t)ncand * w.maxDst);
     w.trace  = trace;
     w.live   = nullptr;
+    w.heard  = reinterpret_cast<unsigned long long *>(c.hostCounts + kHostStep);
+    *(volatile unsigned long long *)w.heard = 0; // (tags start at 1)
     if (c.clock.on) {
         w.live = c.arena.get<unsigned long long>("icp.live", 1);
         SM_CUDA(cudaMemsetAsync(w.live, 0, sizeof(unsigned long long), c.stream));

@@ -167,9 +167,10 @@ struct KernelClock {
 };
 
 // A context's page-locked scratch, in ints: counts first, from kHostResult on a match's results
-// (some 1100 candidates).
+// (some 1100 candidates), last the word in which a refinement step reports its candidates.
 constexpr int kHostResult = 64;
-constexpr int kHostInts   = kHostResult + 16384;
+constexpr int kHostStep   = kHostResult + 16384;
+constexpr int kHostInts   = kHostStep + 32;
 
 struct Ctx {
     int          device    = 0;
@@ -199,6 +200,7 @@ struct Ctx {
         int                 cap    = 0;
         unsigned            epoch  = 0;
     } scan;
+    unsigned    stepTag = 0; // the last refinement step launched (icp.cu)
     KernelClock clock; // opt-in per-launch timing (sm_context_kernel_clock)
     // launches of this context are chained to the previous kernel of its stream (see
     // launch_chained); off for the batch and serving workers, many of which run at once

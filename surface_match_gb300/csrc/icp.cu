@@ -629,7 +629,7 @@ __global__ void k_stage_end(Work w, int last, int failStatus) {
 // lane each, and adds to a candidate's count once per 32 (two launches of the large scene in
 // reference order 250 -> 158 us).
 template <bool TREE>
-__global__ void __launch_bounds__(kT, TREE ? 3 : 6)
+__global__ void __launch_bounds__(kT, TREE ? 3 : 5)
     k_inliers(Work w, const float4 *__restrict__ src, int n, int last, HGridView F, float r2,
               smk::KdView t, int treeM, const int *__restrict__ treePos,
               const float *__restrict__ exc) {
@@ -807,7 +807,7 @@ void icp_all(Ctx &c, const Model &m, const IcpScene &sc, const IcpParams &p, con
     const float sc2  = p.scoreDist * p.scoreDist;
     const bool tree = sc.tree != nullptr;
     auto inliers = [&](const float4 *src, int n, int last) {
-        const int g = wave(c, (long long)ncand * n, tree ? 3 : 6);
+        const int g = wave(c, (long long)ncand * n, tree ? 3 : 5);
         if (tree)
             launch_chained(c, k_inliers<true>, g, kT, 0, w, src, n, last, sc.full.view(), sc2,
                            sc.tree->view(nullptr, sc.pos, nullptr, sc.tpF), sc.tree->m,

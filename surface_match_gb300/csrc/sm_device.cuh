@@ -303,6 +303,11 @@ __device__ __forceinline__ bool warp_band(const HGridView &g, float qx, float qy
                                           const int c[3], int lo, int hi, B &&bound, V &&visit) {
     const int lane = threadIdx.x & 31;
     const int w = 2 * hi + 1, w2 = w * w, N = w2 * w;
+    // cell t = base + 32 j + lane of the cube, carried as (tx, ty, tz): 32 cells on are (sx, sy,
+    // sz) with carries (with two divisions a cell the large scene's correspondences took 201 us
+    // in ten launches, now 174)
+    const int sz = 32 / w2, sy = (32 - sz * w2) / w, sx = 32 - sz * w2 - sy * w;
+    int       tz = lane / w2, ty = (lane - tz * w2) / w, tx = lane - tz * w2 - ty * w;
     for (int base = 0; base < N; base += 256) {
         const float b2 = bound();
         // candidates of this lane (bit j: cell base + 32 j + lane), then their occupancy
@@ -314,7 +319,6 @@ __device__ __forceinline__ bool warp_band(const HGridView &g, float qx, float qy
             const int t = base + j * 32 + lane;
             key[j]      = 0u;
             if (t < N) {
-                const int tz = t / w2, ty = (t - tz * w2) / w, tx = t - tz * w2 - ty * w;
                 const int dx = tx - hi, dy = ty - hi, dz = tz - hi;
                 const int r  = max(abs(dx), max(abs(dy), abs(dz)));
                 const int x = c[0] + dx, y = c[1] + dy, z = c[2] + dz;
@@ -323,6 +327,17 @@ __device__ __forceinline__ bool warp_band(const HGridView &g, float qx, float qy
                     m |= 1u << j;
                     key[j] = (uint32_t)g.key_of(x, y, z);
                 }
+            }
+            tx += sx;
+            ty += sy;
+            tz += sz;
+            if (tx >= w) {
+                tx -= w;
+                ty++;
+            }
+            if (ty >= w) {
+                ty -= w;
+                tz++;
             }
         }
         if (g.dense) {
@@ -363,8 +378,8 @@ __device__ __forceinline__ bool warp_band(const HGridView &g, float qx, float qy
                     om &= om - 1u;
                 const int j  = __ffs(om) - 1;
                 const int t  = base + j * 32 + own;
-                const int tz = t / w2, ty = (t - tz * w2) / w, tx = t - tz * w2 - ty * w;
-                const unsigned long long k = g.key_of(c[0] + tx - hi, c[1] + ty - hi, c[2] + tz - hi);
+                const int oz = t / w2, oy = (t - oz * w2) / w, ox = t - oz * w2 - oy * w;
+                const unsigned long long k = g.key_of(c[0] + ox - hi, c[1] + oy - hi, c[2] + oz - hi);
                 if (g.dense) {
                     const int2 v = __ldg(&g.dense[k]);
                     b            = v.x;

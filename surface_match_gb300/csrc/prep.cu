@@ -835,22 +835,33 @@ __device__ __forceinline__ unsigned long long hkey(const float4 &p, const GridPa
            (unsigned)cx;
 }
 
-// Hashed grid, three passes over one table of uint4 {key low, key high, first point, points - 1},
-// all ones where empty (so that one fill clears it): points claim their cell's slot by its
-// 64-bit key and take a place in the cell, then every occupied cell takes its points' range from
-// a counter (a CTA's at once; the cells' order in the point arrays does not matter), then the
-// points go to their places. (A key table, a count table, their scan, a copy of the scan and a
-// pack into the slots moved twice the bytes: 81 us a grid of 0.92 M points against 57 us now.)
+// Grid, three passes over one table: points count themselves into their cell's entry, then every
+// occupied cell takes its points' range from a counter (a CTA's at once; the cells' order in the
+// point arrays does not matter), then the points go to their places. The table is a direct one
+// where the cell box is small (DIRECT: {first, count}), else hashed: slots of {key low, key high,
+// first point, points - 1}, all ones where empty (so that one fill clears it), claimed by the
+// cell's 64-bit key, half as many again as points. Bounded by the table's bytes and two atomics a
+// point. (A key table, a count table, their scan, a copy of the scan and a pack into the slots
+// moved twice the bytes; the slots rounded up to a power of two, with a CTA and its add to the
+// counter per 256 of them, took 25 us in the second pass of 0.92 M points' grid, now 10, and 71 us
+// in all, now 55. Both tables beside each other cost the small clouds, which read the direct one
+// only, a third more.)
+constexpr int kHgRun = 8; // entries a thread of the second pass
+template <bool DIRECT>
 __global__ void k_hg_insert(const float4 *__restrict__ pos, const int *__restrict__ ids, int m,
-                            GridParams gp, uint4 *__restrict__ slot, uint32_t mask,
-                            int2 *__restrict__ place) {
+                            GridParams gp, uint4 *__restrict__ slot, uint32_t slots,
+                            int2 *__restrict__ dense, int2 *__restrict__ place) {
     chain_enter(); // launched chained
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m)
         return;
     const unsigned long long key = hkey(pos[ids[i]], gp);
-    uint32_t                 h   = (uint32_t)smm::mix64(key) & mask;
-    for (uint32_t p = 0; p <= mask; p++) {
+    if (DIRECT) {
+        place[i] = make_int2((int)key, atomicAdd(&dense[key].y, 1));
+        return;
+    }
+    uint32_t h = hg_slot(key, slots);
+    for (uint32_t p = 0; p < slots; p++) {
         unsigned long long      *k    = reinterpret_cast<unsigned long long *>(&slot[h]);
         const unsigned long long prev = atomicCAS(k, ~0ull, key);
         if (prev == ~0ull || prev == key) {
@@ -858,41 +869,64 @@ __global__ void k_hg_insert(const float4 *__restrict__ pos, const int *__restric
             place[i] = make_int2((int)h, (int)(atomicAdd(&slot[h].w, 1u) + 1u));
             return;
         }
-        h = (h + 1) & mask;
+        h = h + 1 < slots ? h + 1 : 0;
     }
 }
 
-// Ranges of the occupied cells, their occupancy bits and direct-table entries.
+// Ranges of the occupied cells (of T entries), and the hashed ones' occupancy bits.
+template <bool DIRECT>
 __global__ void __launch_bounds__(256)
-    k_hg_ranges(uint4 *__restrict__ slot, uint32_t T, int *__restrict__ next,
-                uint32_t *__restrict__ occ, int2 *__restrict__ dense) {
+    k_hg_ranges(uint4 *__restrict__ slot, uint32_t T, int2 *__restrict__ dense,
+                int *__restrict__ next, uint32_t *__restrict__ occ) {
     chain_enter(); // launched chained
     __shared__ int sh[33];
     __shared__ int sBase;
-    const uint32_t t   = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint4    v   = t < T ? slot[t] : make_uint4(~0u, ~0u, ~0u, ~0u);
-    const int      cnt = (int)(v.w + 1u);
-    int            tot;
-    const int      ex = block_excl_scan(cnt, sh, &tot);
+    const uint32_t     t0 = blockIdx.x * (256u * kHgRun) + threadIdx.x;
+    int                cnt[kHgRun], sum = 0;
+    unsigned long long key[kHgRun];
+#pragma unroll
+    for (int r = 0; r < kHgRun; r++) {
+        const uint32_t t = t0 + 256u * r;
+        if (DIRECT) {
+            cnt[r] = t < T ? dense[t].y : 0;
+        } else {
+            const uint4 v = t < T ? slot[t] : make_uint4(~0u, ~0u, ~0u, ~0u);
+            cnt[r]        = (int)(v.w + 1u);
+            key[r]        = ((unsigned long long)v.y << 32) | v.x;
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < kHgRun; r++)
+        sum += cnt[r];
+    int       tot;
+    const int ex = block_excl_scan(sum, sh, &tot);
     if (tot == 0)
         return; // (uniform)
     if (threadIdx.x == 0)
         sBase = atomicAdd(next, tot);
     __syncthreads();
-    if (cnt == 0)
-        return;
-    const int                first = sBase + ex;
-    const unsigned long long k     = ((unsigned long long)v.y << 32) | v.x;
-    slot[t].z                      = (uint32_t)first;
-    if (occ)
-        atomicOr(&occ[k >> 5], 1u << (k & 31));
-    if (dense)
-        dense[k] = make_int2(first, cnt);
+    int first = sBase + ex;
+#pragma unroll
+    for (int r = 0; r < kHgRun; r++) {
+        if (cnt[r] == 0)
+            continue;
+        const uint32_t t = t0 + 256u * r;
+        if (DIRECT) {
+            dense[t].x = first;
+        } else {
+            slot[t].z = (uint32_t)first;
+            if (occ)
+                atomicOr(&occ[key[r] >> 5], 1u << (key[r] & 31));
+        }
+        first += cnt[r];
+    }
 }
 
+template <bool DIRECT>
 __global__ void k_hg_scatter(const float4 *__restrict__ pos, const int *__restrict__ ids,
-                             const uint4 *__restrict__ slot, const int2 *__restrict__ place, int m,
-                             float4 *__restrict__ pts, int wIsRank) {
+                             const uint4 *__restrict__ slot, const int2 *__restrict__ dense,
+                             const int2 *__restrict__ place, int m, float4 *__restrict__ pts,
+                             int wIsRank) {
     chain_enter(); // launched chained
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m)
@@ -900,7 +934,8 @@ __global__ void k_hg_scatter(const float4 *__restrict__ pos, const int *__restri
     const int    id = ids[i];
     const float4 p  = pos[id];
     const int2   at = place[i];
-    pts[slot[at.x].z + at.y] = make_float4(p.x, p.y, p.z, __int_as_float(wIsRank ? i : id));
+    const int    first = DIRECT ? dense[at.x].x : (int)slot[at.x].z;
+    pts[first + at.y]  = make_float4(p.x, p.y, p.z, __int_as_float(wIsRank ? i : id));
 }
 
 // Rank-ordered copies of a subset's positions and normals: out[r] = in[ids[r]].
@@ -1157,37 +1192,44 @@ void build_hgrid(Ctx &c, const float4 *pos, const int *ids, int m, const Box &bo
         H.org[a] = box.mn[a];
         H.dim[a] = smg::dim_of(box.ext(a), g);
     }
-    uint32_t T = 1024;
-    while (T < 2u * (uint32_t)std::max(m, 1))
-        T <<= 1;
-    H.mask = T - 1;
-    H.m    = m;
+    H.m         = m;
     int  *next  = c.arena.get<int>(tag + ".next", 1);
     int2 *place = c.arena.get<int2>(tag + ".place", std::max(m, 1));
     H.pts       = c.arena.get<float4>(tag + ".pts", std::max(m, 1));
-    H.slot      = c.arena.get<uint4>(tag + ".slot", T);
-    // occupancy bits over the cell box, when it has at most 2^28 cells (32 MB), and a direct
-    // {first, count} table too when it has at most 2^22 cells (32 MB); all cleared with the
-    // slots and the counter in one launch
-    const unsigned long long ncell = (unsigned long long)H.dim[0] * H.dim[1] * H.dim[2];
-    const size_t             words = (size_t)((ncell + 31) / 32);
-    H.occ   = ncell <= (1ull << 28) ? c.arena.get<uint32_t>(tag + ".occ", words) : nullptr;
-    H.dense = ncell <= (1ull << 22) ? c.arena.get<int2>(tag + ".dense", (size_t)ncell) : nullptr;
+    // a direct {first, count} table over a cell box of at most 2^22 cells (32 MB), else the hashed
+    // one, with occupancy bits over a box of at most 2^28 cells (32 MB); cleared with the counter
+    // in one launch
+    const unsigned long long ncell  = (unsigned long long)H.dim[0] * H.dim[1] * H.dim[2];
+    const size_t             words  = (size_t)((ncell + 31) / 32);
+    const bool               direct = ncell <= (1ull << 22);
+    H.slots = direct ? 0u : (uint32_t)m + (uint32_t)m / 2u + 64u;
+    H.dense = direct ? c.arena.get<int2>(tag + ".dense", (size_t)ncell) : nullptr;
+    H.slot  = direct ? nullptr : c.arena.get<uint4>(tag + ".slot", H.slots);
+    H.occ   = !direct && ncell <= (1ull << 28) ? c.arena.get<uint32_t>(tag + ".occ", words) : nullptr;
     FillSet clear;
-    clear.add(H.slot, (size_t)T * sizeof(uint4), 0xffffffffu);
     clear.add(next, sizeof(int), 0u);
-    if (H.occ)
-        clear.add(H.occ, words * 4, 0u);
     if (H.dense)
         clear.add(H.dense, (size_t)ncell * sizeof(int2), 0u);
+    if (H.slot)
+        clear.add(H.slot, (size_t)H.slots * sizeof(uint4), 0xffffffffu);
+    if (H.occ)
+        clear.add(H.occ, words * 4, 0u);
     fill(c, clear);
     if (m <= 0)
         return;
-    const GridParams gp = grid_params(box, g, H.dim);
-    launch_chained(c, k_hg_insert, nblocks(m, 256), 256, 0, pos, ids, m, gp, H.slot, H.mask, place);
-    launch_chained(c, k_hg_ranges, nblocks(T, 256), 256, 0, H.slot, T, next, H.occ, H.dense);
-    launch_chained(c, k_hg_scatter, nblocks(m, 256), 256, 0, pos, ids, H.slot, place, m, H.pts,
-                   wIsRank ? 1 : 0);
+    const GridParams gp  = grid_params(box, g, H.dim);
+    const uint32_t   T   = direct ? (uint32_t)ncell : H.slots;
+    const int        gm  = nblocks(m, 256), gt = nblocks(T, 256 * kHgRun);
+    const int        isR = wIsRank ? 1 : 0;
+    if (direct) {
+        launch_chained(c, k_hg_insert<true>, gm, 256, 0, pos, ids, m, gp, H.slot, H.slots, H.dense, place);
+        launch_chained(c, k_hg_ranges<true>, gt, 256, 0, H.slot, T, H.dense, next, H.occ);
+        launch_chained(c, k_hg_scatter<true>, gm, 256, 0, pos, ids, H.slot, H.dense, place, m, H.pts, isR);
+    } else {
+        launch_chained(c, k_hg_insert<false>, gm, 256, 0, pos, ids, m, gp, H.slot, H.slots, H.dense, place);
+        launch_chained(c, k_hg_ranges<false>, gt, 256, 0, H.slot, T, H.dense, next, H.occ);
+        launch_chained(c, k_hg_scatter<false>, gm, 256, 0, pos, ids, H.slot, H.dense, place, m, H.pts, isR);
+    }
 }
 
 void gather_subset(Ctx &c, const float4 *pos, const float4 *nrm, const int *ids, int m,

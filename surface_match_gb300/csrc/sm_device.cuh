@@ -21,13 +21,17 @@ constexpr int kKnnMaxShell = 24; // shells a k-nearest walk visits before it sca
 // and the table stays small enough to live in L2. The points of a cell are contiguous in
 // `pts` (position, point index in w), so a search reads them without an indirection, and
 // an occupancy bitmap over the cell box lets searches skip empty cells without a probe.
-// Small cell boxes also get a direct table of {first, count} per cell, read in one load.
+// Small cell boxes get a direct table of {first, count} per cell instead, read in one load.
+__device__ __forceinline__ uint32_t hg_slot(unsigned long long key, uint32_t slots) {
+    return __umulhi((uint32_t)smm::mix64(key), slots);
+}
+
 struct HGridView {
     float         org[3];
     float         g;
     int           dim[3];
-    const uint4  *slot;
-    uint32_t      mask;
+    const uint4  *slot; // the hashed table (not built beside a direct one)
+    uint32_t      slots;
     const float4 *pts;
     const uint32_t *occ;   // one bit per cell of the dim box (nullptr: not built)
     const int2     *dense; // {first, count} per cell of the dim box (nullptr: not built)
@@ -38,8 +42,8 @@ struct HGridView {
     }
     // the table entry of an occupied cell (s = e = 0 when the cell holds no point)
     __device__ __forceinline__ void lookup(unsigned long long key, int &s, int &e) const {
-        uint32_t h = (uint32_t)smm::mix64(key) & mask;
-        for (uint32_t p = 0; p <= mask; p++) {
+        uint32_t h = hg_slot(key, slots);
+        for (uint32_t p = 0; p < slots; p++) {
             const uint4 v = slot[h];
             if (v.w == 0xffffffffu)
                 break;
@@ -48,7 +52,7 @@ struct HGridView {
                 e = (int)(v.z + v.w + 1u);
                 return;
             }
-            h = (h + 1) & mask;
+            h = h + 1 < slots ? h + 1 : 0;
         }
         s = e = 0;
     }

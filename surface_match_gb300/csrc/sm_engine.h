@@ -114,10 +114,10 @@ struct HGrid {
     float     org[3] = {0, 0, 0};
     float     g      = 1;
     int       dim[3] = {1, 1, 1};
-    uint4    *slot   = nullptr;
-    uint32_t  mask   = 0;
+    uint4    *slot   = nullptr; // hashed table (nullptr beside a direct one)
+    uint32_t  slots  = 0;
     float4   *pts    = nullptr; // positions in cell order, point index in w (bit pattern)
-    uint32_t *occ    = nullptr; // occupancy bit per cell (nullptr when the cell box is too large)
+    uint32_t *occ    = nullptr; // occupancy bit per cell (nullptr: too large a cell box, or direct)
     int2     *dense  = nullptr; // {first, count} per cell (nullptr unless the cell box is small)
     int       m      = 0;
     smd::HGridView view() const {
@@ -128,7 +128,7 @@ struct HGrid {
         }
         v.g    = g;
         v.slot = slot;
-        v.mask = mask;
+        v.slots = slots;
         v.pts  = pts;
         v.occ   = occ;
         v.dense = dense;

@@ -3,10 +3,10 @@
 //
 // Both clusterings are greedy first fits: in order, an entry joins the first earlier head (leader)
 // it is compatible with, or becomes one. Taken one after the other they are a chain as long as the
-// list (a warp's walk over 8083 poses took 9 ms; all the clustering takes 0.33 ms now), so they are resolved a chunk of kClBs entries at a
-// time from the compatibility bits of the chunk's pairs, in parallel rounds that reproduce the
-// sequential decisions (greedy_chunk), after the entries that fit a head of an earlier chunk
-// were taken out.
+// list (a warp's walk over 8083 poses took 9 ms; all the clustering takes 0.33 ms now), so they
+// are resolved a chunk of kClBs entries at a time from the compatibility bits of the chunk's pairs,
+// in parallel rounds that reproduce the sequential decisions (greedy_chunk), after the entries that
+// fit a head of an earlier chunk were taken out.
 //
 // k_cluster_rank (all CTAs): stable rank-by-counting sort on (votes desc, list position).
 // k_cluster_bits (all CTAs): the compatibility of every pose with the earlier ones of its chunk.

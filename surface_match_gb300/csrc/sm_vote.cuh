@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <type_traits>
 
 #include "sm_device.cuh"
 #include "sm_icp.h"
@@ -91,17 +92,104 @@ __device__ __forceinline__ uint32_t probe(const uint4 *__restrict__ tab, uint32_
     return 0;
 }
 
+// One vote in cell c of the accumulator at shared address acc. One increment per vote: a warp's
+// votes rarely share a cell (a bucket's entries are different pairs), so aggregating them first
+// measured 2.8x slower on the large scene.
+template <bool NARROW> __device__ __forceinline__ void cast_vote(uint32_t acc, uint32_t c) {
+    const uint32_t at = NARROW ? acc + ((c * 2u) & ~3u) : acc + c * 4u;
+    const uint32_t by = NARROW ? (c & 1u) * 65535u + 1u : 1u;
+    asm volatile("red.relaxed.cta.shared.add.u32 [%0], %1;" : : "r"(at), "r"(by) : "memory");
+}
+
 // Votes of the hits hOff/hCnt/hAs/hAsT[0..nHits) into the shared accumulator of reference
-// points [r0, r1). A hit's bucket is cut into items of kItem consecutive entries (cPre:
-// prefix of items per hit, T in all) and each warp takes a contiguous range of items.
-// Within an item the hit's values are warp-uniform registers, lane l owns entries l, l+32,
-// ... and issues all its kVoteU loads before the first use, so one L2 latency covers 256
-// votes and the loads coalesce. `narrow`: two 16-bit counters per 32-bit word.
+// points [r0, r1) (ALL: of every one). A hit's bucket is cut into items of kItem consecutive
+// entries (cPre: prefix of items per hit, T in all) and each warp takes a contiguous range of
+// items. Within an item the hit's values are warp-uniform registers, lane l owns entries l, l+32,
+// ..., so the loads coalesce, and issues up to kVoteU of them before the first use. NARROW: two
+// 16-bit counters per 32-bit word. Bound by a vote's instructions and the bank conflicts of its
+// increments (5.4 wavefronts a round of 32 random cells): a round inside the bucket's 8-lane
+// blocks has no tests of its own, whole batches of rounds no predicated loads, and the bin is
+// smm::vote_bin's of such an entry (whose floor the conversion to an unsigned number is). With
+// tests and predicates on every entry (39 instructions a round) 2.9e9 votes of 3,349 keypoints
+// took 4.36 ms, now 2.65; the large scene's 35e6 0.125 ms, now 0.098. Loads of the next item
+// taken over vote by vote (a fuller pipeline) measured slower, 3.7 against 3.5 ms at that point.
+template <bool ALL, bool NARROW>
+__device__ __forceinline__ void cast_items(const VoteArgs &a, uint32_t acc, const int *hOff,
+                                           const int *hCnt, const float *hAs, const float *hAsT,
+                                           const int *cPre, int h, int i0, int i1, int r0, int r1) {
+    const int      lane = threadIdx.x & 31;
+    const uint32_t A = (uint32_t)a.A, last = A - 1u;
+    const float    smax = a.smax;
+    for (int item = i0; item < i1; item++) {
+        while (cPre[h + 1] <= item)
+            h++;
+        const int    B   = hCnt[h], e0 = (item - cPre[h]) * kItem;
+        const int    n   = min(B - e0, kItem);                // entries of the item
+        const int    vec = B - B % smm::kLanes - e0;          // and those inside the blocks
+        const float  as  = hAs[h], vs = as - smm::kPiF;
+        const uint2 *src = a.entries + hOff[h] + e0 + lane;
+        auto         fast = [&](const uint2 &ent) {
+            float v = __uint_as_float(ent.y) - vs;
+            if (v > smm::k2PiF)
+                v = v - smm::k2PiF;
+            if (v < 0.0f)
+                v = v + smm::k2PiF;
+            // (at most A - 1: the bound keeps the index in range whatever the entry)
+            const uint32_t bin = min(__float2uint_rz(smax * v), last);
+            if (ALL || ((int)ent.x >= r0 && (int)ent.x < r1))
+                cast_vote<NARROW>(acc, (ALL ? ent.x : ent.x - (uint32_t)r0) * A + bin);
+        };
+        auto batch = [&](auto rounds, int u0) {
+            uint2 ent[rounds.value];
+#pragma unroll
+            for (int u = 0; u < rounds.value; u++)
+                ent[u] = src[(u0 + u) * 32];
+#pragma unroll
+            for (int u = 0; u < rounds.value; u++)
+                fast(ent[u]);
+        };
+        const int full = min(n, vec) >> 5; // rounds inside the blocks
+        if (full == kVoteU) {
+            batch(std::integral_constant<int, kVoteU>(), 0);
+            continue;
+        }
+        // the last entries' load goes out first
+        uint2 end = make_uint2(0u, 0u);
+        if (full * 32 + lane < n)
+            end = src[full * 32];
+        if (full & 4)
+            batch(std::integral_constant<int, 4>(), 0);
+        if (full & 2)
+            batch(std::integral_constant<int, 2>(), full & 4);
+        if (full & 1)
+            batch(std::integral_constant<int, 1>(), full & 6);
+        for (int t = full * 32 + lane; t < n; t += 32) {
+            const int ref = (int)end.x;
+            if (ALL || (ref >= r0 && ref < r1)) {
+                const uint32_t bin =
+                    smm::vote_bin(t < vec, __uint_as_float(end.y), as, hAsT[h], smax);
+                cast_vote<NARROW>(acc, (uint32_t)(ALL ? ref : ref - r0) * A + min(bin, last));
+            }
+            if (t + 32 < n) // (a round cut by the end of the blocks, and what is beyond it)
+                end = src[t + 32 - lane];
+        }
+    }
+}
+
+// The rarer forms, out of line: inlined they take the common one's registers.
+template <bool NARROW>
+static __device__ __noinline__ void cast_items_call(const VoteArgs &a, uint32_t acc, const int *hOff,
+                                                    const int *hCnt, const float *hAs,
+                                                    const float *hAsT, const int *cPre, int h, int i0,
+                                                    int i1, int r0, int r1) {
+    cast_items<false, NARROW>(a, acc, hOff, hCnt, hAs, hAsT, cPre, h, i0, i1, r0, r1);
+}
+
 __device__ __forceinline__ void cast_votes(const VoteArgs &a, uint32_t *acc, const int *hOff,
                                            const int *hCnt, const float *hAs, const float *hAsT,
                                            const int *cPre, int nHits, int T, int r0, int r1,
                                            bool narrow) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int i0 = (int)((long long)T * w / nw), i1 = (int)((long long)T * (w + 1) / nw);
     if (i0 >= i1)
         return;
@@ -113,48 +201,14 @@ __device__ __forceinline__ void cast_votes(const VoteArgs &a, uint32_t *acc, con
         else
             hi = mid - 1;
     }
-    int        h       = lo;
-    const bool allRefs = r0 == 0 && r1 == a.ns; // one pass holds every reference point
-    for (int item = i0; item < i1; item++) {
-        while (cPre[h + 1] <= item)
-            h++;
-        const int    B    = hCnt[h];
-        const float  as   = hAs[h];
-        const float  asT  = hAsT[h];
-        const int    e0   = (item - cPre[h]) * kItem;
-        const int    eEnd = min(B, e0 + kItem);
-        const int    vecB = B - B % smm::kLanes;
-        const uint2 *src  = a.entries + hOff[h];
-        uint2        ent[kVoteU];
-#pragma unroll
-        for (int u = 0; u < kVoteU; u++) {
-            const int e = e0 + u * 32 + lane;
-            ent[u]      = e < eEnd ? src[e] : make_uint2(0xffffffffu, 0u);
-        }
-#pragma unroll
-        for (int u = 0; u < kVoteU; u++) {
-            const int  e   = e0 + u * 32 + lane;
-            const int  ref = (int)ent[u].x;
-            const bool ok  = !(e >= eEnd || (!allRefs && (ref < r0 || ref >= r1)));
-            if (!ok)
-                continue;
-            const float am = __uint_as_float(ent[u].y);
-            uint32_t    bin;
-            if (e0 + u * 32 + 32 <= vecB) // warp-uniform: the round lies in the 8-lane blocks
-                bin = smm::vote_bin(true, am, as, asT, a.smax);
-            else
-                bin = smm::vote_bin(e < vecB, am, as, asT, a.smax);
-            bin         = min(bin, (uint32_t)(a.A - 1)); // unreachable; keeps the index in range
-            const int c = (ref - r0) * a.A + (int)bin;
-            // one increment per vote: a warp's votes rarely share a cell (a bucket's
-            // entries are different pairs), so aggregating them first measured 2.8x
-            // slower on the large scene
-            if (narrow)
-                atomicAdd(&acc[c >> 1], 1u << ((c & 1) * 16));
-            else
-                atomicAdd(&acc[c], 1u);
-        }
-    }
+    const uint32_t at  = (uint32_t)__cvta_generic_to_shared(acc);
+    const bool     all = r0 == 0 && r1 == a.ns; // one pass holds every reference point
+    if (all && narrow)
+        cast_items<true, true>(a, at, hOff, hCnt, hAs, hAsT, cPre, lo, i0, i1, r0, r1);
+    else if (narrow)
+        cast_items_call<true>(a, at, hOff, hCnt, hAs, hAsT, cPre, lo, i0, i1, r0, r1);
+    else
+        cast_items_call<false>(a, at, hOff, hCnt, hAs, hAsT, cPre, lo, i0, i1, r0, r1);
 }
 
 __device__ __forceinline__ int acc_get(const uint32_t *acc, int e, bool narrow) {

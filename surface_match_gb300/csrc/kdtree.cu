@@ -716,7 +716,7 @@ __device__ __forceinline__ bool reaches(const SampleArgs &a, const float4 &q, co
     if (d < sure)
         return true;
     uint64_t key;
-    return smk::kd_reaches(a.t, qq, ip, a.r2, &key);
+    return smk::kd_sure(a.t, qq, ip, a.r2) || smk::kd_reaches(a.t, qq, ip, a.r2, &key);
 }
 
 // The cell of each tree position (noCell where reduce() excluded it).

@@ -386,7 +386,7 @@ __device__ __forceinline__ int warp_kd_knearest(const KdView &t, int m, const sm
         // every one of them reached even with the final worst distance, and no two at one
         // distance (nor a further point at the last one's): the order is that of the distances
         uint64_t    key;
-        const bool  in    = lane >= n || kd_reaches(t, q, pos, B, &key);
+        const bool  in    = lane >= n || kd_sure(t, q, pos, B) || kd_reaches(t, q, pos, B, &key);
         const float dn    = __shfl_down_sync(0xffffffffu, d, 1);
         const int   idn   = __shfl_down_sync(0xffffffffu, *id, 1);
         const bool  equal = lane < n && lane < 31 && idn != -1 && dn == d;

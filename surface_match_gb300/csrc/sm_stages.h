@@ -304,6 +304,7 @@ struct KdTree {
         v.pos      = pos;
         v.nonEmpty = nonEmpty;
         v.tpos     = tpos;
+        v.leafOf   = leafOf;
         return v;
     }
 };

@@ -163,7 +163,9 @@ __global__ void __launch_bounds__(kKpWarps * 32) k_kp_radius(VoteArgs a, PipeBuf
             if (lane < n) {
                 const int e = queue[w][nq - n + lane], k = e >> 16, j = e & 0xffff;
                 uint64_t  key;
-                if (smk::kd_reaches(b.tree.view, kx[w][k], b.tree.posOf[t0 + j], a.sqDiam, &key))
+                const int at = b.tree.posOf[t0 + j];
+                if (smk::kd_sure(b.tree.view, kx[w][k], at, a.sqDiam) ||
+                    smk::kd_reaches(b.tree.view, kx[w][k], at, a.sqDiam, &key))
                     atomicOr(&words[w][k][j >> 5], 1u << (j & 31));
             }
             nq -= n;

@@ -183,11 +183,12 @@ __device__ __forceinline__ int4 leaf_node(int l, int r) { return make_int4(l, r,
 // Control words: nodes, small ranges, error, then per level its open ranges and whether a
 // point lies on a cut (else the second pass has nothing to do). The levels' launches are chained
 // and sized by bounds; the host looks at the counts every kKdLevels levels only. (One round trip,
-// two counter copies, a flag kernel per pass and ordinary launches a level: 3.3 ms for 0.92 M
-// points, now 1.9 ms.)
+// two counter copies, a flag kernel per pass and ordinary launches a level a call on 0.92 M
+// points took 9.35 ms, with these 8.82; the build is some 2.2 ms of launches.)
 enum { kKdNodes = 0, kKdSmallN = 1, kKdErr = 2, kKdOpen = 8, kKdOnCut = 8 + 2 * smk::kMaxDepth };
 constexpr int kKdCtl    = kKdOnCut + 2 * smk::kMaxDepth;
 constexpr int kKdLevels = 4;
+static_assert((63 - kKdOpen) % kKdLevels != 0, "the counts' word 63 is sync_checked's");
 
 __global__ void k_kd_root(Seg *seg, Seg *small, int m, Box box, int4 *nd, int *parent, int *ctl) {
     Seg s{};

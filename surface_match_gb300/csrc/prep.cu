@@ -804,8 +804,9 @@ __global__ void k_mark_todo(const int *__restrict__ ids, int m, const float4 *__
 
 // One warp per query (exact k nearest neighbours, sm_device.cuh warp_knn_sorted) of part `part`
 // of the list; lane j writes the j-th neighbour, and with `grow` lists it when it still needs a
-// normal.
-__global__ void __launch_bounds__(256, 6)
+// normal. Five CTAs an SM: at six the ring search spills, at four the large scene's queries took
+// 85 + 82 us, at five 77 + 74.
+__global__ void __launch_bounds__(256, 5)
     k_knn(NormalList L, int part, HGridView G, const float4 *__restrict__ pos, int k, bool grow,
           const float4 *__restrict__ nrm) {
     chain_enter(); // launched chained

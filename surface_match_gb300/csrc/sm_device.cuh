@@ -244,7 +244,8 @@ __device__ __forceinline__ bool warp_block27(const HGridView &g, float qx, float
 // screened 256 cells at a time - each lane computes 8 cells' bounds and issues their 8
 // occupancy-bit loads together - and only the occupied survivors, compacted over the warp,
 // are looked up in the table: a deep search costs a few rounds of independent loads instead
-// of one dependent probe round per 32 cells. Returns visit's "done".
+// of one dependent probe round per 32 cells. Callers stop at kKnnMaxShell rings, so the cube's
+// cells are counted in 32 bits. Returns visit's "done".
 template <class B, class V>
 __device__ __forceinline__ bool warp_band(const HGridView &g, float qx, float qy, float qz,
                                           const int c[3], int lo, int hi, B &&bound, V &&visit) {
@@ -368,7 +369,6 @@ __device__ __forceinline__ bool knn_enters(unsigned long long key, unsigned long
 // it saw k points, else the k-th of a strided sample of the points; a merge runs only for a
 // round with a point below the current k-th. It runs for few queries and is kept lean (two
 // loads in flight per lane) so that the search's register count stays as it is.
-template <bool TIES>
 static __device__ __noinline__ void knn_scan_all(const HGridView &g, float qx, float qy, float qz, int k,
                                           unsigned long long &best, int &seen) {
     const int lane  = threadIdx.x & 31;
@@ -406,7 +406,7 @@ static __device__ __noinline__ void knn_scan_all(const HGridView &g, float qx, f
             if ((unsigned)(key >> 32) > bound)
                 key = ~0ull;
             seen += __popc(__ballot_sync(0xffffffffu, r < g.m));
-            if (__any_sync(0xffffffffu, knn_enters<TIES>(key, __shfl_sync(0xffffffffu, best, k - 1))))
+            if (__any_sync(0xffffffffu, key < __shfl_sync(0xffffffffu, best, k - 1)))
                 best = warp_merge_low(best, warp_bitonic_sort(key));
         }
     }
@@ -423,7 +423,9 @@ static __device__ __noinline__ void knn_scan_all(const HGridView &g, float qx, f
 // the k-th distance (warp_band). (Shell by shell, every cell looked up, 18,000 queries of a
 // scene with uniform clutter took 152 us, now 108.) Returns the number found (<= k); lane j < that count gets the j-th neighbour's index in *id and
 // squared distance in *d. With TIES points at the k-th distance are never skipped: for k < 32
-// lane k holds one more of them (index >= 0, the same distance) if there is one.
+// lane k holds one more of them (index >= 0, the same distance) if there is one; and a search that
+// the rings up to kKnnMaxShell do not decide ends with -1 there: its caller has the tree, whose
+// search costs a far point no more than any other, instead of every point of the grid.
 template <bool TIES = false>
 __device__ __forceinline__ int warp_knn_sorted(const HGridView &g, float qx, float qy, float qz,
                                                int k, int *id, float *d) {
@@ -495,7 +497,9 @@ __device__ __forceinline__ int warp_knn_sorted(const HGridView &g, float qx, flo
         if (d < rb * rb || done >= ms)
             break;
         if (done >= kKnnMaxShell) {
-            knn_scan_all<TIES>(g, qx, qy, qz, k, best, seen);
+            if (TIES)
+                return -1;
+            knn_scan_all(g, qx, qy, qz, k, best, seen);
             break;
         }
         // (while fewer than k are found the next ring, from the third on three at once: a band's
@@ -518,9 +522,12 @@ __device__ __forceinline__ int warp_knn_sorted(const HGridView &g, float qx, flo
 // until the nearest is below the ring bound or the ring bound passes limit2. A point
 // farther than limit2 may be returned (callers test the distance); -1 when none was found.
 // A caller that knows a point of the grid at squared distance u from q may pass limit2 <= u:
-// the nearest is then found exactly with fewer cells visited. All lanes return the result.
+// the nearest is then found exactly with fewer cells visited. All lanes return the result. Beyond
+// kKnnMaxShell rings (a query thrown far off by a bad pose: the rings' cubes grow with the fourth
+// power of the distance) every point is looked at instead.
 __device__ __forceinline__ int warp_nn_walk(const HGridView &g, float qx, float qy, float qz,
                                             float limit2, float &outd) {
+    const int          lane  = threadIdx.x & 31;
     unsigned long long best  = ~0ull;
     auto               visit = [&](const float4 &p, bool valid) {
         if (valid) {
@@ -545,6 +552,11 @@ __device__ __forceinline__ int warp_nn_walk(const HGridView &g, float qx, float 
         const float rb = smg::ring_bound(done, g.g);
         if (d < rb * rb || rb * rb > limit2 || done >= ms)
             break;
+        if (done >= kKnnMaxShell) {
+            for (int r = lane; r < g.m; r += 32)
+                visit(g.pts[r], true);
+            break;
+        }
         const int hi = band_end(done, ms, fminf(d, limit2), g.g);
         warp_band(g, qx, qy, qz, c, done + 1, hi, [&]() { return fminf(bd(), limit2); }, visit);
         done = hi;

@@ -158,9 +158,15 @@ __device__ __forceinline__ unsigned warp_kd_restricted(const int4 *__restrict__ 
     return met;
 }
 
+// Rings that a walk here goes out to before it leaves the query to the tree's own search. The
+// rings' cubes grow with the fourth power of the distance, so a lone point some hundred cells from
+// its neighbours would keep its warp for seconds; the tree's search does not depend on it.
+constexpr int kMaxShell = smd::kKnnMaxShell;
+constexpr int kFar      = -2; // a nearest search that gave up there
+
 // All points of grid g within squared distance B of q (<=), ascending by (distance, index) over
-// the lanes: lane j gets the j-th key. Returns their number; above 32 only the 32 nearest are
-// held.
+// the lanes: lane j gets the j-th key. Returns their number; above 32, or where B reaches beyond
+// kMaxShell rings, 33 and no points.
 __device__ __forceinline__ int warp_collect(const smd::HGridView &g, float qx, float qy, float qz,
                                             float B, unsigned long long *key) {
     unsigned long long best = ~0ull;
@@ -177,26 +183,27 @@ __device__ __forceinline__ int warp_collect(const smd::HGridView &g, float qx, f
             n += c;
             best = smd::warp_merge_low(best, smd::warp_bitonic_sort(kk));
         }
-        return false;
+        return n > 32;
     };
     int c[3];
     smd::grid_cc(g, qx, qy, qz, c);
     const int ms = max(smd::grid_max_shell(g, c), 1);
-    smd::warp_block27(g, qx, qy, qz, c, B, visit);
-    for (int done = 1;;) {
+    bool      over = smd::warp_block27(g, qx, qy, qz, c, B, visit);
+    for (int done = 1; !over;) {
         const float rb = smg::ring_bound(done, g.g);
         if (rb * rb > B || done >= ms)
             break;
         const int hi = smd::band_end(done, ms, B, g.g);
-        smd::warp_band(g, qx, qy, qz, c, done + 1, hi, [&]() { return B; }, visit);
+        over = done >= kMaxShell ||
+               smd::warp_band(g, qx, qy, qz, c, done + 1, hi, [&]() { return B; }, visit);
         done = hi;
     }
     *key = best;
-    return n;
+    return over ? 33 : n;
 }
 
 // Nearest point of g by squared distance as smd::warp_nn_walk (bounded by limit2), and whether
-// another point lies at the same distance.
+// another point lies at the same distance. kFar: not found within kMaxShell rings.
 __device__ __forceinline__ int warp_nn_tie(const smd::HGridView &g, float qx, float qy, float qz,
                                            float limit2, float &outd, bool &tie) {
     unsigned long long gb = ~0ull, mine = ~0ull; // warp's best so far; lane's since then
@@ -240,6 +247,8 @@ __device__ __forceinline__ int warp_nn_tie(const smd::HGridView &g, float qx, fl
         const float rb = smg::ring_bound(done, g.g);
         if (d < rb * rb || rb * rb > limit2 || done >= ms)
             break;
+        if (done >= kMaxShell)
+            return kFar;
         const int hi = smd::band_end(done, ms, fminf(d, limit2), g.g);
         smd::warp_band(g, qx, qy, qz, c, done + 1, hi, [&]() { return fminf(fold(), limit2); }, visit);
         done = hi;
@@ -251,6 +260,12 @@ __device__ __forceinline__ int warp_nn_tie(const smd::HGridView &g, float qx, fl
     }
     outd = __uint_as_float((unsigned)(gb >> 32));
     return (int)(unsigned)(gb & 0xffffffffu);
+}
+
+// Whether the nearest point's squared distance d is one that the reference's search returns and
+// its caller asks for (the search starts from the largest float: d may have overflowed).
+__device__ __forceinline__ bool in_limit(float d, float limit2) {
+    return d <= limit2 && d < 3.402823466e38f;
 }
 
 // What the reference's one-nearest search of tree `t` (m positions, reduced to the points of
@@ -269,13 +284,13 @@ __device__ __forceinline__ int warp_kd_nearest(const KdView &t, int m, const smd
         return -1; // no distance from it is below the search's start
     bool tie;
     const int   j = warp_nn_tie(g, qx, qy, qz, limit2, *d, tie);
-    if (j < 0 || *d > limit2)
+    if (j != kFar && (j < 0 || !in_limit(*d, limit2)))
         return -1; // the reference's result is no nearer
     float B     = *d;
     float dl    = *d;
     int   name  = j;
     int   count = 1;
-    for (int it = 0; it < kMaxRaise; it++) {
+    for (int it = 0; j != kFar && it < kMaxRaise; it++) {
         if (it > 0 || tie) {
             unsigned long long key;
             count = warp_collect(g, qx, qy, qz, B, &key);
@@ -349,8 +364,11 @@ __device__ __forceinline__ int lanes_kd_nearest(const KdView &t, int m, const sm
         }
     }
     bool open = false;
-    if (j >= 0 && *d > limit2) {
-        j = -1; // the reference's result is no nearer
+    if (j == kFar) {
+        open = true;
+    } else if (j >= 0 && !in_limit(*d, limit2)) {
+        j  = -1; // the reference's result is no nearer
+        *d = 3.402823466e38f;
     } else if (j >= 0) {
         uint64_t    key;
         const float q[3] = {qx, qy, qz};
@@ -379,8 +397,12 @@ __device__ __forceinline__ int warp_kd_knearest(const KdView &t, int m, const sm
     const float q[3] = {qx, qy, qz};
     float       d;
     const int   n = smd::warp_knn_sorted<true>(g, qx, qy, qz, k, id, &d);
+    if (n < 0)
+        return -1; // far from its neighbours
     // fewer than k points in all: the search's worst distance stays at the start
     float B = n < k ? 3.402823466e38f : __shfl_sync(0xffffffffu, d, k - 1);
+    if (__any_sync(0xffffffffu, lane < n && !(d < 3.402823466e38f)))
+        return -1; // (distances that overflow: a search from the largest float leaves them out)
     int   pos = lane < n ? treePos[*id] : -1;
     {
         // every one of them reached even with the final worst distance, and no two at one

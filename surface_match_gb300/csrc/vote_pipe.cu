@@ -58,6 +58,7 @@ struct PipeBufs {
     VoteTree            tree;    // reference order
     int                *tail;    // reference order: K x 8, the tail rows' candidates (else -1)
     int                *rowOff;  // K + 1
+    unsigned long long *rowSum;  // reference order: all rows (their 32-bit prefixes may wrap)
     int4               *hits;    // per row segment: {bucket offset, count, alpha bits, 0}
     int                *hitCnt;  // K
     unsigned long long *votes;   // K
@@ -130,6 +131,8 @@ __global__ void __launch_bounds__(kKpWarps * 32) k_kp_radius(VoteArgs a, PipeBuf
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int c0   = (blockIdx.x * kKpWarps + w) * kKpPer;
     const int i0 = blockIdx.y * per, i1 = min(a.ncand, i0 + per);
+    if (TREE && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
+        *b.rowSum = 0ull; // (k_kp_info adds to it)
     int       self[kKpPer], S[kKpPer], R[kKpPer]; // self: the keypoint's id, TREE: its candidate
     float     x[kKpPer], y[kKpPer], z[kKpPer];
 #pragma unroll
@@ -342,6 +345,8 @@ template <bool TREE> __global__ void k_kp_info(VoteArgs a, PipeBufs b, int *__re
     b.info[c]         = info;
     b.rt[c]           = smm::transform_rt(p1.x, p1.y, p1.z, n1.x, n1.y, n1.z);
     cnt[c]            = info.y;
+    if (TREE)
+        atomicAdd(b.rowSum, (unsigned long long)info.y);
     b.hitCnt[c]       = 0;
     b.votes[c]        = 0ull;
     b.bound[c]        = 0ull;
@@ -744,9 +749,12 @@ void vote(Ctx &c, const Model &m, const float4 *pos, const float4 *nrm, const in
     if (K <= 0)
         return;
     // rows (keypoint, neighbour) are counted and offset in 32-bit ints: at most K x ncand in
-    // radius mode (every candidate a neighbour of every keypoint)
-    if (!nbrOff && !tree && (long long)K * (long long)ncand > 0x7fffffffll)
-        throw Error(SM_ERR_CAPACITY, "too many keypoint x sampled point pairs for one call");
+    // radius mode (every candidate a neighbour of every keypoint). Grid order refuses what could
+    // be more, reference order what is.
+    const char *const tooMany = "too many keypoint x sampled point pairs for one call";
+    const bool        many    = !nbrOff && (long long)K * (long long)ncand > 0x7fffffffll;
+    if (many && !tree)
+        throw Error(SM_ERR_CAPACITY, tooMany);
     VoteArgs a{};
     fill_vote_model(m, minScore, a);
     a.pos    = pos;
@@ -812,6 +820,7 @@ void vote(Ctx &c, const Model &m, const float4 *pos, const float4 *nrm, const in
         if (tree) {
             b.tree = *tree;
             b.tail = c.arena.get<int>("v.tail", (size_t)K * 8);
+            b.rowSum = c.arena.get<unsigned long long>("v.rowsum", 1);
             launch_chained(c, k_kp_radius<true>, dim3(gx, b.splits), kKpWarps * 32, 0, a, b, per);
             launch_chained(c, k_kp_info<true>, gi, 256, 0, a, b, cnt);
         } else {
@@ -819,7 +828,13 @@ void vote(Ctx &c, const Model &m, const float4 *pos, const float4 *nrm, const in
             launch_chained(c, k_kp_info<false>, gi, 256, 0, a, b, cnt);
         }
     }
+    unsigned long long *rowSum = reinterpret_cast<unsigned long long *>(c.hostCounts + 2);
+    *rowSum                    = 0ull;
+    if (many) // (read with the scan's total)
+        SM_CUDA(cudaMemcpyAsync(rowSum, b.rowSum, sizeof(*rowSum), cudaMemcpyDeviceToHost, c.stream));
     const int rtot = scan_excl(c, cnt, b.rowOff, (long long)K + 1, "v.scan", true);
+    if (*rowSum > 0x7fffffffull)
+        throw Error(SM_ERR_CAPACITY, tooMany);
     b.hits = c.arena.get<int4>("v.hits", std::max(rtot, 1));
     SM_CUDA(cudaEventRecord(c.ev[10], c.stream));
     if (rtot > 0) {

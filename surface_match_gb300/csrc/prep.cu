@@ -1184,7 +1184,8 @@ void build_hgrid(Ctx &c, const float4 *pos, const int *ids, int m, const Box &bo
     // (any cell side gives the same results: without a wanted one, some 1000 cells an axis)
     if (!(g > 0.0f))
         g = std::max(std::max(box.ext(0), box.ext(1)), std::max(box.ext(2), 1e-30f)) / 1024.0f;
-    // cells per axis stay below 2^20 so that cell keys fit 60 bits (coarser cells if needed)
+    // cells per axis stay below 2^20 so that cell keys fit 60 bits (coarser cells if needed; the
+    // loop ends: dim_of is 1 where the side overflows)
     while (smg::dim_of(box.ext(0), g) >= (1 << 20) || smg::dim_of(box.ext(1), g) >= (1 << 20) ||
            smg::dim_of(box.ext(2), g) >= (1 << 20))
         g = g * 2.0f;

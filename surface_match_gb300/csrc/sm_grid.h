@@ -17,11 +17,17 @@ namespace smg {
 
 constexpr long long kMaxCells = 1ll << 22; // dense grid size cap (4M cells, 16 MB of u32)
 
-SM_HD int dim_of(float extent, float g) { return (int)smm::ffloor(smm::fdiv(extent, g)) + 1; }
+// Cells along an axis, at most 2^30 (a stray point, or one with a huge number in the place of a
+// missing value, can lie beyond what an int counts); one where both overflow.
+SM_HD int dim_of(float extent, float g) {
+    const float q = smm::ffloor(smm::fdiv(extent, g));
+    return q < 1073741823.0f ? (int)q + 1 : q == q ? 1 << 30 : 1;
+}
 
+// Cells of the box, at most 2^62.
 SM_HD long long cells_of(const float ext[3], float g) {
-    return (long long)dim_of(ext[0], g) * (long long)dim_of(ext[1], g) *
-           (long long)dim_of(ext[2], g);
+    const long long a = (long long)dim_of(ext[0], g) * dim_of(ext[1], g), c = dim_of(ext[2], g);
+    return a <= (1ll << 62) / c ? a * c : 1ll << 62;
 }
 
 // Cell side of the grid-order greedy sampler at `step`: slightly larger than the step so

@@ -655,21 +655,40 @@ constexpr int       kSpSleep    = 100;
 constexpr int       kSpCtl      = 32;
 constexpr int       kSpUnlinked = -2;      // a filed cell's link until it is stored
 constexpr long long kSpCells    = 1ll << 25; // most cells of the dense table (128 MB)
+constexpr float     kSpCoarse   = 1.5f;      // above so many steps a side its cells are hashed ones
+
+// Hashed cells, where a dense table of cells just above the step would not fit: a cell's number is
+// its slot in an open-addressed table of its key, 21 bits of each coordinate. Coordinates count
+// cells from 0 and wrap, so a cell can hold points 2^21 cells apart, which are no more than further
+// candidates; beyond 2^50 cells, where points within the step share the coordinate itself, they are
+// drawn from its bits. So cells stay just above the step whatever the extent. (Coarser cells of the
+// dense table instead, as the extent grows: every decision goes through all points of 27 cells, and
+// two points 100 m away made the sampling of 10,000 others at 1.4 mm take 842 ms, against 0.2 ms.)
+constexpr int                kSpWrap = 21;
+constexpr unsigned long long kSpMask = (1ull << kSpWrap) - 1;
+__device__ __forceinline__ unsigned long long sp_wrapped(float x, double perCell) {
+    const double q = floor((double)x * perCell);
+    return (fabs(q) < 1125899906842624.0 ? (unsigned long long)(long long)q
+                                         : smm::mix64((unsigned long long)__float_as_uint(x))) &
+           kSpMask;
+}
 
 struct SampleArgs {
     KdView          t;
     int             dim[3];
+    const unsigned long long *keys; // hashed cells: slot -> key (all ones: empty)
+    uint32_t        slotMask;
     const float4   *ent;      // cell runs: {x, y, z, tree position bits}, tree order in a run
     const float    *sure;     // the entries' sure_reach
-    const int      *cellRank; // dense cell -> occupied rank (-1: empty)
-    const int      *cellList; // occupied rank -> dense cell
+    const int      *cellRank; // cell -> occupied rank (-1: empty)
+    const int      *cellList; // occupied rank -> cell
     const int      *cellEnd;  // occupied rank -> end of its run of the entries
     // occupied rank -> an entry of its run that no open one comes before, and its tree position
     unsigned long long *cur;
     int            *dec;      // per entry: 0 open, 1 kept, 2 dropped
     int            *filed;    // per entry: first cell filed under it (-1: none)
     int            *nextCell; // per occupied rank: the next cell filed under the same entry
-    int            *ring;     // queue of dense cells (-1: slot not written)
+    int            *ring;     // queue of cells (-1: slot not written)
     unsigned        ringMask;
     int            *head, *tail;
     int            *open;     // cells with points not yet decided
@@ -735,6 +754,33 @@ __global__ void k_sp_keys(const int *__restrict__ vaccA, const float4 *__restric
         const int    cy = smg::coord(p.y, gp.org[1], gp.g, gp.dim[1]);
         const int    cz = smg::coord(p.z, gp.org[2], gp.g, gp.dim[2]);
         k               = (uint32_t)((cz * gp.dim[1] + cy) * gp.dim[0] + cx);
+    }
+    key[i] = k;
+    val[i] = (uint32_t)i;
+}
+
+// The same with hashed cells, which enter the table (of at least twice as many slots as points).
+__global__ void k_sp_keys_hashed(const int *__restrict__ vaccA, const float4 *__restrict__ pos, int m,
+                                 double perCell, unsigned long long *__restrict__ keys,
+                                 uint32_t slotMask, uint32_t noCell, uint32_t *__restrict__ key,
+                                 uint32_t *__restrict__ val) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m)
+        return;
+    const int id = vaccA[i];
+    uint32_t  k  = noCell;
+    if (id >= 0) {
+        const float4             p = pos[id];
+        const unsigned long long w = sp_wrapped(p.x, perCell) | sp_wrapped(p.y, perCell) << kSpWrap |
+                                     sp_wrapped(p.z, perCell) << (2 * kSpWrap);
+        uint32_t h = (uint32_t)smm::mix64(w) & slotMask;
+        for (uint32_t q = 0; q <= slotMask; q++) {
+            const unsigned long long prev = atomicCAS(&keys[h], ~0ull, w);
+            if (prev == ~0ull || prev == w)
+                break;
+            h = (h + 1) & slotMask;
+        }
+        k = h;
     }
     key[i] = k;
     val[i] = (uint32_t)i;
@@ -862,15 +908,33 @@ struct SpRuns {
     int nr, nend;      // occupied rank, end of its run
     int from, pos;     // its first open entry (or one before it) and that one's tree position
     int nb, excl, tot; // this pass's begin, exclusive prefix of the lengths and their sum
-    __device__ __forceinline__ void find(const SampleArgs &a, int cid) {
+    template <bool HASHED> __device__ __forceinline__ void find(const SampleArgs &a, int cid) {
         const int lane = threadIdx.x & 31;
-        const int cx = cid % a.dim[0], cy = (cid / a.dim[0]) % a.dim[1],
-                  cz = cid / (a.dim[0] * a.dim[1]);
-        const int x = cx + lane % 3 - 1, y = cy + (lane / 3) % 3 - 1, z = cz + lane / 9 - 1;
+        const int dx = lane % 3 - 1, dy = (lane / 3) % 3 - 1, dz = lane / 9 - 1;
         nr   = -1;
         nend = from = pos = 0;
-        if (lane < 27 && x >= 0 && y >= 0 && z >= 0 && x < a.dim[0] && y < a.dim[1] && z < a.dim[2])
-            nr = a.cellRank[(z * a.dim[1] + y) * a.dim[0] + x];
+        if (HASHED) {
+            const unsigned long long c = a.keys[cid];
+            const unsigned long long w =
+                ((c + (long long)dx) & kSpMask) |
+                (((c >> kSpWrap) + (long long)dy) & kSpMask) << kSpWrap |
+                (((c >> (2 * kSpWrap)) + (long long)dz) & kSpMask) << (2 * kSpWrap);
+            uint32_t           h = (uint32_t)smm::mix64(w) & a.slotMask;
+            unsigned long long k = lane < 27 ? a.keys[h] : ~0ull;
+            while (k != w && k != ~0ull) { // (a free slot ends every probe)
+                h = (h + 1) & a.slotMask;
+                k = a.keys[h];
+            }
+            if (k != ~0ull)
+                nr = a.cellRank[h];
+        } else {
+            const int cx = cid % a.dim[0], cy = (cid / a.dim[0]) % a.dim[1],
+                      cz = cid / (a.dim[0] * a.dim[1]);
+            const int x = cx + dx, y = cy + dy, z = cz + dz;
+            if (lane < 27 && x >= 0 && y >= 0 && z >= 0 && x < a.dim[0] && y < a.dim[1] &&
+                z < a.dim[2])
+                nr = a.cellRank[(z * a.dim[1] + y) * a.dim[0] + x];
+        }
         if (nr >= 0)
             nend = a.cellEnd[nr];
         look(a);
@@ -990,13 +1054,13 @@ __device__ __forceinline__ unsigned sp_drop(const SampleArgs &a, SpRuns &R, int 
 // its first point, or queues it. (Through the queue these are a third of its takes, each with the
 // queue's fences: the large scene's last sampling took 1.79 ms in k_sp_run alone, now 0.08 ms here
 // and 1.27 ms there.)
-__global__ void __launch_bounds__(kSpBs) k_sp_first(SampleArgs a) {
+template <bool HASHED> __global__ void __launch_bounds__(kSpBs) k_sp_first(SampleArgs a) {
     const int lane = threadIdx.x & 31;
     const int n = *a.open, nw = gridDim.x * (kSpBs / 32);
     for (int r = blockIdx.x * (kSpBs / 32) + (threadIdx.x >> 5); r < n; r += nw) {
-        SpRuns R;
+        SpRuns R{};
         const int cid = a.cellList[r];
-        R.find(a, cid);
+        R.find<HASHED>(a, cid);
         const int    k = __shfl_sync(0xffffffffu, R.from, kSpOwn);
         const float4 p = a.ent[k];
         const int    j = sp_blocker(a, R, k, p, __float_as_int(p.w));
@@ -1009,15 +1073,15 @@ __global__ void __launch_bounds__(kSpBs) k_sp_first(SampleArgs a) {
     }
 }
 
-__global__ void __launch_bounds__(kSpBs) k_sp_run(SampleArgs a) {
+template <bool HASHED> __global__ void __launch_bounds__(kSpBs) k_sp_run(SampleArgs a) {
     const int lane = threadIdx.x & 31;
     for (;;) {
         const int cid = __shfl_sync(0xffffffffu, lane == 0 ? sp_take(a) : 0, 0);
         if (cid < 0)
             return;
         __syncwarp(); // (lane 0's acquire holds for the warp)
-        SpRuns R;
-        R.find(a, cid);
+        SpRuns R{};
+        R.find<HASHED>(a, cid);
         const int r = __shfl_sync(0xffffffffu, R.nr, kSpOwn);
         const int e = __shfl_sync(0xffffffffu, R.nend, kSpOwn);
         int       k = __shfl_sync(0xffffffffu, R.from, kSpOwn);
@@ -1322,21 +1386,25 @@ int kd_sample(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
         return 0;
     const int *vaccA = vaccActive ? vaccActive : T.vacc;
     float      ext[3] = {box.ext(0), box.ext(1), box.ext(2)};
+    unsigned   ring   = 1024;
+    while (ring < 2u * (unsigned)m)
+        ring <<= 1;
     GridParamsK gp;
-    // cells just above the step, coarser where a dense table would not fit
+    // a dense table where cells just above the step fit it (5 % faster than hashed ones on 0.9 M
+    // points: 1.59 against 1.68 ms), else hashed ones (0.9 M points in an extent of twice and four
+    // times what fits: 1.76 and 1.58 ms; cells of twice and four times the side 2.15 and 4.87)
     gp.g = smg::sample_cell(step, ext, kSpCells);
     for (int a = 0; a < 3; a++) {
         gp.org[a] = box.mn[a];
         gp.dim[a] = smg::dim_of(ext[a], gp.g);
     }
-    const long long nc     = (long long)gp.dim[0] * gp.dim[1] * gp.dim[2];
+    const float     want   = step * (1.0f + 1.0f / 1024.0f);
+    const bool      hashed = gp.g > kSpCoarse * want;
+    const long long nc     = hashed ? (long long)ring : (long long)gp.dim[0] * gp.dim[1] * gp.dim[2];
     const uint32_t  noCell = (uint32_t)nc;
     int             bits   = 1;
     while ((nc >> bits) != 0)
         bits++;
-    unsigned ring = 1024;
-    while (ring < 2u * (unsigned)m)
-        ring <<= 1;
     uint32_t *key   = c.arena.get<uint32_t>(tag + ".key", m);
     uint32_t *val   = c.arena.get<uint32_t>(tag + ".val", m);
     int      *head  = c.arena.get<int>(tag + ".head", (size_t)m + 1);
@@ -1369,7 +1437,16 @@ int kd_sample(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
     a.r2       = step * step;
     a.keptFlag = flag;
     a.err      = ctl + 3 * kSpCtl;
-    k_sp_keys<<<nblocks(m, 256), 256, 0, c.stream>>>(vaccA, pos, m, gp, noCell, key, val);
+    if (hashed) {
+        auto *keys = c.arena.get<unsigned long long>(tag + ".keys", nc);
+        a.keys     = keys;
+        a.slotMask = (uint32_t)(nc - 1);
+        SM_CUDA(cudaMemsetAsync(keys, 0xff, (size_t)nc * 8, c.stream));
+        k_sp_keys_hashed<<<nblocks(m, 256), 256, 0, c.stream>>>(vaccA, pos, m, 1.0 / (double)want, keys,
+                                                                a.slotMask, noCell, key, val);
+    } else {
+        k_sp_keys<<<nblocks(m, 256), 256, 0, c.stream>>>(vaccA, pos, m, gp, noCell, key, val);
+    }
     SM_LAUNCH_CHECK();
     radix_sort_pairs(c, key, val, m, bits, tag);
     k_sp_heads<<<nblocks((long long)m + 1, 256), 256, 0, c.stream>>>(key, m, noCell, head);
@@ -1384,9 +1461,17 @@ int kd_sample(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
     SM_LAUNCH_CHECK();
     int nsm = 0;
     SM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device));
-    k_sp_first<<<std::min(nblocks(m, kSpBs / 32), nsm * 8), kSpBs, 0, c.stream>>>(a);
+    const int gFirst = std::min(nblocks(m, kSpBs / 32), nsm * 8);
+    const int gRun   = std::min(nblocks(m, kSpBs / 32), nsm * kSpCtas);
+    if (hashed)
+        k_sp_first<true><<<gFirst, kSpBs, 0, c.stream>>>(a);
+    else
+        k_sp_first<false><<<gFirst, kSpBs, 0, c.stream>>>(a);
     SM_LAUNCH_CHECK();
-    k_sp_run<<<std::min(nblocks(m, kSpBs / 32), nsm * kSpCtas), kSpBs, 0, c.stream>>>(a);
+    if (hashed)
+        k_sp_run<true><<<gRun, kSpBs, 0, c.stream>>>(a);
+    else
+        k_sp_run<false><<<gRun, kSpBs, 0, c.stream>>>(a);
     SM_LAUNCH_CHECK();
     int *pre = c.arena.get<int>(tag + ".pre", (size_t)m + 1);
     scan_excl(c, flag, pre, (long long)m + 1, tag + ".os", false);

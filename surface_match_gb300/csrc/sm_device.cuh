@@ -14,6 +14,11 @@ namespace smd {
 
 constexpr int kMaxKnn      = 32; // largest supported knnNormal
 constexpr int kKnnMaxShell = 24; // shells a k-nearest walk visits before it scans every point
+// The same where the k-d tree's own search, by one lane, takes over. (0.92 M points in reference
+// order, with three stray points 1 m and 10 m away: 8.6 and 9.6 ms a call with 9, 9.1 and 10.2 with
+// 12, 17.4 and 18.5 with 24, 7.2 without them. At 3 the ordinary queries of a scene with uniform
+// clutter are slower too, 4.09 ms against 3.90; at 6 as at 9.)
+constexpr int kTreeShell = 9;
 
 // Device view of a hashed uniform grid: only occupied cells are stored, in an
 // open-addressed table of uint4 {key low, key high, first point, point count - 1} (all ones in
@@ -424,8 +429,8 @@ static __device__ __noinline__ void knn_scan_all(const HGridView &g, float qx, f
 // scene with uniform clutter took 152 us, now 108.) Returns the number found (<= k); lane j < that count gets the j-th neighbour's index in *id and
 // squared distance in *d. With TIES points at the k-th distance are never skipped: for k < 32
 // lane k holds one more of them (index >= 0, the same distance) if there is one; and a search that
-// the rings up to kKnnMaxShell do not decide ends with -1 there: its caller has the tree, whose
-// search costs a far point no more than any other, instead of every point of the grid.
+// the rings up to kTreeShell do not decide ends with -1 there: its caller has the tree, whose
+// search does not count empty cells.
 template <bool TIES = false>
 __device__ __forceinline__ int warp_knn_sorted(const HGridView &g, float qx, float qy, float qz,
                                                int k, int *id, float *d) {
@@ -496,9 +501,9 @@ __device__ __forceinline__ int warp_knn_sorted(const HGridView &g, float qx, flo
         const float d = kd(), rb = smg::ring_bound(done, g.g);
         if (d < rb * rb || done >= ms)
             break;
+        if (TIES && done >= kTreeShell)
+            return -1;
         if (done >= kKnnMaxShell) {
-            if (TIES)
-                return -1;
             knn_scan_all(g, qx, qy, qz, k, best, seen);
             break;
         }

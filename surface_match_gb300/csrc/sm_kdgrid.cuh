@@ -158,10 +158,10 @@ __device__ __forceinline__ unsigned warp_kd_restricted(const int4 *__restrict__ 
     return met;
 }
 
-// Rings that a walk here goes out to before it leaves the query to the tree's own search. The
+// Rings that a walk here goes out to before it leaves the query to the tree's own search: the
 // rings' cubes grow with the fourth power of the distance, so a lone point some hundred cells from
-// its neighbours would keep its warp for seconds; the tree's search does not depend on it.
-constexpr int kMaxShell = smd::kKnnMaxShell;
+// its neighbours would keep its warp for seconds.
+constexpr int kMaxShell = smd::kTreeShell;
 constexpr int kFar      = -2; // a nearest search that gave up there
 
 // All points of grid g within squared distance B of q (<=), ascending by (distance, index) over

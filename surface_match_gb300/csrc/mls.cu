@@ -368,8 +368,12 @@ void estimate_normals_mls(Ctx &c, const float4 *pos, const int *valid, int nvali
     const float r2 = radius * radius;
     if (m <= 0 || nvalid <= 0 || !(r2 > 0.0f))
         return; // no point has a neighbour within a zero radius
+    // (coarser where the rounding of cell coordinates is more than the two hundredths)
+    float g = r * 1.02f;
+    while (box.slack(g) > smg::kCellSlack && !(r <= g * (1.0f - 2.0f * box.slack(g))) && g < 1e37f)
+        g *= 1.25f;
     HGrid G;
-    build_hgrid(c, pos, valid, nvalid, box, r * 1.02f, G, "mls.g");
+    build_hgrid(c, pos, valid, nvalid, box, g, G, "mls.g");
     MlsArgs a;
     a.g      = G.view();
     a.pos    = pos;

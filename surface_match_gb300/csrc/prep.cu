@@ -1194,6 +1194,7 @@ void build_hgrid(Ctx &c, const float4 *pos, const int *ids, int m, const Box &bo
         H.org[a] = box.mn[a];
         H.dim[a] = smg::dim_of(box.ext(a), g);
     }
+    H.slack     = box.slack(g);
     H.m         = m;
     int  *next  = c.arena.get<int>(tag + ".next", 1);
     int2 *place = c.arena.get<int2>(tag + ".place", std::max(m, 1));

@@ -34,6 +34,7 @@ __device__ __forceinline__ uint32_t hg_slot(unsigned long long key, uint32_t slo
 struct HGridView {
     float         org[3];
     float         g;
+    float         slack, slack1; // smg::cell_slack in cells, and 1 more
     int           dim[3];
     const uint4  *slot; // the hashed table (not built beside a direct one)
     uint32_t      slots;
@@ -211,8 +212,8 @@ __device__ __forceinline__ bool warp_visit_cells(const G &g, int b, int e, V &&v
 }
 
 // Lower bound of the squared distance from q to any point filed under cell (x, y, z): the
-// distance to the cell's box grown by the 1% cell margin that covers the rounding of cell
-// coordinates (as in ring_bound).
+// distance to the cell's box grown by the margin that covers the rounding of cell coordinates
+// (smg::cell_slack, as in ring_bound).
 __device__ __forceinline__ float cell_lb2(const HGridView &g, float qx, float qy, float qz, int x,
                                           int y, int z) {
     const float q[3] = {qx, qy, qz};
@@ -220,8 +221,8 @@ __device__ __forceinline__ float cell_lb2(const HGridView &g, float qx, float qy
     float       s    = 0.0f;
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        const float lo  = g.org[a] + ((float)k[a] - 0.01f) * g.g;
-        const float hi  = g.org[a] + ((float)k[a] + 1.01f) * g.g;
+        const float lo  = g.org[a] + ((float)k[a] - g.slack) * g.g;
+        const float hi  = g.org[a] + ((float)k[a] + g.slack1) * g.g;
         const float gap = fmaxf(0.0f, fmaxf(lo - q[a], q[a] - hi));
         s += gap * gap;
     }
@@ -350,10 +351,10 @@ __device__ __forceinline__ bool warp_band(const HGridView &g, float qx, float qy
 
 // The last ring of the next band after ring `done`: the first ring whose bound passes b2
 // (rings beyond it cannot hold a point within b2), at most 3 rings on and never past ms.
-__device__ __forceinline__ int band_end(int done, int ms, float b2, float g) {
+__device__ __forceinline__ int band_end(int done, int ms, float b2, const HGridView &g) {
     int hi = done + 1;
     while (hi < ms && hi < done + 3) {
-        const float rb = smg::ring_bound(hi, g);
+        const float rb = smg::ring_bound(hi, g.g, g.slack);
         if (rb * rb > b2)
             break;
         hi++;
@@ -498,7 +499,7 @@ __device__ __forceinline__ int warp_knn_sorted(const HGridView &g, float qx, flo
         return seen >= k ? f : kInf;
     };
     for (int done = 1;;) {
-        const float d = kd(), rb = smg::ring_bound(done, g.g);
+        const float d = kd(), rb = smg::ring_bound(done, g.g, g.slack);
         if (d < rb * rb || done >= ms)
             break;
         if (TIES && done >= kTreeShell)
@@ -509,7 +510,7 @@ __device__ __forceinline__ int warp_knn_sorted(const HGridView &g, float qx, flo
         }
         // (while fewer than k are found the next ring, from the third on three at once: a band's
         // cube is counted through whole)
-        const int hi = min(d < kInf ? band_end(done, ms, d, g.g) : done < 3 ? done + 1 : done + 3, ms);
+        const int hi = min(d < kInf ? band_end(done, ms, d, g) : done < 3 ? done + 1 : done + 3, ms);
         warp_band(g, qx, qy, qz, c, done + 1, hi, kd, [&](const float4 &p, bool valid) {
             visit(p, valid);
             return false;
@@ -554,7 +555,7 @@ __device__ __forceinline__ int warp_nn_walk(const HGridView &g, float qx, float 
     warp_block27(g, qx, qy, qz, c, limit2, visit);
     for (int done = 1;;) {
         const float d  = bd();
-        const float rb = smg::ring_bound(done, g.g);
+        const float rb = smg::ring_bound(done, g.g, g.slack);
         if (d < rb * rb || rb * rb > limit2 || done >= ms)
             break;
         if (done >= kKnnMaxShell) {
@@ -562,7 +563,7 @@ __device__ __forceinline__ int warp_nn_walk(const HGridView &g, float qx, float 
                 visit(g.pts[r], true);
             break;
         }
-        const int hi = band_end(done, ms, fminf(d, limit2), g.g);
+        const int hi = band_end(done, ms, fminf(d, limit2), g);
         warp_band(g, qx, qy, qz, c, done + 1, hi, [&]() { return fminf(bd(), limit2); }, visit);
         done = hi;
     }
@@ -611,10 +612,10 @@ __device__ __forceinline__ bool warp_any_within(const HGridView &g, float qx, fl
     const int ms = max(grid_max_shell(g, c), 1);
     warp_block27(g, qx, qy, qz, c, r2, visit);
     for (int done = 1;;) {
-        const float rb = smg::ring_bound(done, g.g);
+        const float rb = smg::ring_bound(done, g.g, g.slack);
         if (hit || rb * rb >= r2 || done >= ms)
             break;
-        const int hi = band_end(done, ms, r2, g.g);
+        const int hi = band_end(done, ms, r2, g);
         warp_band(g, qx, qy, qz, c, done + 1, hi, [&]() { return r2; }, visit);
         done = hi;
     }

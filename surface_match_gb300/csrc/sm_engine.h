@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+#include <cmath>
 #include <map>
 #include <mutex>
 #include <stdexcept>
@@ -120,14 +122,17 @@ struct HGrid {
     uint32_t *occ    = nullptr; // occupancy bit per cell (nullptr: too large a cell box, or direct)
     int2     *dense  = nullptr; // {first, count} per cell (nullptr unless the cell box is small)
     int       m      = 0;
+    float     slack  = smg::kCellSlack;
     smd::HGridView view() const {
         smd::HGridView v;
         for (int a = 0; a < 3; a++) {
             v.org[a] = org[a];
             v.dim[a] = dim[a];
         }
-        v.g    = g;
-        v.slot = slot;
+        v.g      = g;
+        v.slack  = slack;
+        v.slack1 = 1.0f + slack;
+        v.slot   = slot;
         v.slots = slots;
         v.pts  = pts;
         v.occ   = occ;
@@ -140,6 +145,16 @@ struct HGrid {
 struct Box {
     float mn[3], mx[3];
     float ext(int a) const { return mx[a] - mn[a]; }
+    // margin of a search grid of side g over the box (cell_slack)
+    float slack(float g) const {
+        int   d = 1;
+        float t = 0.0f;
+        for (int a = 0; a < 3; a++) {
+            d = std::max(d, smg::dim_of(ext(a), g));
+            t = std::max(t, std::max(std::fabs(mn[a]), std::fabs(mx[a])));
+        }
+        return smg::cell_slack(d, t, g);
+    }
     // Eigen norm order of the box size: x*x + (y*y + z*z)
     float diameter() const {
         const float x = ext(0), y = ext(1), z = ext(2);

@@ -83,9 +83,22 @@ SM_HD int coord(float x, float origin, float g, int dim) {
 
 SM_HD int phase_of(int cx, int cy, int cz) { return (cx & 1) | ((cy & 1) << 1) | ((cz & 1) << 2); }
 
+// How far, in cells, a point may lie outside the cell it is filed under, and what that does to the
+// distance of two points' cells: its coordinate is rounded twice (x - origin, / g), a cell's
+// bounds once against their number and once against the coordinates themselves. 1 % of a cell
+// covers up to 20,000 cells an axis and coordinates up to 40,000 cells from zero; a stray point, or
+// a cloud far from zero, takes more. dim: the longest axis; top: the largest coordinate.
+constexpr float kCellSlack = 0.01f;
+SM_HD float cell_slack(int dim, float top, float g) {
+    const float s = (float)dim * (1.0f / 2097152.0f) + smm::fdiv(top, g) * (1.0f / 4194304.0f);
+    return s > kCellSlack ? s : kCellSlack;
+}
+
 // After the cells within Chebyshev radius s of the query's cell have been searched, every
-// other point lies at least s cells' width away from the query: lower bound s * g, less a
-// 1% cell margin for the rounding of cell coordinates.
-SM_HD float ring_bound(int s, float g) { return s <= 0 ? 0.0f : ((float)s - 0.01f) * g; }
+// other point lies at least s cells' width away from the query: lower bound s * g, less the
+// margin for the rounding of cell coordinates.
+SM_HD float ring_bound(int s, float g, float slack = kCellSlack) {
+    return (float)s <= slack ? 0.0f : ((float)s - slack) * g;
+}
 
 } // namespace smg

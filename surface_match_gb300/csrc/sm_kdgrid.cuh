@@ -190,10 +190,10 @@ __device__ __forceinline__ int warp_collect(const smd::HGridView &g, float qx, f
     const int ms = max(smd::grid_max_shell(g, c), 1);
     bool      over = smd::warp_block27(g, qx, qy, qz, c, B, visit);
     for (int done = 1; !over;) {
-        const float rb = smg::ring_bound(done, g.g);
+        const float rb = smg::ring_bound(done, g.g, g.slack);
         if (rb * rb > B || done >= ms)
             break;
-        const int hi = smd::band_end(done, ms, B, g.g);
+        const int hi = smd::band_end(done, ms, B, g);
         over = done >= kMaxShell ||
                smd::warp_band(g, qx, qy, qz, c, done + 1, hi, [&]() { return B; }, visit);
         done = hi;
@@ -244,12 +244,12 @@ __device__ __forceinline__ int warp_nn_tie(const smd::HGridView &g, float qx, fl
     smd::warp_block27(g, qx, qy, qz, c, limit2, visit);
     for (int done = 1;;) {
         const float d  = fold();
-        const float rb = smg::ring_bound(done, g.g);
+        const float rb = smg::ring_bound(done, g.g, g.slack);
         if (d < rb * rb || rb * rb > limit2 || done >= ms)
             break;
         if (done >= kMaxShell)
             return kFar;
-        const int hi = smd::band_end(done, ms, fminf(d, limit2), g.g);
+        const int hi = smd::band_end(done, ms, fminf(d, limit2), g);
         smd::warp_band(g, qx, qy, qz, c, done + 1, hi, [&]() { return fminf(fold(), limit2); }, visit);
         done = hi;
     }

@@ -838,7 +838,10 @@ __device__ __forceinline__ int nb_entry(int t, int excl, int nb) {
 // Memory order. A cell moves between warps through the ring: pushed after a fence, taken by an
 // acquire. Filing stores the link and then looks at the entry's decision, deciding stores the
 // decision and then looks at the entry's list, each with a sequentially consistent fence
-// between: whichever comes second sees the other.
+// between: whichever comes second sees the other. A kept point's mark is a release by one lane
+// after a warp barrier, so that it covers the drops of all lanes; a warp that finds no blocker
+// fences and meets at a barrier before one lane looks at the point's own state, so that any lane's
+// look at such a mark counts.
 __device__ __forceinline__ void fence_sc() { asm volatile("fence.sc.gpu;" ::: "memory"); }
 __device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 __device__ __forceinline__ int  exch_acquire(int *p, int v) {
@@ -850,6 +853,9 @@ __device__ __forceinline__ int exch_release(int *p, int v) {
     int o;
     asm volatile("atom.release.gpu.global.exch.b32 %0, [%1], %2;" : "=r"(o) : "l"(p), "r"(v) : "memory");
     return o;
+}
+__device__ __forceinline__ void st_release(int *p, int v) {
+    asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 // Queues the cells filed under entry j. A slot is written once its last reader has emptied it:
 // at most every cell is queued, and the ring holds twice as many.
@@ -1132,15 +1138,15 @@ template <bool HASHED> __global__ void __launch_bounds__(kSpBs) k_sp_run(SampleA
             // no open earlier point within the step. A kept point drops before it counts as
             // decided, so p's own state is final now
             fence_acq_rel();
+            __syncwarp();
             if (__shfl_sync(0xffffffffu, lane == 0 ? ld_vol(&a.dec[k]) : 0, 0) != 0)
                 continue; // dropped meanwhile: on to the cell's next open entry
             const unsigned drop = sp_drop(a, R, k, p, ip);
             const unsigned any  = __reduce_or_sync(0xffffffffu, drop);
-            fence_acq_rel();
-            __syncwarp();
+            __syncwarp(); // (every lane's drops)
             if (lane == 0) {
-                a.keptFlag[ip]             = 1;
-                *(volatile int *)&a.dec[k] = 1;
+                a.keptFlag[ip] = 1;
+                st_release(&a.dec[k], 1);
             }
             fence_sc();
             for (unsigned m = any; m; m &= m - 1u) {

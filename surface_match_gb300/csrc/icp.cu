@@ -35,6 +35,7 @@ constexpr int kR  = smi::kIcpThreads; // reduction CTAs: a slot per thread
 constexpr int kRW = kR / 32;
 constexpr int kRC = smi::kIcpBlocks;  // reduction CTAs per candidate: one thread-block cluster
 constexpr int kFitU = 4;              // pairs whose loads a reduction thread has in flight
+constexpr int kStepLists = 3;         // candidate lists that a stage's steps take in turn
 constexpr int kTraceIters  = 32;
 constexpr int kTraceFloats = 2 * kTraceIters * 4 + 2;
 
@@ -77,24 +78,26 @@ struct Work {
     int                 maxSrc, maxDst;
     float              *trace;  // ncand x kTraceFloats (nullable)
     unsigned long long *live;   // (candidate, source point) searches of K1 (nullable: not counted)
-    // the candidates of each step of a stage (any order): iteration it refines those in
-    // list[it * ncand ..], cnt[it] of them; step `iters` holds those the stage leaves active
+    // a stage's candidate lists (any order), list l at list[l * ncand ..], cnt[l] of them: step `it`
+    // refines list it % kStepLists and lists those that go on in the next one, while the third is
+    // cleared; list kStepLists holds those the stage leaves active
     int                *cnt, *list;
     int                 ncand;
     unsigned long long *heard; // page-locked: {tag, candidates} of the last step begun
 };
 
-// The candidates of step `it`: their number and the k-th.
-__device__ __forceinline__ int  step_count(const Work &w, int it) { return w.cnt[it]; }
-__device__ __forceinline__ int  step_cand(const Work &w, int it, int k) { return w.list[it * w.ncand + k]; }
-// Candidate and source point of item k of the step's candidates times n source points.
-__device__ __forceinline__ void step_item(const Work &w, int it, long long k, int n, int &ci, int &i) {
+// The candidates of list l: their number and the k-th.
+__device__ __forceinline__ int step_list(int it) { return it % kStepLists; }
+__device__ __forceinline__ int step_count(const Work &w, int l) { return w.cnt[l]; }
+__device__ __forceinline__ int step_cand(const Work &w, int l, int k) { return w.list[l * w.ncand + k]; }
+// Candidate and source point of item k of the list's candidates times n source points.
+__device__ __forceinline__ void step_item(const Work &w, int l, long long k, int n, int &ci, int &i) {
     const int c = k < (1ll << 31) ? (int)((unsigned)k / (unsigned)n) : (int)(k / n);
-    ci          = step_cand(w, it, c);
+    ci          = step_cand(w, l, c);
     i           = (int)(k - (long long)c * n);
 }
-__device__ __forceinline__ void step_add(const Work &w, int it, int ci) {
-    w.list[it * w.ncand + atomicAdd(&w.cnt[it], 1)] = ci;
+__device__ __forceinline__ void step_add(const Work &w, int l, int ci) {
+    w.list[l * w.ncand + atomicAdd(&w.cnt[l], 1)] = ci;
 }
 
 __device__ __forceinline__ unsigned long long win_key(float d, int i) {
@@ -129,10 +132,12 @@ __global__ void __launch_bounds__(kT, TREE ? 3 : 4)
     k_corr(Work w, Stage s, int it, unsigned tag) {
     chain_enter(); // launched chained
     const int       lane  = threadIdx.x & 31;
-    const long long items = (long long)step_count(w, it) * s.n;
+    const int       l     = step_list(it);
+    const long long items = (long long)step_count(w, l) * s.n;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
+        w.cnt[step_list(it + 2)] = 0; // (the last step's: k_update adds to the next one's)
         *(volatile unsigned long long *)w.heard =
-            ((unsigned long long)tag << 32) | (unsigned)step_count(w, it);
+            ((unsigned long long)tag << 32) | (unsigned)step_count(w, l);
         if (w.live)
             atomicAdd(w.live, (unsigned long long)items);
     }
@@ -142,7 +147,7 @@ __global__ void __launch_bounds__(kT, TREE ? 3 : 4)
         const bool      have = k < items;
         int             ci = 0, i = 0;
         if (have)
-            step_item(w, it, k, s.n, ci, i);
+            step_item(w, l, k, s.n, ci, i);
         const size_t o   = (size_t)ci * w.maxSrc + i;
         const Cand  &C   = w.cand[ci];
         float4       x   = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -305,9 +310,10 @@ __global__ void __cluster_dims__(kRC, 1, 1) __launch_bounds__(kR) k_fit(Work w, 
     __shared__ int   sTotal;
     cg::cluster_group cl = cg::this_cluster();
     const int         rk = (int)cl.block_rank();
-    if ((int)(blockIdx.x / kRC) >= step_count(w, it))
+    const int         l  = step_list(it);
+    if ((int)(blockIdx.x / kRC) >= step_count(w, l))
         return; // (the whole cluster: one candidate)
-    const int     ci   = step_cand(w, it, blockIdx.x / kRC);
+    const int     ci   = step_cand(w, l, blockIdx.x / kRC);
     Cand         &C    = w.cand[ci];
     int          *nnId = w.nnId + (size_t)ci * w.maxSrc;
     const int    *nnR  = w.nnR + (size_t)ci * w.maxSrc;
@@ -448,14 +454,15 @@ __global__ void __cluster_dims__(kRC, 1, 1) __launch_bounds__(kR) k_fit(Work w, 
 template <bool TREE>
 __global__ void __launch_bounds__(kT, TREE ? 3 : 5) k_resid(Work w, Stage s, int it) {
     chain_enter(); // launched chained
-    const long long items = (long long)step_count(w, it) * s.n;
+    const int       l     = step_list(it);
+    const long long items = (long long)step_count(w, l) * s.n;
     const long long warps = (long long)gridDim.x * kW;
     for (long long base = blockIdx.x * kW + (threadIdx.x >> 5); base < items; base += 32 * warps) {
         const long long k    = base + (threadIdx.x & 31) * warps;
         bool            have = k < items;
         int             ci = 0, i = 0;
         if (have)
-            step_item(w, it, k, s.n, ci, i);
+            step_item(w, l, k, s.n, ci, i);
         const size_t o = (size_t)ci * w.maxSrc + i;
         float        y0 = 0.f, y1 = 0.f, y2 = 0.f, lim = 0.f, d;
         if (have) {
@@ -485,9 +492,10 @@ __global__ void __cluster_dims__(kRC, 1, 1) __launch_bounds__(kR) k_update(Work 
     __shared__ float part[1][2];
     cg::cluster_group cl = cg::this_cluster();
     const int         rk = (int)cl.block_rank();
-    if ((int)(blockIdx.x / kRC) >= step_count(w, it))
+    const int         l  = step_list(it);
+    if ((int)(blockIdx.x / kRC) >= step_count(w, l))
         return;
-    const int  ci   = step_cand(w, it, blockIdx.x / kRC);
+    const int  ci   = step_cand(w, l, blockIdx.x / kRC);
     Cand      &C    = w.cand[ci];
     const int  slot = rk * kR + threadIdx.x;
     const int  lane = threadIdx.x & 31;
@@ -566,15 +574,14 @@ __global__ void __cluster_dims__(kRC, 1, 1) __launch_bounds__(kR) k_update(Work 
         if (cnt >= 6)
             C.iterations = done + 1;
         if (!stop && done + 1 < s.iters)
-            step_add(w, it + 1, ci);
+            step_add(w, step_list(it + 1), ci);
     }
 }
 
-__global__ void k_init(Work w, const float *__restrict__ cands, float voteThreshold, int sparse,
-                       int steps) {
+__global__ void k_init(Work w, const float *__restrict__ cands, float voteThreshold, int sparse) {
     const int ci = blockIdx.x * blockDim.x + threadIdx.x;
-    for (int k = ci; k < steps; k += gridDim.x * blockDim.x)
-        w.cnt[k] = 0; // the candidate counts of every step of both stages
+    if (ci < 2 * (kStepLists + 1))
+        w.cnt[ci] = 0; // the candidate counts of both stages
     if (ci >= w.ncand)
         return;
     Cand        &C = w.cand[ci];
@@ -606,7 +613,7 @@ __global__ void k_stage_begin(Work w, int iters) {
 
 // After a refinement: failed candidates get their status; converged ones keep the pose and are
 // listed for the scoring.
-__global__ void k_stage_end(Work w, int last, int failStatus) {
+__global__ void k_stage_end(Work w, int failStatus) {
     chain_enter(); // launched chained
     const int ci = blockIdx.x * blockDim.x + threadIdx.x;
     if (ci >= w.ncand)
@@ -619,22 +626,22 @@ __global__ void k_stage_end(Work w, int last, int failStatus) {
         C.active = 0;
     } else {
         C.keep = C.M;
-        step_add(w, last, ci);
+        step_add(w, kStepLists, ci);
     }
 }
 
-// Inliers of each candidate left (step `last`): source points with a scene point closer than the
+// Inliers of each candidate left (list kStepLists): source points with a scene point closer than the
 // scoring distance (warp_any_within); with TREE the scene point that the reference's search of the
 // whole tree returns (inliner, util.cpp:628-641). A warp takes consecutive points, 32 at a time a
 // lane each, and adds to a candidate's count once per 32 (two launches of the large scene in
 // reference order 250 -> 158 us).
 template <bool TREE>
 __global__ void __launch_bounds__(kT, TREE ? 3 : 5)
-    k_inliers(Work w, const float4 *__restrict__ src, int n, int last, HGridView F, float r2,
+    k_inliers(Work w, const float4 *__restrict__ src, int n, HGridView F, float r2,
               smk::KdView t, int treeM, const int *__restrict__ treePos,
               const float *__restrict__ exc) {
     chain_enter(); // launched chained
-    const long long items = (long long)step_count(w, last) * n;
+    const long long items = (long long)step_count(w, kStepLists) * n;
     const long long warps = (long long)gridDim.x * kW, per = (items + warps - 1) / warps;
     long long       k   = (blockIdx.x * (long long)kW + (threadIdx.x >> 5)) * per;
     const long long end = k + per < items ? k + per : items;
@@ -644,7 +651,7 @@ __global__ void __launch_bounds__(kT, TREE ? 3 : 5)
         int        ci = -1, i = 0;
         float      x = 0.f, y = 0.f, z = 0.f;
         if (have) {
-            step_item(w, last, k + lane, n, ci, i);
+            step_item(w, kStepLists, k + lane, n, ci, i);
             const float4 p = src[i];
             smi::pose_apply(w.cand[ci].M, p.x, p.y, p.z, x, y, z);
         }
@@ -793,27 +800,25 @@ void icp_all(Ctx &c, const Model &m, const IcpScene &sc, const IcpParams &p, con
         w.live = c.arena.get<unsigned long long>("icp.live", 1);
         SM_CUDA(cudaMemsetAsync(w.live, 0, sizeof(unsigned long long), c.stream));
     }
-    // steps of the sparse stage (5 iterations and the scoring), then of the dense one
     constexpr int sparseIters = 5;
-    const int     sparseLast = sparseIters, denseLast = std::max(p.denseSteps, 0);
-    const int     steps = sparseLast + 1 + denseLast + 1;
+    constexpr int lists       = kStepLists + 1; // of the sparse stage, then of the dense one
     w.ncand = ncand;
-    w.cnt   = c.arena.get<int>("icp.cnt", steps);
-    w.list  = c.arena.get<int>("icp.list", (size_t)steps * ncand);
+    w.cnt   = c.arena.get<int>("icp.cnt", 2 * lists);
+    w.list  = c.arena.get<int>("icp.list", (size_t)2 * lists * ncand);
     SM_CUDA(cudaMemsetAsync(w.win, 0xff, (size_t)ncand * w.maxDst * 8, c.stream));
-    k_init<<<nblocks(ncand, 128), 128, 0, c.stream>>>(w, cands, p.voteThreshold, p.sparse, steps);
+    k_init<<<nblocks(ncand, 128), 128, 0, c.stream>>>(w, cands, p.voteThreshold, p.sparse);
     SM_LAUNCH_CHECK();
     const float rej2 = p.rejectDist * p.rejectDist;
     const float sc2  = p.scoreDist * p.scoreDist;
     const bool tree = sc.tree != nullptr;
-    auto inliers = [&](const float4 *src, int n, int last) {
+    auto inliers = [&](const float4 *src, int n) {
         const int g = wave(c, (long long)ncand * n, tree ? 3 : 5);
         if (tree)
-            launch_chained(c, k_inliers<true>, g, kT, 0, w, src, n, last, sc.full.view(), sc2,
+            launch_chained(c, k_inliers<true>, g, kT, 0, w, src, n, sc.full.view(), sc2,
                            sc.tree->view(nullptr, sc.pos, nullptr, sc.tpF), sc.tree->m,
                            (const int *)sc.tree->treePos, sc.exc + 2);
         else
-            launch_chained(c, k_inliers<false>, g, kT, 0, w, src, n, last, sc.full.view(), sc2,
+            launch_chained(c, k_inliers<false>, g, kT, 0, w, src, n, sc.full.view(), sc2,
                            smk::KdView{}, 0, (const int *)nullptr, (const float *)nullptr);
     };
     if (p.sparse) {
@@ -827,8 +832,8 @@ void icp_all(Ctx &c, const Model &m, const IcpScene &sc, const IcpParams &p, con
             s.exc    = sc.exc;
         }
         run_stage(c, w, s);
-        launch_chained(c, k_stage_end, nblocks(ncand, 128), 128, 0, w, sparseLast, 2);
-        inliers(m.sp, m.ns, sparseLast);
+        launch_chained(c, k_stage_end, nblocks(ncand, 128), 128, 0, w, 2);
+        inliers(m.sp, m.ns);
         launch_chained(c, k_score, nblocks(ncand, 128), 128, 0, w, ncand, m.ns, p.minScore, 3,
                        0);
         if (p.dense) {
@@ -841,11 +846,11 @@ void icp_all(Ctx &c, const Model &m, const IcpScene &sc, const IcpParams &p, con
                 d.tposOf = sc.tposR;
                 d.exc    = sc.exc + 1;
             }
-            w.cnt += sparseLast + 1;
-            w.list += (size_t)(sparseLast + 1) * ncand;
+            w.cnt += lists;
+            w.list += (size_t)lists * ncand;
             run_stage(c, w, d);
-            launch_chained(c, k_stage_end, nblocks(ncand, 128), 128, 0, w, denseLast, 4);
-            inliers(m.rp, m.nr, denseLast);
+            launch_chained(c, k_stage_end, nblocks(ncand, 128), 128, 0, w, 4);
+            inliers(m.rp, m.nr);
             launch_chained(c, k_score, nblocks(ncand, 128), 128, 0, w, ncand, m.nr, p.minScore,
                            5, 1);
         }

@@ -24,16 +24,15 @@
 // definite (Eigen's LLT then reports a numerical issue and its solve returns an unspecified
 // vector) the point keeps the PCA normal, as for a non-finite solution.
 //
-// Two kernels over a hashed grid of cell just above the radius, so that the 3x3x3 block holds
+// Three kernels over a hashed grid of cell just above the radius, so that the 3x3x3 block holds
 // every neighbour. k_mls_near, a warp per listed point, collects its neighbours; k_mls_fit, a
-// thread per point, makes everything of them. The work is FP64 (eigenvector, Cholesky) and a
-// few dozen sums, and GB300 issues an FP64 warp instruction at the same cost for one active
-// lane as for 32 and has no cheap way to spread one point's sums over a warp: with a warp per
-// point for all of it, 50,000 points of 30 neighbours at order 2 took 2080 us, now 300 us (the
-// call 2640 -> 710 us). Sums are FP32
-// Kahan per point, read out with their compensation in FP64; the fit runs in coordinates
-// scaled by 1/r (the same polynomial, better conditioned); the small systems are solved in
-// FP64.
+// thread per point, makes everything of them; k_mls_wide, a warp per point, does it for points with
+// too many. The work is FP64 (eigenvector, Cholesky) and a few dozen sums, and GB300 issues an FP64
+// warp instruction at the same cost for one active lane as for 32: with a warp per point for all of
+// it, 50,000 points of 30 neighbours at order 2 took 2080 us of a call's 2640, now the call takes
+// 340. Sums are FP32 Kahan per point, read out with their compensation in FP64; the fit runs in
+// coordinates scaled by 1/r (the same polynomial, better conditioned); the small systems are solved
+// in FP64.
 #include <cmath>
 
 #include "sm_device.cuh"
@@ -113,11 +112,48 @@ template <int N> __device__ bool cholesky_solve(double (&G)[N][N], double (&b)[N
     return true;
 }
 
+// The same in loops, for a system in shared memory.
+__device__ bool cholesky_solve(double *G, double *b, int n) {
+    for (int j = 0; j < n; j++) {
+        double d = G[j * n + j];
+        for (int k = 0; k < j; k++)
+            d -= G[j * n + k] * G[j * n + k];
+        if (!(d > 0.0))
+            return false;
+        const double s = sqrt(d);
+        G[j * n + j]   = s;
+        for (int i = j + 1; i < n; i++) {
+            double v = G[i * n + j];
+            for (int k = 0; k < j; k++)
+                v -= G[i * n + k] * G[j * n + k];
+            G[i * n + j] = v / s;
+        }
+    }
+    for (int i = 0; i < n; i++) { // L y = b
+        double v = b[i];
+        for (int k = 0; k < i; k++)
+            v -= G[i * n + k] * b[k];
+        b[i] = v / G[i * n + i];
+    }
+    for (int i = n - 1; i >= 0; i--) { // L^T c = y
+        double v = b[i];
+        for (int k = i + 1; k < n; k++)
+            v -= G[k * n + i] * b[k];
+        b[i] = v / G[i * n + i];
+        if (!isfinite(b[i]))
+            return false;
+    }
+    return true;
+}
+
 // The neighbours of listed point i0 + t (places in g.pts) in the lists' order: neighbour j of
-// the points of a warp of k_mls_fit is one line of near; cnt[t] their number, also above the
-// list's length.
+// the points of a warp of k_mls_fit is one line of near; cnt[t] their number, or more than the
+// list's length where they are more: such points are named in wide[], counted on from base in
+// *nwide.
 __global__ void __launch_bounds__(kMlsWarps * 32)
-    k_mls_near(MlsArgs a, int i0, int n, int *__restrict__ near, int *__restrict__ cnt) {
+    k_mls_near(MlsArgs a, int i0, int n, int *__restrict__ near, int *__restrict__ cnt,
+               int *__restrict__ wide, int *__restrict__ nwide, int base) {
+    smd::chain_enter(); // launched chained
     const int lane = threadIdx.x & 31;
     const int t    = blockIdx.x * kMlsWarps + (threadIdx.x >> 5);
     if (t >= n)
@@ -138,8 +174,8 @@ __global__ void __launch_bounds__(kMlsWarps * 32)
         const int excl = incl - (e - b);
         const int T    = __shfl_sync(0xffffffffu, incl, 31);
         int      *L    = near + (size_t)(t >> 5) * (32 * kMlsNear) + (t & 31);
-        for (int base = 0; base < T; base += 32) {
-            const int r   = base + lane;
+        for (int r0 = 0; r0 < T && num <= kMlsNear; r0 += 32) {
+            const int r   = r0 + lane;
             int       own = 0; // the lane whose cell holds point r: last lane with excl <= r
 #pragma unroll
             for (int step = 16; step >= 1; step >>= 1)
@@ -158,8 +194,11 @@ __global__ void __launch_bounds__(kMlsWarps * 32)
             num += __popc(m);
         }
     }
-    if (lane == 0)
+    if (lane == 0) {
         cnt[t] = num;
+        if (num > kMlsNear)
+            wide[atomicAdd(nwide, 1) - base] = t;
+    }
 }
 
 // fn(p) for every neighbour p of q: the listed ones, or by a walk over the 3x3x3 block.
@@ -199,17 +238,239 @@ __device__ __forceinline__ void each_near(const MlsArgs &a, const float4 &q, con
 
 __device__ __forceinline__ double sum_of(const smi::KahanF &k) { return (double)k.s - (double)k.c; }
 
+// The tangent frame of normal n.
+__device__ __forceinline__ void mls_frame(const float n[3], float u[3], float v[3]) {
+    if (!(fabsf(n[0]) <= fabsf(n[2]) * 1e-5f) || !(fabsf(n[1]) <= fabsf(n[2]) * 1e-5f)) {
+        const float h = smm::fdiv(1.0f, smm::fsqrt(n[0] * n[0] + n[1] * n[1]));
+        v[0]          = -n[1] * h;
+        v[1]          = n[0] * h;
+        v[2]          = 0.0f;
+    } else {
+        const float h = smm::fdiv(1.0f, smm::fsqrt(n[1] * n[1] + n[2] * n[2]));
+        v[0]          = 0.0f;
+        v[1]          = -n[2] * h;
+        v[2]          = n[1] * h;
+    }
+    u[0] = n[1] * v[2] - n[2] * v[1];
+    u[1] = n[2] * v[0] - n[0] * v[2];
+    u[2] = n[0] * v[1] - n[1] * v[0];
+}
+
+// 4. The fit's coefficients b back in unscaled coordinates (c0 scales by r, the linear terms are
+// slopes and do not change), and with them the point and its normal.
+template <int ORDER>
+__device__ __forceinline__ void mls_write(const MlsArgs &a, int id, const double *b, const float m[3],
+                                          const float n[3], const float u[3], const float v[3]) {
+    const float c0 = (float)(b[0] * (double)a.r);
+    const float cv = (float)b[1], cu = (float)b[ORDER + 1];
+    const float px = m[0] + c0 * n[0], py = m[1] + c0 * n[1], pz = m[2] + c0 * n[2];
+    float       nx = n[0] - cu * u[0] - cv * v[0], ny = n[1] - cu * u[1] - cv * v[1],
+          nz = n[2] - cu * u[2] - cv * v[2];
+    const float nn = nx * nx + ny * ny + nz * nz;
+    if (nn > 0.0f) {
+        const float s = smm::fsqrt(nn);
+        nx            = smm::fdiv(nx, s);
+        ny            = smm::fdiv(ny, s);
+        nz            = smm::fdiv(nz, s);
+    }
+    const float d = a.hasVp ? nx * (a.vx - px) + ny * (a.vy - py) + nz * (a.vz - pz) : nz;
+    if (a.invert ? d > 0.0f : d < 0.0f) {
+        nx = -nx;
+        ny = -ny;
+        nz = -nz;
+    }
+    float *outN = a.outNrm + 3 * (size_t)id;
+    float *outP = a.outXyz + 3 * (size_t)id;
+    outP[0]     = px;
+    outP[1]     = py;
+    outP[2]     = pz;
+    outN[0]     = nx;
+    outN[1]     = ny;
+    outN[2]     = nz;
+}
+
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1)
+        v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// The place of moment u^i v^j (i + j <= D, i outer): rows 0 .. i - 1 come before it.
+template <int D> __device__ __forceinline__ constexpr int moment_at(int i, int j) {
+    return i * (D + 1) - i * (i - 1) / 2 + j;
+}
+
+// Exponents of monomial k of total degree <= order, u's outer.
+__device__ __forceinline__ void monomial(int k, int order, int &i, int &j) {
+    for (i = 0; k > order - i; i++)
+        k -= order - i + 1;
+    j = k;
+}
+
+// Which points of a launch of n a warp takes each (wide: how many have more neighbours than are
+// listed): those, up to as many as the warps work off in the time that a thread takes for one; and
+// all points of a small launch with such, so that no thread's chain follows the warps'. A thread
+// walks the 27 cells for three sums, tens of thousands of loads one after the other: order 2, 1000
+// neighbours, of 16,000 points in all, by threads and by warps: 40 points 2695 and 603 us, 5000
+// 2625 and 1191, 10,000 2685 and 1833, 16,000 2709 and 2774; 300 neighbours: 967 and 291, 1164 and
+// 637, 1164 and 959, 1204 and 1397. Order 4, 300 neighbours, 2000 points: 1508 and 953, 5000: 1503
+// and 1854; 5000 neighbours of 100,000 points, 5000 points: 20911 and 8244.
+enum MlsBy { kMlsThreads, kMlsWideByWarps, kMlsAllByWarps };
+constexpr int kMlsSmall = 2048, kMlsWideCtas = 3; // (CTAs per SM)
+__device__ __forceinline__ MlsBy mls_by(int n, int wide, int order) {
+    if (wide > 0 && n <= kMlsSmall)
+        return kMlsAllByWarps;
+    const int most = order == 1 ? 32768 : order == 2 ? 12288 : order == 3 ? 8192 : 6144;
+    return wide <= most ? kMlsWideByWarps : kMlsThreads;
+}
+
+// The points that a warp takes each, which walks the 3x3x3 block for each sum: lane l owns the fit's
+// sums l, l + 32, ... (the moments of the Gram matrix, then the right-hand side) and takes every
+// neighbour.
+template <int ORDER>
+__global__ void __launch_bounds__(kMlsWarps * 32, kMlsWideCtas)
+    k_mls_wide(MlsArgs a, int i0, int n, const int *__restrict__ num, const int *__restrict__ wide,
+               const int *__restrict__ nwide, int base) {
+    smd::chain_enter(); // launched chained
+    constexpr int D = 2 * ORDER, NM = (D + 1) * (D + 2) / 2, NC = (ORDER + 1) * (ORDER + 2) / 2;
+    constexpr int PER = (NM + NC + 31) / 32;
+    __shared__ double sMom[kMlsWarps][NM + NC], sGram[kMlsWarps][NC * NC];
+    const int         lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int         nw = *nwide - base;
+    const MlsBy       by = mls_by(n, nw, ORDER);
+    if (nw == 0 || by == kMlsThreads)
+        return;
+    const float r2 = a.r2, invR = smm::fdiv(1.0f, a.r);
+    // the lane's sums: exponents of u and v, whether the term carries the height
+    int  eu[PER], ev[PER];
+    bool rhs[PER];
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+        const int e = lane + 32 * k;
+        rhs[k]      = e >= NM;
+        monomial(rhs[k] ? min(e - NM, NC - 1) : e, rhs[k] ? ORDER : D, eu[k], ev[k]);
+    }
+    const int last = by == kMlsAllByWarps ? n : nw;
+    for (int k0 = blockIdx.x * kMlsWarps + wid; k0 < last; k0 += gridDim.x * kMlsWarps) {
+        const int t = by == kMlsAllByWarps ? k0 : wide[k0];
+        if (num[t] < 3)
+            continue;
+        const int    id = a.ids[i0 + t];
+        const float4 q  = a.pos[id];
+        int          c[3];
+        smd::grid_cc(a.g, q.x, q.y, q.z, c);
+        auto each = [&](auto &&fn) { // fn(p, whether the lane's p is a neighbour), by all lanes
+            smd::warp_block27(a.g, q.x, q.y, q.z, c, r2, [&](const float4 &p, bool valid) {
+                fn(p, valid && smm::dist2(q.x, q.y, q.z, p.x, p.y, p.z) < r2);
+                return false;
+            });
+        };
+        smi::KahanF s0[3];
+        int         cnt = 0;
+        for (int d = 0; d < 3; d++)
+            s0[d].init();
+        each([&](const float4 &p, bool in) {
+            if (in) {
+                cnt++;
+                s0[0].add(p.x - q.x);
+                s0[1].add(p.y - q.y);
+                s0[2].add(p.z - q.z);
+            }
+        });
+        cnt              = __reduce_add_sync(0xffffffffu, cnt);
+        const double inv = 1.0 / (double)cnt;
+        const float  cx  = (float)((double)q.x + warp_sum(sum_of(s0[0])) * inv);
+        const float  cy  = (float)((double)q.y + warp_sum(sum_of(s0[1])) * inv);
+        const float  cz  = (float)((double)q.z + warp_sum(sum_of(s0[2])) * inv);
+        smi::KahanF  s1[6];
+        for (int e = 0; e < 6; e++)
+            s1[e].init();
+        each([&](const float4 &p, bool in) {
+            if (in) {
+                const float dx = p.x - cx, dy = p.y - cy, dz = p.z - cz;
+                s1[0].add(dx * dx);
+                s1[1].add(dx * dy);
+                s1[2].add(dx * dz);
+                s1[3].add(dy * dy);
+                s1[4].add(dy * dz);
+                s1[5].add(dz * dz);
+            }
+        });
+        double C[6];
+        for (int e = 0; e < 6; e++)
+            C[e] = warp_sum(sum_of(s1[e]));
+        float n3[3], u[3], v[3];
+        sml::normal_from_cov(C, n3);
+        if (lane < 3)
+            a.outNrm[3 * (size_t)id + lane] = lane == 0 ? n3[0] : lane == 1 ? n3[1] : n3[2];
+        if (ORDER <= 1 && NC > cnt)
+            continue;
+        const float dist = n3[0] * (q.x - cx) + n3[1] * (q.y - cy) + n3[2] * (q.z - cz);
+        const float m[3] = {q.x - dist * n3[0], q.y - dist * n3[1], q.z - dist * n3[2]};
+        mls_frame(n3, u, v);
+        smi::KahanF acc[PER];
+#pragma unroll
+        for (int k = 0; k < PER; k++)
+            acc[k].init();
+        each([&](const float4 &p, bool in) {
+            float w = 0.0f, uc = 0.0f, vc = 0.0f, fc = 0.0f;
+            if (in) {
+                const float dx = p.x - m[0], dy = p.y - m[1], dz = p.z - m[2];
+                w  = expf(-smm::fdiv(dx * dx + dy * dy + dz * dz, r2));
+                uc = (dx * u[0] + dy * u[1] + dz * u[2]) * invR;
+                vc = (dx * v[0] + dy * v[1] + dz * v[2]) * invR;
+                fc = (dx * n3[0] + dy * n3[1] + dz * n3[2]) * invR;
+            }
+            for (unsigned live = __ballot_sync(0xffffffffu, w > 0.0f); live; live &= live - 1u) {
+                const int   j  = __ffs(live) - 1;
+                const float wj = __shfl_sync(0xffffffffu, w, j);
+                const float uj = __shfl_sync(0xffffffffu, uc, j);
+                const float vj = __shfl_sync(0xffffffffu, vc, j);
+                const float fj = __shfl_sync(0xffffffffu, fc, j);
+#pragma unroll
+                for (int k = 0; k < PER; k++) {
+                    const float term = wj * powi(uj, eu[k]) * powi(vj, ev[k]);
+                    acc[k].add(rhs[k] ? term * fj : term);
+                }
+            }
+        });
+        __syncwarp(); // (the last point's solve has read them)
+#pragma unroll
+        for (int k = 0; k < PER; k++)
+            if (lane + 32 * k < NM + NC)
+                sMom[wid][lane + 32 * k] = sum_of(acc[k]);
+        __syncwarp();
+        for (int e = lane; e < NC * NC; e += 32) {
+            int i, j, i2, j2;
+            monomial(e / NC, ORDER, i, j);
+            monomial(e % NC, ORDER, i2, j2);
+            sGram[wid][e] = sMom[wid][moment_at<D>(i + i2, j + j2)];
+        }
+        __syncwarp();
+        if (lane == 0) {
+            double *b = &sMom[wid][NM];
+            if (cholesky_solve(sGram[wid], b, NC))
+                mls_write<ORDER>(a, id, b, m, n3, u, v);
+        }
+    }
+}
+
+// The listed points by a thread each, but for those that k_mls_wide takes.
 template <int ORDER>
 __global__ void __launch_bounds__(kMlsFitBs)
-    k_mls_fit(MlsArgs a, int i0, int n, const int *__restrict__ near, const int *__restrict__ num) {
+    k_mls_fit(MlsArgs a, int i0, int n, const int *__restrict__ near, const int *__restrict__ num,
+              const int *__restrict__ nwide, int base) {
+    smd::chain_enter(); // launched chained
     constexpr int D  = 2 * ORDER;               // the Gram entries are moments of degree <= D
     constexpr int NM = (D + 1) * (D + 2) / 2;   // u^i v^j, i + j <= D, i outer
     constexpr int NC = (ORDER + 1) * (ORDER + 2) / 2;
-    const int     t  = blockIdx.x * kMlsFitBs + threadIdx.x;
+    const int t = blockIdx.x * kMlsFitBs + threadIdx.x;
     if (t >= n)
         return;
-    const int cnt = num[t];
-    if (cnt < 3)
+    const int   cnt = num[t];
+    const MlsBy by  = mls_by(n, *nwide - base, ORDER);
+    if (cnt < 3 || by == kMlsAllByWarps || (by == kMlsWideByWarps && cnt > kMlsNear))
         return;
     const int    id = a.ids[i0 + t];
     const float4 q  = a.pos[id];
@@ -217,14 +478,16 @@ __global__ void __launch_bounds__(kMlsFitBs)
 
     // 1. centroid (offsets from q), then the covariance about it
     smi::KahanF s0[3];
+    int         found = 0; // (cnt, where they are listed)
     for (int d = 0; d < 3; d++)
         s0[d].init();
     each_near(a, q, L, cnt, [&](const float4 &p) {
+        found++;
         s0[0].add(p.x - q.x);
         s0[1].add(p.y - q.y);
         s0[2].add(p.z - q.z);
     });
-    const double inv = 1.0 / (double)cnt;
+    const double inv = 1.0 / (double)found;
     const float  cx  = (float)((double)q.x + sum_of(s0[0]) * inv);
     const float  cy  = (float)((double)q.y + sum_of(s0[1]) * inv);
     const float  cz  = (float)((double)q.z + sum_of(s0[2]) * inv);
@@ -246,28 +509,15 @@ __global__ void __launch_bounds__(kMlsFitBs)
     float n3[3];
     sml::normal_from_cov(C, n3);
     float *outN = a.outNrm + 3 * (size_t)id;
-    float *outP = a.outXyz + 3 * (size_t)id;
     outN[0]     = n3[0];
     outN[1]     = n3[1];
     outN[2]     = n3[2];
 
     // 2. projection on the plane and the tangent frame
     const float dist = n3[0] * (q.x - cx) + n3[1] * (q.y - cy) + n3[2] * (q.z - cz);
-    const float mx = q.x - dist * n3[0], my = q.y - dist * n3[1], mz = q.z - dist * n3[2];
-    float       v[3];
-    if (!(fabsf(n3[0]) <= fabsf(n3[2]) * 1e-5f) || !(fabsf(n3[1]) <= fabsf(n3[2]) * 1e-5f)) {
-        const float h = smm::fdiv(1.0f, smm::fsqrt(n3[0] * n3[0] + n3[1] * n3[1]));
-        v[0]          = -n3[1] * h;
-        v[1]          = n3[0] * h;
-        v[2]          = 0.0f;
-    } else {
-        const float h = smm::fdiv(1.0f, smm::fsqrt(n3[1] * n3[1] + n3[2] * n3[2]));
-        v[0]          = 0.0f;
-        v[1]          = -n3[2] * h;
-        v[2]          = n3[1] * h;
-    }
-    const float u[3] = {n3[1] * v[2] - n3[2] * v[1], n3[2] * v[0] - n3[0] * v[2],
-                        n3[0] * v[1] - n3[1] * v[0]};
+    const float m[3] = {q.x - dist * n3[0], q.y - dist * n3[1], q.z - dist * n3[2]};
+    float       u[3], v[3];
+    mls_frame(n3, u, v);
     if (ORDER <= 1 && NC > cnt)
         return;
 
@@ -281,7 +531,7 @@ __global__ void __launch_bounds__(kMlsFitBs)
         rhs[k].init();
     const float invR = smm::fdiv(1.0f, a.r);
     each_near(a, q, L, cnt, [&](const float4 &p) {
-        const float dx = p.x - mx, dy = p.y - my, dz = p.z - mz;
+        const float dx = p.x - m[0], dy = p.y - m[1], dz = p.z - m[2];
         const float w  = expf(-smm::fdiv(dx * dx + dy * dy + dz * dz, a.r2));
         const float uc = (dx * u[0] + dy * u[1] + dz * u[2]) * invR;
         const float vc = (dx * v[0] + dy * v[1] + dz * v[2]) * invR;
@@ -318,39 +568,24 @@ __global__ void __launch_bounds__(kMlsFitBs)
 #pragma unroll
                     for (int j2 = 0; j2 <= ORDER - i2; j2++, l++)
                         if (l <= k) {
-                            const int A = i + i2, B = j + j2; // moments of rows 0 .. A-1 before it
-                            G[k][l] = sum_of(mom[A * (D + 1) - A * (A - 1) / 2 + B]);
+                            G[k][l] = sum_of(mom[moment_at<D>(i + i2, j + j2)]);
                         }
             }
     }
     if (!cholesky_solve(G, b))
         return;
-    // 4. coefficients back to unscaled coordinates: c0 scales by r, the linear terms are
-    // slopes and do not change
-    const float c0 = (float)(b[0] * (double)a.r);
-    const float cv = (float)b[1], cu = (float)b[ORDER + 1];
-    const float px = mx + c0 * n3[0], py = my + c0 * n3[1], pz = mz + c0 * n3[2];
-    float       nx = n3[0] - cu * u[0] - cv * v[0], ny = n3[1] - cu * u[1] - cv * v[1],
-          nz = n3[2] - cu * u[2] - cv * v[2];
-    const float nn = nx * nx + ny * ny + nz * nz;
-    if (nn > 0.0f) {
-        const float s = smm::fsqrt(nn);
-        nx            = smm::fdiv(nx, s);
-        ny            = smm::fdiv(ny, s);
-        nz            = smm::fdiv(nz, s);
-    }
-    const float d = a.hasVp ? nx * (a.vx - px) + ny * (a.vy - py) + nz * (a.vz - pz) : nz;
-    if (a.invert ? d > 0.0f : d < 0.0f) {
-        nx = -nx;
-        ny = -ny;
-        nz = -nz;
-    }
-    outP[0] = px;
-    outP[1] = py;
-    outP[2] = pz;
-    outN[0] = nx;
-    outN[1] = ny;
-    outN[2] = nz;
+    mls_write<ORDER>(a, id, b, m, n3, u, v);
+}
+
+template <int ORDER>
+void fit(Ctx &c, const MlsArgs &a, int i0, int n, const int *near, const int *num, const int *wide,
+         const int *nwide, int base) {
+    int nsm = 0;
+    SM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device));
+    launch_chained(c, k_mls_wide<ORDER>, std::min(nblocks(n, kMlsWarps), kMlsWideCtas * nsm), kMlsWarps * 32, 0, a,
+                   i0, n, num, wide, nwide, base);
+    launch_chained(c, k_mls_fit<ORDER>, nblocks(n, kMlsFitBs), kMlsFitBs, 0, a, i0, n, near, num, nwide,
+                   base);
 }
 
 __global__ void k_fill_nan(float *x, long long n) {
@@ -389,15 +624,26 @@ void estimate_normals_mls(Ctx &c, const float4 *pos, const int *valid, int nvali
     a.outNrm = outNrm;
     const int chunk = std::min(m, kMlsChunk);
     int      *near  = c.arena.get<int>("mls.near", (size_t)((chunk + 31) / 32) * 32 * kMlsNear);
-    int      *num   = c.arena.get<int>("mls.num", chunk);
-    void (*const fit[kMlsMaxOrder])(MlsArgs, int, int, const int *, const int *) = {
-        k_mls_fit<1>, k_mls_fit<2>, k_mls_fit<3>, k_mls_fit<4>};
+    int      *num   = c.arena.get<int>("mls.num", (size_t)chunk * 2);
+    int      *wide  = num + chunk;
+    // the built grid's range counter, at the number of its points, goes on as the wide points'
+    int *nwide = G.next, base = nvalid;
     for (int i0 = 0; i0 < m; i0 += chunk) {
         const int n = std::min(chunk, m - i0);
-        k_mls_near<<<nblocks(n, kMlsWarps), kMlsWarps * 32, 0, c.stream>>>(a, i0, n, near, num);
-        SM_LAUNCH_CHECK();
-        fit[order - 1]<<<nblocks(n, kMlsFitBs), kMlsFitBs, 0, c.stream>>>(a, i0, n, near, num);
-        SM_LAUNCH_CHECK();
+        if (i0 > 0) {
+            SM_CUDA(cudaMemsetAsync(nwide, 0, sizeof(int), c.stream));
+            base = 0;
+        }
+        launch_chained(c, k_mls_near, nblocks(n, kMlsWarps), kMlsWarps * 32, 0, a, i0, n, near, num, wide,
+                       nwide, base);
+        if (order == 1)
+            fit<1>(c, a, i0, n, near, num, wide, nwide, base);
+        else if (order == 2)
+            fit<2>(c, a, i0, n, near, num, wide, nwide, base);
+        else if (order == 3)
+            fit<3>(c, a, i0, n, near, num, wide, nwide, base);
+        else
+            fit<4>(c, a, i0, n, near, num, wide, nwide, base);
     }
 }
 

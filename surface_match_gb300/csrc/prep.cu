@@ -1199,6 +1199,7 @@ void build_hgrid(Ctx &c, const float4 *pos, const int *ids, int m, const Box &bo
     int  *next  = c.arena.get<int>(tag + ".next", 1);
     int2 *place = c.arena.get<int2>(tag + ".place", std::max(m, 1));
     H.pts       = c.arena.get<float4>(tag + ".pts", std::max(m, 1));
+    H.next      = next;
     // a direct {first, count} table over a cell box of at most 2^22 cells (32 MB), else the hashed
     // one, with occupancy bits over a box of at most 2^28 cells (32 MB); cleared with the counter
     // in one launch

@@ -123,6 +123,7 @@ struct HGrid {
     int2     *dense  = nullptr; // {first, count} per cell (nullptr unless the cell box is small)
     int       m      = 0;
     float     slack  = smg::kCellSlack;
+    int      *next   = nullptr; // the ranges' counter: m once the grid is built
     smd::HGridView view() const {
         smd::HGridView v;
         for (int a = 0; a < 3; a++) {

@@ -67,7 +67,6 @@ struct Stage {
 
 struct Work {
     Cand               *cand;
-    const float4       *pos, *nrm;
     int                *nnId;   // ncand x maxSrc: subset rank of the pair's scene point (-1 none)
     int                *nnR;    // ncand x maxSrc: the same, kept through pair selection
     int                *nnPrev; // ncand x maxSrc: nearest subset point of the last iteration
@@ -780,8 +779,6 @@ void icp_all(Ctx &c, const Model &m, const IcpScene &sc, const IcpParams &p, con
     if (ncand <= 0)
         return;
     Work w;
-    w.pos    = sc.pos;
-    w.nrm    = sc.nrm;
     w.maxSrc = std::max(std::max(m.ns, m.nr), 1);
     w.maxDst = std::max(std::max(sc.sampled.m, sc.resampled.m), 1);
     w.cand   = c.arena.get<Cand>("icp.cand", ncand);

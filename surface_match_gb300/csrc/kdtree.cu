@@ -794,7 +794,8 @@ __global__ void k_sp_heads(const uint32_t *__restrict__ key, int m, uint32_t noC
     head[k] = (k < m && key[k] != noCell && (k == 0 || key[k - 1] != key[k])) ? 1 : 0;
 }
 
-// The cells' runs, and the runs' points in run order: {x, y, z, tree position bits}, with the distance a search surely reaches it at.
+// The cells' runs, and the runs' points in run order: {x, y, z, tree position bits}, with the
+// distance a search surely reaches it at.
 __global__ void k_sp_cells(const uint32_t *__restrict__ key, const uint32_t *__restrict__ sortPos,
                            int m, uint32_t noCell, const int *__restrict__ head,
                            const int *__restrict__ rank, const float *__restrict__ nodeBox,
@@ -1179,11 +1180,10 @@ __global__ void k_sp_out(const int *__restrict__ flag, const int *__restrict__ p
 // first found), and how many: by a thread over the tree.
 __device__ __forceinline__ void kd_knn_query(const KdView &t, const float q[3], int k,
                                              int *__restrict__ nbr, float *__restrict__ dist,
-                                             int *__restrict__ cnt, int *__restrict__ err) {
+                                             int *__restrict__ cnt) {
     smk::KnnSet<kMaxKnn> rs;
     rs.init(k);
-    if (!smk::kd_search(t, q, rs))
-        atomicExch(err, 1);
+    smk::kd_search(t, q, rs); // (no tree is deeper than its stack: the build refuses them)
     for (int j = 0; j < k; j++) {
         nbr[j] = j < rs.count ? rs.idx[j] : -1;
         if (dist)
@@ -1195,14 +1195,13 @@ __device__ __forceinline__ void kd_knn_query(const KdView &t, const float q[3], 
 
 // One query per thread, at qpos[t].
 __global__ void k_kd_knn(KdView t, const float4 *__restrict__ qpos, const int *__restrict__ nq,
-                         int k, int *__restrict__ nbr, float *__restrict__ dist,
-                         int *__restrict__ err) {
+                         int k, int *__restrict__ nbr, float *__restrict__ dist) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= *nq)
         return;
     const float4 p    = qpos[i];
     const float  q[3] = {p.x, p.y, p.z};
-    kd_knn_query(t, q, k, nbr + (size_t)i * k, dist + (size_t)i * k, nullptr, err);
+    kd_knn_query(t, q, k, nbr + (size_t)i * k, dist + (size_t)i * k, nullptr);
 }
 
 // One query per warp over part `part` of a normal estimation's list, answered on the grid of the
@@ -1210,8 +1209,7 @@ __global__ void k_kd_knn(KdView t, const float4 *__restrict__ qpos, const int *_
 constexpr int kKnnBs = 256;
 __global__ void __launch_bounds__(kKnnBs)
     k_kd_knn_grid(KdView t, int m, HGridView g, const int *__restrict__ treePos, NormalList L,
-                  int part, int k, bool grow, int *__restrict__ err,
-                  const float4 *__restrict__ nrm) {
+                  int part, int k, bool grow, const float4 *__restrict__ nrm) {
     const int lane = threadIdx.x & 31;
     const int i    = L.begin(part) +
                   (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -1224,7 +1222,7 @@ __global__ void __launch_bounds__(kKnnBs)
     if (n < 0) {
         if (lane == 0) {
             const float q[3] = {p.x, p.y, p.z};
-            kd_knn_query(t, q, k, out, nullptr, L.nbrCnt + i, err);
+            kd_knn_query(t, q, k, out, nullptr, L.nbrCnt + i);
         }
         __syncwarp();
         n  = L.nbrCnt[i];
@@ -1499,12 +1497,10 @@ void kd_knn(Ctx &c, const KdTree &T, const int *vaccActive, const float4 *pos,
         return;
     if (k < 1 || k > kMaxKnn)
         throw Error(SM_ERR_RANGE, "knnNormal larger than " + std::to_string(kMaxKnn) + " is not supported");
-    int    *err  = c.arena.get<int>("kd.knn.err", 1);
     float4 *tpos = c.arena.get<float4>("kd.knn.tpos", T.m);
-    SM_CUDA(cudaMemsetAsync(err, 0, sizeof(int), c.stream));
     kd_tree_positions(c, T, vaccActive, pos, tpos);
     k_kd_knn<<<nblocks(nqMax, 128), 128, 0, c.stream>>>(T.view(vaccActive, pos, nullptr, tpos), qpos,
-                                                        nq, k, nbr, dist, err);
+                                                        nq, k, nbr, dist);
     SM_LAUNCH_CHECK();
 }
 
@@ -1513,10 +1509,8 @@ void kd_knn_points(Ctx &c, const KdTree &T, const HGrid &g, const float4 *pos,
                    const float4 *nrm) {
     if (nqMax <= 0 || T.m <= 0)
         return;
-    int *err = c.arena.get<int>("kd.knn.err", 1);
-    SM_CUDA(cudaMemsetAsync(err, 0, sizeof(int), c.stream));
     k_kd_knn_grid<<<nblocks((long long)nqMax * 32, kKnnBs), kKnnBs, 0, c.stream>>>(
-        T.view(nullptr, pos), T.m, g.view(), T.treePos, L, part, k, grow, err, nrm);
+        T.view(nullptr, pos), T.m, g.view(), T.treePos, L, part, k, grow, nrm);
     SM_LAUNCH_CHECK();
 }
 

@@ -48,11 +48,11 @@ struct ScanInts {
 
 // What a scan writes: kPrefix, out[i] = sum of the values before i; kSelect (0/1 flags), the
 // places i of set flags packed into out; kSelectIds, ids[i] for these. A thread's eight prefixes
-// are two 16-byte stores where the array is aligned to them. (Values and prefixes one by one, and with the selected places written by a second kernel from the stored prefixes, 0.92 M
-// flags took 11 + 7 us, a table of 2 M counts 20 us.)
+// are two 16-byte stores where the array is aligned to them. (Values and prefixes one by one, and
+// with the selected places written by a second kernel from the stored prefixes, 0.92 M flags took
+// 11 + 7 us, a table of 2 M counts 20 us.)
 enum ScanOut { kPrefix, kSelect, kSelectIds };
 
-//
 // The values come from IN: skip(), uniform over the launch, ends it before it takes a ticket or
 // writes anything; load() gives each thread its eight consecutive values of the tile from `base`
 // (0 from n on), called by the whole CTA.

@@ -34,7 +34,7 @@ __device__ __forceinline__ uint32_t hg_slot(unsigned long long key, uint32_t slo
 struct HGridView {
     float         org[3];
     float         g;
-    float         slack, slack1; // smg::cell_slack in cells, and 1 more
+    float         slack, half; // smg::cell_slack in cells; half a cell and that, in its units
     int           dim[3];
     const uint4  *slot; // the hashed table (not built beside a direct one)
     uint32_t      slots;
@@ -213,7 +213,7 @@ __device__ __forceinline__ bool warp_visit_cells(const G &g, int b, int e, V &&v
 
 // Lower bound of the squared distance from q to any point filed under cell (x, y, z): the
 // distance to the cell's box grown by the margin that covers the rounding of cell coordinates
-// (smg::cell_slack, as in ring_bound).
+// (smg::cell_slack, as in ring_bound), both counted from the grid's origin as cell coordinates are.
 __device__ __forceinline__ float cell_lb2(const HGridView &g, float qx, float qy, float qz, int x,
                                           int y, int z) {
     const float q[3] = {qx, qy, qz};
@@ -221,9 +221,9 @@ __device__ __forceinline__ float cell_lb2(const HGridView &g, float qx, float qy
     float       s    = 0.0f;
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        const float lo  = g.org[a] + ((float)k[a] - g.slack) * g.g;
-        const float hi  = g.org[a] + ((float)k[a] + g.slack1) * g.g;
-        const float gap = fmaxf(0.0f, fmaxf(lo - q[a], q[a] - hi));
+        float u; // (not kept over a search's cells: the three registers spill in k_knn)
+        asm volatile("sub.rn.f32 %0, %1, %2;" : "=f"(u) : "f"(q[a]), "f"(g.org[a]));
+        const float gap = fmaxf(0.0f, fabsf(u - ((float)k[a] + 0.5f) * g.g) - g.half);
         s += gap * gap;
     }
     return s;

@@ -6,7 +6,6 @@
 #include <stdint.h>
 
 #include <algorithm>
-#include <cmath>
 #include <map>
 #include <mutex>
 #include <stdexcept>
@@ -132,7 +131,7 @@ struct HGrid {
         }
         v.g      = g;
         v.slack  = slack;
-        v.slack1 = 1.0f + slack;
+        v.half   = (0.5f + slack) * g;
         v.slot   = slot;
         v.slots = slots;
         v.pts  = pts;
@@ -148,13 +147,10 @@ struct Box {
     float ext(int a) const { return mx[a] - mn[a]; }
     // margin of a search grid of side g over the box (cell_slack)
     float slack(float g) const {
-        int   d = 1;
-        float t = 0.0f;
-        for (int a = 0; a < 3; a++) {
+        int d = 1;
+        for (int a = 0; a < 3; a++)
             d = std::max(d, smg::dim_of(ext(a), g));
-            t = std::max(t, std::max(std::fabs(mn[a]), std::fabs(mx[a])));
-        }
-        return smg::cell_slack(d, t, g);
+        return smg::cell_slack(d);
     }
     // Eigen norm order of the box size: x*x + (y*y + z*z)
     float diameter() const {

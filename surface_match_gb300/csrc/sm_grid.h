@@ -84,13 +84,15 @@ SM_HD int coord(float x, float origin, float g, int dim) {
 SM_HD int phase_of(int cx, int cy, int cz) { return (cx & 1) | ((cy & 1) << 1) | ((cz & 1) << 2); }
 
 // How far, in cells, a point may lie outside the cell it is filed under, and what that does to the
-// distance of two points' cells: its coordinate is rounded twice (x - origin, / g), a cell's
-// bounds once against their number and once against the coordinates themselves. 1 % of a cell
-// covers up to 20,000 cells an axis and coordinates up to 40,000 cells from zero; a stray point, or
-// a cloud far from zero, takes more. dim: the longest axis; top: the largest coordinate.
+// distance of two points' cells: coordinates are taken from the origin on both sides, so that every
+// rounding is one of a number of at most dim cells - a point's coordinate twice (x - origin, / g), a
+// cell's bounds twice, the query's coordinate once, half a unit of 2^-23 each. 1 % of a cell covers
+// up to 20,000 cells an axis; a stray point takes more. dim: the longest axis. (Bounds in the
+// cloud's own coordinates are rounded by those: a cloud far from zero needed a margin of many
+// cells, and every search looked at as many rings of them.)
 constexpr float kCellSlack = 0.01f;
-SM_HD float cell_slack(int dim, float top, float g) {
-    const float s = (float)dim * (1.0f / 2097152.0f) + smm::fdiv(top, g) * (1.0f / 4194304.0f);
+SM_HD float cell_slack(int dim) {
+    const float s = (float)dim * (1.0f / 2097152.0f);
     return s > kCellSlack ? s : kCellSlack;
 }
 

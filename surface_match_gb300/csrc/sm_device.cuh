@@ -426,12 +426,13 @@ static __device__ __noinline__ void knn_scan_all(const HGridView &g, float qx, f
 // (no point there can enter the list, not even by the index tie-break). The search ends
 // after shell s once k points were seen and the k-th distance is below the ring bound of s
 // (every unvisited point is farther); further shells come in bands, their cells screened against
-// the k-th distance (warp_band). (Shell by shell, every cell looked up, 18,000 queries of a
-// scene with uniform clutter took 152 us, now 108.) Returns the number found (<= k); lane j < that
-// count gets the j-th neighbour's index in *id and squared distance in *d. With TIES points at the k-th distance are never skipped: for k < 32
-// lane k holds one more of them (index >= 0, the same distance) if there is one; and a search that
-// the rings up to kTreeShell do not decide ends with -1 there: its caller has the tree, whose
-// search does not count empty cells.
+// the k-th distance (warp_band), and after kKnnMaxShell of them all points are scanned. (Shell by
+// shell, every cell looked up, 18,000 queries of a scene with uniform clutter took 152 us, now 108.)
+// Returns the number found (<= k); lane j < that count gets the j-th neighbour's index in *id and
+// squared distance in *d. With TIES points at the k-th distance are never skipped: for k < 32 lane
+// k holds one more of them (index >= 0, the same distance) if there is one; and a search that the
+// rings up to kTreeShell do not decide ends with -1 there: its caller has the tree, whose search
+// does not count empty cells.
 template <bool TIES = false>
 __device__ __forceinline__ int warp_knn_sorted(const HGridView &g, float qx, float qy, float qz,
                                                int k, int *id, float *d) {

@@ -381,10 +381,10 @@ void train(Ctx &c, Model &m, const float *xyzIn, const float *nrmIn, int64_t n64
         const KdTree *tree = m.order == SM_ORDER_REFERENCE ? &T : nullptr;
         HGrid         q;
         const float   gq = knn_cell(nvalid, n1, sampleStep, tp.knnNormal);
-        build_hgrid(c, pos, valid, nvalid, box, gq, q, "t.q");
+        build_hgrid(c, pos, valid, nvalid, box, gq, q, "t.q", false, tree != nullptr);
         estimate_normals(c, pos, nrm, n, idx1, n1, q, tp.knnNormal, tp.smoothNormal != 0, false,
                          nullptr, "t.n1", tree);
-        build_hgrid(c, pos, valid, nvalid, box, gq, q, "t.q");
+        build_hgrid(c, pos, valid, nvalid, box, gq, q, "t.q", false, tree != nullptr);
         estimate_normals(c, pos, nrm, n, idx2, n2, q, tp.knnNormal, tp.smoothNormal != 0, false,
                          nullptr, "t.n2", tree);
     }
@@ -557,7 +557,7 @@ void match(Ctx &c, const Model &m, const float *xyzIn, const float *nrmIn, int64
     }
     gq = knn_cell(nvalid, ns, sampleStep, mp.knnNormal);
     if (!hasN) {
-        build_hgrid(c, pos, valid, nvalid, box, gq, q, "m.q");
+        build_hgrid(c, pos, valid, nvalid, box, gq, q, "m.q", false, ref);
         estimate_normals(c, pos, nrm, n, sampled, ns, q, mp.knnNormal, mp.smoothNormal != 0,
                          mp.invertNormal != 0, vp, "m.n1", ref ? &T : nullptr);
     }
@@ -604,7 +604,7 @@ void match(Ctx &c, const Model &m, const float *xyzIn, const float *nrmIn, int64
                        : sample_points(d, P, n, valid, nvalid, box, reSampleStep, resampled, "m.s3");
             if (!hasN) {
                 HGrid q2;
-                build_hgrid(d, P, valid, nvalid, box, gq, q2, "m.q");
+                build_hgrid(d, P, valid, nvalid, box, gq, q2, "m.q", false, ref);
                 estimate_normals(d, P, N, n, resampled, nres, q2, mp.knnNormal, false,
                                  mp.invertNormal != 0, vp, "m.n2", ref ? &T : nullptr);
             }
@@ -653,10 +653,11 @@ void match(Ctx &c, const Model &m, const float *xyzIn, const float *nrmIn, int64
         // (in grid order the subsets are ascending, so rank order is index order), and the
         // refinement reads rank-ordered copies of the subsets.
         build_hgrid(d, P, sampled, ns, box, std::max(sampleStep, refDist / 2.98f), s.sampled,
-                    "m.gS", true);
+                    "m.gS", true, ref);
         build_hgrid(d, P, resampled, nres, box, std::max(2.0f * reSampleStep, refDist / 2.98f),
-                    s.resampled, "m.gR", true);
-        build_hgrid(d, P, valid, nvalid, box, std::max(scoreDist * 1.02f, gq), s.full, "m.gF");
+                    s.resampled, "m.gR", true, ref);
+        build_hgrid(d, P, valid, nvalid, box, std::max(scoreDist * 1.02f, gq), s.full, "m.gF",
+                    false, ref);
         float4 *posS = d.arena.get<float4>("m.posS", std::max(ns, 1));
         float4 *nrmS = d.arena.get<float4>("m.nrmS", std::max(ns, 1));
         float4 *posR = d.arena.get<float4>("m.posR", std::max(nres, 1));

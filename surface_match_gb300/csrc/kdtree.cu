@@ -1237,6 +1237,28 @@ __global__ void __launch_bounds__(kKnnBs)
         L.add_neighbour(lane < n, id, nrm);
 }
 
+// The same by the tree's own search, a thread per query, where the grid's cells are coarse.
+__global__ void k_kd_knn_list(KdView t, NormalList L, int part, int k, bool grow,
+                              const float4 *__restrict__ nrm) {
+    const int lane = threadIdx.x & 31;
+    const int i0   = L.begin(part) + (blockIdx.x * blockDim.x + threadIdx.x - lane);
+    const int end  = L.end(part);
+    if (i0 >= end)
+        return;
+    if (i0 + lane < end) {
+        const float4 p    = t.pos[L.list[i0 + lane]];
+        const float  q[3] = {p.x, p.y, p.z};
+        kd_knn_query(t, q, k, L.nbr + (size_t)(i0 + lane) * k, nullptr, L.nbrCnt + i0 + lane);
+    }
+    if (!grow)
+        return;
+    __syncwarp();
+    for (int i = i0; i < min(i0 + 32, end); i++) {
+        const bool in = lane < L.nbrCnt[i];
+        L.add_neighbour(in, in ? L.nbr[(size_t)i * k + lane] : -1, nrm);
+    }
+}
+
 // ---- the voting stage's candidates (ppf.cpp:273-276) --------------------------------------
 // Candidate r (id cand[r], the reduced tree's r-th point): its tree position, and the squared
 // distance below which a radius search of radius^2 r2 surely reaches it: the search's bound
@@ -1509,6 +1531,12 @@ void kd_knn_points(Ctx &c, const KdTree &T, const HGrid &g, const float4 *pos,
                    const float4 *nrm) {
     if (nqMax <= 0 || T.m <= 0)
         return;
+    if (g.coarse) {
+        k_kd_knn_list<<<nblocks(nqMax, 128), 128, 0, c.stream>>>(T.view(nullptr, pos), L, part, k, grow,
+                                                                 nrm);
+        SM_LAUNCH_CHECK();
+        return;
+    }
     k_kd_knn_grid<<<nblocks((long long)nqMax * 32, kKnnBs), kKnnBs, 0, c.stream>>>(
         T.view(nullptr, pos), T.m, g.view(), T.treePos, L, part, k, grow, nrm);
     SM_LAUNCH_CHECK();

@@ -1179,23 +1179,36 @@ void compact_known(Ctx &c, const int *flags, int n, int count, int *outIds) {
         scan_launch<kSelect>(c, flags, outIds, n, nullptr, nullptr);
 }
 
+// With a tree beside it a grid is not built where the extent (a stray point some 2^20 cells off, or a
+// huge number in the place of a missing value) makes its cells more than kCoarse times the wanted
+// ones: a cell's points grow with their square, and the tree's own searches, a thread each, do not
+// depend on the extent. (0.92 M points with strays 4, 8, 16, 32 and 64 km and 1000 km away: on the
+// grid 10.6, 12.5, 21.9, 48, 113 and 868 ms a call, on the tree 16.6 to 18.1 up to 64 km; 0.1 M
+// points 4.6, 4.7, 5.6, 8.7, 23 and 61 against 6.3 to 6.5. Far less than four times, the grid is
+// faster; without a stray it takes 7.5 against 13.4 ms.)
+constexpr float kCoarse = 4.0f;
+
 void build_hgrid(Ctx &c, const float4 *pos, const int *ids, int m, const Box &box, float g,
-                 HGrid &H, const std::string &tag, bool wIsRank) {
+                 HGrid &H, const std::string &tag, bool wIsRank, bool tree) {
     // (any cell side gives the same results: without a wanted one, some 1000 cells an axis)
     if (!(g > 0.0f))
         g = std::max(std::max(box.ext(0), box.ext(1)), std::max(box.ext(2), 1e-30f)) / 1024.0f;
+    const float want = g;
     // cells per axis stay below 2^20 so that cell keys fit 60 bits (coarser cells if needed; the
     // loop ends: dim_of is 1 where the side overflows)
     while (smg::dim_of(box.ext(0), g) >= (1 << 20) || smg::dim_of(box.ext(1), g) >= (1 << 20) ||
            smg::dim_of(box.ext(2), g) >= (1 << 20))
         g = g * 2.0f;
-    H.g = g;
+    H.g      = g;
+    H.coarse = tree && g > kCoarse * want;
     for (int a = 0; a < 3; a++) {
         H.org[a] = box.mn[a];
         H.dim[a] = smg::dim_of(box.ext(a), g);
     }
     H.slack     = box.slack(g);
     H.m         = m;
+    if (H.coarse)
+        return;
     int  *next  = c.arena.get<int>(tag + ".next", 1);
     int2 *place = c.arena.get<int2>(tag + ".place", std::max(m, 1));
     H.pts       = c.arena.get<float4>(tag + ".pts", std::max(m, 1));

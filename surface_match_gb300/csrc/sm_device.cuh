@@ -42,6 +42,7 @@ struct HGridView {
     const uint32_t *occ;   // one bit per cell of the dim box (nullptr: not built)
     const int2     *dense; // {first, count} per cell of the dim box (nullptr: not built)
     int             m;     // points in pts
+    bool            coarse; // not built: the points' k-d tree is searched instead
     __device__ __forceinline__ unsigned long long key_of(int x, int y, int z) const {
         return ((unsigned long long)z * (unsigned)dim[1] + (unsigned)y) * (unsigned)dim[0] +
                (unsigned)x;

@@ -121,6 +121,7 @@ struct HGrid {
     uint32_t *occ    = nullptr; // occupancy bit per cell (nullptr: too large a cell box, or direct)
     int2     *dense  = nullptr; // {first, count} per cell (nullptr unless the cell box is small)
     int       m      = 0;
+    bool      coarse = false;   // not built: the points' k-d tree is searched instead
     float     slack  = smg::kCellSlack;
     int      *next   = nullptr; // the ranges' counter: m once the grid is built
     smd::HGridView view() const {
@@ -138,6 +139,7 @@ struct HGrid {
         v.occ   = occ;
         v.dense = dense;
         v.m     = m;
+        v.coarse = coarse;
         return v;
     }
 };

@@ -268,6 +268,18 @@ __device__ __forceinline__ bool in_limit(float d, float limit2) {
     return d <= limit2 && d < 3.402823466e38f;
 }
 
+// The search itself, by one lane: the point's name (-1: none, or one farther than limit2) and its
+// squared distance.
+__device__ __forceinline__ int tree_nearest(const KdView &t, const int *__restrict__ nameOf, float exc,
+                                            float qx, float qy, float qz, float limit2, float *d) {
+    const float q[3] = {qx, qy, qz};
+    NnSet       rs;
+    rs.init(nn_bound(nn_bound(limit2, exc), exc));
+    kd_search(t, q, rs);
+    *d = rs.dist;
+    return !rs.count ? -1 : nameOf ? nameOf[rs.idx] : rs.idx;
+}
+
 // What the reference's one-nearest search of tree `t` (m positions, reduced to the points of
 // grid g; t.tpos their leaf records) returns from q, provided its squared distance is at most
 // limit2: the point's name in g (pts.w) and its squared distance *d. Else -1, or a point farther
@@ -323,13 +335,8 @@ __device__ __forceinline__ int warp_kd_nearest(const KdView &t, int m, const smd
     // the search itself, by one lane
     int   id = -1;
     float dd = 0.0f;
-    if (lane == 0) {
-        NnSet rs;
-        rs.init(nn_bound(nn_bound(limit2, exc), exc));
-        kd_search(t, q, rs);
-        id = rs.count ? (nameOf ? nameOf[rs.idx] : rs.idx) : -1;
-        dd = rs.dist;
-    }
+    if (lane == 0)
+        id = tree_nearest(t, nameOf, exc, qx, qy, qz, limit2, &dd);
     *d = __shfl_sync(0xffffffffu, dd, 0);
     return __shfl_sync(0xffffffffu, id, 0);
 }
@@ -351,6 +358,12 @@ __device__ __forceinline__ int lanes_kd_nearest(const KdView &t, int m, const sm
     *d = 3.402823466e+38f;
     // (no distance from a point that is not finite is below the search's start)
     need = need && isfinite(qx) && isfinite(qy) && isfinite(qz);
+    if (g.coarse) { // (uniform) the search itself, a lane for each query
+        if (need)
+            j = tree_nearest(t, nameOf, exc, qx, qy, qz, limit2, d);
+        __syncwarp();
+        return j;
+    }
     for (unsigned w = __ballot_sync(0xffffffffu, need); w; w &= w - 1u) {
         const int src = __ffs(w) - 1;
         bool      tie;

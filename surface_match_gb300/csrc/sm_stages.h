@@ -257,9 +257,11 @@ unsigned scan_state(Ctx &c, int nparts);
 int compact(Ctx &c, const int *flags, int n, int *outIds, const std::string &tag);
 // The same when the count is known already (no host round trip).
 void compact_known(Ctx &c, const int *flags, int n, int count, int *outIds);
-// Hashed grid over points ids[0..m) with cell side g (fine cells at any scene extent).
+// Hashed grid over points ids[0..m) with cell side g (fine cells at any scene extent). With `tree`
+// the points have a k-d tree too, and a grid whose cells the extent would make coarse is not built
+// (H.coarse: its searches are the tree's).
 void build_hgrid(Ctx &c, const float4 *pos, const int *ids, int m, const Box &box, float g,
-                 HGrid &H, const std::string &tag, bool wIsRank = false);
+                 HGrid &H, const std::string &tag, bool wIsRank = false, bool tree = false);
 // subPos[r] = pos[ids[r]], subNrm[r] = nrm[ids[r]] for r < m.
 void gather_subset(Ctx &c, const float4 *pos, const float4 *nrm, const int *ids, int m,
                    float4 *subPos, float4 *subNrm);

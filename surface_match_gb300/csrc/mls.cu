@@ -46,6 +46,7 @@ namespace {
 constexpr int kMlsWarps = 8;       // points per CTA of the neighbour kernel
 constexpr int kMlsFitBs = 64;      // threads per CTA of the fit kernel
 constexpr int kMlsNear  = 128;     // neighbours listed per point; a point with more walks the grid
+constexpr int kMlsCount = 288;     // neighbours counted, of a point with more than are listed
 constexpr int kMlsChunk = 1 << 18; // points per launch pair (128 MB of lists)
 
 struct MlsArgs {
@@ -147,9 +148,11 @@ __device__ bool cholesky_solve(double *G, double *b, int n) {
 }
 
 // The neighbours of listed point i0 + t (places in g.pts) in the lists' order: neighbour j of
-// the points of a warp of k_mls_fit is one line of near; cnt[t] their number, or more than the
-// list's length where they are more: such points are named in wide[], counted on from base in
-// *nwide.
+// the points of a warp of k_mls_fit is one line of near; cnt[t] their number, counted to
+// some kMlsCount. Points with more than are listed are named in wide[], counted on from base in
+// nwide[0], and their numbers added to nwide[1]. (Counting on costs up to 5 %: 50,000 points of 200
+// neighbours 1291 -> 1358 us. Their number estimated from what the list's end left of the block
+// misses the line of mls_by by too much.)
 __global__ void __launch_bounds__(kMlsWarps * 32)
     k_mls_near(MlsArgs a, int i0, int n, int *__restrict__ near, int *__restrict__ cnt,
                int *__restrict__ wide, int *__restrict__ nwide, int base) {
@@ -174,7 +177,7 @@ __global__ void __launch_bounds__(kMlsWarps * 32)
         const int excl = incl - (e - b);
         const int T    = __shfl_sync(0xffffffffu, incl, 31);
         int      *L    = near + (size_t)(t >> 5) * (32 * kMlsNear) + (t & 31);
-        for (int r0 = 0; r0 < T && num <= kMlsNear; r0 += 32) {
+        for (int r0 = 0; r0 < T && num <= kMlsCount; r0 += 32) {
             const int r   = r0 + lane;
             int       own = 0; // the lane whose cell holds point r: last lane with excl <= r
 #pragma unroll
@@ -196,8 +199,10 @@ __global__ void __launch_bounds__(kMlsWarps * 32)
     }
     if (lane == 0) {
         cnt[t] = num;
-        if (num > kMlsNear)
+        if (num > kMlsNear) {
             wide[atomicAdd(nwide, 1) - base] = t;
+            atomicAdd(nwide + 1, num);
+        }
     }
 }
 
@@ -308,21 +313,28 @@ __device__ __forceinline__ void monomial(int k, int order, int &i, int &j) {
     j = k;
 }
 
-// Which points of a launch of n a warp takes each (wide: how many have more neighbours than are
-// listed): those, up to as many as the warps work off in the time that a thread takes for one; and
-// all points of a small launch with such, so that no thread's chain follows the warps'. A thread
-// walks the 27 cells for three sums, tens of thousands of loads one after the other: order 2, 1000
-// neighbours, of 16,000 points in all, by threads and by warps: 40 points 2695 and 603 us, 5000
-// 2625 and 1191, 10,000 2685 and 1833, 16,000 2709 and 2774; 300 neighbours: 967 and 291, 1164 and
-// 637, 1164 and 959, 1204 and 1397. Order 4, 300 neighbours, 2000 points: 1508 and 953, 5000: 1503
-// and 1854; 5000 neighbours of 100,000 points, 5000 points: 20911 and 8244.
+// Which points of a launch of n a warp takes each: those with more neighbours than are listed, where
+// they have enough more of them (W points, `sum` neighbours) for their warps to be done sooner than
+// the threads' walks are; and all points of a small launch then, so that no thread's chain follows
+// the warps'. A thread walks the 27 cells for three sums, loads one after the other, beside the other
+// points' threads; the warps' kernel comes before those, with a chain of its own (a solve by one
+// lane: some 130 us at order 3, 450 at order 4) and a time per point. By threads and by warps, of
+// 16,000 points, W of them taken: order 2, mean 133 neighbours, W 273 350 and 369 us; 137, 3915 522
+// and 576; 145, 1400 658 and 264; 182, 7300 898 and 683; 1000, 40 2695 and 603, 10,000 2685 and
+// 1833. Order 3, 130, 4 332 and 458; 145, 5200 788 and 1001; 300, 8000 1331 and 1269. Order 4, 133,
+// 273 518 and 1207; 300, 2000 1508 and 953. The line fits 393 such cases of clouds of 3,000 to
+// 50,000 points, few of them more than 5 % slower than by threads.
 enum MlsBy { kMlsThreads, kMlsWideByWarps, kMlsAllByWarps };
 constexpr int kMlsSmall = 2048, kMlsWideCtas = 3; // (CTAs per SM)
-__device__ __forceinline__ MlsBy mls_by(int n, int wide, int order) {
-    if (wide > 0 && n <= kMlsSmall)
-        return kMlsAllByWarps;
-    const int most = order == 1 ? 32768 : order == 2 ? 12288 : order == 3 ? 8192 : 6144;
-    return wide <= most ? kMlsWideByWarps : kMlsThreads;
+__device__ __forceinline__ MlsBy mls_by(int n, const int *wide, int base, int order) {
+    const int   W = wide[0] - base, sum = wide[1];
+    const int   most = order == 1 ? 32768 : order == 2 ? 12288 : order == 3 ? 8192 : 6144;
+    const float perWide = order == 1 ? 0.0f : order <= 3 ? 0.002f : 0.02f;
+    const float perOther = order == 1 ? 0.0f : order == 2 ? 0.002f : 0.004f;
+    if (W == 0 || W > most ||
+        (float)sum < (float)W * ((float)kMlsNear + perWide * (float)W + perOther * (float)min(n - W, 16000)))
+        return kMlsThreads;
+    return n <= kMlsSmall ? kMlsAllByWarps : kMlsWideByWarps;
 }
 
 // The points that a warp takes each, which walks the 3x3x3 block for each sum: lane l owns the fit's
@@ -338,8 +350,8 @@ __global__ void __launch_bounds__(kMlsWarps * 32, kMlsWideCtas)
     __shared__ double sMom[kMlsWarps][NM + NC], sGram[kMlsWarps][NC * NC];
     const int         lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int         nw = *nwide - base;
-    const MlsBy       by = mls_by(n, nw, ORDER);
-    if (nw == 0 || by == kMlsThreads)
+    const MlsBy       by = mls_by(n, nwide, base, ORDER);
+    if (by == kMlsThreads)
         return;
     const float r2 = a.r2, invR = smm::fdiv(1.0f, a.r);
     // the lane's sums: exponents of u and v, whether the term carries the height
@@ -469,7 +481,7 @@ __global__ void __launch_bounds__(kMlsFitBs)
     if (t >= n)
         return;
     const int   cnt = num[t];
-    const MlsBy by  = mls_by(n, *nwide - base, ORDER);
+    const MlsBy by  = mls_by(n, nwide, base, ORDER);
     if (cnt < 3 || by == kMlsAllByWarps || (by == kMlsWideByWarps && cnt > kMlsNear))
         return;
     const int    id = a.ids[i0 + t];
@@ -626,12 +638,13 @@ void estimate_normals_mls(Ctx &c, const float4 *pos, const int *valid, int nvali
     int      *near  = c.arena.get<int>("mls.near", (size_t)((chunk + 31) / 32) * 32 * kMlsNear);
     int      *num   = c.arena.get<int>("mls.num", (size_t)chunk * 2);
     int      *wide  = num + chunk;
-    // the built grid's range counter, at the number of its points, goes on as the wide points'
+    // the built grid's range counter, at the number of its points, goes on as the wide points', and
+    // the word behind it, clear, as their neighbours'
     int *nwide = G.next, base = nvalid;
     for (int i0 = 0; i0 < m; i0 += chunk) {
         const int n = std::min(chunk, m - i0);
         if (i0 > 0) {
-            SM_CUDA(cudaMemsetAsync(nwide, 0, sizeof(int), c.stream));
+            SM_CUDA(cudaMemsetAsync(nwide, 0, 2 * sizeof(int), c.stream));
             base = 0;
         }
         launch_chained(c, k_mls_near, nblocks(n, kMlsWarps), kMlsWarps * 32, 0, a, i0, n, near, num, wide,

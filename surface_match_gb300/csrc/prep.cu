@@ -1209,7 +1209,7 @@ void build_hgrid(Ctx &c, const float4 *pos, const int *ids, int m, const Box &bo
     H.m         = m;
     if (H.coarse)
         return;
-    int  *next  = c.arena.get<int>(tag + ".next", 1);
+    int  *next  = c.arena.get<int>(tag + ".next", 2);
     int2 *place = c.arena.get<int2>(tag + ".place", std::max(m, 1));
     H.pts       = c.arena.get<float4>(tag + ".pts", std::max(m, 1));
     H.next      = next;
@@ -1224,7 +1224,7 @@ void build_hgrid(Ctx &c, const float4 *pos, const int *ids, int m, const Box &bo
     H.slot  = direct ? nullptr : c.arena.get<uint4>(tag + ".slot", H.slots);
     H.occ   = !direct && ncell <= (1ull << 28) ? c.arena.get<uint32_t>(tag + ".occ", words) : nullptr;
     FillSet clear;
-    clear.add(next, sizeof(int), 0u);
+    clear.add(next, 2 * sizeof(int), 0u);
     if (H.dense)
         clear.add(H.dense, (size_t)ncell * sizeof(int2), 0u);
     if (H.slot)

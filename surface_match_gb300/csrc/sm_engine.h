@@ -123,7 +123,7 @@ struct HGrid {
     int       m      = 0;
     bool      coarse = false;   // not built: the points' k-d tree is searched instead
     float     slack  = smg::kCellSlack;
-    int      *next   = nullptr; // the ranges' counter: m once the grid is built
+    int      *next   = nullptr; // the ranges' counter, m once the grid is built, and a word at 0
     smd::HGridView view() const {
         smd::HGridView v;
         for (int a = 0; a < 3; a++) {
